@@ -187,7 +187,8 @@ __global__ void __launch_bounds__(kGtThreads)
   if (warp == 0) tp_tmem_free(tmem, BN);
 }
 
-int gemm_operand_map(const void *base, long rows, int cols, long pitch, int box, CUtensorMap *out) {
+int tensor_map_2d(const void *base, CUtensorMapDataType type, long rows, long cols, long pitch, int box_rows, int box_cols,
+                  CUtensorMapSwizzle swizzle, CUtensorMap *out) {
   typedef CUresult (*encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                 const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                                 CUtensorMapFloatOOBfill);
@@ -204,14 +205,17 @@ int gemm_operand_map(const void *base, long rows, int cols, long pitch, int box,
     }
   }
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)pitch * 2};
-  const cuuint32_t boxes[2] = {kGtKStep, (cuuint32_t)box};
+  const cuuint64_t strides[1] = {(cuuint64_t)pitch};
+  const cuuint32_t boxes[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, boxes, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  BLOK_REQUIRE(r == CUDA_SUCCESS, BLOK_ERR_CUDA, "gemm: no tensor map (%d) for a matrix of %ld x %d, pitch %ld", (int)r, rows, cols, pitch);
+  const CUresult r = encode(out, type, 2, const_cast<void *>(base), dims, strides, boxes, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  BLOK_REQUIRE(r == CUDA_SUCCESS, BLOK_ERR_CUDA, "gemm: no tensor map (%d) for a matrix of %ld x %ld, pitch %ld bytes", (int)r, rows, cols, pitch);
   return BLOK_OK;
+}
+
+int gemm_operand_map(const void *base, long rows, int cols, long pitch, int box, CUtensorMap *out) {
+  return tensor_map_2d(base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rows, cols, pitch * 2, box, kGtKStep, CU_TENSOR_MAP_SWIZZLE_128B, out);
 }
 
 template <int BN, int ACT, bool F32>

@@ -10,6 +10,11 @@ namespace blok {
 enum { GEMM_ACT_NONE = 0, GEMM_ACT_RELU2 = 1, GEMM_ACT_SILU = 2, GEMM_ACT_SWIGLU = 3 };
 constexpr int kGtTileRows = 128;  // rows of x per tile
 
+// A 2-D tensor map: rows of `cols` elements, `pitch` bytes apart (a multiple of 16; base 16-byte aligned), copied in boxes
+// of box_rows x box_cols; elements past the ends read as zeros.
+int tensor_map_2d(const void *base, CUtensorMapDataType type, long rows, long cols, long pitch, int box_rows, int box_cols,
+                  CUtensorMapSwizzle swizzle, CUtensorMap *out);
+
 // A matrix operand: bf16 [rows, cols], rows `pitch` elements apart (pitch a multiple of 8, base 16-byte aligned).
 // `box`: rows per copied box (128 for x, 128 or 256 for weights).
 int gemm_operand_map(const void *base, long rows, int cols, long pitch, int box, CUtensorMap *out);

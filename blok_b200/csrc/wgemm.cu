@@ -58,7 +58,6 @@ __global__ void __launch_bounds__(kWgThreads) wgemm_kernel(const WgArgs a) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int e = a.tile_expert[tile], p0 = a.tile_start[tile], cnt = a.tile_count[tile];
-  if (a.small_max && cnt <= (a.small_limit ? *a.small_limit : a.small_max)) return;  // a small group: wgemv_small.cu has it
   const int ntiles = (cnt + 7) >> 3;
 
   // the lane's two weight rows
@@ -203,20 +202,9 @@ static int wgemm_forced_impl() {  // read at every launch, so that a test can sw
   return 0;
 }
 
-int launch_wgemm(int mode, const WgArgs &args_in, int max_tiles, cudaStream_t stream) {
+int launch_wgemm(int mode, const WgArgs &args, int max_tiles, cudaStream_t stream) {
   const int forced = wgemm_forced_impl();
   const bool i4 = mode == WG_I4_SWIGLU || mode == WG_I4_PLAIN;
-  WgArgs args = args_in;
-  {
-    // groups of a few tokens first, through the mat-vec-style kernel; the kernel below then skips them
-    // (not when one GEMM kernel is forced: a forced run wants every row through the same arithmetic, whatever shares
-    // its group, which is what the expert-parallel parity checks compare bit for bit)
-    const char *sm = getenv("BLOK_WGEMM_SMALL");
-    if (i4 && forced == 0 && !(sm && sm[0] == '0') && wgemv_small_supports(mode, args, max_tiles)) {
-      if (int rc = launch_wgemv_small(mode, args, stream)) return rc;
-      args.small_max = kWgSmallTokens;
-    }
-  }
   const bool swiglu = mode == WG_BF16_SWIGLU || mode == WG_I4_SWIGLU;
   if (!i4 && forced == 0 && wgemm_stream_supports(mode, args)) {
     int nz = 1;
@@ -225,7 +213,7 @@ int launch_wgemm(int mode, const WgArgs &args_in, int max_tiles, cudaStream_t st
   }
   // bf16: the tcgen05 kernel's 256-token tiles leave most SMs idle below about 650 tokens (shared expert: 376 us from
   // 128 to 1,024 tokens, against 106 / 162 / 297 / 585 us for the K-split mma.sync kernel at 128 / 256 / 512 / 1,024)
-  const bool enough = args.n_rows >= (i4 ? 256 : 640);
+  const bool enough = args.n_rows >= 640;
   if (forced != 1 && (forced == 2 || enough) && wgemm_tc_supports(mode, args)) return launch_wgemm_tc(mode, args, max_tiles, stream);
   const size_t smem = wgemm_smem_bytes();
   const int rows_per_cta = swiglu ? 8 * kWgWarps : 16 * kWgWarps;
@@ -250,6 +238,23 @@ int launch_wgemm(int mode, const WgArgs &args_in, int max_tiles, cudaStream_t st
 #undef BLOK_WG_LAUNCH
   if (int rc = launch_status("wgemm_kernel")) return rc;
   return grid.z > 1 ? launch_wgemm_splitk_reduce(mode, args, (int)grid.z, stream) : BLOK_OK;
+}
+
+int launch_wgemm_experts(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream) {
+  const int forced = wgemm_forced_impl();
+  const char *sm = getenv("BLOK_WGEMM_SMALL");
+  // The mat-vec-style kernel deals a handful of groups out evenly, where the tcgen05 kernel's units of 256 rows fill the SMs
+  // unevenly; its work grows with the tokens, the tcgen05 kernel's does not.  Layer pass, us, mat-vec-style / tcgen05: 32
+  // assignments over 128 experts of 2048 x 1024 101 / 106, 64 129 / 117, 96 150 / 129; over 384 experts of 7168 x 2048 48
+  // 303 / 300, 72 403 / 424, 96 499 / 504, 128 703 / 644, 192 914 / 829.
+  if (forced == 0 && !(sm && sm[0] == '0') && rows <= kWgSmallRows && wgemv_small_supports(WG_I4_SWIGLU, up, max_tiles) &&
+      wgemv_small_supports(WG_I4_PLAIN, down, max_tiles)) {
+    if (int rc = launch_wgemv_small(WG_I4_SWIGLU, up, stream)) return rc;
+    return launch_wgemv_small(WG_I4_PLAIN, down, stream);
+  }
+  if (forced != 1 && wgemm_i4_supports(up, down)) return launch_wgemm_i4(up, down, xs, rows, max_tiles, stream);
+  if (int rc = launch_wgemm(WG_I4_SWIGLU, up, max_tiles, stream)) return rc;
+  return launch_wgemm(WG_I4_PLAIN, down, max_tiles, stream);
 }
 
 }  // namespace blok

@@ -9,7 +9,9 @@ namespace blok {
 enum { WG_BF16_PLAIN = 0, WG_BF16_SWIGLU = 1, WG_I4_SWIGLU = 2, WG_I4_PLAIN = 3 };
 constexpr int kWgTileTokens = 64;
 constexpr int kWgStreamTokens = 64;  // bf16 weights over up to this many rows take the weight-streaming kernel (wgemm_stream.cu)
-constexpr int kWgSmallTokens = 8;  // groups of up to this many tokens take the mat-vec-style kernel (wgemv_small.cu: four per pass)
+// Grouped INT4 products of up to this many assignments take the mat-vec-style kernel (wgemv_small.cu: four tokens per pass),
+// more take the tcgen05 kernel
+constexpr int kWgSmallRows = 40;
 
 struct WgArgs {
   const void *w_a;
@@ -30,17 +32,12 @@ struct WgArgs {
   const int *out_index;
   int identity_tiles = 0;  // the tiles are consecutive 64-row blocks of x (one group: a dense layer over n_rows tokens)
   int n_rows = 0;  // rows of x the launch covers (tokens, or token-expert assignments): picks the kernel
-  int small_max = 0;  // > 0: tiles of at most this many tokens are somebody else's (wgemv_small.cu) and are skipped
-  // INT4 modes, optional: a device word in which the small-group kernel leaves the group size up to which it took the
-  // launch's tiles (it takes every group when the larger ones are few); the GEMM kernel behind it skips those
-  int *small_limit = nullptr;
   // bf16 modes over identity tiles: scratch for the K-split partial sums, see wgemm_splitk_bytes; NULL: no split
   float *splitk_ws = nullptr;
   size_t splitk_bytes = 0;
 };
 
-// Picks the kernels of a launch.  INT4 modes: the small-group kernel first (wgemv_small.cu), then for what it left the
-// tcgen05 kernel (wgemm_tc.cu) from 256 assignments on, below that the mma.sync kernel.  bf16 modes: up to
+// Picks the kernel of a launch.  INT4 modes: the mma.sync kernel (see launch_wgemm_experts for the others).  bf16 modes: up to
 // kWgStreamTokens rows of a dense product the weight-streaming kernel (wgemm_stream.cu); from 640 tokens on the tcgen05
 // kernel; in between, and for shapes the others do not cover, the mma.sync kernel with its K-split.
 // BLOK_WGEMM_IMPL=mma / =tc in the environment forces one GEMM kernel for every row (no small-group or streaming kernel).
@@ -57,9 +54,8 @@ size_t wgemm_splitk_bytes(int mode, int K, int R, int max_rows);
 // Fills the tile arrays with consecutive 64-row tiles of T rows (one group, expert 0): a dense layer.
 int launch_identity_tiles(int T, int *tile_expert, int *tile_start, int *tile_count, int *num_tiles, cudaStream_t stream);
 
-// The INT4 modes for groups of up to kWgSmallTokens tokens (every group when the larger ones are few, see
-// WgArgs::small_limit): streams the weights like the batch-1 decode kernel and leaves the other groups alone.  launch_wgemm runs it in front of the kernel that takes the rest
-// (BLOK_WGEMM_SMALL=0 in the environment: every group through the GEMM kernels).
+// The INT4 modes over few assignments: streams the weights like the batch-1 decode kernel (BLOK_WGEMM_SMALL=0 in the
+// environment: through the GEMM kernels as well).
 bool wgemv_small_supports(int mode, const WgArgs &args, int max_tiles);
 int launch_wgemv_small(int mode, const WgArgs &args, cudaStream_t stream);
 
@@ -75,6 +71,14 @@ int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t 
 // fp32 output) or the SwiGLU front half of (w_a = gate, w_b = up) (mode WG_BF16_SWIGLU), for 1 <= T <= kWgStreamTokens.
 int launch_wgemm_rows(int mode, const void *w_a, const void *w_b, const uint16_t *x, uint16_t *out_bf16, float *out_f32, int R, int K,
                       int T, float *splitk_ws, size_t splitk_bytes, cudaStream_t stream);
+
+// Both products of the grouped experts, INT4: mid = SwiGLU front half of x (up: WG_I4_SWIGLU), then the down projection
+// (down: WG_I4_PLAIN, its x is up's output).  Up to kWgSmallRows rows through the mat-vec-style kernel (wgemv_small.cu), else
+// through the tcgen05 kernel (wgemm_tc.cu) where it covers the shapes; else, or with BLOK_WGEMM_IMPL=mma, launch_wgemm twice.  xs: scratch of `rows` x up.K values, where `rows` is the number of sorted
+// positions that up.out_bf16 and xs hold (it may be the buffer of down's output).
+int launch_wgemm_experts(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream);
+bool wgemm_i4_supports(const WgArgs &up, const WgArgs &down);
+int launch_wgemm_i4(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream);
 
 bool wgemm_tc_supports(int mode, const WgArgs &args);
 int launch_wgemm_tc(int mode, const WgArgs &args, int max_tiles, cudaStream_t stream);

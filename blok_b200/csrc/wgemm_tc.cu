@@ -1,25 +1,15 @@
-// Weight-streaming grouped GEMM on the 5th-generation tensor cores (tcgen05, accumulators
-// in tensor memory) for the INT4 experts of the batched routed-MoE layer:
+// Grouped GEMM on the 5th-generation tensor cores (tcgen05, accumulators in tensor memory) for the INT4 experts of the
+// batched routed-MoE layer:
 //   out[token, row] = sum_c bf16(q[row, c] * scale[row, c / 32]) * x[token, c]
-// Reference arithmetic: matvec_i4_bf16_scale_k (src/kimi_exec.cu:300-323) applied per
-// token; the dequantised weight is the reference's bf16(q * s) bit for bit (:312).
-//
-// One CTA = one tile of up to 64 tokens of one expert x two 128-row blocks of weights (gate
-// and up rows of the same indices, or rows r and r + 128 of the down projection).  The
-// weight rows are the M = 128 dimension of tcgen05.mma, the tokens the N dimension, so
-// a weight byte is read from HBM and dequantised once per tile whatever the token
-// count.  Eight producer warps (one weight row per thread) copy 256 packed columns and
-// their scales per step into shared memory with coalesced cp.async (rows XOR-swizzled
-// against bank conflicts), dequantise them exactly and write them to TENSOR MEMORY with
-// tcgen05.st as the A operand, 64 columns per pipeline stage; the tile's activations go
-// to shared memory in the K-major core-matrix layout the instruction reads (no swizzle:
-// 8 rows x 16 bytes per core matrix) as the B operand.  A ninth warp's first lane issues
-// the MMAs; producers arrive on a `full` mbarrier per stage, tcgen05.commit on an `empty`
-// mbarrier frees it.  Every mbarrier wait is bounded; on a timeout the CTA records an
-// error, still releases its tensor memory and returns.
+// Reference arithmetic: matvec_i4_bf16_scale_k (src/kimi_exec.cu:300-323) applied per token; the dequantised weight is the
+// reference's bf16(q * s) bit for bit (:312).  The weight rows are the M = 128 dimension of tcgen05.mma, the tokens the N
+// dimension, so a weight byte is read from HBM and dequantised once per tile whatever the token count.  Every mbarrier wait
+// is bounded; on a timeout the CTA records an error, waits for its copies, releases its tensor memory and returns.
 #include <algorithm>
 
 #include "common.cuh"
+#include "gemm_tma.h"
+#include "tc_pipe.cuh"
 #include "wgemm.h"
 
 namespace blok {
@@ -28,43 +18,42 @@ constexpr int kTcProducers = 256;    // threads that unpack weights: one weight 
 constexpr int kTcThreads = kTcProducers + 32;  // plus one warp whose first lane issues the MMAs
 constexpr int kTcN = kWgTileTokens;  // token columns of a tile
 constexpr int kTcKC = 64;            // weight columns per pipeline step
-constexpr int kTcStages = 2;
 constexpr int kTcSbo = 128;          // bytes between 8-token groups of the activation tile
-constexpr int kTcBLbo = 1040;        // 8 token groups x 128 B, plus 16 B so that the 8 K-slices of a token hit 8 banks
-constexpr int kTcBBytes = (kTcKC / 8) * kTcBLbo;
-constexpr int kTcStageBytes = ((kTcBBytes + 127) / 128) * 128;  // shared memory per stage: the activation tile only
-constexpr int kTcSuper = 256;        // weight columns per copy step: 128 packed bytes and 8 scales of each row
-constexpr int kTcRing = 2;           // copy steps resident per CTA: one being unpacked, one in flight
-constexpr int kTcRawBytes = kTcProducers * 128 + kTcProducers * 16;  // 256 rows x (128 B of words + 16 B of scales)
-constexpr int kTcACols = kTcKC / 2;                       // tensor-memory columns of one 128-row block of one step (2 bf16 per column)
-constexpr int kTcTmemCols = 256;                          // 2 accumulators x 64 columns + 2 stages x 2 blocks x 32 columns of weights
 constexpr unsigned kTcSpinLimit = 1u << 22;
 
 __device__ unsigned g_wgemm_tc_error = 0;
 
-__device__ __forceinline__ uint32_t tc_bf16x2_sub(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
 __device__ __forceinline__ uint32_t tc_bf16x2_mul(uint32_t a, uint32_t b) {
   uint32_t r;
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
+__device__ __forceinline__ uint32_t tc_bf16x2_fma(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t r;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+  return r;
+}
 
-// Exact dequantised pairs of one packed word: (bf16(q_j * s), bf16(q_{j+4} * s)), j = 0..3,
-// i.e. the word's eight columns in the order 0 4 1 5 2 6 3 7 (the activations get the same order).
-__device__ __forceinline__ uint4 tc_dequant_word(uint32_t w, uint32_t s2) {
-  constexpr uint32_t kMask = 0x000f000fu, kMagic = 0x43004300u, kOff = 0x43084308u;  // 128.0 | nibble, 136.0
-  uint32_t o[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    uint32_t v;
-    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(v) : "r"(w >> (4 * j)), "r"(kMask), "r"(kMagic));
-    o[j] = tc_bf16x2_mul(tc_bf16x2_sub(v, kOff), s2);
-  }
-  return make_uint4(o[0], o[1], o[2], o[3]);
+// Dequantisation with one instruction per pair of weights besides the masks.  The bits of a nibble n = q + 8 in the low four
+// bits of a bf16 are the number n 2^-133, in the next four n 2^-129 (below and just above the smallest normal number the
+// encoding is linear), so w & 0x000f000f and w & 0x00f000f0 are pairs of nibbles as they lie, and
+//   fma(n 2^-129, s 2^100, -s 2^-26) = bf16(q s 2^-29) = 2^-29 bf16(q s)
+// with one rounding, the reference's (:312): a power of two does not change it while s 2^104 is finite and q s 2^-29 normal
+// (2^-97 <= |s| < 2^24).  The epilogue takes the 2^29 back, exactly.  (Adding an exponent to the nibble, subtracting 136 and
+// multiplying took 15 instructions a word instead of 9.)
+constexpr uint32_t kI4Hi = 0x71807180u, kI4Lo = 0x73807380u, kI4Off = 0xb280b280u;  // 2^100, 2^104, -2^-26
+constexpr float kI4Unscale = 536870912.f;                                           // 2^29
+struct I4Scale {
+  uint32_t hi, lo, off;
+  __device__ __forceinline__ explicit I4Scale(uint32_t s2) : hi(tc_bf16x2_mul(s2, kI4Hi)), lo(tc_bf16x2_mul(s2, kI4Lo)), off(tc_bf16x2_mul(s2, kI4Off)) {}
+};
+// The pairs (q_j s, q_{j+4} s), j = 0..3, of one packed word: its eight columns in the order 0 4 1 5 2 6 3 7.
+__device__ __forceinline__ void i4_dequant(uint32_t w, const I4Scale &s, uint32_t *o) {
+  const uint32_t t = w >> 8;
+  o[0] = tc_bf16x2_fma(w & 0x000f000fu, s.lo, s.off);
+  o[1] = tc_bf16x2_fma(w & 0x00f000f0u, s.hi, s.off);
+  o[2] = tc_bf16x2_fma(t & 0x000f000fu, s.lo, s.off);
+  o[3] = tc_bf16x2_fma(t & 0x00f000f0u, s.hi, s.off);
 }
 
 // Shared-memory matrix descriptor, K-major, no swizzle: start address, leading (K) and
@@ -80,28 +69,6 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t adesc, uint
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same with the A operand (128 rows x 16 columns of bf16) taken from tensor memory.
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n" ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, "
-      "%19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
-      "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
-      "r"(r[31])
       : "memory");
 }
 
@@ -140,10 +107,6 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 __device__ __forceinline__ void tc_cp_async16(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void tc_cp_async4(uint32_t dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-
 // Epilogue of a tile: lane l of warp w (8 warps) holds accumulator row 32 (w % 4) + l of both row blocks (its
 // tensor-memory lane); warps 0..3 take the even 16-token column blocks, warps 4..7 the odd ones.
 template <bool SWIGLU>
@@ -179,223 +142,333 @@ __device__ __forceinline__ void tc_epilogue(const WgArgs &a, uint32_t tmem, int 
   }
 }
 
-template <bool SWIGLU>
-__global__ void __launch_bounds__(kTcThreads, 2) wgemm_tc_kernel(const WgArgs a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) unsigned long long s_mbar[2 * kTcStages];
-  __shared__ uint32_t s_tmem_base;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // The grid's y extent is a fixed number of tile slots, not the worst-case tile count (tokens / 64 + experts, most of
-  // which a launch does not use or leaves to the small-group kernel: 6,000-11,000 CTAs that only start and leave cost
-  // 36-58 us per launch); a CTA walks the tiles slot, slot + slots, ...
-  const int ntiles = *a.num_tiles;
-  const int skip_upto = a.small_max ? (a.small_limit ? *a.small_limit : a.small_max) : 0;  // groups wgemv_small.cu has taken
-  bool have_tmem = false;
-  uint32_t tmem = 0;
-  for (int tile = blockIdx.y; tile < ntiles; tile += gridDim.y) {
-  const int e = a.tile_expert[tile], p0 = a.tile_start[tile], cnt = a.tile_count[tile];
-  if (cnt <= skip_upto) continue;  // nothing is allocated yet
-  const int N = max(16, (cnt + 15) & ~15);  // token columns the MMAs cover
+// ---- INT4 weights ----
+//
+// A unit is (tile of up to 64 tokens of one expert) x 256 weight rows (128 gate + 128 up rows of the same indices, or 256
+// rows of the down projection); a persistent CTA per SM walks the units, and every role runs ahead across their boundaries:
+//   warps 0, 1    MMAs of row block 0 and 1: 4 K = 16 steps per 64-column piece
+//   warp 2        activations by TMA: four slots of 128 columns
+//   warp 3        weights and scales by TMA: four stages of 256 rows x 128 bytes, scales 32 bytes (512 columns) per row
+//   warps 4..7    epilogue of the unit before (two accumulator buffers)
+//   warps 8..     unpack: sets of eight warps take the pieces in turn; a thread owns one row of one block and writes
+//                 the piece's exact bf16(q * s) to TENSOR MEMORY as the MMA's A operand
+// The activations arrive in sorted order with the columns of every packed word in the order 0 4 1 5 2 6 3 7 (the order the
+// unpacking leaves the weights in): i4_rows_kernel lays them out once per launch, the SwiGLU epilogue writes them so.
+//
+// Bound: the weight stream where a group has few tokens, then the tensor cores and the power of both.  What it took, gate/up
+// product of 384 experts of 7168 x 2048 over 4,136 assignments (6.3 GB): cp.async producers that also fetched the activations,
+// two CTAs per SM 1,447 us and 835 us more for the groups of up to 8 (mat-vec-style kernel); TMA, roles, one CTA 1,687 us;
+// dequantisation in 9 instead of 15 instructions a word 1,437; MMAs of the two blocks by two warps 1,389; scales on the
+// weights' barrier 1,301; operands of the MMAs in uniform registers 1,255; pieces of 128 columns instead of 64 and 16
+// unpacking warps instead of 24 1,138 us (5.6 TB/s).  With a hand-over every 64 columns the MMA warps' waits were the limit,
+// whatever the others did.  At 16,384 assignments 2,190 us before, 1,537 now; at 512 1,017 before, 800 now.
+constexpr int kI4Unpack = 16, kI4Epi = 4;                       // warps
+constexpr int kI4FirstUnpack = 4 + kI4Epi;
+constexpr int kI4Threads = (kI4FirstUnpack + kI4Unpack) * 32;
+constexpr int kI4Cols = 256;                                    // columns per weight stage
+constexpr int kI4WStages = 4, kI4WBytes = 256 * (kI4Cols / 2);  // 32 KB
+constexpr int kI4SStages = 3, kI4SBytes = 256 * 32;             // scales of 512 columns: whole 32-byte sectors
+constexpr int kI4XStages = 4, kI4XHalf = kTcN * 128, kI4XBytes = 2 * kI4XHalf;  // 64 tokens x 2 x 64 columns
+constexpr int kI4Smem = kI4WStages * kI4WBytes + kI4SStages * kI4SBytes + kI4XStages * kI4XBytes + 1024;
+constexpr int kI4Piece = 2;                                     // 64-column parts per piece
+constexpr int kI4Pieces = 4 / kI4Piece;                         // per weight stage; each has its own tensor-memory buffer
+constexpr int kI4TmemCols = 512;                                // 2 x 2 accumulators of 64 columns, 4 pieces x 2 blocks x 32 columns of weights
+constexpr int kI4ACol = 4 * kTcN;
 
-  // ---- this thread unpacks weight row r of block blk: threads 0..127 block 0 (gate rows / rows r), 128..255 block 1 ----
-  const int blk = tid >> 7, r = tid & 127;
-  const int rows_per_cta = SWIGLU ? 128 : 256;
-  const int row0 = blockIdx.x * rows_per_cta;
-  const size_t rowbytes = (size_t)a.K / 2;  // packed bytes per weight row
-  const size_t srowbytes = (size_t)a.K / 16;  // scale bytes per weight row
-  const size_t grow0 = (size_t)e * a.expert_stride_rows + row0;
-  const unsigned char *wbase0 = reinterpret_cast<const unsigned char *>(a.w_a) + grow0 * rowbytes;
-  const unsigned char *wbase1 = SWIGLU ? reinterpret_cast<const unsigned char *>(a.w_b) + grow0 * rowbytes : wbase0 + 128 * rowbytes;
-  const unsigned char *sbase0 = reinterpret_cast<const unsigned char *>(a.s_a) + grow0 * srowbytes;
-  const unsigned char *sbase1 = SWIGLU ? reinterpret_cast<const unsigned char *>(a.s_b) + grow0 * srowbytes : sbase0 + 128 * srowbytes;
-  // ---- this thread's two pieces of the activation tile: token (tid / 8) + 32 i, K-slice tid % 8 ----
-  const int ki = tid & 7;
-  const uint4 *xp[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int tok = (tid >> 3) + 32 * i;
-    xp[i] = nullptr;
-    if (tok < cnt) {
-      const size_t xr = a.x_index ? (size_t)a.x_index[p0 + tok] : (size_t)(p0 + tok);
-      xp[i] = reinterpret_cast<const uint4 *>(a.x + xr * a.K) + ki;
-    }
+struct I4Args {
+  uint16_t *out;
+  const int *out_index, *tile_expert, *tile_start, *tile_count, *num_tiles;
+  int K, R, stride_rows;
+};
+
+__device__ __forceinline__ uint4 i4_lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t i4_lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+// Bounded wait; a warp that has time (SLEEP ns between tries) leaves the issue slots to the unpacking warps.
+template <int SLEEP>
+__device__ __forceinline__ bool i4_wait(uint32_t mbar, uint32_t parity) {
+  for (unsigned it = 0; it < (1u << 21); ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if (SLEEP) __nanosleep(SLEEP);
   }
-  // Packed words and scales reach shared memory in copy steps of 256 columns: 8 neighbouring lanes copy the 128
-  // contiguous bytes of one row (16 bytes each), so a warp's cp.async touches 4 cache lines, not 32.  Piece p of row
-  // q lands at q * 128 + ((p ^ (q & 7)) * 16): both the copy and the later per-row reads are free of bank conflicts.
-  // The activations (L2 resident, shared by all row blocks of the expert) are fetched one step ahead into registers.
-  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
-  const uint32_t raw0 = sbase + kTcStages * kTcStageBytes;
-  const unsigned char *rawp = smem + kTcStages * kTcStageBytes;
-  const int nchunks = a.K / kTcKC;
-  const int nsuper = a.K / kTcSuper;
-  const bool producer = tid < kTcProducers;
-  auto issue = [&](int sc) {
-    if (sc < nsuper) {
-      const uint32_t slot = raw0 + (uint32_t)(sc % kTcRing) * kTcRawBytes;
-      const int q0 = tid >> 3, pc = tid & 7;
+  return false;
+}
+
+// A ring's position: slot and the parity of the slot's current use.
+template <int N>
+struct I4Ring {
+  int slot = 0;
+  uint32_t turn = 0;
+  __device__ __forceinline__ void next() {
+    if (++slot == N) slot = 0, turn ^= 1;
+  }
+};
+
+struct I4Mma {
+  uint32_t x_full, x_empty, a_full, a_empty, d_full, d_empty, xbase;
+};
+// The MMAs of one row block; false: a wait gave up.  The whole warp walks the pieces and one lane issues: every address is
+// a constant or a loop variable and stays in uniform registers.
+template <int BLK>
+__device__ __forceinline__ bool i4_mma(const I4Mma &m, const I4Args &a, int units, int blocks, int stages) {
+  const bool issues = tp_elect();
+  I4Ring<kI4XStages> xr;
+  I4Ring<2> dr;
+  uint32_t aturn = 0;
+  for (int u = blockIdx.x; u < units; u += gridDim.x) {
+    const uint32_t idesc = tp_idesc_bf16(((__ldg(a.tile_count + u / blocks) + 15) >> 4) << 4);
+    if (!__all_sync(0xffffffffu, i4_wait<0>(m.d_empty + 8 * dr.slot, dr.turn ^ 1))) return false;
+    const uint32_t d = (uint32_t)(dr.slot * 2 + BLK) * kTcN;
+    for (int st = 0; st < stages; ++st) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int q = q0 + 32 * i;  // 0..255: block q / 128, row q % 128
-        const unsigned char *src = (i < 4 ? wbase0 : wbase1) + (size_t)(q & 127) * rowbytes + (size_t)sc * 128 + pc * 16;
-        tc_cp_async16(slot + q * 128 + ((pc ^ (q & 7)) * 16), src);
+      for (int c = 0; c < kI4Pieces; ++c) {
+        const bool first = kI4Piece == 2 || !(c & 1), last = kI4Piece == 2 || (c & 1);  // of the piece's 128 columns of activations
+        bool ok = !first || i4_wait<0>(m.x_full + 8 * xr.slot, xr.turn);
+        ok = ok && i4_wait<0>(m.a_full + 16 * c + 8 * BLK, aturn);
+        if (!__all_sync(0xffffffffu, ok)) return false;
+        tc_fence_after();
+        const uint64_t bd = tp_desc_k_sw128(m.xbase + xr.slot * kI4XBytes);
+        constexpr uint32_t ta = kI4ACol + BLK * 32;
+        if (issues) {
+#pragma unroll
+          for (int z = 0; z < kI4Piece; ++z)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              tp_mma_ts(d, ta + (c * kI4Piece + z) * 64 + 8 * k, bd + (uint64_t)(((c * kI4Piece + z) & 1) * (kI4XHalf / 16) + 2 * k), idesc,
+                        (st | c | z | k) ? 1u : 0u);
+          tp_commit(m.a_empty + 16 * c + 8 * BLK);
+          if (last) tp_commit(m.x_empty + 8 * xr.slot);
+          if (c == kI4Pieces - 1 && st == stages - 1) tp_commit(m.d_full + 8 * dr.slot);
+        }
+        if (last) xr.next();
       }
-      tc_cp_async16(slot + kTcProducers * 128 + tid * 16, (blk ? sbase1 : sbase0) + (size_t)r * srowbytes + (size_t)sc * 16);
+      aturn ^= 1;
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  auto fetch_x = [&](int c, uint4 (&xv)[2]) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) xv[i] = xp[i] ? __ldg(xp[i] + (size_t)c * (kTcKC / 8)) : make_uint4(0, 0, 0, 0);
-  };
-  if (producer) issue(0);
+    dr.next();
+  }
+  return true;
+}
 
-  // ---- barriers and tensor memory: full[s] counts the 8 producer warps, empty[s] the MMAs' commit ----
-  const uint32_t mbar_full = (uint32_t)__cvta_generic_to_shared(&s_mbar[0]);
-  const uint32_t mbar_empty = mbar_full + 8 * kTcStages;
+template <bool SWIGLU>
+__global__ void __launch_bounds__(kI4Threads, 1)
+    wgemm_tc_kernel(const __grid_constant__ CUtensorMap mwa, const __grid_constant__ CUtensorMap mwb, const __grid_constant__ CUtensorMap msa,
+                    const __grid_constant__ CUtensorMap msb, const __grid_constant__ CUtensorMap mx, const I4Args a) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long s_bar[2 * (kI4WStages + kI4XStages + 8 + 2)];
+  __shared__ uint32_t s_tmem;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int kRows = SWIGLU ? 128 : 256;
+  const int blocks = a.R / kRows, units = *a.num_tiles * blocks;
+  const int stages = a.K / kI4Cols;
+  const uint32_t wbase = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023u) & ~1023u;
+  const uint32_t sbase = wbase + kI4WStages * kI4WBytes, xbase = sbase + kI4SStages * kI4SBytes;
+  const uint32_t w_full = (uint32_t)__cvta_generic_to_shared(&s_bar[0]), w_empty = w_full + 8 * kI4WStages;
+  const uint32_t x_full = w_empty + 8 * kI4WStages, x_empty = x_full + 8 * kI4XStages;
+  const uint32_t a_full = x_empty + 8 * kI4XStages, a_empty = a_full + 64, d_full = a_empty + 64, d_empty = d_full + 16;
   if (tid == 0) {
-#pragma unroll
-    for (int s = 0; s < kTcStages; ++s) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar_full + 8 * s), "r"(kTcProducers / 32) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_empty + 8 * s) : "memory");
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int s = 0; s < kI4WStages; ++s) tp_mbar_init(w_full + 8 * s, 1), tp_mbar_init(w_empty + 8 * s, kI4Pieces * 8);
+    for (int s = 0; s < kI4XStages; ++s) tp_mbar_init(x_full + 8 * s, 1), tp_mbar_init(x_empty + 8 * s, 2);
+    for (int s = 0; s < 8; ++s) tp_mbar_init(a_full + 8 * s, 4), tp_mbar_init(a_empty + 8 * s, 1);  // [piece of a stage][row block]
+    for (int s = 0; s < 2; ++s) tp_mbar_init(d_full + 8 * s, 2), tp_mbar_init(d_empty + 8 * s, kI4Epi);
+    tp_mbar_init_fence();
   }
-  if (warp == 0 && !have_tmem) {  // once per CTA, at its first tile; the columns serve every tile the CTA walks
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(&s_tmem_base)),
-                 "r"((uint32_t)kTcTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  have_tmem = true;
-  uint4 xnext[2];
-  if (producer) fetch_x(0, xnext);
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if (warp == 0) tp_tmem_alloc((uint32_t)__cvta_generic_to_shared(&s_tmem), kI4TmemCols);
+  tc_fence_before();
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  tmem = s_tmem_base;
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
-
+  tc_fence_after();
+  constexpr uint32_t tmem = 0;  // all columns are this CTA's, so they start at 0: a constant keeps the MMAs' operands in uniform registers
   bool failed = false;
-  if (producer) {
-    // ---- producers: unpack step c into stage c % 2 as soon as the MMAs of step c - 2 have released it ----
-    for (int sc = 0; sc < nsuper; ++sc) {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");  // this thread's copies of the step have landed
-      // producers' barrier: everybody's copies have landed and the other slot is no longer read.  It also ORs the
-      // threads' failure flags, so that after a timeout all of them leave together and nobody waits here alone.
-      uint32_t anyfail;
-      asm volatile(
-          "{\n\t"
-          ".reg .pred p, q;\n\t"
-          "setp.ne.u32 q, %1, 0;\n\t"
-          "bar.red.or.pred p, 1, %2, q;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t"
-          "}\n"
-          : "=r"(anyfail)
-          : "r"((uint32_t)failed), "n"(kTcProducers)
-          : "memory");
-      if (anyfail) {
+
+  if (warp >= kI4FirstUnpack) {
+    const int set = (warp - kI4FirstUnpack) >> 3, blk = (warp >> 2) & 1, row = 32 * (warp & 3) + lane;
+    const uint32_t wrow = wbase + (uint32_t)(blk * (128 * 128) + row * 128);
+    const uint32_t srow = sbase + (uint32_t)(blk * (128 * 32) + row * 32);
+    const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(kI4ACol + blk * 32);
+    const int pieces = (int)blockIdx.x < units ? ((units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * kI4Pieces * stages : 0;
+    for (int p = set; p < pieces; p += kI4Unpack / 8) {
+      const int st = p / kI4Pieces, c = p % kI4Pieces;  // c: the piece of its stage, and the tensor-memory buffer it goes to
+      const int ws = st % kI4WStages, ss = (st >> 1) % kI4SStages;
+      if (!__all_sync(0xffffffffu, i4_wait<0>(w_full + 8 * ws, (uint32_t)(st / kI4WStages) & 1))) {
         failed = true;
         break;
       }
-      issue(sc + 1);
-      const unsigned char *raw = rawp + (size_t)(sc % kTcRing) * kTcRawBytes;
-      const uint4 scq = *reinterpret_cast<const uint4 *>(raw + kTcProducers * 128 + tid * 16);  // the row's 8 scales
-      const uint32_t scw[4] = {scq.x, scq.y, scq.z, scq.w};
+      uint4 q[2 * kI4Piece];
+      uint32_t sc[kI4Piece];
 #pragma unroll
-      for (int j = 0; j < kTcSuper / kTcKC; ++j) {
-        const int c = sc * (kTcSuper / kTcKC) + j;
-        uint4 xcur[2];
+      for (int h = 0; h < 2 * kI4Piece; ++h) q[h] = i4_lds128(wrow + ws * kI4WBytes + (((2 * kI4Piece * c + h) ^ (row & 7)) << 4));
 #pragma unroll
-        for (int i = 0; i < 2; ++i) xcur[i] = xnext[i];
-        if (c + 1 < nchunks) fetch_x(c + 1, xnext);
-        const int s = c % kTcStages;
-        if (c >= kTcStages && !tc_mbar_wait(mbar_empty + 8 * s, (uint32_t)((c / kTcStages - 1) & 1))) {
-          failed = true;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        unsigned char *B = smem + (size_t)s * kTcStageBytes;
-        // The row's 64 dequantised weights of this step go to tensor memory as the MMA's A operand: lane = row, two
-        // bf16 per 32-bit column, 8 columns per K = 16 step (column pairs in the order 0 4 1 5 2 6 3 7 of each word).
+      for (int h = 0; h < kI4Piece; ++h) sc[h] = i4_lds32(srow + ss * kI4SBytes + (((st & 1) ^ ((row >> 2) & 1)) << 4) + (c * kI4Piece + h) * 4);
+      __syncwarp();
+      if (lane == 0) tp_arrive(w_empty + 8 * ws);
+#pragma unroll
+      for (int z = 0; z < kI4Piece; ++z) {
         uint32_t av[32];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const uint32_t s2 = __byte_perm(scw[j], scw[j], h ? 0x3232 : 0x1010);
-          const uint4 q = *reinterpret_cast<const uint4 *>(raw + tid * 128 + (((2 * j + h) ^ (tid & 7)) * 16));
-          const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+          const I4Scale s2(__byte_perm(sc[z], 0, h ? 0x3232 : 0x1010));
+          const uint32_t w[4] = {q[2 * z + h].x, q[2 * z + h].y, q[2 * z + h].z, q[2 * z + h].w};
 #pragma unroll
-          for (int w = 0; w < 4; ++w) {
-            const uint4 d = tc_dequant_word(qw[w], s2);
-            av[(h * 4 + w) * 4 + 0] = d.x;
-            av[(h * 4 + w) * 4 + 1] = d.y;
-            av[(h * 4 + w) * 4 + 2] = d.z;
-            av[(h * 4 + w) * 4 + 3] = d.w;
-          }
+          for (int k = 0; k < 4; ++k) i4_dequant(w[k], s2, av + (h * 4 + k) * 4);
         }
-        tc_st32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 2 * kTcN + (uint32_t)(s * 2 + blk) * kTcACols, av);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          if (32 * i < N) {
-            const uint4 v = xcur[i];
-            uint4 o;  // columns 0 4 1 5 2 6 3 7, as the weights
-            o.x = __byte_perm(v.x, v.z, 0x5410);
-            o.y = __byte_perm(v.x, v.z, 0x7632);
-            o.z = __byte_perm(v.y, v.w, 0x5410);
-            o.w = __byte_perm(v.y, v.w, 0x7632);
-            const int tok = (tid >> 3) + 32 * i;
-            *reinterpret_cast<uint4 *>(B + ki * kTcBLbo + (tok >> 3) * kTcSbo + (tok & 7) * 16) = o;
+        if (z == 0) {
+          if (!__all_sync(0xffffffffu, i4_wait<0>(a_empty + 16 * c + 8 * blk, ((uint32_t)st & 1) ^ 1))) {  // the first use finds it free
+            failed = true;
+            break;
           }
+          tc_fence_after();
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the activation tile is read by the tensor core's proxy
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar_full + 8 * s) : "memory");
+        tmem_st32(ta + (c * kI4Piece + z) * 64, av);
       }
+      if (failed) break;
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tp_arrive(a_full + 16 * c + 8 * blk);
     }
-    // all MMAs have completed once the last step's commit has arrived
-    if (!failed) {
-      const int last = nchunks - 1;
-      failed = !tc_mbar_wait(mbar_empty + 8 * (last % kTcStages), (uint32_t)((last / kTcStages) & 1));
-    }
-  } else if (lane == 0) {
-    // ---- the MMA thread: 4 K = 16 steps x 2 row blocks per stage, then the commit that releases the stage ----
-    for (int c = 0; c < nchunks; ++c) {
-      const int s = c % kTcStages;
-      if (!tc_mbar_wait(mbar_full + 8 * s, (uint32_t)((c / kTcStages) & 1))) {
+  } else if (warp >= 4) {
+    const int quarter = warp & 3, row = 32 * quarter + lane;
+    I4Ring<2> dr;
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+      const int tile = u / blocks, row0 = (u - tile * blocks) * kRows;
+      const int p0 = a.tile_start[tile], cnt = a.tile_count[tile];
+      if (!__all_sync(0xffffffffu, i4_wait<400>(d_full + 8 * dr.slot, dr.turn))) {
         failed = true;
         break;
       }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t b = sbase + (uint32_t)s * kTcStageBytes;
-      const uint32_t ta = tmem + 2 * kTcN + (uint32_t)(s * 2) * kTcACols;
+      tc_fence_after();
+      const uint32_t td = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(dr.slot * 2 * kTcN);
+      // a row of the intermediate vector is a column of the down projection's activations
+      const int col = row0 + (SWIGLU ? (row & ~7) | ((row & 3) << 1) | ((row >> 2) & 1) : row);
+      for (int n0 = 0; n0 < cnt; n0 += 16) {
+        uint32_t ra[16], rb[16];
+        tmem_ld16(td + n0, ra);
+        tmem_ld16(td + kTcN + n0, rb);
+        tmem_wait_ld();
 #pragma unroll
-      for (int j = 0; j < kTcKC / 16; ++j) {
-        const uint32_t acc = (c > 0 || j > 0) ? 1u : 0u;
-        const uint64_t bd = tc_smem_desc(b + j * 2 * kTcBLbo, kTcBLbo, kTcSbo);
-        tc_mma_f16_ts(tmem, ta + 8 * j, bd, idesc, acc);
-        tc_mma_f16_ts(tmem + kTcN, ta + kTcACols + 8 * j, bd, idesc, acc);
+        for (int j = 0; j < 16; ++j) {
+          const int tok = n0 + j;
+          if (tok < cnt) {
+            const size_t p = a.out_index ? (size_t)a.out_index[p0 + tok] : (size_t)(p0 + tok);
+            const float va = __uint_as_float(ra[j]) * kI4Unscale, vb = __uint_as_float(rb[j]) * kI4Unscale;
+            if (SWIGLU) {
+              const float gv = round_bf16(va), uv = round_bf16(vb);
+              a.out[p * a.R + col] = f32_to_bf16_bits(round_bf16(gv / (1.0f + expf(-gv))) * uv);
+            } else {
+              a.out[p * a.R + col] = f32_to_bf16_bits(va);
+              a.out[p * a.R + col + 128] = f32_to_bf16_bits(vb);
+            }
+          }
+        }
       }
-      tc_commit(mbar_empty + 8 * s);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tp_arrive(d_empty + 8 * dr.slot);
+      dr.next();
+    }
+  } else if (warp == 3) {
+    if (lane == 0) {
+      I4Ring<kI4WStages> wr;
+      I4Ring<kI4SStages> sr;
+      long issued = 0;
+      for (int u = blockIdx.x; u < units && !failed; u += gridDim.x) {
+        const int tile = u / blocks, row0 = (u - tile * blocks) * kRows;
+        const int r = a.tile_expert[tile] * a.stride_rows + row0, rb = SWIGLU ? r : r + 128;
+        for (int st = 0; st < stages; ++st) {
+          if (!i4_wait<100>(w_empty + 8 * wr.slot, wr.turn ^ 1)) {
+            failed = true;
+            break;
+          }
+          const uint32_t dst = wbase + wr.slot * kI4WBytes, bar = w_full + 8 * wr.slot;
+          tp_expect_tx(bar, kI4WBytes + (st & 1 ? 0 : kI4SBytes));
+          if (!(st & 1)) {
+            // scales ride with the even stage; the slot's last readers, stages st - 6 and st - 5, left before stage st - 1 was asked for
+            const uint32_t sdst = sbase + sr.slot * kI4SBytes;
+            tp_load_2d(sdst, &msa, st * (kI4Cols / 16), r, bar);
+            tp_load_2d(sdst + kI4SBytes / 2, SWIGLU ? &msb : &msa, st * (kI4Cols / 16), rb, bar);
+            sr.next();
+          }
+          tp_load_2d(dst, &mwa, st * (kI4Cols / 2), r, bar);
+          tp_load_2d(dst + kI4WBytes / 2, SWIGLU ? &mwb : &mwa, st * (kI4Cols / 2), rb, bar);
+          wr.next();
+          ++issued;
+        }
+      }
+      // no copy may be in flight when the CTA leaves: the last use of every slot
+      for (long c = issued > kI4WStages ? issued - kI4WStages : 0; c < issued; ++c)
+        i4_wait<0>(w_full + 8 * (int)(c % kI4WStages), (uint32_t)((c / kI4WStages) & 1));
+    }
+  } else if (warp == 2) {
+    if (lane == 0) {
+      I4Ring<kI4XStages> xr;
+      long issued = 0;
+      for (int u = blockIdx.x; u < units && !failed; u += gridDim.x) {
+        const int tile = u / blocks, p0 = a.tile_start[tile], rows16 = (a.tile_count[tile] + 15) >> 4;
+        for (int c = 0; c < 2 * stages; ++c) {
+          if (!i4_wait<20>(x_empty + 8 * xr.slot, xr.turn ^ 1)) {
+            failed = true;
+            break;
+          }
+          const uint32_t dst = xbase + xr.slot * kI4XBytes, bar = x_full + 8 * xr.slot;
+          tp_expect_tx(bar, rows16 * 4096);
+          for (int n = 0; n < rows16; ++n) {
+            tp_load_2d(dst + n * 2048, &mx, c * 128, p0 + 16 * n, bar);
+            tp_load_2d(dst + kI4XHalf + n * 2048, &mx, c * 128 + 64, p0 + 16 * n, bar);
+          }
+          xr.next();
+          ++issued;
+        }
+      }
+      for (long c = issued > kI4XStages ? issued - kI4XStages : 0; c < issued; ++c)
+        i4_wait<0>(x_full + 8 * (int)(c % kI4XStages), (uint32_t)((c / kI4XStages) & 1));
+    }
+  } else {
+    const I4Mma m = {x_full, x_empty, a_full, a_empty, d_full, d_empty, xbase};
+    failed = warp ? !i4_mma<1>(m, a, units, blocks, stages) : !i4_mma<0>(m, a, units, blocks, stages);
+  }
+  if (failed) atomicExch(&g_wgemm_tc_error, 1u);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tp_tmem_free(tmem, kI4TmemCols);
+}
+
+// xs[p] = x[x_index ? x_index[p] : p] for the sorted positions p of every tile, the columns of each packed word in the
+// order 0 4 1 5 2 6 3 7.  grid = (tile slots, parts of a tile).
+__global__ void __launch_bounds__(256) i4_rows_kernel(const uint16_t *__restrict__ x, const int *__restrict__ x_index, int K,
+                                                      const int *__restrict__ tile_start, const int *__restrict__ tile_count,
+                                                      const int *__restrict__ num_tiles, uint16_t *__restrict__ xs) {
+  const int ntiles = *num_tiles, per_row = K / 8;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int p0 = tile_start[tile], n = tile_count[tile] * per_row;
+    for (int u = blockIdx.y * 256 + threadIdx.x; u < n; u += gridDim.y * 256) {
+      const int r = u / per_row, c = u - r * per_row;
+      const size_t src = x_index ? (size_t)x_index[p0 + r] : (size_t)(p0 + r);
+      const uint4 v = reinterpret_cast<const uint4 *>(x + src * K)[c];
+      uint4 o;
+      o.x = __byte_perm(v.x, v.z, 0x5410);
+      o.y = __byte_perm(v.x, v.z, 0x7632);
+      o.z = __byte_perm(v.y, v.w, 0x5410);
+      o.w = __byte_perm(v.y, v.w, 0x7632);
+      reinterpret_cast<uint4 *>(xs + (size_t)(p0 + r) * K)[c] = o;
     }
   }
-  failed = __any_sync(0xffffffffu, failed);  // warp-uniform: the tensor-memory loads below are warp-wide
-  if (failed && lane == 0) atomicExch(&g_wgemm_tc_error, 1u);
-
-  if (producer && !failed) tc_epilogue<SWIGLU>(a, tmem, kTcN, warp, lane, N, cnt, p0, row0);
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  // a CTA that gave up on a barrier stops here (every warp: the flag goes through the barrier's OR)
-  if (__syncthreads_or(failed ? 1 : 0)) break;
-  // the next tile sets the barriers up afresh
-  if (tid == 0) {
-#pragma unroll
-    for (int s = 0; s < 2 * kTcStages; ++s) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(mbar_full + 8 * s) : "memory");
-  }
-  __syncthreads();
-  }
-  if (have_tmem && warp == 0)  // block-uniform: every thread walked the same tiles
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTcTmemCols) : "memory");
 }
 
 // ---- bf16 weights (shared expert): both operands come straight from global memory into the core-matrix layout
@@ -564,45 +637,73 @@ __global__ void __launch_bounds__(kTcThreads, 1) wgemm_tc_bf16_kernel(const WgAr
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kBfTmemCols) : "memory");
 }
 
-size_t wgemm_tc_smem_bytes() { return (size_t)kTcStages * kTcStageBytes + (size_t)kTcRing * kTcRawBytes; }
-
-// True when the tcgen05 kernel covers this mode and shape.
+// True when the tcgen05 kernel for bf16 weights covers this mode and shape.
 bool wgemm_tc_supports(int mode, const WgArgs &args) {
-  const bool swiglu = mode == WG_I4_SWIGLU || mode == WG_BF16_SWIGLU;
-  const int rows_per_cta = swiglu ? 128 : 256;
-  return args.R % rows_per_cta == 0 && args.K % kTcSuper == 0 && args.K / kTcKC >= kBfMinSteps;
+  if (mode != WG_BF16_PLAIN && mode != WG_BF16_SWIGLU) return false;
+  return args.R % (mode == WG_BF16_SWIGLU ? 128 : 256) == 0 && args.K % kTcKC == 0 && args.K / kTcKC >= kBfMinSteps;
+}
+
+static bool tc_aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+bool wgemm_i4_supports(const WgArgs &up, const WgArgs &down) {
+  if (up.K % 512 || up.R % 512 || down.K != up.R || down.R != up.K) return false;
+  for (const void *p : {up.w_a, up.w_b, down.w_a, (const void *)up.s_a, (const void *)up.s_b, (const void *)down.s_a, (const void *)up.x,
+                        (const void *)up.out_bf16})
+    if (!tc_aligned16(p)) return false;
+  return true;
+}
+
+static int i4_launch(bool swiglu, const WgArgs &g, const uint16_t *x, long x_rows, cudaStream_t stream) {
+  // rows past the last expert are never addressed: the coordinates come from the tile table
+  constexpr long kRows = 1l << 31;
+  CUtensorMap wa, wb, sa, sb, mx;
+  int rc;
+  if ((rc = tensor_map_2d(g.w_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, kRows, g.K / 2, g.K / 2, 128, kI4Cols / 2, CU_TENSOR_MAP_SWIZZLE_128B, &wa))) return rc;
+  if ((rc = tensor_map_2d(g.s_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, kRows, g.K / 16, g.K / 16, 128, 32, CU_TENSOR_MAP_SWIZZLE_32B, &sa))) return rc;
+  wb = wa;
+  sb = sa;
+  if (swiglu) {
+    if ((rc = tensor_map_2d(g.w_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, kRows, g.K / 2, g.K / 2, 128, kI4Cols / 2, CU_TENSOR_MAP_SWIZZLE_128B, &wb))) return rc;
+    if ((rc = tensor_map_2d(g.s_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, kRows, g.K / 16, g.K / 16, 128, 32, CU_TENSOR_MAP_SWIZZLE_32B, &sb))) return rc;
+  }
+  if ((rc = tensor_map_2d(x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x_rows, g.K, (long)g.K * 2, 16, 64, CU_TENSOR_MAP_SWIZZLE_128B, &mx))) return rc;
+  const I4Args a = {g.out_bf16, g.out_index, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.K, g.R, (int)g.expert_stride_rows};
+  if (swiglu) {
+    BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kI4Smem));
+    wgemm_tc_kernel<true><<<sm_count(), kI4Threads, kI4Smem, stream>>>(wa, wb, sa, sb, mx, a);
+  } else {
+    BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kI4Smem));
+    wgemm_tc_kernel<false><<<sm_count(), kI4Threads, kI4Smem, stream>>>(wa, wb, sa, sb, mx, a);
+  }
+  return launch_status("wgemm_tc_kernel");
+}
+
+int launch_wgemm_i4(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream) {
+  // a tile's rows are shared by a few CTAs: 64 rows of 7,168 columns are 57,344 16-byte pieces
+  i4_rows_kernel<<<dim3(std::min(max_tiles, 1024), 4), 256, 0, stream>>>(up.x, up.x_index, up.K, up.tile_start, up.tile_count, up.num_tiles, xs);
+  int rc = launch_status("i4_rows_kernel");
+  if (rc) return rc;
+  if ((rc = i4_launch(true, up, xs, rows, stream))) return rc;
+  return i4_launch(false, down, up.out_bf16, rows, stream);
 }
 
 int launch_wgemm_tc(int mode, const WgArgs &args, int max_tiles, cudaStream_t stream) {
-  const bool swiglu = mode == WG_I4_SWIGLU || mode == WG_BF16_SWIGLU;
+  const bool swiglu = mode == WG_BF16_SWIGLU;
   dim3 grid(args.R / (swiglu ? 128 : 256), max_tiles);
-  if (mode == WG_BF16_SWIGLU || mode == WG_BF16_PLAIN) {
 #define BLOK_BF_LAUNCH(SW, NT)                                                                                                 \
   {                                                                                                                            \
     const size_t bsmem = (size_t)BfCfg<NT>::kStages * BfCfg<NT>::kStageBytes;                                                  \
     BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_bf16_kernel<SW, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));    \
     wgemm_tc_bf16_kernel<SW, NT><<<grid, kTcThreads, bsmem, stream>>>(args);                                                   \
   }
-    if (args.identity_tiles) {
-      grid.y = (args.n_rows + 255) / 256;
-      if (swiglu) BLOK_BF_LAUNCH(true, 256) else BLOK_BF_LAUNCH(false, 256)
-    } else {
-      if (swiglu) BLOK_BF_LAUNCH(true, 64) else BLOK_BF_LAUNCH(false, 64)
-    }
-#undef BLOK_BF_LAUNCH
-    return launch_status("wgemm_tc_bf16_kernel");
-  }
-  const size_t smem = wgemm_tc_smem_bytes();
-  // tile slots: about eight rounds of CTAs (two per SM); a CTA walks the tiles of its slot
-  const dim3 igrid(grid.x, std::min(max_tiles, std::max(1, 8 * 2 * sm_count() / (int)grid.x)));
-  if (swiglu) {
-    BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    wgemm_tc_kernel<true><<<igrid, kTcThreads, smem, stream>>>(args);
+  if (args.identity_tiles) {
+    grid.y = (args.n_rows + 255) / 256;
+    if (swiglu) BLOK_BF_LAUNCH(true, 256) else BLOK_BF_LAUNCH(false, 256)
   } else {
-    BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    wgemm_tc_kernel<false><<<igrid, kTcThreads, smem, stream>>>(args);
+    if (swiglu) BLOK_BF_LAUNCH(true, 64) else BLOK_BF_LAUNCH(false, 64)
   }
-  return launch_status("wgemm_tc_kernel");
+#undef BLOK_BF_LAUNCH
+  return launch_status("wgemm_tc_bf16_kernel");
 }
 
 // Non-zero once any tcgen05 GEMM CTA gave up on a barrier; cleared by the read.

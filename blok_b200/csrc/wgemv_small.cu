@@ -12,9 +12,7 @@
 // one group (a group of 5..8 tokens is two passes over its weights): the pass's activations are quantised to block
 // integers in shared memory once per task run, then each warp streams one row-block over the whole K in chunks of 14 or
 // 16 k-blocks (the scales of a chunk are staged whole, as in moe_fused.cu).  Tasks are dealt out in contiguous ranges, so
-// a CTA restages activations about twice per launch.  Larger groups are left to the tcgen05 kernel, which skips what this
-// kernel took (WgArgs::small_max, ::small_limit) - unless they are so few (48 passes' worth) that the GEMM kernel would
-// spend a CTA's whole latency, about 100 us per product, on a handful of tiles: then this kernel takes every group.
+// a CTA restages activations about twice per launch.  launch_wgemm_experts (wgemm.cu) sends it products of few assignments.
 //
 // Measured at T = 64 (284 groups, 7.05 GB of expert weights): gate/up and down together about 1.6 ms (4.4 TB/s); with
 // every lane loading a token's operands (24 of 32 read the zero block) 1.75 ms; with a run-time token loop and pointer
@@ -35,8 +33,7 @@ constexpr int kGsDepth = 5;                               // ring steps of 1 KB 
 constexpr int kGsMaxChunk = 16;                           // most k-blocks whose scales are staged together
 constexpr int kGsScaleRow = kGsMaxChunk * 8 + 16;         // bytes per row of the scale stage (36 words: rows 4 banks apart)
 constexpr int kGsWarpBytes = kGsDepth * 1024 + 16 * kGsScaleRow;
-constexpr int kGsBigPasses = 48;                          // most passes of larger groups this kernel takes over from the GEMM kernel
-constexpr int kGsMaxGroups = 2048;                        // small groups a launch can hold in its shared-memory list
+constexpr int kGsMaxGroups = 2048;                        // passes a launch can hold in its shared-memory list
 
 __device__ __forceinline__ void gs_cp16(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -205,7 +202,7 @@ template <bool SWIGLU>
 __global__ void __launch_bounds__(kGsThreads, 1) wgemv_small_kernel(const WgArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ unsigned short s_group[kGsMaxGroups];  // the launch's passes: tile index | pass of the tile << 12
-  __shared__ int s_ngroups, s_limit;
+  __shared__ int s_ngroups;
   __shared__ int s_wcount[kGsWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -213,34 +210,14 @@ __global__ void __launch_bounds__(kGsThreads, 1) wgemv_small_kernel(const WgArgs
   const size_t xbytes = imma_stage_bytes(K);
   const uint32_t smem_addr = (uint32_t)__cvta_generic_to_shared(smem);
 
-  // ---- which groups are this kernel's: those of up to kWgSmallTokens tokens, or every group when the larger ones are so
-  // few that the GEMM kernel behind this one would spend a CTA's whole latency (about 100 us per product) on a handful
-  // of tiles, while their passes here are spread over every SM (about 5 us each) ----
   const int ntiles = *a.num_tiles;
-  {
-    int mine = 0;
-    for (int i = tid; i < ntiles; i += kGsThreads) {
-      const int c = a.tile_count[i];
-      if (c > kWgSmallTokens) mine += (c + kGsPass - 1) / kGsPass;
-    }
-    for (int o = 16; o; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-    if (lane == 0) s_wcount[warp] = mine;
-    __syncthreads();
-    if (tid == 0) {
-      int tot = 0;
-      for (int w = 0; w < kGsWarps; ++w) tot += s_wcount[w];
-      s_limit = (a.small_limit && tot <= kGsBigPasses) ? kWgTileTokens : kWgSmallTokens;
-      if (a.small_limit && blockIdx.x == 0) *a.small_limit = s_limit;  // the GEMM kernel skips what this one takes
-      s_ngroups = 0;
-    }
-    __syncthreads();
-  }
-  const int limit = s_limit;
+  if (tid == 0) s_ngroups = 0;
+  __syncthreads();
   // ---- the passes in tile order, up to kGsPass tokens each (every CTA builds the same list) ----
   for (int i0 = 0; i0 < ntiles; i0 += kGsThreads) {
     const int i = i0 + tid;
     const int c = i < ntiles ? a.tile_count[i] : 0;
-    const int np = (c >= 1 && c <= limit) ? (c + kGsPass - 1) / kGsPass : 0;
+    const int np = (c + kGsPass - 1) / kGsPass;
     // positions by a block-wide ordered count: a scan inside the warp, then the warps in order
     int incl = np;
     for (int o = 1; o < 32; o <<= 1) {
@@ -334,10 +311,10 @@ __global__ void __launch_bounds__(kGsThreads, 1) wgemv_small_kernel(const WgArgs
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// max_tiles: the most tiles the launch's table can hold; every pass of every tile must fit the kernel's list (two passes
-// per tile of up to kWgSmallTokens tokens, kGsBigPasses more when it takes the larger groups too) and its 12-bit tile index
+// max_tiles: the most tiles the launch's table can hold; every pass of every tile must fit the kernel's list and its 12-bit
+// tile index
 bool wgemv_small_supports(int mode, const WgArgs &a, int max_tiles) {
-  if (max_tiles > 4096 || 2 * max_tiles + kGsBigPasses > kGsMaxGroups) return false;
+  if (max_tiles > 4096 || max_tiles + a.n_rows / kGsPass > kGsMaxGroups) return false;
   if (mode != WG_I4_SWIGLU && mode != WG_I4_PLAIN) return false;
   if (a.identity_tiles || a.K % 256 || a.R % 16) return false;  // 16-byte scale copies: an even number of k-blocks per row
   return wgemv_small_smem_bytes(a.K) <= 200 * 1024;
