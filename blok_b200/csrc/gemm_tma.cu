@@ -48,11 +48,13 @@ __device__ __forceinline__ float gt_act(float v) {
 
 template <int BN, int ACT, bool F32>
 __global__ void __launch_bounds__(kGtThreads)
-    gemm_tma_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw, const GtArgs a) {
+    gemm_tma_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mup,
+                    const GtArgs a) {
   using Cfg = GtCfg<BN>;
   constexpr int S = Cfg::kStages;
   // a pair of 128-row boxes, gate and up, makes 128 output columns
-  constexpr int kCols = ACT == GEMM_ACT_SWIGLU ? BN / 2 : BN;
+  constexpr bool kGated = ACT == GEMM_ACT_SWIGLU || ACT == GEMM_ACT_SWIGLU_REF;
+  constexpr int kCols = kGated ? BN / 2 : BN;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long s_bar[2 * S + 1];
   __shared__ uint32_t s_tmem;
@@ -84,7 +86,8 @@ __global__ void __launch_bounds__(kGtThreads)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_tmem;
-  const int nsteps = (a.K + kGtKStep - 1) / kGtKStep;
+  const int all_steps = (a.K + kGtKStep - 1) / kGtKStep;
+  const int first = (int)((long)all_steps * blockIdx.z / gridDim.z), nsteps = (int)((long)all_steps * (blockIdx.z + 1) / gridDim.z) - first;
   bool failed = false;
 
   if (warp == 4) {
@@ -98,9 +101,10 @@ __global__ void __launch_bounds__(kGtThreads)
         }
         const uint32_t dst = sbase + (uint32_t)s * Cfg::kStageBytes;
         tp_expect_tx(full + 8 * s, Cfg::kStageBytes);
-        tp_load_2d(dst, &mx, c * kGtKStep, row0, full + 8 * s);
-        tp_load_2d(dst + Cfg::kABytes, &mw, c * kGtKStep, wrow, full + 8 * s);
-        if (ACT == GEMM_ACT_SWIGLU) tp_load_2d(dst + Cfg::kABytes + kCols * 128, &mw, c * kGtKStep, a.up_row + wrow, full + 8 * s);
+        const int k = (first + c) * kGtKStep;
+        tp_load_2d(dst, &mx, k, row0, full + 8 * s);
+        tp_load_2d(dst + Cfg::kABytes, &mw, k, wrow, full + 8 * s);
+        if (kGated) tp_load_2d(dst + Cfg::kABytes + kCols * 128, &mup, k, a.up_row + wrow, full + 8 * s);
         issued = c + 1;
       }
       // no copy may be in flight when the CTA leaves; the MMA lane has seen all of them unless a wait gave up
@@ -134,9 +138,9 @@ __global__ void __launch_bounds__(kGtThreads)
     if (!failed) {
       tc_fence_after();
       const int r = 32 * warp + lane;
-      const size_t o = (size_t)(row0 + r) * a.ldo;
+      const size_t o = ((size_t)blockIdx.z * a.T + row0 + r) * a.ldo;
       const int n0 = blockIdx.x * kCols;
-      if constexpr (ACT == GEMM_ACT_SWIGLU) {
+      if constexpr (kGated) {
 #pragma unroll 1
         for (int c0 = 0; c0 < kCols; c0 += 16) {
           if (n0 + c0 >= a.R) break;
@@ -150,9 +154,21 @@ __global__ void __launch_bounds__(kGtThreads)
             for (int j = 0; j < 16; j += 4) {
               const int col = n0 + c0 + j;
               if (col < a.R) {
+                if (F32) {  // the parts of a K split
+                  *reinterpret_cast<uint4 *>(static_cast<float *>(a.out) + o + col) = make_uint4(gate[j], gate[j + 1], gate[j + 2], gate[j + 3]);
+                  *reinterpret_cast<uint4 *>(static_cast<float *>(a.out) + o + a.R + col) = make_uint4(up[j], up[j + 1], up[j + 2], up[j + 3]);
+                  continue;
+                }
                 float f[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) f[i] = gt_act<GEMM_ACT_SILU>(__uint_as_float(gate[j + i])) * __uint_as_float(up[j + i]);
+                for (int i = 0; i < 4; ++i) {
+                  if (ACT == GEMM_ACT_SWIGLU_REF) {
+                    const float g = round_bf16(__uint_as_float(gate[j + i]));
+                    f[i] = round_bf16(g / (1.0f + expf(-g))) * round_bf16(__uint_as_float(up[j + i]));
+                  } else {
+                    f[i] = gt_act<GEMM_ACT_SILU>(__uint_as_float(gate[j + i])) * __uint_as_float(up[j + i]);
+                  }
+                }
                 *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(a.out) + o + col) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
               }
             }
@@ -222,12 +238,20 @@ template <int BN, int ACT, bool F32>
 static int gt_launch(const GemmTma &g, dim3 grid, cudaStream_t stream) {
   const GtArgs a = {g.out, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.T, g.R, g.K, g.ldo, g.act_cols, g.up_row};
   BLOK_CUDA(cudaFuncSetAttribute(gemm_tma_kernel<BN, ACT, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, GtCfg<BN>::kSmem));
-  gemm_tma_kernel<BN, ACT, F32><<<grid, kGtThreads, GtCfg<BN>::kSmem, stream>>>(*g.x, BN == 128 || ACT == GEMM_ACT_SWIGLU ? *g.w128 : *g.w256, a);
+  gemm_tma_kernel<BN, ACT, F32><<<grid, kGtThreads, GtCfg<BN>::kSmem, stream>>>(
+      *g.x, BN == 128 || ACT == GEMM_ACT_SWIGLU || ACT == GEMM_ACT_SWIGLU_REF ? *g.w128 : *g.w256, g.up128 ? *g.up128 : *g.w128, a);
   return launch_status("gemm_tma_kernel");
 }
 
 int launch_gemm_tma(const GemmTma &g, cudaStream_t stream) {
   BLOK_REQUIRE(g.x && g.w128 && g.out && g.R % 4 == 0 && g.K % 8 == 0 && g.T >= 1, BLOK_ERR_SHAPE, "gemm: T %d, R %d, K %d", g.T, g.R, g.K);
+  BLOK_REQUIRE(g.splits == 1 || (g.out_f32 && !g.tile_start && (g.act == GEMM_ACT_NONE || g.act == GEMM_ACT_SWIGLU_REF)), BLOK_ERR_SHAPE,
+               "gemm: a K split leaves plain fp32 sums");
+  if (g.act == GEMM_ACT_SWIGLU_REF) {
+    BLOK_REQUIRE(g.up128 && !g.tile_start && (g.splits > 1) == g.out_f32, BLOK_ERR_SHAPE, "gemm: a gated product is bf16 and not grouped");
+    const dim3 grid((g.R + 127) / 128, (g.T + kGtTileRows - 1) / kGtTileRows, g.splits);
+    return g.out_f32 ? gt_launch<256, GEMM_ACT_SWIGLU_REF, true>(g, grid, stream) : gt_launch<256, GEMM_ACT_SWIGLU_REF, false>(g, grid, stream);
+  }
   if (g.act == GEMM_ACT_SWIGLU) {
     BLOK_REQUIRE(!g.out_f32 && !g.tile_start, BLOK_ERR_SHAPE, "gemm: a gated product is bf16 and not grouped");
     return gt_launch<256, GEMM_ACT_SWIGLU, false>(g, dim3((g.R + 127) / 128, (g.T + kGtTileRows - 1) / kGtTileRows), stream);
@@ -236,7 +260,7 @@ int launch_gemm_tma(const GemmTma &g, cudaStream_t stream) {
   // the wide tile reads fewer bytes from shared memory per product; it needs enough tiles to fill the GPU
   const long wide = (long)((g.R + 255) / 256) * (g.tile_start ? (g.T + kGtTileRows - 1) / kGtTileRows : tiles);
   const bool use256 = g.w256 && wide >= sm_count();
-  const dim3 grid((g.R + (use256 ? 255 : 127)) / (use256 ? 256 : 128), tiles);
+  const dim3 grid((g.R + (use256 ? 255 : 127)) / (use256 ? 256 : 128), tiles, g.splits);
   if (g.act == GEMM_ACT_SILU) {
     BLOK_REQUIRE(!g.out_f32 && g.act_cols % 4 == 0, BLOK_ERR_SHAPE, "gemm: SiLU on %d columns of an fp32 output", g.act_cols);
     return use256 ? gt_launch<256, GEMM_ACT_SILU, false>(g, grid, stream) : gt_launch<128, GEMM_ACT_SILU, false>(g, grid, stream);

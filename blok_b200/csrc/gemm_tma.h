@@ -7,7 +7,8 @@
 
 namespace blok {
 
-enum { GEMM_ACT_NONE = 0, GEMM_ACT_RELU2 = 1, GEMM_ACT_SILU = 2, GEMM_ACT_SWIGLU = 3 };
+// GEMM_ACT_SWIGLU_REF: the gated product with the reference's rounding points (both products, SiLU and the result to bf16).
+enum { GEMM_ACT_NONE = 0, GEMM_ACT_RELU2 = 1, GEMM_ACT_SILU = 2, GEMM_ACT_SWIGLU = 3, GEMM_ACT_SWIGLU_REF = 4 };
 constexpr int kGtTileRows = 128;  // rows of x per tile
 
 // A 2-D tensor map: rows of `cols` elements, `pitch` bytes apart (a multiple of 16; base 16-byte aligned), copied in boxes
@@ -31,6 +32,11 @@ struct GemmTma {
   int act_cols = 0;                            // GEMM_ACT_SILU: the first so many columns (a multiple of 4) only; bf16 output
   // GEMM_ACT_SWIGLU: out[t, r] = silu(row r) * (row up_row + r), bf16 (R counts the outputs; the weights hold both halves)
   int up_row = 0;
+  // GEMM_ACT_SWIGLU_REF: the up weights, a matrix of their own (w128: the gate weights)
+  const CUtensorMap *up128 = nullptr;
+  // > 1: K is cut into so many parts (grid.z), `out` is fp32 [splits][T][ldo] and holds the parts' sums (of both products, gate
+  // columns then up columns, ldo = 2 R, for a gated product); no activation
+  int splits = 1;
   // Grouped form: tile i covers rows [tile_start[i], + tile_count[i]) of x (at most kGtTileRows) and weight rows
   // [tile_expert[i] * R, + R); at most max_tiles tiles, *num_tiles of them valid.  NULL: consecutive tiles of one matrix.
   const int *tile_expert = nullptr, *tile_start = nullptr, *tile_count = nullptr, *num_tiles = nullptr;

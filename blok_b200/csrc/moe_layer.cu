@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "moe_layer.h"
+#include "gemm_tma.h"
 #include "wgemm.h"
 
 namespace blok {
@@ -224,9 +225,10 @@ extern "C" int blok_moe_layer_check(blok_moe_layer_t *L, blok_stream_t stream_) 
   BLOK_REQUIRE(L, BLOK_ERR_ARG, "blok_moe_layer_check: null pointer");
   cudaStream_t stream = (cudaStream_t)stream_;
   BLOK_CUDA(cudaStreamSynchronize(stream));
-  unsigned tc_err = 0;
+  unsigned tc_err = 0, gt_err = 0;
   if (int rc = wgemm_tc_take_error(&tc_err)) return rc;
-  if (tc_err) {
+  if (int rc = gemm_tma_take_error(&gt_err)) return rc;
+  if (tc_err || gt_err) {
     set_error("blok_moe_batched: a tensor-core GEMM tile gave up waiting for its MMAs");
     return BLOK_ERR_TIMEOUT;
   }

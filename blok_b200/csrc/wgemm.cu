@@ -13,6 +13,7 @@
 // to the reference's exact bf16 values bf16(q * scale) (one subtract and one
 // multiply on packed bf16 pairs) and reused across the tile's token columns.
 #include "common.cuh"
+#include "gemm_tma.h"
 #include "wgemm.h"
 #include <algorithm>
 #include <cstdlib>
@@ -202,6 +203,45 @@ static int wgemm_forced_impl() {  // read at every launch, so that a test can sw
   return 0;
 }
 
+static bool wg_aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// A dense product the TMA-fed GEMM covers (gemm_tma.cu).
+static bool wgemm_tma_supports(int mode, const WgArgs &a) {
+  if (!a.identity_tiles || a.x_index || a.out_index || a.K % 8 || a.R % 8 || a.n_rows < 1) return false;
+  return wg_aligned16(a.w_a) && wg_aligned16(a.x) && wg_aligned16(a.out_bf16) && wg_aligned16(a.out_f32) &&
+         (mode != WG_BF16_SWIGLU || wg_aligned16(a.w_b));
+}
+
+// forced: no K split, so that a row's sums do not depend on how many rows the launch has
+static int launch_wgemm_tma(int mode, const WgArgs &a, int forced, cudaStream_t stream) {
+  const bool swiglu = mode == WG_BF16_SWIGLU;
+  CUtensorMap mx, mw, mw256, mup;
+  int rc;
+  if ((rc = gemm_operand_map(a.x, a.n_rows, a.K, a.K, kGtTileRows, &mx))) return rc;
+  if ((rc = gemm_operand_map(a.w_a, a.R, a.K, a.K, 128, &mw))) return rc;
+  if ((rc = gemm_operand_map(swiglu ? a.w_b : a.w_a, a.R, a.K, a.K, swiglu ? 128 : 256, swiglu ? &mup : &mw256))) return rc;
+  GemmTma g;
+  g.x = &mx;
+  g.w128 = &mw;
+  if (swiglu) g.up128 = &mup;
+  else g.w256 = &mw256;
+  g.T = a.n_rows; g.R = a.R; g.K = a.K; g.ldo = a.R;
+  g.act = swiglu ? GEMM_ACT_SWIGLU_REF : GEMM_ACT_NONE;
+  g.out = a.out_f32 ? (void *)a.out_f32 : (void *)a.out_bf16;
+  g.out_f32 = a.out_f32 != nullptr;
+  const int cols = swiglu ? 2 * a.R : a.R;
+  const int nz = forced || !a.splitk_ws ? 1 : std::min<long>(wgemm_tma_split(mode, a.K, a.R, a.n_rows), a.splitk_bytes / ((size_t)a.n_rows * cols * sizeof(float)));
+  if (nz > 1) {
+    g.splits = nz;
+    g.out = a.splitk_ws;
+    g.out_f32 = true;
+    g.ldo = cols;
+    if ((rc = launch_gemm_tma(g, stream))) return rc;
+    return launch_wgemm_splitk_reduce(mode, a, nz, stream);
+  }
+  return launch_gemm_tma(g, stream);
+}
+
 int launch_wgemm(int mode, const WgArgs &args, int max_tiles, cudaStream_t stream) {
   const int forced = wgemm_forced_impl();
   const bool i4 = mode == WG_I4_SWIGLU || mode == WG_I4_PLAIN;
@@ -211,10 +251,8 @@ int launch_wgemm(int mode, const WgArgs &args, int max_tiles, cudaStream_t strea
     if (int rc = launch_wgemm_stream(mode, args, &nz, stream)) return rc;
     return nz > 1 ? launch_wgemm_splitk_reduce(mode, args, nz, stream) : BLOK_OK;
   }
-  // bf16: the tcgen05 kernel's 256-token tiles leave most SMs idle below about 650 tokens (shared expert: 376 us from
-  // 128 to 1,024 tokens, against 106 / 162 / 297 / 585 us for the K-split mma.sync kernel at 128 / 256 / 512 / 1,024)
-  const bool enough = args.n_rows >= 640;
-  if (forced != 1 && (forced == 2 || enough) && wgemm_tc_supports(mode, args)) return launch_wgemm_tc(mode, args, max_tiles, stream);
+  // the mma.sync kernel with its K-split, over the shared expert of 2048 x 7168 at 517 tokens: 235 + 121 us
+  if (!i4 && forced != 1 && wgemm_tma_supports(mode, args)) return launch_wgemm_tma(mode, args, forced, stream);
   const size_t smem = wgemm_smem_bytes();
   const int rows_per_cta = swiglu ? 8 * kWgWarps : 16 * kWgWarps;
   BLOK_REQUIRE(args.R % rows_per_cta == 0 && args.K % kWgChunk == 0, BLOK_ERR_SHAPE,

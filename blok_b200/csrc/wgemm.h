@@ -38,8 +38,8 @@ struct WgArgs {
 };
 
 // Picks the kernel of a launch.  INT4 modes: the mma.sync kernel (see launch_wgemm_experts for the others).  bf16 modes: up to
-// kWgStreamTokens rows of a dense product the weight-streaming kernel (wgemm_stream.cu); from 640 tokens on the tcgen05
-// kernel; in between, and for shapes the others do not cover, the mma.sync kernel with its K-split.
+// kWgStreamTokens rows of a dense product the weight-streaming kernel (wgemm_stream.cu); more, the TMA-fed tcgen05 GEMM
+// (gemm_tma.cu), K split where its tiles are few; for shapes the others do not cover the mma.sync kernel with its K-split.
 // BLOK_WGEMM_IMPL=mma / =tc in the environment forces one GEMM kernel for every row (no small-group or streaming kernel).
 int launch_wgemm(int mode, const WgArgs &args, int max_tiles, cudaStream_t stream);
 
@@ -50,6 +50,7 @@ int launch_wgemm(int mode, const WgArgs &args, int max_tiles, cudaStream_t strea
 // the same bits.  wgemm_splitk_bytes: the scratch that serves every launch of up to max_rows rows.
 int wgemm_splitk_factor(int mode, int K, int R, int tiles);
 size_t wgemm_splitk_bytes(int mode, int K, int R, int max_rows);
+int wgemm_tma_split(int mode, int K, int R, int rows);  // the same for the TMA-fed GEMM
 
 // Fills the tile arrays with consecutive 64-row tiles of T rows (one group, expert 0): a dense layer.
 int launch_identity_tiles(int T, int *tile_expert, int *tile_start, int *tile_count, int *num_tiles, cudaStream_t stream);
@@ -80,8 +81,6 @@ int launch_wgemm_experts(const WgArgs &up, const WgArgs &down, uint16_t *xs, lon
 bool wgemm_i4_supports(const WgArgs &up, const WgArgs &down);
 int launch_wgemm_i4(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream);
 
-bool wgemm_tc_supports(int mode, const WgArgs &args);
-int launch_wgemm_tc(int mode, const WgArgs &args, int max_tiles, cudaStream_t stream);
 // *out becomes non-zero if a tcgen05 GEMM CTA has given up on a barrier since the last call (the flag is cleared).
 int wgemm_tc_take_error(unsigned *out);
 

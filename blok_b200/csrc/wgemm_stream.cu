@@ -242,11 +242,23 @@ int wgemm_splitk_factor(int mode, int K, int R, int tiles) {
   const int ctas = R / rows_per_cta * tiles, chunks = K / 512;
   return std::max(1, std::min(chunks, 2 * sm_count() / ctas));
 }
+// The TMA-fed GEMM has tiles of 128 rows of x by 128 outputs (256 where that fills the GPU) and two CTAs per SM: parts of at
+// least 16 of its 64-column steps, so that its pipeline fills (the 384-expert router over 517 tokens: 15 tiles, 7 parts).
+int wgemm_tma_split(int mode, int K, int R, int rows) {
+  if (mode != WG_BF16_PLAIN && mode != WG_BF16_SWIGLU) return 1;
+  const int ctas = (R + 127) / 128 * ((rows + 127) / 128);
+  return std::max(1, std::min((K + 63) / 64 / 16, 2 * sm_count() / ctas));
+}
 size_t wgemm_splitk_bytes(int mode, int K, int R, int max_rows) {
   size_t worst = 0;
+  for (int rows = 128; max_rows > kWgStreamTokens; rows += 128) {
+    const int nz = wgemm_tma_split(mode, K, R, rows);
+    if (nz > 1) worst = std::max(worst, (size_t)nz * std::min(rows, max_rows) * (mode == WG_BF16_SWIGLU ? 2 * R : R) * sizeof(float));
+    if (nz <= 1 || rows >= max_rows) break;  // the factor falls as the rows grow
+  }
   {  // the weight-streaming kernel over up to kWgStreamTokens rows
     const int nz = wgemm_stream_split(mode, K, R);
-    if (nz > 1) worst = (size_t)nz * std::min(max_rows, kWgStreamTokens) * (mode == WG_BF16_SWIGLU ? 2 * R : R) * sizeof(float);
+    if (nz > 1) worst = std::max(worst, (size_t)nz * std::min(max_rows, kWgStreamTokens) * (mode == WG_BF16_SWIGLU ? 2 * R : R) * sizeof(float));
   }
   for (int tiles = 1; tiles <= (max_rows + kWgTileTokens - 1) / kWgTileTokens; ++tiles) {
     const int nz = wgemm_splitk_factor(mode, K, R, tiles);

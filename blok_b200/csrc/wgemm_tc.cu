@@ -14,13 +14,7 @@
 
 namespace blok {
 
-constexpr int kTcProducers = 256;    // threads that unpack weights: one weight row each
-constexpr int kTcThreads = kTcProducers + 32;  // plus one warp whose first lane issues the MMAs
 constexpr int kTcN = kWgTileTokens;  // token columns of a tile
-constexpr int kTcKC = 64;            // weight columns per pipeline step
-constexpr int kTcSbo = 128;          // bytes between 8-token groups of the activation tile
-constexpr unsigned kTcSpinLimit = 1u << 22;
-
 __device__ unsigned g_wgemm_tc_error = 0;
 
 __device__ __forceinline__ uint32_t tc_bf16x2_mul(uint32_t a, uint32_t b) {
@@ -56,94 +50,6 @@ __device__ __forceinline__ void i4_dequant(uint32_t w, const I4Scale &s, uint32_
   o[3] = tc_bf16x2_fma(t & 0x00f000f0u, s.hi, s.off);
 }
 
-// Shared-memory matrix descriptor, K-major, no swizzle: start address, leading (K) and
-// stride (M/N) byte offsets in 16-byte units, descriptor version 1.
-__device__ __forceinline__ uint64_t tc_smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
-}
-
-__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_commit(uint32_t mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
-
-// Bounded wait for the given phase parity of an mbarrier; false on timeout.
-__device__ __forceinline__ bool tc_mbar_wait(uint32_t mbar, uint32_t parity) {
-  for (unsigned it = 0; it < kTcSpinLimit; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(mbar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    __nanosleep(64);  // a failed try already waited out the hardware's own time slice; do not burn issue slots
-  }
-  return false;
-}
-
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_cp_async16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-// Epilogue of a tile: lane l of warp w (8 warps) holds accumulator row 32 (w % 4) + l of both row blocks (its
-// tensor-memory lane); warps 0..3 take the even 16-token column blocks, warps 4..7 the odd ones.
-template <bool SWIGLU>
-__device__ __forceinline__ void tc_epilogue(const WgArgs &a, uint32_t tmem, int acc1_col, int warp, int lane, int N, int cnt, int p0,
-                                            int row0) {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const int lg = warp & 3, row = 32 * lg + lane;
-  const uint32_t trow = tmem + ((uint32_t)(32 * lg) << 16);
-  for (int n0 = 16 * (warp >> 2); n0 < N; n0 += 32) {
-    uint32_t ra[16], rb[16];
-    tc_ld16(trow + n0, ra);
-    tc_ld16(trow + acc1_col + n0, rb);
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int tok = n0 + j;
-      if (tok < cnt) {
-        const size_t p = a.out_index ? (size_t)a.out_index[p0 + tok] : (size_t)(p0 + tok);
-        const float va = __uint_as_float(ra[j]), vb = __uint_as_float(rb[j]);
-        if (SWIGLU) {
-          const float gv = round_bf16(va), uv = round_bf16(vb);
-          const float m = round_bf16(round_bf16(gv / (1.0f + expf(-gv))) * uv);
-          a.out_bf16[p * a.R + row0 + row] = f32_to_bf16_bits(m);
-        } else if (a.out_f32) {
-          a.out_f32[p * a.R + row0 + row] = va;
-          a.out_f32[p * a.R + row0 + 128 + row] = vb;
-        } else {
-          a.out_bf16[p * a.R + row0 + row] = f32_to_bf16_bits(va);
-          a.out_bf16[p * a.R + row0 + 128 + row] = f32_to_bf16_bits(vb);
-        }
-      }
-    }
-  }
-}
-
-// ---- INT4 weights ----
-//
 // A unit is (tile of up to 64 tokens of one expert) x 256 weight rows (128 gate + 128 up rows of the same indices, or 256
 // rows of the down projection); a persistent CTA per SM walks the units, and every role runs ahead across their boundaries:
 //   warps 0, 1    MMAs of row block 0 and 1: 4 K = 16 steps per 64-column piece
@@ -471,178 +377,6 @@ __global__ void __launch_bounds__(256) i4_rows_kernel(const uint16_t *__restrict
   }
 }
 
-// ---- bf16 weights (shared expert): both operands come straight from global memory into the core-matrix layout
-// with 16-byte cp.async copies, one per (row, 8-column slice); no registers, no permutation.  kBfStages steps of
-// 2 x 128 weight rows + the token tile are in flight per CTA. ----
-constexpr int kBfMinSteps = 4;       // fewest 64-column steps the pipelines below are written for
-constexpr int kBfALbo = 2048 + 16;   // + 16 B: the 8 K-slices of a row, copied by 8 neighbouring lanes, hit 8 banks
-constexpr int kBfABytes = (kTcKC / 8) * kBfALbo;
-// NT = token columns per tile: 64 for tiles of an expert group, 256 for a dense layer (every token, same weights),
-// where the larger tile halves the bytes fetched from L2 per flop.  STAGES steps are resident per CTA.
-template <int NT>
-struct BfCfg {
-  static constexpr int kBLbo = (NT / 8) * 128 + 16;
-  static constexpr int kBBytes = (kTcKC / 8) * kBLbo;
-  static constexpr int kStageBytes = ((2 * kBfABytes + kBBytes + 127) / 128) * 128;
-  static constexpr int kStages = NT == 64 ? 4 : 3;
-  static constexpr int kTmemCols = 2 * NT;
-};
-
-__device__ __forceinline__ void tc_cp_async16_zfill(uint32_t dst, const void *src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-
-template <bool SWIGLU, int NT>
-__global__ void __launch_bounds__(kTcThreads, 1) wgemm_tc_bf16_kernel(const WgArgs a) {
-  using Cfg = BfCfg<NT>;
-  constexpr int kBfStages = Cfg::kStages;
-  constexpr int kBfStageBytes = Cfg::kStageBytes;
-  constexpr int kBfTmemCols = Cfg::kTmemCols;
-  constexpr int kBLbo = Cfg::kBLbo;
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) unsigned long long s_mbar[2 * kBfStages];
-  __shared__ uint32_t s_tmem_base;
-  const int tile = blockIdx.y;
-  int e, p0, cnt;
-  if (a.identity_tiles) {  // dense: tile t covers rows [NT t, NT t + NT) of x
-    e = 0;
-    p0 = NT * tile;
-    cnt = min(NT, a.n_rows - p0);
-    if (cnt <= 0) return;
-  } else {
-    if (tile >= *a.num_tiles) return;
-    e = a.tile_expert[tile], p0 = a.tile_start[tile], cnt = a.tile_count[tile];
-  }
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int N = max(16, (cnt + 15) & ~15);
-  const int rows_per_cta = SWIGLU ? 128 : 256;
-  const int row0 = blockIdx.x * rows_per_cta;
-  const bool producer = tid < kTcProducers;
-  const int nchunks = a.K / kTcKC;
-  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
-
-  // this thread's pieces: weight rows (tid / 8) + 32 i of both blocks (i < 4), tokens (tid / 8) + 32 i (i < 2), K-slice tid % 8
-  const int ki = tid & 7, r0 = tid >> 3;
-  const size_t rowbytes = (size_t)a.K * 2;
-  const unsigned char *wa = reinterpret_cast<const unsigned char *>(a.w_a) + ((size_t)e * a.expert_stride_rows + row0 + r0) * rowbytes + ki * 16;
-  const unsigned char *wb = SWIGLU ? reinterpret_cast<const unsigned char *>(a.w_b) + ((size_t)e * a.expert_stride_rows + row0 + r0) * rowbytes + ki * 16
-                                   : wa + 128 * rowbytes;
-  constexpr int kXPieces = NT / 32;  // activation pieces per thread and step
-  const unsigned char *xs[kXPieces];
-  uint32_t xbytes[kXPieces];
-#pragma unroll
-  for (int i = 0; i < kXPieces; ++i) {
-    const int tok = r0 + 32 * i;
-    xs[i] = reinterpret_cast<const unsigned char *>(a.x);
-    xbytes[i] = 0;  // rows beyond the tile's tokens are filled with zeros
-    if (tok < cnt) {
-      const size_t xr = a.x_index ? (size_t)a.x_index[p0 + tok] : (size_t)(p0 + tok);
-      xs[i] = reinterpret_cast<const unsigned char *>(a.x) + xr * rowbytes + ki * 16;
-      xbytes[i] = 16;
-    }
-  }
-  auto issue = [&](int c) {
-    if (c < nchunks) {
-      const uint32_t st = sbase + (uint32_t)(c % kBfStages) * kBfStageBytes;
-      const size_t koff = (size_t)c * (kTcKC * 2);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int row = r0 + 32 * i;
-        const uint32_t d = (uint32_t)(ki * kBfALbo + (row >> 3) * kTcSbo + (row & 7) * 16);
-        tc_cp_async16(st + d, wa + (size_t)(32 * i) * rowbytes + koff);
-        tc_cp_async16(st + kBfABytes + d, wb + (size_t)(32 * i) * rowbytes + koff);
-      }
-#pragma unroll
-      for (int i = 0; i < kXPieces; ++i) {
-        const int tok = r0 + 32 * i;
-        if (32 * i < N)
-          tc_cp_async16_zfill(st + 2 * kBfABytes + (uint32_t)(ki * kBLbo + (tok >> 3) * kTcSbo + (tok & 7) * 16),
-                              xs[i] + (xbytes[i] ? koff : 0), xbytes[i]);
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  if (producer) {
-#pragma unroll
-    for (int c = 0; c < kBfStages - 1; ++c) issue(c);
-  }
-
-  const uint32_t mbar_full = (uint32_t)__cvta_generic_to_shared(&s_mbar[0]);
-  const uint32_t mbar_empty = mbar_full + 8 * kBfStages;
-  if (tid == 0) {
-#pragma unroll
-    for (int s = 0; s < kBfStages; ++s) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar_full + 8 * s), "r"(kTcProducers / 32) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_empty + 8 * s) : "memory");
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(&s_tmem_base)),
-                 "r"((uint32_t)kBfTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = s_tmem_base;
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
-
-  bool failed = false;
-  if (producer) {
-    for (int c = 0; c < nchunks; ++c) {
-      // hand step c to the MMA thread as soon as this thread's pieces of it have landed ...
-      asm volatile("cp.async.wait_group %0;" ::"n"(kBfStages - 2) : "memory");
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar_full + 8 * (c % kBfStages)) : "memory");
-      // ... and only then wait for the stage that step c + kBfStages - 1 goes to: the MMAs of step c - 1 read it
-      if (c >= 1 && c + kBfStages - 1 < nchunks &&
-          !tc_mbar_wait(mbar_empty + 8 * ((c - 1) % kBfStages), (uint32_t)(((c - 1) / kBfStages) & 1))) {
-        failed = true;
-        break;
-      }
-      issue(c + kBfStages - 1);
-    }
-    if (!failed) {
-      const int last = nchunks - 1;
-      failed = !tc_mbar_wait(mbar_empty + 8 * (last % kBfStages), (uint32_t)((last / kBfStages) & 1));
-    }
-  } else if (lane == 0) {
-    for (int c = 0; c < nchunks; ++c) {
-      const int s = c % kBfStages;
-      if (!tc_mbar_wait(mbar_full + 8 * s, (uint32_t)((c / kBfStages) & 1))) {
-        failed = true;
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a0 = sbase + (uint32_t)s * kBfStageBytes, a1 = a0 + kBfABytes, b = a1 + kBfABytes;
-#pragma unroll
-      for (int j = 0; j < kTcKC / 16; ++j) {
-        const uint32_t acc = (c > 0 || j > 0) ? 1u : 0u;
-        const uint64_t bd = tc_smem_desc(b + j * 2 * kBLbo, kBLbo, kTcSbo);
-        tc_mma_f16(tmem, tc_smem_desc(a0 + j * 2 * kBfALbo, kBfALbo, kTcSbo), bd, idesc, acc);
-        tc_mma_f16(tmem + NT, tc_smem_desc(a1 + j * 2 * kBfALbo, kBfALbo, kTcSbo), bd, idesc, acc);
-      }
-      tc_commit(mbar_empty + 8 * s);
-    }
-  }
-  failed = __any_sync(0xffffffffu, failed);
-  if (failed && lane == 0) atomicExch(&g_wgemm_tc_error, 1u);
-  if (producer && !failed) tc_epilogue<SWIGLU>(a, tmem, NT, warp, lane, N, cnt, p0, row0);
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kBfTmemCols) : "memory");
-}
-
-// True when the tcgen05 kernel for bf16 weights covers this mode and shape.
-bool wgemm_tc_supports(int mode, const WgArgs &args) {
-  if (mode != WG_BF16_PLAIN && mode != WG_BF16_SWIGLU) return false;
-  return args.R % (mode == WG_BF16_SWIGLU ? 128 : 256) == 0 && args.K % kTcKC == 0 && args.K / kTcKC >= kBfMinSteps;
-}
-
 static bool tc_aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 bool wgemm_i4_supports(const WgArgs &up, const WgArgs &down) {
@@ -685,25 +419,6 @@ int launch_wgemm_i4(const WgArgs &up, const WgArgs &down, uint16_t *xs, long row
   if (rc) return rc;
   if ((rc = i4_launch(true, up, xs, rows, stream))) return rc;
   return i4_launch(false, down, up.out_bf16, rows, stream);
-}
-
-int launch_wgemm_tc(int mode, const WgArgs &args, int max_tiles, cudaStream_t stream) {
-  const bool swiglu = mode == WG_BF16_SWIGLU;
-  dim3 grid(args.R / (swiglu ? 128 : 256), max_tiles);
-#define BLOK_BF_LAUNCH(SW, NT)                                                                                                 \
-  {                                                                                                                            \
-    const size_t bsmem = (size_t)BfCfg<NT>::kStages * BfCfg<NT>::kStageBytes;                                                  \
-    BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_bf16_kernel<SW, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));    \
-    wgemm_tc_bf16_kernel<SW, NT><<<grid, kTcThreads, bsmem, stream>>>(args);                                                   \
-  }
-  if (args.identity_tiles) {
-    grid.y = (args.n_rows + 255) / 256;
-    if (swiglu) BLOK_BF_LAUNCH(true, 256) else BLOK_BF_LAUNCH(false, 256)
-  } else {
-    if (swiglu) BLOK_BF_LAUNCH(true, 64) else BLOK_BF_LAUNCH(false, 64)
-  }
-#undef BLOK_BF_LAUNCH
-  return launch_status("wgemm_tc_bf16_kernel");
 }
 
 // Non-zero once any tcgen05 GEMM CTA gave up on a barrier; cleared by the read.

@@ -1,4 +1,5 @@
-"""The grouped INT4 product on tcgen05 (csrc/wgemm_tc.cu) at the edges of its tiles, and its dequantisation on the CPU."""
+"""The batched layer's products on tcgen05 at the edges of their tiles (csrc/wgemm_tc.cu, csrc/gemm_tma.cu), and the INT4
+dequantisation on the CPU."""
 import numpy as np
 import pytest
 import torch
@@ -65,4 +66,27 @@ def test_grouped_experts_at_tile_edges(cuda, monkeypatch, hidden, inter, counts,
     assert torch.equal(out["tc"], layer.experts_grouped(x, e, rows).float())
     # without a row index the rows are taken as they come
     assert torch.equal(out["tc"], layer.experts_grouped(x[rows.long()].contiguous(), e).float())
+    layer.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,hidden,shared", [(65, 1024, 512), (128, 2048, 1024), (129, 7168, 2048), (1153, 1024, 1024)])
+def test_dense_products_of_a_batch(cuda, monkeypatch, T, hidden, shared):
+    """The router and the shared expert over more than 64 tokens (TMA-fed GEMM, K split where its tiles are few) against the
+    mma.sync kernel: the same operands and rounding points, fp32 sums in another order (as above)."""
+    from blok_b200 import lib, synth
+    w = synth.moe_layer_weights(cuda, seed=9, hidden=hidden, inter=512, experts=128, shared_inter=shared)
+    x = synth.activations(T, hidden, cuda, 10)
+    layer = lib.MoeLayer(w, max_tokens=T)
+    out = {}
+    for impl in ("mma", ""):
+        monkeypatch.setenv("BLOK_WGEMM_IMPL", impl)
+        y, ids, wts = layer.batched(x, return_routing=True)
+        out[impl] = y.float(), layer.shared(x).float(), ids.view(torch.int16).clone(), wts.clone()
+        layer.check()
+    (y0, s0, i0, w0), (y1, s1, i1, w1) = out["mma"], out[""]
+    assert float(((s1 - s0).abs() / s0.abs().amax(dim=1, keepdim=True)).max()) <= 2.0 ** -7
+    same = (i0 == i1).all(dim=1)  # two scores closer than the sums' noise may change places
+    assert float(same.float().mean()) > 0.98 and torch.allclose(w0[same], w1[same], rtol=1e-4)
+    assert float(((y1 - y0).abs() / y0.abs().amax(dim=1, keepdim=True))[same].max()) <= 2.0 ** -6
     layer.close()
