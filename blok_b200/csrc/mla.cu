@@ -169,8 +169,6 @@ struct blok_mla_layer {
   int *seq = nullptr;          // [B]
   unsigned *err = nullptr;     // [1] 1 + b when entry b of a call had a position outside its sequence's rows
   int *chunk_pos = nullptr;    // [B] positions of a prefill chunk's tokens
-  int *tiles = nullptr;        // tile table of the weight-streaming GEMM (projections of 16 or more entries)
-  int n_tiles = 0;
   void *sk_ws = nullptr;       // split-K partial sums and tickets of the projections (zeroed at create)
   size_t sk_bytes = 0;
   float *wg_ws = nullptr;      // K-split partial sums of the projections over 9..64 entries (wgemm_stream.cu)
@@ -241,8 +239,6 @@ extern "C" int blok_mla_layer_create(const blok_mla_weights *w, int max_batch, i
   size_t o_seq = take((size_t)max_batch * 4);
   size_t o_cpos = take((size_t)max_batch * 4);
   size_t o_err = take(4);
-  L->n_tiles = (max_batch + kWgTileTokens - 1) / kWgTileTokens;
-  size_t o_tiles = take((size_t)(3 * L->n_tiles + 1) * sizeof(int));
   size_t o_po = take((size_t)(L->max_splits + max_batch) * w->heads * w->kv_rank * 4);
   size_t o_pml = take((size_t)(L->max_splits + max_batch) * w->heads * 2 * 4);
   L->sk_bytes = bf16_gemv_splitk_workspace_bytes(std::max(std::max(w->q_rank, lat_w), std::max(w->heads * qk_head, w->hidden)));
@@ -277,7 +273,6 @@ extern "C" int blok_mla_layer_create(const blok_mla_weights *w, int max_batch, i
   L->seq = reinterpret_cast<int *>(b + o_seq);
   L->chunk_pos = reinterpret_cast<int *>(b + o_cpos);
   L->err = reinterpret_cast<unsigned *>(b + o_err);
-  L->tiles = reinterpret_cast<int *>(b + o_tiles);
   L->part_o = reinterpret_cast<float *>(b + o_po);
   L->part_ml = reinterpret_cast<float *>(b + o_pml);
   L->sk_ws = b + o_sk;
@@ -434,11 +429,10 @@ static int project(blok_mla_layer *L, const uint16_t *w, const uint16_t *x, uint
     return launch_wgemm_rows(WG_BF16_PLAIN, w, nullptr, x, y, nullptr, rows, cols, B, L->wg_ws, L->wg_bytes, stream);
   if (tiles_ready && rows % 128 == 0 && cols % 512 == 0) {
     const int tiles = (B + kWgTileTokens - 1) / kWgTileTokens;
-    int *tab = L->tiles;
     WgArgs r;
     r.w_a = w; r.w_b = nullptr; r.s_a = r.s_b = nullptr; r.expert_stride_rows = 0; r.x = x; r.x_index = nullptr;
     r.K = cols; r.R = rows; r.out_bf16 = y; r.out_f32 = nullptr;
-    r.tile_expert = tab; r.tile_start = tab + L->n_tiles; r.tile_count = tab + 2 * L->n_tiles; r.num_tiles = tab + 3 * L->n_tiles;
+    r.tile_expert = r.tile_start = r.tile_count = r.num_tiles = nullptr;
     r.out_index = nullptr; r.n_rows = B; r.identity_tiles = 1;
     return launch_wgemm(WG_BF16_PLAIN, r, tiles, stream);
   }
@@ -460,10 +454,8 @@ static int decode_body(blok_mla_layer *L, const uint16_t *n, const CacheRef &c, 
   const size_t q_row = (size_t)w.heads * qk_head, qf_row = (size_t)w.heads * lat_w, ol_row = (size_t)w.heads * w.kv_rank,
                av_row = (size_t)w.heads * w.v_head;
   int rc;
-  const bool gemm = B > kWgStreamTokens;  // the GEMM form of the projections: needs the identity tile table
+  const bool gemm = B > kWgStreamTokens;  // the GEMM form of the projections
   const bool stream_rows = B > 8 && !gemm;  // 9..64 entries: one pass of the weight-streaming kernel per matrix
-  if (gemm && (rc = launch_identity_tiles(B, L->tiles, L->tiles + L->n_tiles, L->tiles + 2 * L->n_tiles, L->tiles + 3 * L->n_tiles, stream)))
-    return rc;
   // q_a -> RMSNorm -> q_b   (:813-815); kv_a (:816) reads the same activations as q_a and shares its launch where the
   // mat-vec kernel serves both (up to 8 entries per launch)
   if (!gemm && !stream_rows) {

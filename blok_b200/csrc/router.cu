@@ -15,24 +15,28 @@ constexpr int kTopkWarps = 4;
 // reference's rule exactly: k rounds of argmax over sel = sigmoid(logit) + bias
 // with strict '>' scanning ascending indices, i.e. the lowest index wins a tie,
 // and the outputs are in descending sel order.
-__global__ void router_topk_kernel(const float *__restrict__ logits, const float *__restrict__ bias, int T,
+template <int N>
+__global__ void __launch_bounds__(kTopkWarps * 32) router_topk_kernel(const float *__restrict__ logits, const float *__restrict__ bias, int T,
                                    int experts, int topk, float routed_scale, uint16_t *__restrict__ ids,
                                    float *__restrict__ wts, int *__restrict__ local_ids, int expert_base) {
   extern __shared__ float sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tok = blockIdx.x * kTopkWarps + warp;
   if (tok >= T) return;
-  float *score = sm + (size_t)warp * 2 * experts;
-  float *sel = score + experts;
-  for (int i = lane; i < experts; i += 32) {
-    float s = 1.0f / (1.0f + expf(-logits[(size_t)tok * experts + i]));
-    score[i] = s;
-    sel[i] = s + bias[i];
+  float *score = sm + (size_t)warp * experts;
+  float sel[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const int i = 32 * j + lane;
+    const bool live = i < experts;
+    const float s = 1.0f / (1.0f + expf(-(live ? logits[(size_t)tok * experts + i] : 0.f)));
+    if (live) score[i] = s;
+    sel[j] = live ? s + bias[i] : -INFINITY;
   }
   __syncwarp();
   int my_id;
   float my_w;
-  warp_topk(score, sel, experts, topk, routed_scale, lane, my_id, my_w);
+  warp_topk(score, sel, topk, routed_scale, lane, my_id, my_w);
   if (lane < topk) {
     if (ids) ids[(size_t)tok * topk + lane] = (uint16_t)my_id;
     if (local_ids) local_ids[(size_t)tok * topk + lane] = my_id - expert_base;
@@ -42,11 +46,14 @@ __global__ void router_topk_kernel(const float *__restrict__ logits, const float
 
 int launch_router_topk(const float *logits, const float *bias, int T, int experts, int topk, float routed_scale,
                        uint16_t *ids, float *wts, int *local_ids, int expert_base, cudaStream_t stream) {
-  size_t smem = (size_t)kTopkWarps * 2 * experts * sizeof(float);
-  router_topk_kernel<<<(T + kTopkWarps - 1) / kTopkWarps, kTopkWarps * 32, smem, stream>>>(logits, bias, T, experts,
-                                                                                            topk, routed_scale, ids,
-                                                                                            wts, local_ids,
-                                                                                            expert_base);
+  const size_t smem = (size_t)kTopkWarps * experts * sizeof(float);
+  const int grid = (T + kTopkWarps - 1) / kTopkWarps;
+#define BLOK_TOPK(N) \
+  router_topk_kernel<N><<<grid, kTopkWarps * 32, smem, stream>>>(logits, bias, T, experts, topk, routed_scale, ids, wts, local_ids, expert_base)
+  if (experts <= 128) BLOK_TOPK(4);
+  else if (experts <= 384) BLOK_TOPK(12);
+  else BLOK_TOPK(32);
+#undef BLOK_TOPK
   return launch_status("router_topk_kernel");
 }
 
@@ -76,14 +83,12 @@ extern "C" int blok_router(const blok_bf16_t *router_w, const float *bias, const
   if (T > 16 && experts % 128 == 0 && hidden % 512 == 0) {
     // many tokens: one pass of the weight-streaming GEMM over the router matrix instead of T / 8 mat-vec launches
     const int tiles = (T + kWgTileTokens - 1) / kWgTileTokens;
-    int *tab = reinterpret_cast<int *>(static_cast<unsigned char *>(workspace) + router_logits_bytes(T, experts));
-    int rc = launch_identity_tiles(T, tab, tab + tiles, tab + 2 * tiles, tab + 3 * tiles, (cudaStream_t)stream);
-    if (rc) return rc;
     WgArgs r;
     r.w_a = router_w; r.w_b = nullptr; r.s_a = r.s_b = nullptr; r.expert_stride_rows = 0; r.x = x; r.x_index = nullptr;
     r.K = hidden; r.R = experts; r.out_bf16 = nullptr; r.out_f32 = logits;
-    r.tile_expert = tab; r.tile_start = tab + tiles; r.tile_count = tab + 2 * tiles; r.num_tiles = tab + 3 * tiles;
+    r.tile_expert = r.tile_start = r.tile_count = r.num_tiles = nullptr;
     r.out_index = nullptr; r.n_rows = T; r.identity_tiles = 1;
+    int rc;
     if ((rc = launch_wgemm(WG_BF16_PLAIN, r, tiles, (cudaStream_t)stream))) return rc;
     return launch_router_topk(logits, bias, T, experts, topk, routed_scale, ids, wts, nullptr, 0, (cudaStream_t)stream);
   }

@@ -55,10 +55,12 @@ __global__ void __launch_bounds__(kWgThreads) wgemm_kernel(const WgArgs a) {
   constexpr bool kSwiglu = MODE == WG_BF16_SWIGLU || MODE == WG_I4_SWIGLU;
   extern __shared__ __align__(16) unsigned char smem[];
   const int tile = blockIdx.y;
-  if (tile >= *a.num_tiles) return;
+  if (!a.identity_tiles && tile >= *a.num_tiles) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int e = a.tile_expert[tile], p0 = a.tile_start[tile], cnt = a.tile_count[tile];
+  const int e = a.identity_tiles ? 0 : a.tile_expert[tile];
+  const int p0 = a.identity_tiles ? tile * kWgTileTokens : a.tile_start[tile];
+  const int cnt = a.identity_tiles ? min(kWgTileTokens, a.n_rows - p0) : a.tile_count[tile];
   const int ntiles = (cnt + 7) >> 3;
 
   // the lane's two weight rows

@@ -52,9 +52,6 @@ int wgemm_splitk_factor(int mode, int K, int R, int tiles);
 size_t wgemm_splitk_bytes(int mode, int K, int R, int max_rows);
 int wgemm_tma_split(int mode, int K, int R, int rows);  // the same for the TMA-fed GEMM
 
-// Fills the tile arrays with consecutive 64-row tiles of T rows (one group, expert 0): a dense layer.
-int launch_identity_tiles(int T, int *tile_expert, int *tile_start, int *tile_count, int *num_tiles, cudaStream_t stream);
-
 // The INT4 modes over few assignments: streams the weights like the batch-1 decode kernel (BLOK_WGEMM_SMALL=0 in the
 // environment: through the GEMM kernels as well).
 bool wgemv_small_supports(int mode, const WgArgs &args, int max_tiles);

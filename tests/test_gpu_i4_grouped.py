@@ -90,3 +90,72 @@ def test_dense_products_of_a_batch(cuda, monkeypatch, T, hidden, shared):
     assert float(same.float().mean()) > 0.98 and torch.allclose(w0[same], w1[same], rtol=1e-4)
     assert float(((y1 - y0).abs() / y0.abs().amax(dim=1, keepdim=True))[same].max()) <= 2.0 ** -6
     layer.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,experts,topk", [(1, 32, 8), (5, 128, 8), (33, 384, 8), (9, 385, 6), (4, 1024, 16)])
+def test_router_ties_and_special_scores(cuda, T, experts, topk):
+    """Selection by the reference's rule (strict '>' over ascending indices): equal scores by index, +0 and -0 alike, -inf and
+    NaN never, +inf first.  Scores are set through the bias; a zero router matrix makes every sigmoid 0.5."""
+    from blok_b200 import lib
+    g = torch.Generator().manual_seed(experts)
+    bias = torch.randint(-3, 4, (experts,), generator=g).float() * 0.25 - 0.5  # sel = 0.5 + bias: many ties, zeros among them
+    bias[3], bias[7], bias[11] = float("nan"), -float("inf"), float("inf")
+    bias[13] = -0.5
+    x = torch.randn(T, 256, generator=g).to(cuda, torch.bfloat16)
+    ids, wts = lib.router(torch.zeros(experts, 256, dtype=torch.bfloat16, device=cuda), bias.to(cuda), x, topk=topk)
+    sel = (bias + 0.5).numpy()
+    want = []
+    for _ in range(topk):
+        best, at = -np.inf, 0
+        for i, v in enumerate(sel):
+            if v > best:
+                best, at = v, i
+        want.append(at)
+        sel[at] = -np.inf
+    assert all(r == want for r in util.ids_np(ids).reshape(T, topk).tolist())
+    assert torch.allclose(wts.float(), torch.full_like(wts.float(), 2.827 / topk), rtol=1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [1023, 1024, 1025, 4096])
+def test_order_of_assignments(cuda, monkeypatch, N):
+    """Up to 1,024 assignments are sorted by the plan kernel, more by a kernel of their own: each row's result does not depend on
+    which, nor on the rows around it."""
+    from blok_b200 import lib, synth
+    monkeypatch.setenv("BLOK_WGEMM_IMPL", "tc")
+    w = synth.moe_layer_weights(cuda, seed=3, hidden=512, inter=512, experts=128, shared_inter=0)
+    layer = lib.MoeLayer(w, max_tokens=512)
+    g = torch.Generator(device=cuda)
+    g.manual_seed(N)
+    x = synth.activations(N, 512, cuda, 4)
+    e = torch.randint(0, 128, (N,), generator=g, device=cuda).to(torch.int32)
+    y = layer.experts_grouped(x, e)
+    for lo in (0, N // 2):
+        part = slice(lo, lo + 300)
+        assert torch.equal(y[part], layer.experts_grouped(x[part].contiguous(), e[part].contiguous()))
+    layer.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hidden,topk,offset", [(512, 8, 0), (514, 8, 0), (512, 3, 2), (1032, 12, 0)])
+def test_combine_by_16_and_by_4_bytes(cuda, hidden, topk, offset):
+    """bf16(bf16(sum_k w y) + shared) with the sum in slot order, whatever the rows' length and alignment."""
+    from blok_b200 import lib
+    g = torch.Generator(device=cuda)
+    g.manual_seed(hidden)
+    T = 5
+
+    def rand(n):
+        return torch.randn(n + offset, generator=g, device=cuda).bfloat16()[offset:]
+
+    y, s = rand(T * topk * hidden).view(T * topk, hidden), rand(T * hidden).view(T, hidden)
+    wts = torch.rand(T, topk, generator=g, device=cuda)
+    got = lib.moe_combine(y, wts, s)
+    acc = torch.zeros(T, hidden, device=cuda, dtype=torch.float64)
+    for k in range(topk):
+        acc = (acc + y.view(T, topk, hidden)[:, k].double() * wts[:, k:k + 1].double()).float().double()
+    want = (acc.float().bfloat16().float() + s.float()).bfloat16()
+    # one rounding per fused multiply-add; where the emulation's double rounding of the product differs, by one place of bf16
+    assert float((got.float() - want.float()).abs().max() / want.float().abs().max()) <= 2.0 ** -8
+    assert float((got == want).float().mean()) > 0.99
