@@ -27,6 +27,7 @@ __global__ void __launch_bounds__(kBfMaxWarps * 32)
   __shared__ float partial[kBfMaxWarps][16][8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3;
+  pdl_trigger();
   stage_x_bf16(x, smem, cols, T, tid, blockDim.x);
   __syncthreads();
   const size_t wrow = cols / 8;  // uint4 per row
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(128) bf16_gemv16_splitk_kernel(const uint16_t 
   const int ksteps = cols / 32;
   const int kbeg = blockIdx.y * ksteps_per_split;
   const int kn = min(ksteps_per_split, ksteps - kbeg);  // k-steps of this CTA
+  pdl_trigger();
   // stage x[:, 32 kbeg .. 32 (kbeg + kn)) with the row skew of stage_x_bf16
   const int per_row = kn * 4;  // uint4 per token row
   const size_t row_bytes = bf16_x_row_bytes(kn * 32);
@@ -200,6 +202,8 @@ template <bool ADD>
 __global__ void __launch_bounds__(256) rmsnorm_kernel(uint16_t *__restrict__ x, const uint16_t *__restrict__ tadd,
                                                       const uint16_t *__restrict__ w, uint16_t *__restrict__ y, int n, float eps) {
   __shared__ float red[32];
+  pdl_trigger();
+  pdl_wait();
   uint16_t *xr = x + (size_t)blockIdx.x * n;
   const uint16_t *tr = ADD ? tadd + (size_t)blockIdx.x * n : nullptr;
   uint16_t *yr = y + (size_t)blockIdx.x * n;
@@ -379,6 +383,7 @@ __global__ void __launch_bounds__(128)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int head = blockIdx.y;
+  pdl_trigger();
   // blockIdx.z: the group of 8 tokens (the later groups find the head's matrix in L2)
   const int T = min(8, T_all - 8 * (int)blockIdx.z);
   x += (size_t)blockIdx.z * 8 * x_tok_stride;
@@ -491,8 +496,7 @@ extern "C" int blok_rmsnorm(const blok_bf16_t *x, const blok_bf16_t *w, blok_bf1
   BLOK_REQUIRE(x && w && y, BLOK_ERR_ARG, "blok_rmsnorm: null pointer");
   BLOK_REQUIRE(T >= 0 && n > 0, BLOK_ERR_SHAPE, "blok_rmsnorm: bad shape T=%d n=%d", T, n);
   if (T == 0) return BLOK_OK;
-  rmsnorm_kernel<false><<<T, 256, 0, (cudaStream_t)stream>>>(const_cast<uint16_t *>(x), nullptr, w, y, n, eps);
-  return launch_status("rmsnorm_kernel");
+  return launch_pdl("rmsnorm_kernel", rmsnorm_kernel<false>, T, 256, 0, (cudaStream_t)stream, const_cast<uint16_t *>(x), nullptr, w, y, n, eps);
 }
 
 extern "C" int blok_add_rmsnorm(blok_bf16_t *x, const blok_bf16_t *t, const blok_bf16_t *w, blok_bf16_t *y, int T, int n,
@@ -500,8 +504,7 @@ extern "C" int blok_add_rmsnorm(blok_bf16_t *x, const blok_bf16_t *t, const blok
   BLOK_REQUIRE(x && t && w && y, BLOK_ERR_ARG, "blok_add_rmsnorm: null pointer");
   BLOK_REQUIRE(T >= 0 && n > 0, BLOK_ERR_SHAPE, "blok_add_rmsnorm: bad shape T=%d n=%d", T, n);
   if (T == 0) return BLOK_OK;
-  rmsnorm_kernel<true><<<T, 256, 0, (cudaStream_t)stream>>>(x, t, w, y, n, eps);
-  return launch_status("rmsnorm_kernel<add>");
+  return launch_pdl("rmsnorm_kernel<add>", rmsnorm_kernel<true>, T, 256, 0, (cudaStream_t)stream, x, t, w, y, n, eps);
 }
 
 extern "C" int blok_add_bf16(blok_bf16_t *a, const blok_bf16_t *b, long n, blok_stream_t stream) {

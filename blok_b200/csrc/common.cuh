@@ -39,7 +39,32 @@ inline int launch_status(const char *what) {
 
 int sm_count();
 
+// Launches a kernel that begins with pdl_wait(): its blocks may become resident while the kernel before it runs (programmatic
+// dependent launch), which takes the launch and the start of its blocks off the critical path; captured into graphs like any
+// other launch.  For kernels whose blocks fill an SM (shared memory) or are few and small.  Not for the mat-vec kernels: blocks
+// that come early crowd on the SMs that have room, and the stream of weights is then uneven (o_proj over 8 rows 29 -> 80 us).
+template <typename... P, typename... A>
+inline int launch_pdl(const char *what, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  count_launch();
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return e == cudaSuccess ? BLOK_OK : cuda_fail(e, what);
+}
+
 // ---- device helpers ----------------------------------------------------------
+// The kernel behind this one may become resident as soon as every block of this one has started.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Everything before this launch has finished and is visible; nothing that it reads or writes may be touched earlier.  Without the launch attribute both do nothing.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ float bf16_bits_to_f32(uint32_t h) { return __uint_as_float(h << 16); }
 __device__ __forceinline__ float bf16lo(uint32_t pair) { return __uint_as_float(pair << 16); }
 __device__ __forceinline__ float bf16hi(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }

@@ -53,6 +53,8 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(const uint16_t *__restric
                                                        int table_stride, int page_rows, long ctx_cap, unsigned *__restrict__ err) {
   __shared__ float red[32];
   const int b = blockIdx.y, tid = threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   int pos = ctx_len[b];
   // A position outside the sequence's rows (dense: ctx_cap rows; paged: table_stride pages) must not become a store or
   // a read: the row is not written, the attention is kept inside the rows, and the host learns of it from *err.
@@ -376,9 +378,8 @@ static int attend_and_merge(blok_mla_layer *L, const uint16_t *q, const CacheRef
                                                  splits, scale, L->part_o, L->part_ml, stream)
                        : launch_mla_attend(q, c.base, c.seq_stride, seq_len, B, splits, scale, L->part_o, L->part_ml, stream);
   if (rc) return rc;
-  mla_merge_kernel<<<dim3(L->w.heads, B), 128, (size_t)splits * sizeof(float), stream>>>(L->part_o, L->part_ml, splits, L->w.heads, L->w.kv_rank,
-                                                           o_lat);
-  return launch_status("mla_merge_kernel");
+  return launch_pdl("mla_merge_kernel", mla_merge_kernel, dim3(L->w.heads, B), 128, (size_t)splits * sizeof(float), stream, L->part_o, L->part_ml, splits,
+                    L->w.heads, L->w.kv_rank, o_lat, 0, nullptr, 0);
 }
 
 static int check_paged(const char *who, const void *pool, const int *block_table, int table_stride, int page_rows) {
@@ -470,10 +471,9 @@ static int decode_body(blok_mla_layer *L, const uint16_t *n, const CacheRef &c, 
   if ((rc = blok_rmsnorm(L->qa, w.q_a_ln, L->qa, B, w.q_rank, w.rms_eps, stream_))) return rc;
   if ((rc = project(L, w.q_b, L->qa, L->q, w.heads * qk_head, w.q_rank, B, gemm, stream))) return rc;
   // norm of c_kv, RoPE of k_pe and of q's rope part, cache append   (:816-824)
-  mla_prep_kernel<<<dim3(1 + (w.heads * (w.qk_rope / 2) + 255) / 256, B), 256, 0, stream>>>(
-      L->kva, w.kv_a_ln, L->q, L->inv_freq, ctx_len, c.base, c.seq_stride, L->q_full, L->seq, w.heads, w.qk_nope, w.qk_rope,
+  rc = launch_pdl("mla_prep_kernel", mla_prep_kernel, dim3(1 + (w.heads * (w.qk_rope / 2) + 255) / 256, B), 256, 0, stream, L->kva, w.kv_a_ln, L->q, L->inv_freq, ctx_len, c.base, c.seq_stride, L->q_full, L->seq, w.heads, w.qk_nope, w.qk_rope,
       w.kv_rank, w.rms_eps, c.block_table, c.slot_of, c.table_stride, c.page_rows, c.ctx_cap, L->err);
-  if ((rc = launch_status("mla_prep_kernel"))) return rc;
+  if (rc) return rc;
   // q_abs = W_UK^T q_nope
   if ((rc = launch_head_gemv(L->wuk_t, (long)w.kv_rank * w.qk_nope, L->q, (long)q_row, qk_head, L->q_full, (long)qf_row, lat_w, w.kv_rank,
                              w.qk_nope, w.heads, B, stream)))

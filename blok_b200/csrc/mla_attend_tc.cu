@@ -174,6 +174,8 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   __shared__ int s_need[2][4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int split = blockIdx.x, splits = gridDim.x, b = blockIdx.y;
+  pdl_trigger();
+  pdl_wait();
   const int seq = FINE ? min(seq_len[b] + 1, table_stride * page_rows) : seq_len[b];
   const int ntiles = (seq + kTaTile - 1) / kTaTile;
   const int per = (ntiles + splits - 1) / splits;
@@ -637,9 +639,7 @@ int launch_mla_attend_tc(const uint16_t *q, const uint16_t *cache, long ctx_stri
   }
   CUtensorMap map;
   if (int rc = cache_tensor_map(cache, total_rows, &map)) return rc;
-  mla_attend_tc_kernel<false, false><<<dim3(splits, B), kTaThreads, kTaSmemBytes, stream>>>(map, q, cache, ctx_stride, seq_len, scale, part_o,
-                                                                                     part_ml, nullptr, nullptr, 0, 0, trace_buffer(), kTaHeads);
-  return launch_status("mla_attend_tc_kernel");
+  return launch_pdl("mla_attend_tc_kernel", mla_attend_tc_kernel<false, false>, dim3(splits, B), kTaThreads, kTaSmemBytes, stream, map, q, cache, ctx_stride, seq_len, scale, part_o, part_ml, nullptr, nullptr, 0, 0, trace_buffer(), kTaHeads);
 }
 
 // The same over a paged pool of pool_rows rows: page_rows must be a positive multiple of the 64-token tile.
@@ -654,9 +654,7 @@ static int launch_paged(const uint16_t *q, const uint16_t *pool, long pool_rows,
   }
   CUtensorMap map;
   if (int rc = cache_tensor_map(pool, pool_rows, &map)) return rc;
-  mla_attend_tc_kernel<true, FINE><<<dim3(splits, B, (heads + kTaHeads - 1) / kTaHeads), kTaThreads, kTaSmemBytes, stream>>>(
-      map, q, pool, 0, seq_len, scale, part_o, part_ml, block_table, slot_of, table_stride, page_rows, trace_buffer(), heads);
-  return launch_status("mla_attend_tc_kernel(paged)");
+  return launch_pdl("mla_attend_tc_kernel(paged)", mla_attend_tc_kernel<true, FINE>, dim3(splits, B, (heads + kTaHeads - 1) / kTaHeads), kTaThreads, kTaSmemBytes, stream, map, q, pool, 0, seq_len, scale, part_o, part_ml, block_table, slot_of, table_stride, page_rows, trace_buffer(), heads);
 }
 int launch_mla_attend_tc_paged(const uint16_t *q, const uint16_t *pool, long pool_rows, const int *block_table, const int *slot_of,
                                int table_stride, int page_rows, const int *seq_len, int B, int splits, float scale, float *part_o,

@@ -15,6 +15,8 @@ static __global__ void mla_merge_kernel(const float *__restrict__ part_o, const 
                                  const uint16_t *__restrict__ gate = nullptr, int ld_gate = 0) {
   extern __shared__ float s_wt[];  // [splits] weight of every split: exp(m_s - M), 0 for an empty split
   __shared__ float s_red[2][4];
+  pdl_trigger();
+  pdl_wait();
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const float *ml = part_ml + ((size_t)b * splits * heads + h) * 2;  // split s at + s * heads * 2
   float M = -INFINITY;

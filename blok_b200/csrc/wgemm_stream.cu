@@ -52,6 +52,8 @@ __global__ void __launch_bounds__(kStMaxWarps * 32) wgemm_stream_kernel(const Wg
   const uint4 *w_lo = reinterpret_cast<const uint4 *>(a.w_a) + (size_t)(row0 + g) * wrow + (size_t)c_begin * (kStChunk / 8) + t;
   const uint4 *w_hi = SWIGLU ? reinterpret_cast<const uint4 *>(a.w_b) + (size_t)(row0 + g) * wrow + (size_t)c_begin * (kStChunk / 8) + t
                              : w_lo + 8 * wrow;
+  pdl_trigger();
+  pdl_wait();
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
   constexpr uint32_t kBufBytes = 8 * NT * kStPitch;
   const uint32_t ring_lane = sbase + 2 * kBufBytes + (uint32_t)warp * (kStDepth * 1024) + (uint32_t)lane * 16;
@@ -191,7 +193,7 @@ int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t 
 #define BLOK_ST_LAUNCH(NT, SW)                                                                                          \
   {                                                                                                                     \
     BLOK_CUDA(cudaFuncSetAttribute(wgemm_stream_kernel<NT, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    wgemm_stream_kernel<NT, SW><<<grid, warps * 32, smem, stream>>>(args);                                              \
+    if (int rc = launch_pdl("wgemm_stream_kernel", wgemm_stream_kernel<NT, SW>, grid, warps * 32, smem, stream, args)) return rc; \
   }
   if (swiglu) {
     if (nt == 2) BLOK_ST_LAUNCH(2, true) else if (nt == 4) BLOK_ST_LAUNCH(4, true) else BLOK_ST_LAUNCH(8, true)
@@ -200,13 +202,15 @@ int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t 
   }
 #undef BLOK_ST_LAUNCH
   *splits = nz;
-  return launch_status("wgemm_stream_kernel");
+  return BLOK_OK;
 }
 
 // Adds the K-split partial sums in split order and applies the epilogue of the GEMM kernels.  grid = (ceil(R / 256), n_rows).
 template <bool SWIGLU>
 __global__ void wgemm_splitk_reduce_kernel(const WgArgs a, int nz) {
   const int p = blockIdx.y, row = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (row >= a.R) return;
   const int cols = SWIGLU ? 2 * a.R : a.R;
   const float *ps = a.splitk_ws + (size_t)p * cols + row;
@@ -229,9 +233,8 @@ __global__ void wgemm_splitk_reduce_kernel(const WgArgs a, int nz) {
 
 int launch_wgemm_splitk_reduce(int mode, const WgArgs &args, int nz, cudaStream_t stream) {
   const dim3 rg((args.R + 255) / 256, args.n_rows);
-  if (mode == WG_BF16_SWIGLU || mode == WG_I4_SWIGLU) wgemm_splitk_reduce_kernel<true><<<rg, 256, 0, stream>>>(args, nz);
-  else wgemm_splitk_reduce_kernel<false><<<rg, 256, 0, stream>>>(args, nz);
-  return launch_status("wgemm_splitk_reduce_kernel");
+  if (mode == WG_BF16_SWIGLU || mode == WG_I4_SWIGLU) return launch_pdl("wgemm_splitk_reduce_kernel", wgemm_splitk_reduce_kernel<true>, rg, 256, 0, stream, args, nz);
+  return launch_pdl("wgemm_splitk_reduce_kernel", wgemm_splitk_reduce_kernel<false>, rg, 256, 0, stream, args, nz);
 }
 
 // The mma.sync kernel (wgemm.cu) has 128 weight rows per CTA (64 + 64 for SwiGLU) and splits whole 512-column chunks.
