@@ -1,8 +1,7 @@
-// The grouped W4A16 product for groups of a few tokens: a mat-vec-style consumer in place of the dequantising GEMM.
+// The grouped W4A16 product over few assignments: a mat-vec-style consumer in place of the dequantising GEMM.
 //
-// At T = 64 tokens and 384 experts a group holds 1.8 tokens on average, and the tcgen05 kernel (wgemm_tc.cu) still turns
-// every weight into a bf16 operand (about 15 thread-instructions per packed word) for a tile that is nearly empty.  Here
-// the weights stream through a warp-private cp.async ring exactly as in the batch-1 decode kernel and meet the integer
+// With a handful of groups of one or two tokens the tcgen05 kernel (wgemm_tc.cu) has units of 256 rows that fill the SMs
+// unevenly.  Here the weights stream through a warp-private cp.async ring as in the batch-1 decode kernel and meet the integer
 // tensor-core consumer of i4_imma.cuh: a nibble becomes the byte 16 (q + 8) with one mask (unpacked ONCE per k-block),
 // then every token of the group costs four mma.m16n8k32 and one post-scale.  Same arithmetic contract as
 // matvec_i4_bf16_scale_k (src/kimi_exec.cu:300-323) within the floating-point bar (the error model of i4_imma.cuh);
