@@ -87,7 +87,8 @@ __global__ void __launch_bounds__(kGtThreads)
   tc_fence_after();
   const uint32_t tmem = s_tmem;
   const int all_steps = (a.K + kGtKStep - 1) / kGtKStep;
-  const int first = (int)((long)all_steps * blockIdx.z / gridDim.z), nsteps = (int)((long)all_steps * (blockIdx.z + 1) / gridDim.z) - first;
+  const int parts = (int)gridDim.z, z = (int)blockIdx.z;  // no division where K is not cut
+  const int first = parts == 1 ? 0 : all_steps * z / parts, nsteps = parts == 1 ? all_steps : all_steps * (z + 1) / parts - first;
   bool failed = false;
 
   if (warp == 4) {
