@@ -33,8 +33,9 @@ __device__ __forceinline__ uint32_t tc_bf16x2_fma(uint32_t a, uint32_t b, uint32
 // encoding is linear), so w & 0x000f000f and w & 0x00f000f0 are pairs of nibbles as they lie, and
 //   fma(n 2^-129, s 2^100, -s 2^-26) = bf16(q s 2^-29) = 2^-29 bf16(q s)
 // with one rounding, the reference's (:312): a power of two does not change it while s 2^104 is finite and q s 2^-29 normal
-// (2^-97 <= |s| < 2^24).  The epilogue takes the 2^29 back, exactly.  (Adding an exponent to the nibble, subtracting 136 and
-// multiplying took 15 instructions a word instead of 9.)
+// (s = 0 or 2^-97 <= |s| < 2^24).  The epilogue takes the 2^29 back, exactly.  (Adding an exponent to the nibble, subtracting
+// 136 and multiplying took 15 instructions a word instead of 9.)  No checkpoint has other scales, but any bf16 is accepted:
+// i4_outside finds them, and i4_plain_rows takes the place of the unit's epilogue.
 constexpr uint32_t kI4Hi = 0x71807180u, kI4Lo = 0x73807380u, kI4Off = 0xb280b280u;  // 2^100, 2^104, -2^-26
 constexpr float kI4Unscale = 536870912.f;                                           // 2^29
 struct I4Scale {
@@ -68,6 +69,7 @@ __device__ __forceinline__ void i4_dequant(uint32_t w, const I4Scale &s, uint32_
 // weights' barrier 1,301; operands of the MMAs in uniform registers 1,255; pieces of 128 columns instead of 64 and 16
 // unpacking warps instead of 24 1,138 us (5.6 TB/s).  With a hand-over every 64 columns the MMA warps' waits were the limit,
 // whatever the others did.  At 16,384 assignments 2,190 us before, 1,537 now; at 512 1,017 before, 800 now.
+// The test of the scales' range costs the whole layer 0.7 % at 6 tokens (289 us) and 1 to 2.5 % from 64 on.
 constexpr int kI4Unpack = 16, kI4Epi = 4;                       // warps
 constexpr int kI4FirstUnpack = 4 + kI4Epi;
 constexpr int kI4Threads = (kI4FirstUnpack + kI4Unpack) * 32;
@@ -85,7 +87,60 @@ struct I4Args {
   uint16_t *out;
   const int *out_index, *tile_expert, *tile_start, *tile_count, *num_tiles;
   int K, R, stride_rows;
+  const void *w_a, *w_b;  // the operands again, for i4_plain_rows
+  const uint16_t *s_a, *s_b, *x;
 };
+
+// The epilogue of a thread's two sums for one token: gate and up, or two rows of the down projection 128 apart.
+template <bool SWIGLU>
+__device__ __forceinline__ void i4_store(uint16_t *out, float va, float vb) {
+  if (SWIGLU) {
+    const float gv = round_bf16(va), uv = round_bf16(vb);
+    *out = f32_to_bf16_bits(round_bf16(gv / (1.0f + expf(-gv))) * uv);
+  } else {
+    out[0] = f32_to_bf16_bits(va);
+    out[128] = f32_to_bf16_bits(vb);
+  }
+}
+
+// Two scales: |s| 2^24 or more (infinities and NaN too), or below 2^-97 and not zero.  |s| - 1 with the top bit on: zero wraps to
+// the smallest unsigned and the largest signed value.
+__device__ __forceinline__ bool i4_outside(uint32_t s2) {
+  const uint32_t v = (s2 | 0x80008000u) - 0x00010001u;
+  return __vmaxu2(v, 0xcb7ecb7eu) != 0xcb7ecb7eu || __vmins2(v, 0x8eff8effu) != 0x8eff8effu;
+}
+
+// A thread's two rows of a unit that holds scales i4_dequant does not cover, in place of what the MMAs summed: the product q s
+// rounded to bf16 as the reference has it, whatever the scale, in plain loops (a millisecond or two).  row: weight row inside the
+// expert; col: output column.
+template <bool SWIGLU>
+__device__ __noinline__ void i4_plain_rows(const I4Args &a, int tile, int row, int col) {
+  const int p0 = a.tile_start[tile], cnt = a.tile_count[tile], blocks = a.K / 32;
+  const size_t at = ((size_t)a.tile_expert[tile] * a.stride_rows + row) * blocks;
+  const uint4 *w[2] = {reinterpret_cast<const uint4 *>(a.w_a) + at, reinterpret_cast<const uint4 *>(SWIGLU ? a.w_b : a.w_a) + at + (SWIGLU ? 0 : 128 * (size_t)blocks)};
+  const uint16_t *s[2] = {a.s_a + at, (SWIGLU ? a.s_b : a.s_a) + at + (SWIGLU ? 0 : 128 * (size_t)blocks)};
+  for (int tok = 0; tok < cnt; ++tok) {
+    const uint2 *x = reinterpret_cast<const uint2 *>(a.x + (size_t)(p0 + tok) * a.K);
+    float acc[2] = {0.f, 0.f};
+    for (int b = 0; b < blocks; ++b) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t *words = reinterpret_cast<const uint32_t *>(w[h] + b);
+        const float scale = bf16_bits_to_f32(s[h][b]);
+        for (int i = 0; i < 8; ++i) {  // half a word: columns j and j + 4 are neighbours in x
+          const uint2 v = x[8 * b + i];
+          const int q = (int)(words[i >> 1] >> (8 * (i & 1)));
+          acc[h] = fmaf(round_bf16((float)((q & 15) - 8) * scale), bf16lo(v.x), acc[h]);
+          acc[h] = fmaf(round_bf16((float)((q >> 16 & 15) - 8) * scale), bf16hi(v.x), acc[h]);
+          acc[h] = fmaf(round_bf16((float)((q >> 4 & 15) - 8) * scale), bf16lo(v.y), acc[h]);
+          acc[h] = fmaf(round_bf16((float)((q >> 20 & 15) - 8) * scale), bf16hi(v.y), acc[h]);
+        }
+      }
+    }
+    const size_t p = a.out_index ? (size_t)a.out_index[p0 + tok] : (size_t)(p0 + tok);
+    i4_store<SWIGLU>(a.out + p * a.R + col, acc[0], acc[1]);
+  }
+}
 
 __device__ __forceinline__ uint4 i4_lds128(uint32_t addr) {
   uint4 v;
@@ -176,10 +231,11 @@ __device__ __forceinline__ bool i4_mma(const I4Mma &m, const I4Args &a, int unit
 template <bool SWIGLU>
 __global__ void __launch_bounds__(kI4Threads, 1)
     wgemm_tc_kernel(const __grid_constant__ CUtensorMap mwa, const __grid_constant__ CUtensorMap mwb, const __grid_constant__ CUtensorMap msa,
-                    const __grid_constant__ CUtensorMap msb, const __grid_constant__ CUtensorMap mx, const I4Args a) {
+                    const __grid_constant__ CUtensorMap msb, const __grid_constant__ CUtensorMap mx, const __grid_constant__ I4Args a) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long s_bar[2 * (kI4WStages + kI4XStages + 8 + 2)];
   __shared__ uint32_t s_tmem;
+  __shared__ volatile int s_odd[2];  // per accumulator buffer: 1 + the last unit in it that has a scale i4_dequant does not cover
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr int kRows = SWIGLU ? 128 : 256;
   const int blocks = a.R / kRows, units = *a.num_tiles * blocks;
@@ -195,6 +251,7 @@ __global__ void __launch_bounds__(kI4Threads, 1)
     for (int s = 0; s < 8; ++s) tp_mbar_init(a_full + 8 * s, 4), tp_mbar_init(a_empty + 8 * s, 1);  // [piece of a stage][row block]
     for (int s = 0; s < 2; ++s) tp_mbar_init(d_full + 8 * s, 2), tp_mbar_init(d_empty + 8 * s, kI4Epi);
     tp_mbar_init_fence();
+    s_odd[0] = s_odd[1] = 0;
   }
   if (warp == 0) tp_tmem_alloc((uint32_t)__cvta_generic_to_shared(&s_tmem), kI4TmemCols);
   tc_fence_before();
@@ -209,6 +266,8 @@ __global__ void __launch_bounds__(kI4Threads, 1)
     const uint32_t srow = sbase + (uint32_t)(blk * (128 * 32) + row * 32);
     const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(kI4ACol + blk * 32);
     const int pieces = (int)blockIdx.x < units ? ((units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * kI4Pieces * stages : 0;
+    bool odd = false;
+    int unit = blockIdx.x, left = stages, dslot = 0;
     for (int p = set; p < pieces; p += kI4Unpack / 8) {
       const int st = p / kI4Pieces, c = p % kI4Pieces;  // c: the piece of its stage, and the tensor-memory buffer it goes to
       const int ws = st % kI4WStages, ss = (st >> 1) % kI4SStages;
@@ -244,6 +303,15 @@ __global__ void __launch_bounds__(kI4Threads, 1)
         tmem_st32(ta + (c * kI4Piece + z) * 64, av);
       }
       if (failed) break;
+      // while the stores are on their way; exponents that begin 01 are 2^-63 <= |s| < 2, for the few others the exact test
+      if (((sc[0] ^ 0x20002000u) | (sc[1] ^ 0x20002000u)) & 0x60006000u) odd = odd || i4_outside(sc[0]) || i4_outside(sc[1]);
+      if (--left == 0) {  // the unit's last piece of this set
+        if (odd) s_odd[dslot] = unit + 1;
+        odd = false;
+        left = stages;
+        unit += gridDim.x;
+        dslot ^= 1;
+      }
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -274,16 +342,11 @@ __global__ void __launch_bounds__(kI4Threads, 1)
           if (tok < cnt) {
             const size_t p = a.out_index ? (size_t)a.out_index[p0 + tok] : (size_t)(p0 + tok);
             const float va = __uint_as_float(ra[j]) * kI4Unscale, vb = __uint_as_float(rb[j]) * kI4Unscale;
-            if (SWIGLU) {
-              const float gv = round_bf16(va), uv = round_bf16(vb);
-              a.out[p * a.R + col] = f32_to_bf16_bits(round_bf16(gv / (1.0f + expf(-gv))) * uv);
-            } else {
-              a.out[p * a.R + col] = f32_to_bf16_bits(va);
-              a.out[p * a.R + col + 128] = f32_to_bf16_bits(vb);
-            }
+            i4_store<SWIGLU>(a.out + p * a.R + col, va, vb);
           }
         }
       }
+      if (s_odd[dr.slot] == u + 1) i4_plain_rows<SWIGLU>(a, tile, row0 + row, col);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) tp_arrive(d_empty + 8 * dr.slot);
@@ -401,7 +464,8 @@ static int i4_launch(bool swiglu, const WgArgs &g, const uint16_t *x, long x_row
     if ((rc = tensor_map_2d(g.s_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, kRows, g.K / 16, g.K / 16, 128, 32, CU_TENSOR_MAP_SWIZZLE_32B, &sb))) return rc;
   }
   if ((rc = tensor_map_2d(x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x_rows, g.K, (long)g.K * 2, 16, 64, CU_TENSOR_MAP_SWIZZLE_128B, &mx))) return rc;
-  const I4Args a = {g.out_bf16, g.out_index, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.K, g.R, (int)g.expert_stride_rows};
+  const I4Args a = {g.out_bf16, g.out_index, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.K, g.R, (int)g.expert_stride_rows,
+                    g.w_a, g.w_b, g.s_a, g.s_b, x};
   if (swiglu) {
     BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kI4Smem));
     wgemm_tc_kernel<true><<<sm_count(), kI4Threads, kI4Smem, stream>>>(wa, wb, sa, sb, mx, a);

@@ -29,6 +29,19 @@ def test_dequantisation_by_one_rounding():
             assert np.array_equal(got, want)
 
 
+def test_range_of_scales_by_their_bits():
+    """The kernel's two integer tests over every bf16 bit pattern: the exact one says whether s = 0 or 2^-97 <= |s| < 2^24, and what
+    the quick one lets by (exponent bits 01......) is inside."""
+    bits = np.arange(1 << 16, dtype=np.uint32)
+    with np.errstate(invalid="ignore"):
+        s = np.abs((bits << 16).view(np.float32).astype(np.float64))
+    inside = (s == 0) | ((s >= 2.0 ** -97) & (s < 2.0 ** 24))
+    v = ((bits | 0x8000) - 1).astype(np.uint16)
+    outside = (v > np.uint16(0xcb7e)) | (v.view(np.int16) < np.array(0x8eff, dtype=np.uint16).view(np.int16))
+    assert np.array_equal(~outside, inside)
+    assert inside[((bits ^ 0x2000) & 0x6000) == 0].all()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("hidden,inter,counts,scale_octaves", [
     (512, 512, [1, 15, 16, 17, 0, 31, 33, 48], 0),      # two weight stages per product; the token steps of the MMA
@@ -66,6 +79,47 @@ def test_grouped_experts_at_tile_edges(cuda, monkeypatch, hidden, inter, counts,
     assert torch.equal(out["tc"], layer.experts_grouped(x, e, rows).float())
     # without a row index the rows are taken as they come
     assert torch.equal(out["tc"], layer.experts_grouped(x[rows.long()].contiguous(), e).float())
+    layer.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gate,up,down", [
+    (0, 40, -105),      # every up scale above the range of the one-instruction dequantisation, every down scale below it
+    (0, -108, 60),      # and the other way round
+    (-100, 100, 0),
+    (None, None, None),  # single blocks of 32 columns in a few rows: 2^25, 2^-99 and 2^-133 (the smallest there is), and zeros
+])
+def test_grouped_experts_take_any_scale(cuda, monkeypatch, gate, up, down):
+    """Scales outside 2^-97 .. 2^24: the tcgen05 kernel against the mma.sync kernel, which multiplies every nibble by its scale.
+    The same weights, fp32 sums in another order: tolerance as above."""
+    from blok_b200 import lib, synth
+    hidden, inter, N = 1024, 512, 75
+    w = synth.moe_layer_weights(cuda, seed=8, hidden=hidden, inter=inter, experts=128, shared_inter=0)
+    for k, octaves in (("gate_s", gate), ("up_s", up), ("down_s", down)):
+        s = w[k].float() * 8
+        if octaves is None:
+            s[:, 5::64, 3] = 2.0 ** 25
+            s[:, 6::64, 7] = 2.0 ** -99
+            s[:, 7::64, :] = 2.0 ** -133
+            s[:, 8::64, ::2] = 0.0
+        else:
+            s = s * 2.0 ** octaves
+        w[k] = s.bfloat16()
+    layer = lib.MoeLayer(w, max_tokens=16)
+    x = synth.activations(N, hidden, cuda, 6)
+    e = torch.tensor([3] * 66 + [4, 4, 4] + [90] * 6, dtype=torch.int32, device=cuda)
+    out = {}
+    for impl in ("mma", "tc", ""):
+        monkeypatch.setenv("BLOK_WGEMM_IMPL", impl)
+        out[impl] = layer.experts_grouped(x, e).double()  # squares of the largest results overflow fp32
+        layer.check()
+    ref = out["mma"]
+    assert bool(torch.isfinite(ref).all()) and bool((ref.abs().amax(dim=1) > 0).all())
+    for impl in ("tc", ""):
+        assert float(((out[impl] - ref).abs() / ref.abs().amax(dim=1, keepdim=True)).max()) <= 2.0 ** -7
+        # rows of small weights beside rows of large ones
+        rows = ref.abs().amax(dim=0)
+        assert float(((out[impl] - ref).abs().amax(dim=0) / rows.clamp_min(1e-300)).max()) <= 2.0 ** -6
     layer.close()
 
 
