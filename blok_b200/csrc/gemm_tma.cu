@@ -8,8 +8,8 @@
 // the copies and masked at the store, so any T, R and K work.  The grouped form takes its tiles from a device table whose
 // length the host does not know: the grid covers the worst case and surplus CTAs leave at once.
 //
-// Every mbarrier wait is bounded.  A CTA that gives up records it, waits for its own copies in flight, releases its
-// tensor memory and returns.
+// Every mbarrier wait is bounded.  A CTA that gives up records it, stores NaN (0 through max(v, 0)^2), waits for its own copies
+// in flight, releases its tensor memory and returns.
 #include <mutex>
 
 #include "gemm_tma.h"
@@ -34,6 +34,7 @@ struct GtArgs {
   void *out;
   const int *tile_expert, *tile_start, *tile_count, *num_tiles;
   int T, R, K, ldo, act_cols, up_row;
+  unsigned *err;
 };
 
 template <int ACT>
@@ -136,69 +137,75 @@ __global__ void __launch_bounds__(kGtThreads)
   } else {
     failed = !tp_wait(done, 0);
     failed = __any_sync(0xffffffffu, failed);
-    if (!failed) {
-      tc_fence_after();
-      const int r = 32 * warp + lane;
-      const size_t o = ((size_t)blockIdx.z * a.T + row0 + r) * a.ldo;
-      const int n0 = blockIdx.x * kCols;
-      if constexpr (kGated) {
+    tc_fence_after();
+    const int r = 32 * warp + lane;
+    const size_t o = ((size_t)blockIdx.z * a.T + row0 + r) * a.ldo;
+    const int n0 = blockIdx.x * kCols;
+    if constexpr (kGated) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < kCols; c0 += 16) {
-          if (n0 + c0 >= a.R) break;
-          uint32_t gate[16], up[16];
-          const uint32_t at = tmem + ((uint32_t)(32 * warp) << 16) + c0;
-          tmem_ld16(at, gate);
-          tmem_ld16(at + kCols, up);
-          tmem_wait_ld();
-          if (r < count) {
+      for (int c0 = 0; c0 < kCols; c0 += 16) {
+        if (n0 + c0 >= a.R) break;
+        uint32_t gate[16], up[16];
+        const uint32_t at = tmem + ((uint32_t)(32 * warp) << 16) + c0;
+        tmem_ld16(at, gate);
+        tmem_ld16(at + kCols, up);
+        tmem_wait_ld();
+        if (failed) {  // nothing that looks like a result
 #pragma unroll
-            for (int j = 0; j < 16; j += 4) {
-              const int col = n0 + c0 + j;
-              if (col < a.R) {
-                if (F32) {  // the parts of a K split
-                  *reinterpret_cast<uint4 *>(static_cast<float *>(a.out) + o + col) = make_uint4(gate[j], gate[j + 1], gate[j + 2], gate[j + 3]);
-                  *reinterpret_cast<uint4 *>(static_cast<float *>(a.out) + o + a.R + col) = make_uint4(up[j], up[j + 1], up[j + 2], up[j + 3]);
-                  continue;
-                }
-                float f[4];
+          for (int j = 0; j < 16; ++j) gate[j] = up[j] = 0x7fc00000u;
+        }
+        if (r < count) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  if (ACT == GEMM_ACT_SWIGLU_REF) {
-                    const float g = round_bf16(__uint_as_float(gate[j + i]));
-                    f[i] = round_bf16(g / (1.0f + expf(-g))) * round_bf16(__uint_as_float(up[j + i]));
-                  } else {
-                    f[i] = gt_act<GEMM_ACT_SILU>(__uint_as_float(gate[j + i])) * __uint_as_float(up[j + i]);
-                  }
-                }
-                *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(a.out) + o + col) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
+          for (int j = 0; j < 16; j += 4) {
+            const int col = n0 + c0 + j;
+            if (col < a.R) {
+              if (F32) {  // the parts of a K split
+                *reinterpret_cast<uint4 *>(static_cast<float *>(a.out) + o + col) = make_uint4(gate[j], gate[j + 1], gate[j + 2], gate[j + 3]);
+                *reinterpret_cast<uint4 *>(static_cast<float *>(a.out) + o + a.R + col) = make_uint4(up[j], up[j + 1], up[j + 2], up[j + 3]);
+                continue;
               }
+              float f[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                if (ACT == GEMM_ACT_SWIGLU_REF) {
+                  const float g = round_bf16(__uint_as_float(gate[j + i]));
+                  f[i] = round_bf16(g / (1.0f + expf(-g))) * round_bf16(__uint_as_float(up[j + i]));
+                } else {
+                  f[i] = gt_act<GEMM_ACT_SILU>(__uint_as_float(gate[j + i])) * __uint_as_float(up[j + i]);
+                }
+              }
+              *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(a.out) + o + col) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
             }
           }
         }
-      } else {
+      }
+    } else {
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-          if (n0 + c0 >= a.R) break;
-          uint32_t v[32];
-          tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + c0, v);
-          tmem_wait_ld();
-          if (r < count) {
+      for (int c0 = 0; c0 < BN; c0 += 32) {
+        if (n0 + c0 >= a.R) break;
+        uint32_t v[32];
+        tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + c0, v);
+        tmem_wait_ld();
+        if (failed) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const int col = n0 + c0 + j;
-              if (col < a.R) {  // R is a multiple of 4
-                float f0 = __uint_as_float(v[j]), f1 = __uint_as_float(v[j + 1]), f2 = __uint_as_float(v[j + 2]), f3 = __uint_as_float(v[j + 3]);
-                if (ACT != GEMM_ACT_SILU || col < a.act_cols) f0 = gt_act<ACT>(f0), f1 = gt_act<ACT>(f1), f2 = gt_act<ACT>(f2), f3 = gt_act<ACT>(f3);
-                if (F32) *reinterpret_cast<float4 *>(static_cast<float *>(a.out) + o + col) = make_float4(f0, f1, f2, f3);
-                else *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(a.out) + o + col) = make_uint2(pack_bf16x2(f0, f1), pack_bf16x2(f2, f3));
-              }
+          for (int j = 0; j < 32; ++j) v[j] = 0x7fc00000u;
+        }
+        if (r < count) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            const int col = n0 + c0 + j;
+            if (col < a.R) {  // R is a multiple of 4
+              float f0 = __uint_as_float(v[j]), f1 = __uint_as_float(v[j + 1]), f2 = __uint_as_float(v[j + 2]), f3 = __uint_as_float(v[j + 3]);
+              if (ACT != GEMM_ACT_SILU || col < a.act_cols) f0 = gt_act<ACT>(f0), f1 = gt_act<ACT>(f1), f2 = gt_act<ACT>(f2), f3 = gt_act<ACT>(f3);
+              if (F32) *reinterpret_cast<float4 *>(static_cast<float *>(a.out) + o + col) = make_float4(f0, f1, f2, f3);
+              else *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(a.out) + o + col) = make_uint2(pack_bf16x2(f0, f1), pack_bf16x2(f2, f3));
             }
           }
         }
       }
     }
   }
-  if (failed) atomicExch(&g_gemm_tma_error, 1u);
+  if (failed) atomicExch(a.err ? a.err : &g_gemm_tma_error, 1u);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tp_tmem_free(tmem, BN);
@@ -237,7 +244,7 @@ int gemm_operand_map(const void *base, long rows, int cols, long pitch, int box,
 
 template <int BN, int ACT, bool F32>
 static int gt_launch(const GemmTma &g, dim3 grid, cudaStream_t stream) {
-  const GtArgs a = {g.out, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.T, g.R, g.K, g.ldo, g.act_cols, g.up_row};
+  const GtArgs a = {g.out, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.T, g.R, g.K, g.ldo, g.act_cols, g.up_row, g.err};
   BLOK_CUDA(cudaFuncSetAttribute(gemm_tma_kernel<BN, ACT, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, GtCfg<BN>::kSmem));
   gemm_tma_kernel<BN, ACT, F32><<<grid, kGtThreads, GtCfg<BN>::kSmem, stream>>>(
       *g.x, BN == 128 || ACT == GEMM_ACT_SWIGLU || ACT == GEMM_ACT_SWIGLU_REF ? *g.w128 : *g.w256, g.up128 ? *g.up128 : *g.w128, a);

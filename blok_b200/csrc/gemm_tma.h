@@ -37,6 +37,8 @@ struct GemmTma {
   // > 1: K is cut into so many parts (grid.z), `out` is fp32 [splits][T][ldo] and holds the parts' sums (of both products, gate
   // columns then up columns, ldo = 2 R, for a gated product); no activation
   int splits = 1;
+  // Set to 1 by a CTA whose wait gave up (its outputs are NaN); NULL: a word of the process, gemm_tma_take_error.
+  unsigned *err = nullptr;
   // Grouped form: tile i covers rows [tile_start[i], + tile_count[i]) of x (at most kGtTileRows) and weight rows
   // [tile_expert[i] * R, + R); at most max_tiles tiles, *num_tiles of them valid.  NULL: consecutive tiles of one matrix.
   const int *tile_expert = nullptr, *tile_start = nullptr, *tile_count = nullptr, *num_tiles = nullptr;

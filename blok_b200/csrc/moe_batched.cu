@@ -186,7 +186,7 @@ int batched_alloc(blok_moe_layer *L) {
   L->b_splitk_bytes = std::max(wgemm_splitk_bytes(WG_BF16_PLAIN, w.hidden, w.experts, (int)T),
                                std::max(wgemm_splitk_bytes(WG_BF16_SWIGLU, w.hidden, std::max(w.shared_inter, 8), (int)T),
                                         wgemm_splitk_bytes(WG_BF16_PLAIN, std::max(w.shared_inter, 8), w.hidden, (int)T)));
-  size_t o_sk = take(std::max(L->b_splitk_bytes, (size_t)16));
+  size_t o_sk = take(std::max(L->b_splitk_bytes, (size_t)16)), o_err = take(4);
   BLOK_CUDA(cudaMalloc(&L->bws, off));
   unsigned char *b = static_cast<unsigned char *>(L->bws);
   L->b_counts = (int *)(b + o_counts); L->b_offsets = (int *)(b + o_offsets);
@@ -196,6 +196,8 @@ int batched_alloc(blok_moe_layer *L) {
   L->b_mid = (uint16_t *)(b + o_mid); L->b_y = (uint16_t *)(b + o_y);
   L->b_smid = (uint16_t *)(b + o_smid); L->b_sout = (uint16_t *)(b + o_sout);
   L->b_splitk = (float *)(b + o_sk);
+  L->b_err = (unsigned *)(b + o_err);
+  BLOK_CUDA(cudaMemset(L->b_err, 0, sizeof(unsigned)));
   return BLOK_OK;
 }
 
@@ -218,7 +220,7 @@ int grouped_experts(blok_moe_layer *L, const uint16_t *x, const int *x_index, in
   g.w_a = w.gate_w; g.w_b = w.up_w; g.s_a = w.gate_s; g.s_b = w.up_s; g.expert_stride_rows = w.inter;
   g.x = x; g.x_index = L->b_sorted_row; g.K = w.hidden; g.R = w.inter; g.out_bf16 = L->b_mid; g.out_f32 = nullptr;
   g.tile_expert = L->b_tile_expert; g.tile_start = L->b_tile_start; g.tile_count = L->b_tile_count;
-  g.num_tiles = L->b_num_tiles; g.out_index = nullptr; g.n_rows = N;
+  g.num_tiles = L->b_num_tiles; g.out_index = nullptr; g.n_rows = N; g.err = L->b_err;
   const int max_tiles = std::min(L->b_max_tiles, (N + kWgTileTokens - 1) / kWgTileTokens + nl);
   WgArgs d = g;
   d.w_a = w.down_w; d.w_b = nullptr; d.s_a = w.down_s; d.s_b = nullptr; d.expert_stride_rows = w.hidden;
@@ -265,7 +267,7 @@ extern "C" int blok_moe_batched(blok_moe_layer_t *L, const blok_bf16_t *x, int T
   r.K = w.hidden; r.R = w.experts; r.out_bf16 = nullptr; r.out_f32 = L->logits;
   r.tile_expert = r.tile_start = r.tile_count = r.num_tiles = nullptr;
   r.out_index = nullptr; r.n_rows = T; r.identity_tiles = 1;
-  r.splitk_ws = L->b_splitk; r.splitk_bytes = L->b_splitk_bytes;
+  r.splitk_ws = L->b_splitk; r.splitk_bytes = L->b_splitk_bytes; r.err = L->b_err;
   if ((rc = launch_wgemm(WG_BF16_PLAIN, r, tt, stream))) return rc;
   if ((rc = launch_router_topk(L->logits, w.router_bias, T, w.experts, w.topk, w.routed_scale, L->ids, L->wts, L->local_ids,
                                w.expert_base, stream)))
@@ -303,7 +305,7 @@ extern "C" int blok_moe_shared(blok_moe_layer_t *L, const blok_bf16_t *x, int T,
   s.K = w.hidden; s.R = w.shared_inter; s.out_bf16 = L->b_smid; s.out_f32 = nullptr;
   s.tile_expert = s.tile_start = s.tile_count = s.num_tiles = nullptr;
   s.out_index = nullptr; s.n_rows = T; s.identity_tiles = 1;
-  s.splitk_ws = L->b_splitk; s.splitk_bytes = L->b_splitk_bytes;
+  s.splitk_ws = L->b_splitk; s.splitk_bytes = L->b_splitk_bytes; s.err = L->b_err;
   if ((rc = launch_wgemm(WG_BF16_SWIGLU, s, tt, stream))) return rc;
   WgArgs d = s;
   d.w_a = w.shared_down; d.w_b = nullptr; d.x = L->b_smid; d.K = w.shared_inter; d.R = w.hidden; d.out_bf16 = out;

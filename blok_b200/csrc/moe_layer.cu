@@ -7,7 +7,6 @@
 
 #include "common.cuh"
 #include "moe_layer.h"
-#include "gemm_tma.h"
 #include "wgemm.h"
 
 namespace blok {
@@ -225,15 +224,16 @@ extern "C" int blok_moe_layer_check(blok_moe_layer_t *L, blok_stream_t stream_) 
   BLOK_REQUIRE(L, BLOK_ERR_ARG, "blok_moe_layer_check: null pointer");
   cudaStream_t stream = (cudaStream_t)stream_;
   BLOK_CUDA(cudaStreamSynchronize(stream));
-  unsigned tc_err = 0, gt_err = 0;
-  if (int rc = wgemm_tc_take_error(&tc_err)) return rc;
-  if (int rc = gemm_tma_take_error(&gt_err)) return rc;
-  if (tc_err || gt_err) {
-    set_error("blok_moe_batched: a tensor-core GEMM tile gave up waiting for its MMAs");
-    return BLOK_ERR_TIMEOUT;
+  unsigned err = 0;
+  if (L->b_err) {
+    BLOK_CUDA(cudaMemcpy(&err, L->b_err, sizeof(err), cudaMemcpyDeviceToHost));
+    if (err) {
+      BLOK_CUDA(cudaMemset(L->b_err, 0, sizeof(err)));
+      set_error("blok_moe_batched: a tensor-core GEMM tile gave up waiting for its MMAs");
+      return BLOK_ERR_TIMEOUT;
+    }
   }
   if (!L->f_ctrl) return BLOK_OK;
-  unsigned err = 0;
   BLOK_CUDA(cudaMemcpy(&err, L->f_ctrl + 5, sizeof(err), cudaMemcpyDeviceToHost));
   if (err == 0) return BLOK_OK;
   // a bounded wait inside the fused kernel gave up: clear every counter so that the handle stays usable
@@ -244,6 +244,12 @@ extern "C" int blok_moe_layer_check(blok_moe_layer_t *L, blok_stream_t stream_) 
 
 extern "C" int blok_moe_layer_debug_set_error(blok_moe_layer_t *L, unsigned code, blok_stream_t stream) {
   BLOK_REQUIRE(L, BLOK_ERR_ARG, "blok_moe_layer_debug_set_error: null pointer");
+  if (code >= 256) {
+    BLOK_REQUIRE(L->b_err, BLOK_ERR_STATE, "blok_moe_layer_debug_set_error: this layer was created with max_tokens = 1");
+    BLOK_CUDA(cudaMemcpyAsync(L->b_err, &code, sizeof(code), cudaMemcpyHostToDevice, (cudaStream_t)stream));
+    BLOK_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+    return BLOK_OK;
+  }
   BLOK_REQUIRE(L->f_ctrl, BLOK_ERR_STATE, "blok_moe_layer_debug_set_error: this layer has no fused decode kernel (no error word)");
   BLOK_CUDA(cudaMemcpyAsync(L->f_ctrl + 5, &code, sizeof(code), cudaMemcpyHostToDevice, (cudaStream_t)stream));
   BLOK_CUDA(cudaStreamSynchronize((cudaStream_t)stream));

@@ -61,12 +61,11 @@ int launch_router_topk(const float *logits, const float *bias, int T, int expert
 
 using namespace blok;
 
-// fp32 logits [T, experts], then (for more than 16 tokens) the tile table of the weight-streaming GEMM
+// fp32 logits [T, experts], then a word that a product whose wait gave up writes to
 static size_t router_logits_bytes(int T, int experts) { return ((size_t)T * experts * sizeof(float) + 255) / 256 * 256; }
 extern "C" size_t blok_router_workspace_bytes(int T, int experts) {
   if (T <= 0 || experts <= 0) return 0;
-  const size_t tiles = (size_t)(T + kWgTileTokens - 1) / kWgTileTokens;
-  return router_logits_bytes(T, experts) + (3 * tiles + 1) * sizeof(int) + 256;
+  return router_logits_bytes(T, experts) + 256;
 }
 
 extern "C" int blok_router(const blok_bf16_t *router_w, const float *bias, const blok_bf16_t *x, int T, int experts,
@@ -88,6 +87,8 @@ extern "C" int blok_router(const blok_bf16_t *router_w, const float *bias, const
     r.K = hidden; r.R = experts; r.out_bf16 = nullptr; r.out_f32 = logits;
     r.tile_expert = r.tile_start = r.tile_count = r.num_tiles = nullptr;
     r.out_index = nullptr; r.n_rows = T; r.identity_tiles = 1;
+    // no handle to report to: where a wait of the product gave up the logits, and with them the weights, are NaN
+    r.err = reinterpret_cast<unsigned *>(static_cast<unsigned char *>(workspace) + router_logits_bytes(T, experts));
     int rc;
     if ((rc = launch_wgemm(WG_BF16_PLAIN, r, tiles, (cudaStream_t)stream))) return rc;
     return launch_router_topk(logits, bias, T, experts, topk, routed_scale, ids, wts, nullptr, 0, (cudaStream_t)stream);

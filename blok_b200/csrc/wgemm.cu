@@ -231,6 +231,7 @@ static int launch_wgemm_tma(int mode, const WgArgs &a, int forced, cudaStream_t 
   g.act = swiglu ? GEMM_ACT_SWIGLU_REF : GEMM_ACT_NONE;
   g.out = a.out_f32 ? (void *)a.out_f32 : (void *)a.out_bf16;
   g.out_f32 = a.out_f32 != nullptr;
+  g.err = a.err;
   const int cols = swiglu ? 2 * a.R : a.R;
   const int nz = forced || !a.splitk_ws ? 1 : std::min<long>(wgemm_tma_split(mode, a.K, a.R, a.n_rows), a.splitk_bytes / ((size_t)a.n_rows * cols * sizeof(float)));
   if (nz > 1) {

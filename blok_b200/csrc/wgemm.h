@@ -35,6 +35,7 @@ struct WgArgs {
   // bf16 modes over identity tiles: scratch for the K-split partial sums, see wgemm_splitk_bytes; NULL: no split
   float *splitk_ws = nullptr;
   size_t splitk_bytes = 0;
+  unsigned *err = nullptr;  // set to 1 when a tcgen05 kernel's wait gives up: a word of the handle the launch is for
 };
 
 // Picks the kernel of a launch.  INT4 modes: the mma.sync kernel (see launch_wgemm_experts for the others).  bf16 modes: up to
@@ -77,8 +78,5 @@ int launch_wgemm_rows(int mode, const void *w_a, const void *w_b, const uint16_t
 int launch_wgemm_experts(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream);
 bool wgemm_i4_supports(const WgArgs &up, const WgArgs &down);
 int launch_wgemm_i4(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream);
-
-// *out becomes non-zero if a tcgen05 GEMM CTA has given up on a barrier since the last call (the flag is cleared).
-int wgemm_tc_take_error(unsigned *out);
 
 }  // namespace blok

@@ -15,7 +15,6 @@
 namespace blok {
 
 constexpr int kTcN = kWgTileTokens;  // token columns of a tile
-__device__ unsigned g_wgemm_tc_error = 0;
 
 __device__ __forceinline__ uint32_t tc_bf16x2_mul(uint32_t a, uint32_t b) {
   uint32_t r;
@@ -89,6 +88,7 @@ struct I4Args {
   int K, R, stride_rows;
   const void *w_a, *w_b;  // the operands again, for i4_plain_rows
   const uint16_t *s_a, *s_b, *x;
+  unsigned *err;
 };
 
 // The epilogue of a thread's two sums for one token: gate and up, or two rows of the down projection 128 apart.
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(kI4Threads, 1)
     const I4Mma m = {x_full, x_empty, a_full, a_empty, d_full, d_empty, xbase};
     failed = warp ? !i4_mma<1>(m, a, units, blocks, stages) : !i4_mma<0>(m, a, units, blocks, stages);
   }
-  if (failed) atomicExch(&g_wgemm_tc_error, 1u);
+  if (failed && a.err) atomicExch(a.err, 1u);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tp_tmem_free(tmem, kI4TmemCols);
@@ -465,7 +465,7 @@ static int i4_launch(bool swiglu, const WgArgs &g, const uint16_t *x, long x_row
   }
   if ((rc = tensor_map_2d(x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x_rows, g.K, (long)g.K * 2, 16, 64, CU_TENSOR_MAP_SWIZZLE_128B, &mx))) return rc;
   const I4Args a = {g.out_bf16, g.out_index, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.K, g.R, (int)g.expert_stride_rows,
-                    g.w_a, g.w_b, g.s_a, g.s_b, x};
+                    g.w_a, g.w_b, g.s_a, g.s_b, x, g.err};
   if (swiglu) {
     BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kI4Smem));
     wgemm_tc_kernel<true><<<sm_count(), kI4Threads, kI4Smem, stream>>>(wa, wb, sa, sb, mx, a);
@@ -483,15 +483,6 @@ int launch_wgemm_i4(const WgArgs &up, const WgArgs &down, uint16_t *xs, long row
   if (rc) return rc;
   if ((rc = i4_launch(true, up, xs, rows, stream))) return rc;
   return i4_launch(false, down, up.out_bf16, rows, stream);
-}
-
-// Non-zero once any tcgen05 GEMM CTA gave up on a barrier; cleared by the read.
-int wgemm_tc_take_error(unsigned *out) {
-  unsigned v = 0, zero = 0;
-  BLOK_CUDA(cudaMemcpyFromSymbol(&v, g_wgemm_tc_error, sizeof(v)));
-  if (v) BLOK_CUDA(cudaMemcpyToSymbol(g_wgemm_tc_error, &zero, sizeof(zero)));
-  *out = v;
-  return BLOK_OK;
 }
 
 }  // namespace blok

@@ -162,7 +162,8 @@ size_t blok_router_workspace_bytes(int T, int experts);
  * order), w_k = s[id_k] / (sum_k s[id_k] + 1e-20) * routed_scale.  Replaces
  * src/kimi_exec.cu:836-842 (matvec_bf16_f32_k :286, sigmoid_k :377, add_bf16_k
  * :372, router_topk_k :382).  x bf16 [T, hidden]; bias fp32 [experts]; ids uint16
- * [T, topk]; wts fp32 [T, topk].  experts <= 1024, topk <= 32. */
+ * [T, topk]; wts fp32 [T, topk].  experts <= 1024, topk <= 32.  There is no handle to check: should a bounded
+ * device-side wait ever give up (more than 64 tokens), the weights of the tokens concerned are NaN. */
 int blok_router(const blok_bf16_t *router_w, const float *bias, const blok_bf16_t *x, int T, int experts, int hidden,
                 int topk, float routed_scale, uint16_t *ids, float *wts, void *workspace, size_t workspace_bytes,
                 blok_stream_t stream);
@@ -252,14 +253,15 @@ int blok_moe_decode_partial(blok_moe_layer_t *layer, const blok_bf16_t *x, float
 int blok_moe_layer_has_partial(blok_moe_layer_t *layer);
 
 /* Synchronises `stream` and reports whether a device-side wait of an earlier
- * blok_moe_decode on this handle gave up (BLOK_ERR_TIMEOUT; the handle is reset
- * and stays usable).  The reference has no such state: its kernels never wait
+ * blok_moe_decode, blok_moe_batched, blok_moe_experts_grouped or blok_moe_shared on
+ * this handle gave up (BLOK_ERR_TIMEOUT; the handle is reset and stays usable;
+ * other handles report their own).  The reference has no such state: its kernels never wait
  * on one another (src/kimi_exec.cu launches are all on the default stream). */
 int blok_moe_layer_check(blok_moe_layer_t *layer, blok_stream_t stream);
 
 /* Test hook (host-side fault injection; nothing faults or hangs on the device): stores `code` in the handle's device
  * error word exactly as a wait that gave up would, so that the reporting path (blok_moe_layer_check, blok_model_check,
- * blok_moe_decode_host) can be exercised. */
+ * blok_moe_decode_host) can be exercised.  Codes from 256 on: the word of the products over several tokens. */
 int blok_moe_layer_debug_set_error(blok_moe_layer_t *layer, unsigned code, blok_stream_t stream);
 
 /* Diagnostics (no counterpart in the reference): with BLOK_MLA_TRACE=1 in the environment at the first attention

@@ -131,3 +131,24 @@ def test_experts_grouped_handles_empty_and_ragged_groups(cuda, oracle, monkeypat
     with pytest.raises(lib.BlokError):
         layer.experts_grouped(x, torch.zeros(64 * 8 + 1, dtype=torch.int32, device=cuda))
     layer.close()
+
+
+def test_a_product_that_gave_up_is_reported_by_its_own_handle(cuda):
+    """The error word of the products over several tokens belongs to the handle: another layer's check neither reports nor clears
+    it.  The word is set from the host (blok_moe_layer_debug_set_error): no wait is made to run out on the device."""
+    import ctypes as C
+    from blok_b200 import lib, synth
+    w = synth.moe_layer_weights(cuda, seed=41, hidden=512, inter=512, experts=128, shared_inter=0)
+    a, b, one = lib.MoeLayer(w, max_tokens=4), lib.MoeLayer(w, max_tokens=4), lib.MoeLayer(w)
+    assert lib.load().blok_moe_layer_debug_set_error(a._handle, C.c_uint(256), None) == 0
+    b.check()
+    one.check()
+    with pytest.raises(lib.BlokError) as e:
+        a.check()
+    assert e.value.code == -5 and "blok_moe_batched" in str(e.value)
+    a.check()                                   # reported once; the handle stays usable
+    x = synth.activations(4, 512, cuda, 1)
+    assert torch.equal(a.batched(x), b.batched(x))
+    assert lib.load().blok_moe_layer_debug_set_error(one._handle, C.c_uint(256), None) == -4  # no such products on this handle
+    for layer in (a, b, one):
+        layer.close()
