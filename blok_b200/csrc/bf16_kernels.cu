@@ -199,8 +199,7 @@ __global__ void __launch_bounds__(128) bf16_gemv16_splitk_kernel(const uint16_t 
 // the element loop.
 // ADD: first x <- bf16(x + t) (the rounded residual add, src/kimi_exec.cu:248-251), written back, then the norm of it.
 template <bool ADD>
-__global__ void __launch_bounds__(256) rmsnorm_kernel(uint16_t *__restrict__ x, const uint16_t *__restrict__ tadd,
-                                                      const uint16_t *__restrict__ w, uint16_t *__restrict__ y, int n, float eps) {
+__global__ void __launch_bounds__(256) rmsnorm_kernel(uint16_t *x, const uint16_t *tadd, const uint16_t *w, uint16_t *y, int n, float eps) {
   __shared__ float red[32];
   pdl_trigger();
   pdl_wait();
@@ -210,16 +209,20 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(uint16_t *__restrict__ x, 
   const bool vec = (n % 8 == 0) && n <= 8192 && ((reinterpret_cast<uintptr_t>(xr) | reinterpret_cast<uintptr_t>(yr) |
                                                   reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(tr)) & 15) == 0;
   float v = 0.f;
-  uint4 xv[4];
+  uint4 xv[4], tv[4];
   const int nu = n / 8;
   if (vec) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int u = threadIdx.x + k * 256;
       xv[k] = u < nu ? reinterpret_cast<const uint4 *>(xr)[u] : make_uint4(0, 0, 0, 0);
+      if (ADD && u < nu) tv[k] = reinterpret_cast<const uint4 *>(tr)[u];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int u = threadIdx.x + k * 256;
       if (ADD && u < nu) {
-        const uint4 tv = reinterpret_cast<const uint4 *>(tr)[u];
-        const uint32_t a[4] = {xv[k].x, xv[k].y, xv[k].z, xv[k].w}, c[4] = {tv.x, tv.y, tv.z, tv.w};
+        const uint32_t a[4] = {xv[k].x, xv[k].y, xv[k].z, xv[k].w}, c[4] = {tv[k].x, tv[k].y, tv[k].z, tv[k].w};
         uint32_t o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)

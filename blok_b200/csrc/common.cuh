@@ -64,6 +64,8 @@ inline int launch_pdl(const char *what, void (*kernel)(P...), dim3 grid, dim3 bl
 // The kernel behind this one may become resident as soon as every block of this one has started.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Everything before this launch has finished and is visible; nothing that it reads or writes may be touched earlier.  Without the launch attribute both do nothing.
+// The kernel is resident while others write what it will read, so its inputs are plain pointers: const __restrict__ or __ldg would
+// promise that nobody writes them while it lives, and let the compiler and the read-only path fetch them before the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ float bf16_bits_to_f32(uint32_t h) { return __uint_as_float(h << 16); }
 __device__ __forceinline__ float bf16lo(uint32_t pair) { return __uint_as_float(pair << 16); }

@@ -44,12 +44,11 @@ int launch_head_gemv(const uint16_t *w, long w_head_stride, const uint16_t *x, l
 // ---------------------------------------------------------------------------
 // grid = (1 + heads / 8, B), 256 threads: block 0 of a sequence normalises c_kv, rotates k_pe, appends the cache row
 // and publishes seq = ctx_len + 1 (the tokens the attention covers); blocks 1.. rotate the rope part of 8 heads each.
-__global__ void __launch_bounds__(256) mla_prep_kernel(const uint16_t *__restrict__ kva, const uint16_t *__restrict__ kva_ln,
-                                                       const uint16_t *__restrict__ q, const float *__restrict__ inv_freq,
-                                                       const int *__restrict__ ctx_len, uint16_t *__restrict__ cache,
+__global__ void __launch_bounds__(256) mla_prep_kernel(const uint16_t *kva, const uint16_t *kva_ln, const uint16_t *q,
+                                                       const float *__restrict__ inv_freq, const int *ctx_len, uint16_t *__restrict__ cache,
                                                        long ctx_stride, uint16_t *__restrict__ q_full, int *__restrict__ seq,
                                                        int heads, int nope, int rope, int kv_rank, float eps,
-                                                       const int *__restrict__ block_table, const int *__restrict__ slot_of,
+                                                       const int *block_table, const int *slot_of,
                                                        int table_stride, int page_rows, long ctx_cap, unsigned *__restrict__ err) {
   __shared__ float red[32];
   const int b = blockIdx.y, tid = threadIdx.x;

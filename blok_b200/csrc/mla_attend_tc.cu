@@ -163,9 +163,9 @@ size_t mla_attend_tc_smem_bytes() { return kTaSmemBytes; }
 // 64 rows x 64 columns, 128-byte swizzle).  PAGED: page_rows is a multiple of the 64-token tile.
 template <bool PAGED, bool FINE>
 __global__ void __launch_bounds__(kTaThreads, 1)
-    mla_attend_tc_kernel(const __grid_constant__ CUtensorMap tmap, const uint16_t *__restrict__ q, const uint16_t *__restrict__ cache,
-                         long ctx_stride, const int *__restrict__ seq_len, float scale, float *__restrict__ part_o,
-                         float *__restrict__ part_ml, const int *__restrict__ block_table, const int *__restrict__ slot_of,
+    mla_attend_tc_kernel(const __grid_constant__ CUtensorMap tmap, const uint16_t *q, const uint16_t *cache,
+                         long ctx_stride, const int *seq_len, float scale, float *__restrict__ part_o,
+                         float *__restrict__ part_ml, const int *block_table, const int *slot_of,
                          int table_stride, int page_rows, long long *__restrict__ trace, int heads) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long s_bar[11];

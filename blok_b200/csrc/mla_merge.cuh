@@ -10,9 +10,8 @@ namespace blok {
 // Rows of o_lat are ldo values apart (0: heads * kv_rank).  gate, optional: bf16 [B, ld_gate]; head h's output times
 // sigmoid(gate[b][h]).
 // ---------------------------------------------------------------------------
-static __global__ void mla_merge_kernel(const float *__restrict__ part_o, const float *__restrict__ part_ml, int splits,
-                                 int heads, int kv_rank, uint16_t *__restrict__ o_lat, int ldo = 0,
-                                 const uint16_t *__restrict__ gate = nullptr, int ld_gate = 0) {
+static __global__ void mla_merge_kernel(const float *part_o, const float *part_ml, int splits, int heads, int kv_rank,
+                                        uint16_t *__restrict__ o_lat, int ldo = 0, const uint16_t *gate = nullptr, int ld_gate = 0) {
   extern __shared__ float s_wt[];  // [splits] weight of every split: exp(m_s - M), 0 for an empty split
   __shared__ float s_red[2][4];
   pdl_trigger();
@@ -51,7 +50,7 @@ static __global__ void mla_merge_kernel(const float *__restrict__ part_o, const 
     for (; s + 8 <= splits; s += 8) {
       float4 v[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = __ldg(po4 + (size_t)(s + i) * stride4 + j4);
+      for (int i = 0; i < 8; ++i) v[i] = po4[(size_t)(s + i) * stride4 + j4];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float wt = s_wt[s + i];
@@ -62,7 +61,7 @@ static __global__ void mla_merge_kernel(const float *__restrict__ part_o, const 
       }
     }
     for (; s < splits; ++s) {
-      const float4 v = __ldg(po4 + (size_t)s * stride4 + j4);
+      const float4 v = po4[(size_t)s * stride4 + j4];
       const float wt = s_wt[s];
       acc.x = fmaf(wt, v.x, acc.x);
       acc.y = fmaf(wt, v.y, acc.y);
