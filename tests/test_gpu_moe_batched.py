@@ -17,12 +17,13 @@ def _oracle_layer(oracle, w, x, ids_needed, topk=8):
                             shared[2], util.t2np_f32(x), topk=topk, mode=0)
 
 
-# the mma.sync kernel and the tcgen05 kernels, whatever the size; "auto": the library's own choice, which sends groups of
-# up to four tokens through the mat-vec-style kernel (wgemv_small.cu) and the rest through the kernel the size picks
+# the mma.sync kernel and the tcgen05 kernels, whatever the size; "auto": the library's own choice, which takes the mat-vec-style
+# kernel (wgemv_small.cu) up to 40 assignments (T = 5) and the tcgen05 kernel from there
 @pytest.mark.parametrize("impl", ["mma", "tc", "auto"])
 @pytest.mark.parametrize("T,hidden,inter,experts,shared,seed", [(40, 1024, 512, 128, 512, 31), (1, 1024, 512, 128, 512, 32),
                                                                 (64, 7168, 2048, 384, 2048, 2), (130, 512, 512, 128, 0, 33),
-                                                                (7, 1024, 512, 128, 512, 34)])
+                                                                (7, 1024, 512, 128, 512, 34), (2, 2048, 1024, 128, 512, 35),
+                                                                (5, 1536, 512, 128, 0, 36)])
 def test_moe_batched_vs_oracle(cuda, oracle, monkeypatch, impl, T, hidden, inter, experts, shared, seed):
     from blok_b200 import lib, synth
     if impl == "auto":
@@ -106,8 +107,7 @@ def test_moe_batched_2048_tokens_against_the_oracle(cuda, oracle):
 @pytest.mark.parametrize("impl", ["mma", "tc", "auto"])
 def test_experts_grouped_handles_empty_and_ragged_groups(cuda, oracle, monkeypatch, impl):
     """Assignments concentrated on few experts (others get zero tokens), more than one 64-token tile for one expert.
-    Left to itself ("auto") the library sends all of them through the small-group kernel: the larger groups are few, so
-    it takes the 64-token tile (sixteen passes of four tokens) and the group of nine as well."""
+    Left to itself ("auto") the library takes the tcgen05 kernel: there are more than 40 assignments."""
     from blok_b200 import lib, synth
     monkeypatch.setenv("BLOK_WGEMM_IMPL", impl)
     hidden, inter, experts = 512, 512, 128
@@ -130,6 +130,40 @@ def test_experts_grouped_handles_empty_and_ragged_groups(cuda, oracle, monkeypat
     assert layer.experts_grouped(x, e[:0].contiguous(), rows[:0].contiguous()).shape == (0, hidden)
     with pytest.raises(lib.BlokError):
         layer.experts_grouped(x, torch.zeros(64 * 8 + 1, dtype=torch.int32, device=cuda))
+    layer.close()
+
+
+@pytest.mark.parametrize("hidden,inter,groups,small", [
+    (512, 512, {7: 40}, True),                               # ten passes of four tokens over one expert
+    (2048, 1024, {0: 2, 5: 3, 64: 4, 90: 9, 127: 5}, True),  # passes of 1 to 4 tokens; scales staged in chunks of 16 k-blocks
+    (1536, 512, {3: 9, 4: 5, 126: 26}, True),                # 40 assignments; chunks of 14
+    (7168, 512, {2: 1, 3: 2, 383: 6}, True),                 # rows of full length, four whole chunks of 14
+    (1024, 512, {0: 1, 1: 40}, False),                       # one more than the mat-vec-style kernel takes
+])
+def test_few_assignments(cuda, oracle, monkeypatch, hidden, inter, groups, small):
+    """The library's own choice up to 40 assignments, the mat-vec-style kernel (wgemv_small.cu), in passes of up to four tokens of
+    one expert, every assignment against the oracle; the tcgen05 kernel gives other bits below the limit and the same above."""
+    from blok_b200 import lib, synth
+    monkeypatch.delenv("BLOK_WGEMM_IMPL", raising=False)
+    w = synth.moe_layer_weights(cuda, seed=43, hidden=hidden, inter=inter, experts=384, shared_inter=0)
+    if hidden < 7168:
+        for k in ("gate_s", "up_s", "down_s"):
+            w[k] = (w[k].float() * 8).bfloat16()
+    N = sum(groups.values())
+    layer = lib.MoeLayer(w, max_tokens=8)
+    x = synth.activations(N, hidden, cuda, 44)
+    e = torch.tensor([k for k, n in groups.items() for _ in range(n)], dtype=torch.int32, device=cuda)
+    e = e[torch.randperm(N, generator=torch.Generator().manual_seed(N)).to(cuda)].contiguous()
+    got = layer.experts_grouped(x, e)
+    assert torch.equal(got, layer.experts_grouped(x, e))
+    y, xh = util.t2np_f32(got), util.t2np_f32(x)
+    host = {k: [util.t2np_u32(w[n][k]) if n.endswith("_w") else util.t2np_bf16(w[n][k])
+                for n in ("gate_w", "gate_s", "up_w", "up_s", "down_w", "down_s")] for k in groups}
+    for a in range(N):
+        util.assert_close(y[a], oracle.expert_ffn(*host[int(e[a])], xh[a], mode=0, round_out=True), "assignment %d" % a)
+    monkeypatch.setenv("BLOK_WGEMM_IMPL", "tc")
+    assert torch.equal(got, layer.experts_grouped(x, e)) != small
+    layer.check()
     layer.close()
 
 

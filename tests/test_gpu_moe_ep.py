@@ -1,7 +1,7 @@
 """The expert-parallel layer under the C ABI (blok_moe_ep_*) on ONE GPU: with a world of one rank the whole exchange
 (count table, plan, dispatch into the receive buffer, grouped GEMM, combine from the result buffer) runs against the
-rank's own buffers, and the result must equal blok_moe_batched bit for bit: the same kernels compute every row and the
-combine adds the slots in the same order.  (Two ranks: tests/test_gpu_ep.py.)"""
+rank's own buffers, and the result must equal blok_moe_batched bit for bit where the same kernels compute every row (a
+forced GEMM kernel, or more than 40 assignments): the combine adds the slots in the same order.  (Two ranks: tests/test_gpu_ep.py.)"""
 import pytest
 import torch
 
