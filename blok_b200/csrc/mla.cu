@@ -421,21 +421,11 @@ extern "C" int blok_mla_attend_paged(blok_mla_layer_t *L, const blok_bf16_t *q, 
 }
 
 // y[b, :] = bf16(W x[b, :]) for B entries.  Up to 8 entries go through the split-K mat-vec kernel; 9 to 64 through the
-// weight-streaming kernel, one pass over the weights for all entries; more, where the matrix fits its tiling, through the
-// GEMM (`tiles_ready`: the identity tile table for B entries has been written on this stream), else 8 at a time.
-static int project(blok_mla_layer *L, const uint16_t *w, const uint16_t *x, uint16_t *y, int rows, int cols, int B, bool tiles_ready,
-                   cudaStream_t stream) {
-  if (B > 8 && B <= kWgStreamTokens && rows % 16 == 0 && cols % 256 == 0)
+// weight-streaming kernel, one pass over the weights for all entries, where it covers the matrix, else 8 at a time.
+static_assert(kMlaMaxBatch <= kWgStreamTokens, "a call's entries are one pass of the weight-streaming kernel");
+static int project(blok_mla_layer *L, const uint16_t *w, const uint16_t *x, uint16_t *y, int rows, int cols, int B, cudaStream_t stream) {
+  if (B > 8 && rows % 16 == 0 && cols % 256 == 0)
     return launch_wgemm_rows(WG_BF16_PLAIN, w, nullptr, x, y, nullptr, rows, cols, B, L->wg_ws, L->wg_bytes, stream);
-  if (tiles_ready && rows % 128 == 0 && cols % 512 == 0) {
-    const int tiles = (B + kWgTileTokens - 1) / kWgTileTokens;
-    WgArgs r;
-    r.w_a = w; r.w_b = nullptr; r.s_a = r.s_b = nullptr; r.expert_stride_rows = 0; r.x = x; r.x_index = nullptr;
-    r.K = cols; r.R = rows; r.out_bf16 = y; r.out_f32 = nullptr;
-    r.tile_expert = r.tile_start = r.tile_count = r.num_tiles = nullptr;
-    r.out_index = nullptr; r.n_rows = B; r.identity_tiles = 1;
-    return launch_wgemm(WG_BF16_PLAIN, r, tiles, stream);
-  }
   for (int b0 = 0; b0 < B; b0 += 8)
     if (int rc = launch_bf16_gemv_splitk(w, x + (size_t)b0 * cols, y + (size_t)b0 * rows, nullptr, rows, cols, std::min(8, B - b0), L->sk_ws,
                                          L->sk_bytes, stream))
@@ -454,24 +444,20 @@ static int decode_body(blok_mla_layer *L, const uint16_t *n, const CacheRef &c, 
   const size_t q_row = (size_t)w.heads * qk_head, qf_row = (size_t)w.heads * lat_w, ol_row = (size_t)w.heads * w.kv_rank,
                av_row = (size_t)w.heads * w.v_head;
   int rc;
-  const bool gemm = B > kWgStreamTokens;  // the GEMM form of the projections
-  const bool stream_rows = B > 8 && !gemm;  // 9..64 entries: one pass of the weight-streaming kernel per matrix
   // q_a -> RMSNorm -> q_b   (:813-815); kv_a (:816) reads the same activations as q_a and shares its launch where the
   // mat-vec kernel serves both (up to 8 entries per launch)
-  if (!gemm && !stream_rows) {
-    for (int b0 = 0; b0 < B; b0 += 8)
-      if ((rc = launch_bf16_gemv_splitk_pair(w.q_a, w.q_rank, L->qa + (size_t)b0 * w.q_rank, w.kv_a, lat_w, L->kva + (size_t)b0 * lat_w,
-                                             n + (size_t)b0 * w.hidden, w.hidden, std::min(8, B - b0), L->sk_ws, L->sk_bytes, stream)))
-        return rc;
+  if (B <= 8) {
+    if ((rc = launch_bf16_gemv_splitk_pair(w.q_a, w.q_rank, L->qa, w.kv_a, lat_w, L->kva, n, w.hidden, B, L->sk_ws, L->sk_bytes, stream))) return rc;
   } else {
-    if ((rc = project(L, w.q_a, n, L->qa, w.q_rank, w.hidden, B, gemm, stream))) return rc;
-    if ((rc = project(L, w.kv_a, n, L->kva, lat_w, w.hidden, B, gemm, stream))) return rc;
+    if ((rc = project(L, w.q_a, n, L->qa, w.q_rank, w.hidden, B, stream))) return rc;
+    if ((rc = project(L, w.kv_a, n, L->kva, lat_w, w.hidden, B, stream))) return rc;
   }
   if ((rc = blok_rmsnorm(L->qa, w.q_a_ln, L->qa, B, w.q_rank, w.rms_eps, stream_))) return rc;
-  if ((rc = project(L, w.q_b, L->qa, L->q, w.heads * qk_head, w.q_rank, B, gemm, stream))) return rc;
+  if ((rc = project(L, w.q_b, L->qa, L->q, w.heads * qk_head, w.q_rank, B, stream))) return rc;
   // norm of c_kv, RoPE of k_pe and of q's rope part, cache append   (:816-824)
-  rc = launch_pdl("mla_prep_kernel", mla_prep_kernel, dim3(1 + (w.heads * (w.qk_rope / 2) + 255) / 256, B), 256, 0, stream, L->kva, w.kv_a_ln, L->q, L->inv_freq, ctx_len, c.base, c.seq_stride, L->q_full, L->seq, w.heads, w.qk_nope, w.qk_rope,
-      w.kv_rank, w.rms_eps, c.block_table, c.slot_of, c.table_stride, c.page_rows, c.ctx_cap, L->err);
+  rc = launch_pdl("mla_prep_kernel", mla_prep_kernel, dim3(1 + (w.heads * (w.qk_rope / 2) + 255) / 256, B), 256, 0, stream, L->kva, w.kv_a_ln, L->q,
+                  L->inv_freq, ctx_len, c.base, c.seq_stride, L->q_full, L->seq, w.heads, w.qk_nope, w.qk_rope, w.kv_rank, w.rms_eps, c.block_table,
+                  c.slot_of, c.table_stride, c.page_rows, c.ctx_cap, L->err);
   if (rc) return rc;
   // q_abs = W_UK^T q_nope
   if ((rc = launch_head_gemv(L->wuk_t, (long)w.kv_rank * w.qk_nope, L->q, (long)q_row, qk_head, L->q_full, (long)qf_row, lat_w, w.kv_rank,
@@ -482,7 +468,7 @@ static int decode_body(blok_mla_layer *L, const uint16_t *n, const CacheRef &c, 
   if ((rc = launch_head_gemv(w.kv_b + (size_t)w.qk_nope * w.kv_rank, (long)(w.qk_nope + w.v_head) * w.kv_rank, L->o_lat, (long)ol_row,
                              w.kv_rank, L->av, (long)av_row, w.v_head, w.v_head, w.kv_rank, w.heads, B, stream)))
     return rc;
-  return project(L, w.o, L->av, out, w.hidden, w.heads * w.v_head, B, gemm, stream);
+  return project(L, w.o, L->av, out, w.hidden, w.heads * w.v_head, B, stream);
 }
 
 extern "C" int blok_mla_decode(blok_mla_layer_t *L, const blok_bf16_t *n, blok_bf16_t *cache, long ctx_stride,

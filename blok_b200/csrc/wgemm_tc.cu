@@ -77,7 +77,7 @@ constexpr int kI4WStages = 4, kI4WBytes = 256 * (kI4Cols / 2);  // 32 KB
 constexpr int kI4SStages = 3, kI4SBytes = 256 * 32;             // scales of 512 columns: whole 32-byte sectors
 constexpr int kI4XStages = 4, kI4XHalf = kTcN * 128, kI4XBytes = 2 * kI4XHalf;  // 64 tokens x 2 x 64 columns
 constexpr int kI4Smem = kI4WStages * kI4WBytes + kI4SStages * kI4SBytes + kI4XStages * kI4XBytes + 1024;
-constexpr int kI4Piece = 2;                                     // 64-column parts per piece
+constexpr int kI4Piece = 2;                                     // 64-column parts per piece: a slot of the activations
 constexpr int kI4Pieces = 4 / kI4Piece;                         // per weight stage; each has its own tensor-memory buffer
 constexpr int kI4TmemCols = 512;                                // 2 x 2 accumulators of 64 columns, 4 pieces x 2 blocks x 32 columns of weights
 constexpr int kI4ACol = 4 * kTcN;
@@ -201,9 +201,7 @@ __device__ __forceinline__ bool i4_mma(const I4Mma &m, const I4Args &a, int unit
     for (int st = 0; st < stages; ++st) {
 #pragma unroll
       for (int c = 0; c < kI4Pieces; ++c) {
-        const bool first = kI4Piece == 2 || !(c & 1), last = kI4Piece == 2 || (c & 1);  // of the piece's 128 columns of activations
-        bool ok = !first || i4_wait<0>(m.x_full + 8 * xr.slot, xr.turn);
-        ok = ok && i4_wait<0>(m.a_full + 16 * c + 8 * BLK, aturn);
+        const bool ok = i4_wait<0>(m.x_full + 8 * xr.slot, xr.turn) && i4_wait<0>(m.a_full + 16 * c + 8 * BLK, aturn);
         if (!__all_sync(0xffffffffu, ok)) return false;
         tc_fence_after();
         const uint64_t bd = tp_desc_k_sw128(m.xbase + xr.slot * kI4XBytes);
@@ -213,13 +211,13 @@ __device__ __forceinline__ bool i4_mma(const I4Mma &m, const I4Args &a, int unit
           for (int z = 0; z < kI4Piece; ++z)
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              tp_mma_ts(d, ta + (c * kI4Piece + z) * 64 + 8 * k, bd + (uint64_t)(((c * kI4Piece + z) & 1) * (kI4XHalf / 16) + 2 * k), idesc,
+              tp_mma_ts(d, ta + (c * kI4Piece + z) * 64 + 8 * k, bd + (uint64_t)(z * (kI4XHalf / 16) + 2 * k), idesc,
                         (st | c | z | k) ? 1u : 0u);
           tp_commit(m.a_empty + 16 * c + 8 * BLK);
-          if (last) tp_commit(m.x_empty + 8 * xr.slot);
+          tp_commit(m.x_empty + 8 * xr.slot);
           if (c == kI4Pieces - 1 && st == stages - 1) tp_commit(m.d_full + 8 * dr.slot);
         }
-        if (last) xr.next();
+        xr.next();
       }
       aturn ^= 1;
     }
