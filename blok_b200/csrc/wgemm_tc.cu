@@ -68,7 +68,9 @@ __device__ __forceinline__ void i4_dequant(uint32_t w, const I4Scale &s, uint32_
 // weights' barrier 1,301; operands of the MMAs in uniform registers 1,255; pieces of 128 columns instead of 64 and 16
 // unpacking warps instead of 24 1,138 us (5.6 TB/s).  With a hand-over every 64 columns the MMA warps' waits were the limit,
 // whatever the others did.  At 16,384 assignments 2,190 us before, 1,537 now; at 512 1,017 before, 800 now.
-// The test of the scales' range costs the whole layer 0.7 % at 6 tokens (289 us) and 1 to 2.5 % from 64 on.
+// Unpacking is bound by its instructions: the test of the scales' range (four of about 190 a piece) cost the layer 0.7 % at 6
+// tokens and 1 to 2.5 % from 64 on; the walk by pairs of stages, whose slots and parities are constants, took that back: 6 / 64 /
+// 517 / 2,048 tokens 291 / 1,575 / 2,220 / 3,180 us before, 287 / 1,495 / 2,127 / 3,110 now.
 constexpr int kI4Unpack = 16, kI4Epi = 4;                       // warps
 constexpr int kI4FirstUnpack = 4 + kI4Epi;
 constexpr int kI4Threads = (kI4FirstUnpack + kI4Unpack) * 32;
@@ -259,61 +261,66 @@ __global__ void __launch_bounds__(kI4Threads, 1)
   bool failed = false;
 
   if (warp >= kI4FirstUnpack) {
-    const int set = (warp - kI4FirstUnpack) >> 3, blk = (warp >> 2) & 1, row = 32 * (warp & 3) + lane;
+    // c: the piece of every stage that this set takes, and the tensor-memory buffer it goes to.  Two stages at a time: they share
+    // a slot of scales, and the slots and parities inside the pair are constants.
+    const int c = (warp - kI4FirstUnpack) >> 3, blk = (warp >> 2) & 1, row = 32 * (warp & 3) + lane;
     const uint32_t wrow = wbase + (uint32_t)(blk * (128 * 128) + row * 128);
-    const uint32_t srow = sbase + (uint32_t)(blk * (128 * 32) + row * 32);
-    const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(kI4ACol + blk * 32);
-    const int pieces = (int)blockIdx.x < units ? ((units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * kI4Pieces * stages : 0;
-    bool odd = false;
-    int unit = blockIdx.x, left = stages, dslot = 0;
-    for (int p = set; p < pieces; p += kI4Unpack / 8) {
-      const int st = p / kI4Pieces, c = p % kI4Pieces;  // c: the piece of its stage, and the tensor-memory buffer it goes to
-      const int ws = st % kI4WStages, ss = (st >> 1) % kI4SStages;
-      if (!__all_sync(0xffffffffu, i4_wait<0>(w_full + 8 * ws, (uint32_t)(st / kI4WStages) & 1))) {
-        failed = true;
-        break;
-      }
-      uint4 q[2 * kI4Piece];
-      uint32_t sc[kI4Piece];
+    const uint32_t srow = sbase + (uint32_t)(blk * (128 * 32) + row * 32 + c * 4 * kI4Piece);
+    const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(kI4ACol + blk * 32 + c * kI4Piece * 64);
+    const uint32_t ready = a_full + 16 * c + 8 * blk, free = a_empty + 16 * c + 8 * blk;
+    I4Ring<kI4WStages / 2> wr;
+    I4Ring<kI4SStages> sr;
+    int dslot = 0;
+    for (int u = blockIdx.x; u < units && !failed; u += gridDim.x) {
+      bool odd = false;
+      for (int st = 0; st < stages && !failed; st += 2) {
 #pragma unroll
-      for (int h = 0; h < 2 * kI4Piece; ++h) q[h] = i4_lds128(wrow + ws * kI4WBytes + (((2 * kI4Piece * c + h) ^ (row & 7)) << 4));
-#pragma unroll
-      for (int h = 0; h < kI4Piece; ++h) sc[h] = i4_lds32(srow + ss * kI4SBytes + (((st & 1) ^ ((row >> 2) & 1)) << 4) + (c * kI4Piece + h) * 4);
-      __syncwarp();
-      if (lane == 0) tp_arrive(w_empty + 8 * ws);
-#pragma unroll
-      for (int z = 0; z < kI4Piece; ++z) {
-        uint32_t av[32];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const I4Scale s2(__byte_perm(sc[z], 0, h ? 0x3232 : 0x1010));
-          const uint32_t w[4] = {q[2 * z + h].x, q[2 * z + h].y, q[2 * z + h].z, q[2 * z + h].w};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) i4_dequant(w[k], s2, av + (h * 4 + k) * 4);
-        }
-        if (z == 0) {
-          if (!__all_sync(0xffffffffu, i4_wait<0>(a_empty + 16 * c + 8 * blk, ((uint32_t)st & 1) ^ 1))) {  // the first use finds it free
+        for (int e = 0; e < 2; ++e) {
+          const uint32_t ws = 2 * wr.slot + e;
+          if (!__all_sync(0xffffffffu, i4_wait<0>(w_full + 8 * ws, wr.turn))) {
             failed = true;
             break;
           }
-          tc_fence_after();
+          uint4 q[2 * kI4Piece];
+          uint32_t sc[kI4Piece];
+#pragma unroll
+          for (int h = 0; h < 2 * kI4Piece; ++h) q[h] = i4_lds128(wrow + ws * kI4WBytes + (((2 * kI4Piece * c + h) ^ (row & 7)) << 4));
+#pragma unroll
+          for (int h = 0; h < kI4Piece; ++h) sc[h] = i4_lds32(srow + sr.slot * kI4SBytes + ((e ^ ((row >> 2) & 1)) << 4) + h * 4);
+          __syncwarp();
+          if (lane == 0) tp_arrive(w_empty + 8 * ws);
+#pragma unroll
+          for (int z = 0; z < kI4Piece; ++z) {
+            uint32_t av[32];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const I4Scale s2(__byte_perm(sc[z], 0, h ? 0x3232 : 0x1010));
+              const uint32_t w[4] = {q[2 * z + h].x, q[2 * z + h].y, q[2 * z + h].z, q[2 * z + h].w};
+#pragma unroll
+              for (int k = 0; k < 4; ++k) i4_dequant(w[k], s2, av + (h * 4 + k) * 4);
+            }
+            if (z == 0) {
+              if (!__all_sync(0xffffffffu, i4_wait<0>(free, e ^ 1))) {  // the first use finds it free
+                failed = true;
+                break;
+              }
+              tc_fence_after();
+            }
+            tmem_st32(ta + z * 64, av);
+          }
+          if (failed) break;
+          // while the stores are on their way; exponents that begin 01 are 2^-63 <= |s| < 2, for the few others the exact test
+          if (((sc[0] ^ 0x20002000u) | (sc[1] ^ 0x20002000u)) & 0x60006000u) odd = odd || i4_outside(sc[0]) || i4_outside(sc[1]);
+          if (e && st + 2 == stages && odd) s_odd[dslot] = u + 1;
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) tp_arrive(ready);
         }
-        tmem_st32(ta + (c * kI4Piece + z) * 64, av);
+        wr.next();
+        sr.next();
       }
-      if (failed) break;
-      // while the stores are on their way; exponents that begin 01 are 2^-63 <= |s| < 2, for the few others the exact test
-      if (((sc[0] ^ 0x20002000u) | (sc[1] ^ 0x20002000u)) & 0x60006000u) odd = odd || i4_outside(sc[0]) || i4_outside(sc[1]);
-      if (--left == 0) {  // the unit's last piece of this set
-        if (odd) s_odd[dslot] = unit + 1;
-        odd = false;
-        left = stages;
-        unit += gridDim.x;
-        dslot ^= 1;
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) tp_arrive(a_full + 16 * c + 8 * blk);
+      dslot ^= 1;
     }
   } else if (warp >= 4) {
     const int quarter = warp & 3, row = 32 * quarter + lane;
