@@ -281,19 +281,26 @@ int launch_wgemm(int mode, const WgArgs &args, int max_tiles, cudaStream_t strea
   return grid.z > 1 ? launch_wgemm_splitk_reduce(mode, args, (int)grid.z, stream) : BLOK_OK;
 }
 
-int launch_wgemm_experts(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream) {
+int launch_wgemm_experts(const WgArgs &up_in, const WgArgs &down_in, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream) {
   const int forced = wgemm_forced_impl();
   const char *sm = getenv("BLOK_WGEMM_SMALL");
-  // The mat-vec-style kernel deals a handful of groups out evenly, where the tcgen05 kernel's units of 256 rows fill the SMs
-  // unevenly; its work grows with the tokens, the tcgen05 kernel's does not.  Layer pass, us, mat-vec-style / tcgen05: 32
-  // assignments over 128 experts of 2048 x 1024 101 / 106, 64 129 / 117, 96 150 / 129; over 384 experts of 7168 x 2048 48
-  // 303 / 300, 72 403 / 424, 96 499 / 504, 128 703 / 644, 192 914 / 829.
-  if (forced == 0 && !(sm && sm[0] == '0') && rows <= kWgSmallRows && wgemv_small_supports(WG_I4_SWIGLU, up, max_tiles) &&
-      wgemv_small_supports(WG_I4_PLAIN, down, max_tiles)) {
+  const int few = (int)std::min<long>(rows, kWgSmallRows);
+  const bool small = forced == 0 && !(sm && sm[0] == '0') && wgemv_small_supports(WG_I4_SWIGLU, up_in, few) &&
+                     wgemv_small_supports(WG_I4_PLAIN, down_in, few);
+  const bool tc = forced != 1 && wgemm_i4_supports(up_in, down_in);
+  WgArgs up = up_in, down = down_in;
+  if (rows <= kWgSmallRows || !small || !tc) up.total = down.total = nullptr;
+  // The mat-vec-style kernel's work grows with the tokens, the tcgen05 kernel's with the groups.  Grouped experts under random
+  // routing (top 8), us, mat-vec-style / tcgen05: 384 experts of 7168 x 2048 16 assignments 101 / 107, 32 177 / 176, 40 205 / 206,
+  // 48 239 / 240, 64 306 / 297, 96 475 / 417, 128 586 / 558; 128 experts of 2048 x 1024 16 41 / 53, 32 65 / 70, 40 70 / 72, 48 86 / 86,
+  // 64 92 / 87, 128 124 / 91.  With one token in every group, which random routing does not give, the first is ahead to 128 (7168 x
+  // 2048: 96 432 / 502, 128 567 / 664).
+  if (small && (rows <= kWgSmallRows || up.total)) {
     if (int rc = launch_wgemv_small(WG_I4_SWIGLU, up, stream)) return rc;
-    return launch_wgemv_small(WG_I4_PLAIN, down, stream);
+    if (int rc = launch_wgemv_small(WG_I4_PLAIN, down, stream)) return rc;
+    if (rows <= kWgSmallRows) return BLOK_OK;
   }
-  if (forced != 1 && wgemm_i4_supports(up, down)) return launch_wgemm_i4(up, down, xs, rows, max_tiles, stream);
+  if (tc) return launch_wgemm_i4(up, down, xs, rows, max_tiles, stream);
   if (int rc = launch_wgemm(WG_I4_SWIGLU, up, max_tiles, stream)) return rc;
   return launch_wgemm(WG_I4_PLAIN, down, max_tiles, stream);
 }

@@ -35,6 +35,8 @@ struct WgArgs {
   // bf16 modes over identity tiles: scratch for the K-split partial sums, see wgemm_splitk_bytes; NULL: no split
   float *splitk_ws = nullptr;
   size_t splitk_bytes = 0;
+  // INT4 modes, where the host knows only a bound of them: the assignments that pick the kernel, a device word (launch_wgemm_experts)
+  const int *total = nullptr;
   unsigned *err = nullptr;  // set to 1 when a tcgen05 kernel's wait gives up: a word of the handle the launch is for
 };
 
@@ -55,7 +57,7 @@ int wgemm_tma_split(int mode, int K, int R, int rows);  // the same for the TMA-
 
 // The INT4 modes over few assignments: streams the weights like the batch-1 decode kernel (BLOK_WGEMM_SMALL=0 in the
 // environment: through the GEMM kernels as well).
-bool wgemv_small_supports(int mode, const WgArgs &args, int max_tiles);
+bool wgemv_small_supports(int mode, const WgArgs &args, int max_rows);
 int launch_wgemv_small(int mode, const WgArgs &args, cudaStream_t stream);
 
 // The bf16 modes over 1..kWgStreamTokens rows of x (identity tiles): every warp streams its 16 weight rows through a
@@ -73,8 +75,10 @@ int launch_wgemm_rows(int mode, const void *w_a, const void *w_b, const uint16_t
 
 // Both products of the grouped experts, INT4: mid = SwiGLU front half of x (up: WG_I4_SWIGLU), then the down projection
 // (down: WG_I4_PLAIN, its x is up's output).  Up to kWgSmallRows rows through the mat-vec-style kernel (wgemv_small.cu), else
-// through the tcgen05 kernel (wgemm_tc.cu) where it covers the shapes; else, or with BLOK_WGEMM_IMPL=mma, launch_wgemm twice.  xs: scratch of `rows` x up.K values, where `rows` is the number of sorted
-// positions that up.out_bf16 and xs hold (it may be the buffer of down's output).
+// through the tcgen05 kernel (wgemm_tc.cu) where it covers the shapes; else, or with BLOK_WGEMM_IMPL=mma, launch_wgemm twice.
+// With up.total both kernels are launched and the word decides on the device (the other one leaves at once).  xs: scratch of
+// `rows` x up.K values, where `rows` is the number of sorted positions that up.out_bf16 and xs hold (it may be the buffer of
+// down's output).
 int launch_wgemm_experts(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream);
 bool wgemm_i4_supports(const WgArgs &up, const WgArgs &down);
 int launch_wgemm_i4(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream);

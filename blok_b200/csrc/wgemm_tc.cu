@@ -88,6 +88,7 @@ struct I4Args {
   uint16_t *out;
   const int *out_index, *tile_expert, *tile_start, *tile_count, *num_tiles;
   int K, R, stride_rows;
+  const int *total;       // up to kWgSmallRows here: the launch is the mat-vec-style kernel's; NULL: no
   const void *w_a, *w_b;  // the operands again, for i4_plain_rows
   const uint16_t *s_a, *s_b, *x;
   unsigned *err;
@@ -232,6 +233,7 @@ template <bool SWIGLU>
 __global__ void __launch_bounds__(kI4Threads, 1)
     wgemm_tc_kernel(const __grid_constant__ CUtensorMap mwa, const __grid_constant__ CUtensorMap mwb, const __grid_constant__ CUtensorMap msa,
                     const __grid_constant__ CUtensorMap msb, const __grid_constant__ CUtensorMap mx, const __grid_constant__ I4Args a) {
+  if (a.total && *a.total <= kWgSmallRows) return;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long s_bar[2 * (kI4WStages + kI4XStages + 8 + 2)];
   __shared__ uint32_t s_tmem;
@@ -427,7 +429,8 @@ __global__ void __launch_bounds__(kI4Threads, 1)
 // order 0 4 1 5 2 6 3 7.  grid = (tile slots, parts of a tile).
 __global__ void __launch_bounds__(256) i4_rows_kernel(const uint16_t *__restrict__ x, const int *__restrict__ x_index, int K,
                                                       const int *__restrict__ tile_start, const int *__restrict__ tile_count,
-                                                      const int *__restrict__ num_tiles, uint16_t *__restrict__ xs) {
+                                                      const int *__restrict__ num_tiles, const int *__restrict__ total, uint16_t *__restrict__ xs) {
+  if (total && *total <= kWgSmallRows) return;
   const int ntiles = *num_tiles, per_row = K / 8;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int p0 = tile_start[tile], n = tile_count[tile] * per_row;
@@ -469,7 +472,7 @@ static int i4_launch(bool swiglu, const WgArgs &g, const uint16_t *x, long x_row
     if ((rc = tensor_map_2d(g.s_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, kRows, g.K / 16, g.K / 16, 128, 32, CU_TENSOR_MAP_SWIZZLE_32B, &sb))) return rc;
   }
   if ((rc = tensor_map_2d(x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x_rows, g.K, (long)g.K * 2, 16, 64, CU_TENSOR_MAP_SWIZZLE_128B, &mx))) return rc;
-  const I4Args a = {g.out_bf16, g.out_index, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.K, g.R, (int)g.expert_stride_rows,
+  const I4Args a = {g.out_bf16, g.out_index, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.K, g.R, (int)g.expert_stride_rows, g.total,
                     g.w_a, g.w_b, g.s_a, g.s_b, x, g.err};
   if (swiglu) {
     BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kI4Smem));
@@ -483,7 +486,7 @@ static int i4_launch(bool swiglu, const WgArgs &g, const uint16_t *x, long x_row
 
 int launch_wgemm_i4(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream) {
   // a tile's rows are shared by a few CTAs: 64 rows of 7,168 columns are 57,344 16-byte pieces
-  i4_rows_kernel<<<dim3(std::min(max_tiles, 1024), 4), 256, 0, stream>>>(up.x, up.x_index, up.K, up.tile_start, up.tile_count, up.num_tiles, xs);
+  i4_rows_kernel<<<dim3(std::min(max_tiles, 1024), 4), 256, 0, stream>>>(up.x, up.x_index, up.K, up.tile_start, up.tile_count, up.num_tiles, up.total, xs);
   int rc = launch_status("i4_rows_kernel");
   if (rc) return rc;
   if ((rc = i4_launch(true, up, xs, rows, stream))) return rc;

@@ -199,6 +199,7 @@ __device__ __forceinline__ void gs_stream_by_count(int cnt, const GsStream &q, i
 
 template <bool SWIGLU>
 __global__ void __launch_bounds__(kGsThreads, 1) wgemv_small_kernel(const WgArgs a) {
+  if (a.total && *a.total > kWgSmallRows) return;  // the tcgen05 kernel's
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ unsigned short s_group[kGsMaxGroups];  // the launch's passes: tile index | pass of the tile << 12
   __shared__ int s_ngroups;
@@ -310,10 +311,9 @@ __global__ void __launch_bounds__(kGsThreads, 1) wgemv_small_kernel(const WgArgs
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// max_tiles: the most tiles the launch's table can hold; every pass of every tile must fit the kernel's list and its 12-bit
-// tile index
-bool wgemv_small_supports(int mode, const WgArgs &a, int max_tiles) {
-  if (max_tiles > 4096 || max_tiles + a.n_rows / kGsPass > kGsMaxGroups) return false;
+// max_rows: the most assignments a launch that does the work finds; a pass has one at least, and the passes must fit the list
+bool wgemv_small_supports(int mode, const WgArgs &a, int max_rows) {
+  if (max_rows > kGsMaxGroups) return false;
   if (mode != WG_I4_SWIGLU && mode != WG_I4_PLAIN) return false;
   if (a.identity_tiles || a.K % 256 || a.R % 16) return false;  // 16-byte scale copies: an even number of k-blocks per row
   return wgemv_small_smem_bytes(a.K) <= 200 * 1024;
