@@ -30,13 +30,14 @@ __device__ __forceinline__ uint32_t tc_bf16x2_fma(uint32_t a, uint32_t b, uint32
 // Dequantisation with one instruction per pair of weights besides the masks.  The bits of a nibble n = q + 8 in the low four
 // bits of a bf16 are the number n 2^-133, in the next four n 2^-129 (below and just above the smallest normal number the
 // encoding is linear), so w & 0x000f000f and w & 0x00f000f0 are pairs of nibbles as they lie, and
-//   fma(n 2^-129, s 2^100, -s 2^-26) = bf16(q s 2^-29) = 2^-29 bf16(q s)
-// with one rounding, the reference's (:312): a power of two does not change it while s 2^104 is finite and q s 2^-29 normal
-// (s = 0 or 2^-97 <= |s| < 2^24).  The epilogue takes the 2^29 back, exactly.  (Adding an exponent to the nibble, subtracting
+//   fma(n 2^-129, s 2^117, -s 2^-9) = bf16(q s 2^-12) = 2^-12 bf16(q s)
+// with one rounding, the reference's (:312): a power of two does not change it while s 2^121 is finite and q s 2^-12 normal
+// (s = 0 or 2^-114 <= |s| < 2^7).  The epilogue takes the 2^12 back, exactly.  A larger power would cover larger scales and lose
+// smaller sums: with 2^29 results below 1e-31 lost bits, with 2^12 below 1e-36.  (Adding an exponent to the nibble, subtracting
 // 136 and multiplying took 15 instructions a word instead of 9.)  No checkpoint has other scales, but any bf16 is accepted:
 // i4_outside finds them, and i4_plain_rows takes the place of the unit's epilogue.
-constexpr uint32_t kI4Hi = 0x71807180u, kI4Lo = 0x73807380u, kI4Off = 0xb280b280u;  // 2^100, 2^104, -2^-26
-constexpr float kI4Unscale = 536870912.f;                                           // 2^29
+constexpr uint32_t kI4Hi = 0x7a007a00u, kI4Lo = 0x7c007c00u, kI4Off = 0xbb00bb00u;  // 2^117, 2^121, -2^-9
+constexpr float kI4Unscale = 4096.f;                                                // 2^12
 struct I4Scale {
   uint32_t hi, lo, off;
   __device__ __forceinline__ explicit I4Scale(uint32_t s2) : hi(tc_bf16x2_mul(s2, kI4Hi)), lo(tc_bf16x2_mul(s2, kI4Lo)), off(tc_bf16x2_mul(s2, kI4Off)) {}
@@ -106,11 +107,11 @@ __device__ __forceinline__ void i4_store(uint16_t *out, float va, float vb) {
   }
 }
 
-// Two scales: |s| 2^24 or more (infinities and NaN too), or below 2^-97 and not zero.  |s| - 1 with the top bit on: zero wraps to
+// Two scales: |s| 2^7 or more (infinities and NaN too), or below 2^-114 and not zero.  |s| - 1 with the top bit on: zero wraps to
 // the smallest unsigned and the largest signed value.
 __device__ __forceinline__ bool i4_outside(uint32_t s2) {
   const uint32_t v = (s2 | 0x80008000u) - 0x00010001u;
-  return __vmaxu2(v, 0xcb7ecb7eu) != 0xcb7ecb7eu || __vmins2(v, 0x8eff8effu) != 0x8eff8effu;
+  return __vmaxu2(v, 0xc2fec2feu) != 0xc2fec2feu || __vmins2(v, 0x867f867fu) != 0x867f867fu;
 }
 
 // A thread's two rows of a unit that holds scales i4_dequant does not cover, in place of what the MMAs summed: the product q s

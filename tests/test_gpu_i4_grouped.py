@@ -14,30 +14,30 @@ def _bf16(a):
 
 
 def test_dequantisation_by_one_rounding():
-    """fma(n 2^-129, s 2^100, -s 2^-26) and fma(n 2^-133, s 2^104, -s 2^-26), rounded once, are 2^-29 bf16(q s) for every nibble
+    """fma(n 2^-129, s 2^117, -s 2^-9) and fma(n 2^-133, s 2^121, -s 2^-9), rounded once, are 2^-12 bf16(q s) for every nibble
     and every scale mantissa, over the exponents the kernel claims; the bit patterns are the numbers the kernel takes them for."""
     n = np.arange(16)
     for shift, power in ((0, -133), (4, -129)):
         bits = (n << shift).astype(np.uint32) << 16
         assert np.array_equal(bits.view(np.float32).astype(np.float64), np.ldexp(n.astype(np.float64), power))
     mant = 1 + np.arange(128) / 128
-    for e in (-97, -40, -9, 0, 23):
+    for e in (-114, -40, -9, 0, 6):
         s = np.ldexp(mant, e)[:, None] * np.array([[1.0], [-1.0]])[:, None]
-        want = np.ldexp(_bf16((n - 8) * s), -29)
-        for power, scale in ((-129, 100), (-133, 104)):
-            got = _bf16(np.ldexp(n * 1.0, power) * np.ldexp(s, scale) - np.ldexp(s, -26))
+        want = np.ldexp(_bf16((n - 8) * s), -12)
+        for power, scale in ((-129, 117), (-133, 121)):
+            got = _bf16(np.ldexp(n * 1.0, power) * np.ldexp(s, scale) - np.ldexp(s, -9))
             assert np.array_equal(got, want)
 
 
 def test_range_of_scales_by_their_bits():
-    """The kernel's two integer tests over every bf16 bit pattern: the exact one says whether s = 0 or 2^-97 <= |s| < 2^24, and what
+    """The kernel's two integer tests over every bf16 bit pattern: the exact one says whether s = 0 or 2^-114 <= |s| < 2^7, and what
     the quick one lets by (exponent bits 01......) is inside."""
     bits = np.arange(1 << 16, dtype=np.uint32)
     with np.errstate(invalid="ignore"):
         s = np.abs((bits << 16).view(np.float32).astype(np.float64))
-    inside = (s == 0) | ((s >= 2.0 ** -97) & (s < 2.0 ** 24))
+    inside = (s == 0) | ((s >= 2.0 ** -114) & (s < 2.0 ** 7))
     v = ((bits | 0x8000) - 1).astype(np.uint16)
-    outside = (v > np.uint16(0xcb7e)) | (v.view(np.int16) < np.array(0x8eff, dtype=np.uint16).view(np.int16))
+    outside = (v > np.uint16(0xc2fe)) | (v.view(np.int16) < np.array(0x867f, dtype=np.uint16).view(np.int16))
     assert np.array_equal(~outside, inside)
     assert inside[((bits ^ 0x2000) & 0x6000) == 0].all()
 
@@ -83,14 +83,15 @@ def test_grouped_experts_at_tile_edges(cuda, monkeypatch, hidden, inter, counts,
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("gate,up,down", [
-    (0, 40, -105),      # every up scale above the range of the one-instruction dequantisation, every down scale below it
-    (0, -108, 60),      # and the other way round
-    (-100, 100, 0),
-    (None, None, None),  # single blocks of 32 columns in a few rows: 2^25, 2^-99 and 2^-133 (the smallest there is), and zeros
+@pytest.mark.parametrize("gate,up,down,act", [
+    (0, 40, -112, 0),      # every up scale above the range of the one-instruction dequantisation, every down scale below it
+    (0, -112, 60, 0),      # and the other way round
+    (-112, 112, 0, 0),
+    (None, None, None, 0),  # single blocks of 32 columns in a few rows: 2^25, 2^-116 and 2^-133 (the smallest there is), and zeros
+    (0, 0, 0, -59),        # activations whose results lie near the smallest normal numbers
 ])
-def test_grouped_experts_take_any_scale(cuda, monkeypatch, gate, up, down):
-    """Scales outside 2^-97 .. 2^24: the tcgen05 kernel against the mma.sync kernel, which multiplies every nibble by its scale.
+def test_grouped_experts_take_any_scale(cuda, monkeypatch, gate, up, down, act):
+    """Scales outside 2^-114 .. 2^7: the tcgen05 kernel against the mma.sync kernel, which multiplies every nibble by its scale.
     The same weights, fp32 sums in another order: tolerance as above."""
     from blok_b200 import lib, synth
     hidden, inter, N = 1024, 512, 75
@@ -99,14 +100,14 @@ def test_grouped_experts_take_any_scale(cuda, monkeypatch, gate, up, down):
         s = w[k].float() * 8
         if octaves is None:
             s[:, 5::64, 3] = 2.0 ** 25
-            s[:, 6::64, 7] = 2.0 ** -99
+            s[:, 6::64, 7] = 2.0 ** -116
             s[:, 7::64, :] = 2.0 ** -133
             s[:, 8::64, ::2] = 0.0
         else:
             s = s * 2.0 ** octaves
         w[k] = s.bfloat16()
     layer = lib.MoeLayer(w, max_tokens=16)
-    x = synth.activations(N, hidden, cuda, 6)
+    x = (synth.activations(N, hidden, cuda, 6).float() * 2.0 ** act).bfloat16()
     e = torch.tensor([3] * 66 + [4, 4, 4] + [90] * 6, dtype=torch.int32, device=cuda)
     out = {}
     for impl in ("mma", "tc", ""):
