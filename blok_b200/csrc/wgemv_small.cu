@@ -13,14 +13,14 @@
 // 16 k-blocks (the scales of a chunk are staged whole, as in moe_fused.cu).  Tasks are dealt out in contiguous ranges, so
 // a CTA restages activations about twice per launch.  launch_wgemm_experts (wgemm.cu) sends it products of few assignments.
 //
-// Measured at T = 64 (284 groups, 7.05 GB of expert weights): gate/up and down together about 1.6 ms (4.4 TB/s); with
-// every lane loading a token's operands (24 of 32 read the zero block) 1.75 ms; with a run-time token loop and pointer
-// arithmetic per access 2.07 ms (164 warp instructions per 1 KB ring step against 116).
-// Six tokens per pass instead of four: slower (the larger stages cost more than the second pass of the few groups of
-// five or six).  The ring kept running across chunk boundaries (a second scale stage, the next chunk's scales riding
-// with its first weight request): no faster (1.95 ms against 1.93 ms per layer pass; the other fifteen warps of the SM
-// cover a warp's drained ring).  Four warps sharing a row-block with K split between them (better locality in HBM, but
-// the CTA meets at two barriers per 14-step task): slower still (layer 2.70 ms against 2.36 ms then).
+// Measured, 384 experts of 7168 x 2048, plan and both products (24.8 MB a group): 8 groups of one token 64 us, 16 101 us (3.9 TB/s),
+// 37 groups 205 us (4.5 TB/s).  What its form was found with, layers of 64 tokens in 284 groups that the tcgen05 kernel takes today
+// (gate/up and down together): 1.6 ms; with every lane loading a token's operands (24 of 32 read the zero block) 1.75 ms; with a
+// run-time token loop and pointer arithmetic per access 2.07 ms (164 warp instructions per 1 KB ring step against 116).
+// Six tokens per pass instead of four: slower (the larger stages cost more than a second pass).  The ring kept running across chunk
+// boundaries (a second scale stage, the next chunk's scales riding with its first weight request): no faster (the other fifteen warps
+// of the SM cover a warp's drained ring).  Four warps sharing a row-block with K split between them (better locality in HBM, but the
+// CTA meets at two barriers per 14-step task): slower still.
 #include "i4_imma.cuh"
 #include "wgemm.h"
 
