@@ -53,11 +53,11 @@ __device__ __forceinline__ void i4_dequant(uint32_t w, const I4Scale &s, uint32_
 
 // A unit is (tile of up to 64 tokens of one expert) x 256 weight rows (128 gate + 128 up rows of the same indices, or 256
 // rows of the down projection); a persistent CTA per SM walks the units, and every role runs ahead across their boundaries:
-//   warps 0, 1    MMAs of row block 0 and 1: 4 K = 16 steps per 64-column piece
+//   warps 0, 1    MMAs of row block 0 and 1: 8 K = 16 steps per piece of 128 columns
 //   warp 2        activations by TMA: four slots of 128 columns
 //   warp 3        weights and scales by TMA: four stages of 256 rows x 128 bytes, scales 32 bytes (512 columns) per row
 //   warps 4..7    epilogue of the unit before (two accumulator buffers)
-//   warps 8..     unpack: sets of eight warps take the pieces in turn; a thread owns one row of one block and writes
+//   warps 8..     unpack: two sets of eight warps, one for each piece of a stage; a thread owns one row of one block and writes
 //                 the piece's exact bf16(q * s) to TENSOR MEMORY as the MMA's A operand
 // The activations arrive in sorted order with the columns of every packed word in the order 0 4 1 5 2 6 3 7 (the order the
 // unpacking leaves the weights in): i4_rows_kernel lays them out once per launch, the SwiGLU epilogue writes them so.
@@ -115,8 +115,8 @@ __device__ __forceinline__ bool i4_outside(uint32_t s2) {
 }
 
 // A thread's two rows of a unit that holds scales i4_dequant does not cover, in place of what the MMAs summed: the product q s
-// rounded to bf16 as the reference has it, whatever the scale, in plain loops (a millisecond or two).  row: weight row inside the
-// expert; col: output column.
+// rounded to bf16 as the reference has it, whatever the scale, in plain loops (7168 columns: 0.23 ms a token of the tile; four tokens
+// per look at a weight took as long for 64 and longer for one).  row: weight row inside the expert; col: output column.
 template <bool SWIGLU>
 __device__ __noinline__ void i4_plain_rows(const I4Args &a, int tile, int row, int col) {
   const int p0 = a.tile_start[tile], cnt = a.tile_count[tile], blocks = a.K / 32;
@@ -157,10 +157,10 @@ __device__ __forceinline__ uint32_t i4_lds32(uint32_t addr) {
   return v;
 }
 
-// Bounded wait; a warp that has time (SLEEP ns between tries) leaves the issue slots to the unpacking warps.
+// Bounded wait, longer than a unit of i4_plain_rows (64 tokens of 32,768 columns: 70 ms); a warp that has time (SLEEP ns between tries) leaves the issue slots to the unpacking warps.
 template <int SLEEP>
 __device__ __forceinline__ bool i4_wait(uint32_t mbar, uint32_t parity) {
-  for (unsigned it = 0; it < (1u << 21); ++it) {
+  for (unsigned it = 0; it < (1u << 23); ++it) {
     uint32_t ok;
     asm volatile(
         "{\n\t"
