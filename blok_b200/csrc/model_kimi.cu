@@ -377,6 +377,11 @@ static int check(blok_model *m, blok_stream_t stream) {
       message = "layer " + std::to_string(l) + ": " + blok_last_error();
     }
   }
+  if (first == BLOK_OK) {  // the dense layers' and the head's products have no handle
+    unsigned err = 0;
+    if (int rc = wgemm_stream_take_error(&err)) return rc;
+    BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");
+  }
   if (first == BLOK_OK && K->comm) return blok_comm_check(K->comm);
   if (first != BLOK_OK) set_error("%s", message.c_str());
   return first;

@@ -1204,6 +1204,8 @@ int stack_check(blok_model *, blok_stream_t stream) {
   unsigned err = 0;
   TRY(gemm_tma_take_error(&err));
   BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");
+  TRY(wgemm_stream_take_error(&err));
+  BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");
   TRY(prompt_attn_take_error(&err));
   BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "attention over a prompt gave up on a barrier");
   TRY(mla_attend_tc_take_error(&err));

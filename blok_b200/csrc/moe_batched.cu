@@ -277,9 +277,11 @@ extern "C" int blok_moe_batched(blok_moe_layer_t *L, const blok_bf16_t *x, int T
   if (w.shared_inter > 0) {
     WgArgs s = r;
     s.w_a = w.shared_gate; s.w_b = w.shared_up; s.R = w.shared_inter; s.out_bf16 = L->b_smid; s.out_f32 = nullptr;
+    s.weights_early = true;  // the router's launch and others are in between
     if ((rc = launch_wgemm(WG_BF16_SWIGLU, s, tt, stream))) return rc;
     WgArgs d = r;
     d.w_a = w.shared_down; d.x = L->b_smid; d.K = w.shared_inter; d.R = w.hidden; d.out_bf16 = L->b_sout; d.out_f32 = nullptr;
+    d.weights_early = true;
     if ((rc = launch_wgemm(WG_BF16_PLAIN, d, tt, stream))) return rc;
     shared = L->b_sout;
   }

@@ -37,6 +37,13 @@ struct WgArgs {
   size_t splitk_bytes = 0;
   // INT4 modes, where the host knows only a bound of them: the assignments that pick the kernel, a device word (launch_wgemm_experts)
   const int *total = nullptr;
+  // The weight-streaming kernel only.  A second matrix over the same rows (w_b, R2 rows, bf16 to out2): its tiles follow the first's,
+  // its partial sums the first's R columns.  max_splits: a bound of the K split (0: none).  keep_sums: fp32 sums in
+  // splitk_ws also where K is not split.  weights_early: the weights may be fetched
+  // before the kernels in front of this launch have finished (the caller has launched one since they were written, in this call).
+  int R2 = 0, max_splits = 0;
+  uint16_t *out2 = nullptr;
+  bool keep_sums = false, weights_early = false;
   unsigned *err = nullptr;  // set to 1 when a tcgen05 kernel's wait gives up: a word of the handle the launch is for
 };
 
@@ -60,11 +67,15 @@ int wgemm_tma_split(int mode, int K, int R, int rows);  // the same for the TMA-
 bool wgemv_small_supports(int mode, const WgArgs &args, int max_rows);
 int launch_wgemv_small(int mode, const WgArgs &args, cudaStream_t stream);
 
-// The bf16 modes over 1..kWgStreamTokens rows of x (identity tiles): every warp streams its 16 weight rows through a
-// cp.async ring, the activations are double buffered (wgemm_stream.cu).  *splits > 1: K was split and the partial sums
-// wait in args.splitk_ws for wgemm_splitk_reduce_kernel (launch_wgemm runs it).  wgemm_stream_split: the split of a shape.
+// The bf16 modes over 1..kWgStreamTokens rows of x (identity tiles): the weights streamed by TMA as the M side of tcgen05.mma
+// (wgemm_stream.cu).  *splits > 1: K was split and the partial sums wait in args.splitk_ws for wgemm_splitk_reduce_kernel
+// (launch_wgemm runs it) or a kernel that adds them itself.  wgemm_stream_split, _pair_split: the split of a shape at most.
+// wgemm_stream_supports: what launch_wgemm hands to it; the launch itself takes any K % 8 == 0 and R.
 bool wgemm_stream_supports(int mode, const WgArgs &args);
 int wgemm_stream_split(int mode, int K, int R);
+int wgemm_stream_pair_split(int K, int R, int R2);
+// *out becomes non-zero if a CTA without an error word of its own has given up since the last call (the flag is cleared).
+int wgemm_stream_take_error(unsigned *out);
 // The reduction behind a K-split launch: adds the nz partial sums in split order and applies the epilogue.
 int launch_wgemm_splitk_reduce(int mode, const WgArgs &args, int nz, cudaStream_t stream);
 int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t stream);

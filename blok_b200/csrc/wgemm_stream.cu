@@ -1,156 +1,199 @@
-// bf16 weights against 9 to 64 rows of activations (a decode step of 9..64 sequences, a rank's share of a small batch):
+// bf16 weights against up to 64 rows of activations (a decode step, a rank's share of a small batch):
 //   out[token, row] = sum_c W[row, c] * x[token, c]          (matvec_bf16_k, src/kimi_exec.cu:272-284, per token)
 // with the SwiGLU front half as an option (gate and up rows of the same index, :255, :674-686).
 //
-// At these counts the product is bound by the weight stream, not by the tensor cores, and the kernel is built as the
-// batch-1 kernels are: every warp owns 16 weight rows (8 gate + 8 up rows) and pulls them through a private ring of
-// 1 KB steps (16 rows x 64 bytes, cp.async, kStDepth steps in flight), so that a CTA of eight warps keeps 64 KB of
-// requests outstanding whatever the consumers do.  The activations of the CTA's K-range reach shared memory in chunks
-// of 256 columns, double buffered with cp.async (the copy of chunk c + 1 rides with the weight requests of chunk c),
-// one CTA-wide barrier per chunk.  A ring step feeds two mma.sync.m16n8k16 per group of 8 tokens.
+// At these counts the product is the weight stream.  The weights are the M = 128 side of tcgen05.mma and the tokens its N side
+// (16 to 64), so a weight byte passes shared memory once whatever the token count and no warp spends an instruction on it: one
+// thread brings 128 rows x 64 columns of weights and the same columns of the tokens per step by TMA, four to six steps in flight
+// (about 100 KB per CTA, two CTAs per SM), one lane issues the MMAs, four warps store the accumulator (a lane owns a weight row).
 //
-// The mma.sync GEMM (wgemm.cu) loads a k-block's weights right before it uses them and stages the activations
-// between two barriers; over one tile of tokens it reached 0.7-0.8 TB/s (the four projections of the attention block
-// at 32 sequences: 76 us each; the vocabulary projection ran 8 rows at a time, four passes over its 2.35 GB).
+// Matrices with few rows are split over K (blockIdx.y) so that about two CTAs per SM run; the partial sums go to the caller's
+// scratch in the layout of wgemm_splitk_reduce_kernel, which adds them in split order.
 //
-// Matrices with few rows are split over K (blockIdx.y) so that about two CTAs per SM run; the partial sums go to the
-// caller's scratch in the layout of wgemm_splitk_reduce_kernel, which adds them in split order.
+// The mma.sync form before it (a warp's cp.async ring of its own 16 rows, tokens staged in shared memory) read eight times the
+// weights' bytes from shared memory at 64 tokens.  The three projections of the attention block, 202 MB, with what stands between
+// them (mla_heads.cu), us: one sequence 92 -> 67 (mat-vec kernels), 33 sequences 209 -> 140, a 64-token chunk 200 -> 126.
+//
+// The kernel becomes resident while the kernel before it runs (launch_pdl), and where the caller knows that the weights have long
+// been there (WgArgs::weights_early) the first steps' weights are on their way before the wait: the ramp of the stream is hidden
+// behind the kernel before.  Shared memory keeps it at two CTAs per SM, so early CTAs spread evenly.
+//
+// Every wait is bounded; a CTA that gives up sets the error word, stores NaN, waits for its copies and frees its tensor memory.
 #include <algorithm>
 
-#include "bf16_mma.cuh"
+#include "gemm_tma.h"
+#include "tc_pipe.cuh"
 #include "wgemm.h"
 
 namespace blok {
 
-constexpr int kStDepth = 8;                      // ring steps of 1 KB in flight per warp
-constexpr int kStChunk = 256;                    // columns of the activations per buffer (8 ring steps)
-constexpr int kStPitch = kStChunk * 2 + 64;      // bytes per staged token row: two rows of a quarter-warp hit all banks
-constexpr int kStMaxWarps = 8;
+constexpr int kStRows = 128;     // weight rows per CTA (SwiGLU: 64 gate + 64 up rows)
+constexpr int kStCols = 64;      // columns per step
+constexpr int kStMinSteps = 8;   // a split of K has at least so many
+constexpr int kStThreads = 192;  // warps 0..3: stores, 4: copies, 5: MMA
+constexpr int kStMaxStages = 6;
+constexpr int kStTmemCols = 64;
+constexpr uint32_t kStWBytes = kStRows * kStCols * 2;
 
-__device__ __forceinline__ void st_cp16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ uint4 st_lds128(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-  return v;
-}
+__device__ unsigned g_wgemm_stream_error = 0;
 
-// NT = groups of 8 tokens the launch covers (n_rows <= 8 NT).  blockDim.x / 32 warps, each 16 rows (SWIGLU: 8 + 8).
-template <int NT, bool SWIGLU>
-__global__ void __launch_bounds__(kStMaxWarps * 32) wgemm_stream_kernel(const WgArgs a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int T = a.n_rows, K = a.K;
-  const int row0 = (blockIdx.x * nwarps + warp) * (SWIGLU ? 8 : 16);
-  const size_t wrow = (size_t)K / 8;  // uint4 per weight row
-  // whole 256-column chunks of K per split
-  const int chunks = K / kStChunk, nz = gridDim.y, kz = blockIdx.y;
-  const int c_begin = (int)((long)kz * chunks / nz), c_end = (int)((long)(kz + 1) * chunks / nz);
-  const int nchunks = c_end - c_begin, nsteps = nchunks * (kStChunk / 32);
-  const uint4 *w_lo = reinterpret_cast<const uint4 *>(a.w_a) + (size_t)(row0 + g) * wrow + (size_t)c_begin * (kStChunk / 8) + t;
-  const uint4 *w_hi = SWIGLU ? reinterpret_cast<const uint4 *>(a.w_b) + (size_t)(row0 + g) * wrow + (size_t)c_begin * (kStChunk / 8) + t
-                             : w_lo + 8 * wrow;
+struct StArgs {
+  float *part;         // fp32 [split][token][ld] where K is split, else NULL
+  uint16_t *out_bf16;  // [token][R]
+  float *out_f32;
+  uint16_t *out2;      // the second matrix's output (tiles from tiles1 on), bf16; its partial sums follow the first's R columns
+  int T, N, K, R, R2, tiles1, ld, stages, early;
+  unsigned *err;
+};
+
+template <bool SWIGLU>
+__global__ void __launch_bounds__(kStThreads) wgemm_stream_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mwa,
+                                                                  const __grid_constant__ CUtensorMap mwb, const StArgs a) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long s_bar[2 * kStMaxStages + 1];
+  __shared__ uint32_t s_tmem;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // Without early weights the kernels behind this one must not start before everything before it has finished: they may fetch
+  // theirs before their own wait, on the word of a caller who knows this launch to be in between.
+  if (!a.early) pdl_wait();
   pdl_trigger();
-  pdl_wait();
-  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
-  constexpr uint32_t kBufBytes = 8 * NT * kStPitch;
-  const uint32_t ring_lane = sbase + 2 * kBufBytes + (uint32_t)warp * (kStDepth * 1024) + (uint32_t)lane * 16;
-
-  // the CTA's copy of chunk c of the activations (tokens past the last repeat it: their columns of D are never stored)
-  auto stage = [&](int c, int buf) {
-    const uint32_t dst = sbase + (uint32_t)buf * kBufBytes;
-    for (int u = tid; u < 8 * NT * 32; u += blockDim.x) {
-      const int tok = u >> 5, unit = u & 31;
-      const int src_tok = tok < T ? tok : T - 1;
-      st_cp16(dst + (uint32_t)(tok * kStPitch + unit * 16), a.x + (size_t)src_tok * K + (size_t)c * kStChunk + unit * 8);
+  const uint32_t sbase = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023u) & ~1023u;
+  const uint32_t full = (uint32_t)__cvta_generic_to_shared(&s_bar[0]), empty = full + 8 * kStMaxStages, done = full + 16 * kStMaxStages;
+  const int S = a.stages;
+  if (tid == 0) {
+    for (int s = 0; s < S; ++s) {
+      tp_mbar_init(full + 8 * s, 1);
+      tp_mbar_init(empty + 8 * s, 1);
     }
-  };
+    tp_mbar_init(done, 1);
+    tp_mbar_init_fence();
+  }
+  if (warp == 0) tp_tmem_alloc((uint32_t)__cvta_generic_to_shared(&s_tmem), kStTmemCols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = s_tmem;
+  const bool second = !SWIGLU && (int)blockIdx.x >= a.tiles1;
+  const int tile = second ? (int)blockIdx.x - a.tiles1 : (int)blockIdx.x;
+  const int all_steps = (a.K + kStCols - 1) / kStCols, nz = (int)gridDim.y, z = (int)blockIdx.y;
+  const int first = all_steps * z / nz, nsteps = all_steps * (z + 1) / nz - first;
+  const uint32_t xbytes = (uint32_t)a.N * (kStCols * 2), stage = kStWBytes + xbytes;
+  bool failed = false;
 
-  float acc[NT][4];
-#pragma unroll
-  for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-
-  if (nchunks > 0) stage(c_begin, 0);
-  const uint4 *wl = w_lo, *wh = w_hi;  // next ring step to request
-  {
-    uint32_t slot = ring_lane;
-#pragma unroll
-    for (int s = 0; s < kStDepth; ++s) {
-      if (s < nsteps) {
-        st_cp16(slot, wl);
-        st_cp16(slot + 512, wh);
-        wl += 4;
-        wh += 4;
-        slot += 1024;
+  if (warp == 4) {
+    if (lane == 0) {
+      auto weights = [&](int c, uint32_t dst, uint32_t bar) {
+        const int k = (first + c) * kStCols;
+        tp_expect_tx(bar, stage);
+        if (SWIGLU) {
+          tp_load_2d(dst, &mwa, k, tile * (kStRows / 2), bar);
+          tp_load_2d(dst + kStWBytes / 2, &mwb, k, tile * (kStRows / 2), bar);
+        } else {
+          tp_load_2d(dst, second ? &mwb : &mwa, k, tile * kStRows, bar);
+        }
+      };
+      const int pre = min(S, nsteps);
+      for (int c = 0; c < pre; ++c) weights(c, sbase + (uint32_t)c * stage, full + 8 * c);
+      pdl_wait();
+      asm volatile("fence.proxy.async;" ::: "memory");  // the tokens' rows were written by ordinary stores
+      for (int c = 0; c < pre; ++c) tp_load_2d(sbase + (uint32_t)c * stage + kStWBytes, &mx, (first + c) * kStCols, 0, full + 8 * c);
+      int issued = pre, s = 0;
+      uint32_t turn = 0;
+      for (int c = pre; c < nsteps; ++c) {
+        if (!tp_wait(empty + 8 * s, turn)) {
+          failed = true;
+          break;
+        }
+        weights(c, sbase + (uint32_t)s * stage, full + 8 * s);
+        tp_load_2d(sbase + (uint32_t)s * stage + kStWBytes, &mx, (first + c) * kStCols, 0, full + 8 * s);
+        issued = c + 1;
+        if (++s == S) s = 0, turn ^= 1;
       }
-      asm volatile("cp.async.commit_group;" ::: "memory");
+      // no copy may be in flight when the CTA leaves; the MMA lane has seen all of them unless a wait gave up
+      for (int c = max(0, issued - S); c < issued; ++c) tp_wait(full + 8 * (c % S), (uint32_t)((c / S) & 1));
+    }
+  } else if (warp == 5) {
+    // the whole warp walks the steps, so that addresses and descriptors stay warp-uniform; one lane issues
+    const bool issues = tp_elect();
+    const uint32_t idesc = tp_idesc_bf16(a.N);
+    int s = 0;
+    uint32_t turn = 0;
+    for (int c = 0; c < nsteps; ++c) {
+      if (!__all_sync(0xffffffffu, tp_wait(full + 8 * s, turn))) {
+        failed = true;
+        break;
+      }
+      tc_fence_after();
+      const uint64_t ad = tp_desc_k_sw128(sbase + (uint32_t)s * stage), bd = tp_desc_k_sw128(sbase + (uint32_t)s * stage + kStWBytes);
+      if (issues) {
+#pragma unroll
+        for (int k = 0; k < kStCols / 16; ++k) tp_mma(tmem, ad + (uint64_t)(2 * k), bd + (uint64_t)(2 * k), idesc, (c | k) ? 1u : 0u);
+        tp_commit(empty + 8 * s);
+        if (c == nsteps - 1) tp_commit(done);
+      }
+      if (++s == S) s = 0, turn ^= 1;
+    }
+  } else {
+    pdl_wait();  // the kernel before may still read what this one writes
+    failed = __any_sync(0xffffffffu, !tp_wait(done, 0));
+    tc_fence_after();
+    const int r = 32 * warp + lane;
+    const uint32_t at = tmem + ((uint32_t)(32 * warp) << 16);
+    const int R = second ? a.R2 : a.R;
+    if (SWIGLU && !a.part) {
+      // the up half hands its sums over through the ring's memory (every copy into it has been consumed)
+      float *up = reinterpret_cast<float *>(smem_raw);
+      const int row = tile * (kStRows / 2) + (r & 63);
+      for (int half = 1; half >= 0; --half) {
+        if ((warp >> 1) == half) {
+          for (int c0 = 0; c0 < a.N; c0 += 16) {
+            uint32_t v[16];
+            tmem_ld16(at + c0, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const int tok = c0 + j;
+              float f = __uint_as_float(failed ? 0x7fc00000u : v[j]);
+              if (half == 1) {
+                up[tok * 64 + (r & 63)] = f;
+              } else if (tok < a.T && row < R) {
+                f = round_bf16(f);
+                const float m = round_bf16(f / (1.0f + expf(-f))) * round_bf16(up[tok * 64 + r]);
+                a.out_bf16[(size_t)tok * R + row] = f32_to_bf16_bits(round_bf16(m));
+              }
+            }
+          }
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+      }
+    } else {
+      const int row = SWIGLU ? tile * (kStRows / 2) + (r & 63) : tile * kStRows + r;
+      const int col = SWIGLU && r >= 64 ? R + row : (second ? a.R + row : row);  // of the partial sums
+      const size_t ld = a.part ? a.ld : R;
+      float *f32 = a.part ? a.part + (size_t)z * a.T * ld + col : (a.out_f32 && !second ? a.out_f32 + row : nullptr);
+      uint16_t *b16 = (second ? a.out2 : a.out_bf16) + row;
+#pragma unroll 1
+      for (int c0 = 0; c0 < a.T; c0 += 16) {
+        uint32_t v[16];
+        tmem_ld16(at + c0, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (row < R && c0 + j < a.T) {
+            const float f = __uint_as_float(failed ? 0x7fc00000u : v[j]);
+            if (f32) f32[j * ld] = f;
+            else b16[j * ld] = f32_to_bf16_bits(f);
+          }
+        }
+        if (f32) f32 += 16 * ld;
+        else b16 += 16 * ld;
+      }
     }
   }
-  uint32_t slot = ring_lane;
-  int requested = kStDepth;
-  // this lane's activation fragment of token g of group 0, k-step 0 of a buffer
-  const uint32_t xlane = sbase + (uint32_t)(g * kStPitch + t * 16);
-  for (int ci = 0; ci < nchunks; ++ci) {
-    // the chunk's activations were committed at least kStDepth groups ago (with the first ring step of the chunk
-    // before): complete for this thread after the wait, for the CTA after the barrier, which also frees the other buffer
-    asm volatile("cp.async.wait_group %0;" ::"n"(kStDepth - 1) : "memory");
-    __syncthreads();
-    if (ci + 1 < nchunks) stage(c_begin + ci + 1, (ci + 1) & 1);
-    uint32_t xs = xlane + (uint32_t)(ci & 1) * kBufBytes;
-#pragma unroll 2
-    for (int s = 0; s < kStChunk / 32; ++s) {
-      asm volatile("cp.async.wait_group %0;" ::"n"(kStDepth - 1) : "memory");
-      const uint4 wlv = st_lds128(slot), whv = st_lds128(slot + 512);
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const uint4 xb = st_lds128(xs + (uint32_t)(nt * 8 * kStPitch));
-        mma_bf16_16816(acc[nt], wlv.x, whv.x, wlv.y, whv.y, xb.x, xb.y);
-        mma_bf16_16816(acc[nt], wlv.z, whv.z, wlv.w, whv.w, xb.z, xb.w);
-      }
-      if (requested < nsteps) {  // the slot just read takes the step a ring's depth ahead
-        st_cp16(slot, wl);
-        st_cp16(slot + 512, wh);
-        wl += 4;
-        wh += 4;
-      }
-      ++requested;
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      slot += 1024;
-      if (slot == ring_lane + kStDepth * 1024) slot = ring_lane;
-      xs += 64;
-    }
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-
-  // ---- epilogue: the lane holds rows g (acc[.][0..1]) and g + 8 / up row g (acc[.][2..3]) of tokens 8 nt + 2 t, + 1 ----
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int tok = 8 * nt + 2 * t + c;
-      if (tok >= T) continue;
-      if (nz > 1) {  // [split][token][gate rows, then up rows | rows], as wgemm_splitk_reduce_kernel reads it
-        const int cols = SWIGLU ? 2 * a.R : a.R;
-        float *ps = a.splitk_ws + ((size_t)kz * T + tok) * cols;
-        ps[row0 + g] = acc[nt][c];
-        ps[(SWIGLU ? a.R : 8) + row0 + g] = acc[nt][2 + c];
-        continue;
-      }
-      const size_t o = (size_t)tok * a.R + row0 + g;
-      if (SWIGLU) {
-        const float gv = round_bf16(acc[nt][c]), uv = round_bf16(acc[nt][2 + c]);
-        a.out_bf16[o] = f32_to_bf16_bits(round_bf16(round_bf16(gv / (1.0f + expf(-gv))) * uv));
-      } else if (a.out_f32) {
-        a.out_f32[o] = acc[nt][c];
-        a.out_f32[o + 8] = acc[nt][2 + c];
-      } else {
-        a.out_bf16[o] = f32_to_bf16_bits(acc[nt][c]);
-        a.out_bf16[o + 8] = f32_to_bf16_bits(acc[nt][2 + c]);
-      }
-    }
-  }
+  if (failed) atomicExch(a.err ? a.err : &g_wgemm_stream_error, 1u);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tp_tmem_free(tmem, kStTmemCols);
 }
 
 static bool st_aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -158,50 +201,68 @@ static bool st_aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p)
 bool wgemm_stream_supports(int mode, const WgArgs &a) {
   if (mode != WG_BF16_PLAIN && mode != WG_BF16_SWIGLU) return false;
   if (!a.identity_tiles || a.n_rows < 1 || a.n_rows > kWgStreamTokens || a.x_index || a.out_index) return false;
-  if (a.K % kStChunk || a.R % (mode == WG_BF16_SWIGLU ? 8 : 16)) return false;
+  if (a.K % 256 || a.R % (mode == WG_BF16_SWIGLU ? 8 : 16)) return false;
   return st_aligned16(a.w_a) && st_aligned16(a.x) && (mode != WG_BF16_SWIGLU || st_aligned16(a.w_b));
 }
 
-// Warps per CTA (a CTA of w warps covers 16 w rows, or 8 w gate + 8 w up rows): as many as divide the rows while the
-// K-split can still give every SM a CTA; a wide CTA shares one copy of the activations among more weight rows.
-static int st_warps(int mode, int K, int R) {
-  const int blocks = R / (mode == WG_BF16_SWIGLU ? 8 : 16);  // one per warp
-  const int max_split = std::max(1, K / kStChunk / 2);
-  for (int w = kStMaxWarps; w > 1; w >>= 1)
-    if (blocks % w == 0 && (long)(blocks / w) * max_split >= sm_count()) return w;
-  for (int w = kStMaxWarps; w > 1; w >>= 1)
-    if (blocks % w == 0) return w;
-  return 1;
+static int st_tiles(int mode, int R) {
+  const int per = mode == WG_BF16_SWIGLU ? kStRows / 2 : kStRows;
+  return (R + per - 1) / per;
 }
-
+// About two CTAs per SM, at least kStMinSteps steps each.
+static int st_split(int K, int tiles) { return std::max(1, std::min((K + kStCols - 1) / kStCols / kStMinSteps, 2 * sm_count() / tiles)); }
 int wgemm_stream_split(int mode, int K, int R) {
-  if ((mode != WG_BF16_PLAIN && mode != WG_BF16_SWIGLU) || K % kStChunk || R % (mode == WG_BF16_SWIGLU ? 8 : 16)) return 1;
-  const int ctas = R / (mode == WG_BF16_SWIGLU ? 8 : 16) / st_warps(mode, K, R), chunks = K / kStChunk;
-  return std::max(1, std::min(chunks / 2, 2 * sm_count() / ctas));  // at least two chunks per split
+  if (mode != WG_BF16_PLAIN && mode != WG_BF16_SWIGLU) return 1;
+  return st_split(K, st_tiles(mode, R));
 }
+int wgemm_stream_pair_split(int K, int R, int R2) { return st_split(K, st_tiles(WG_BF16_PLAIN, R) + st_tiles(WG_BF16_PLAIN, R2)); }
 
 // Launches the kernel; *splits = the K-split it used (> 1: the partial sums wait in args.splitk_ws for the reduce kernel).
 int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t stream) {
   const bool swiglu = mode == WG_BF16_SWIGLU;
-  const int warps = st_warps(mode, args.K, args.R);
-  int nz = wgemm_stream_split(mode, args.K, args.R);
-  const size_t per_split = (size_t)args.n_rows * (swiglu ? 2 * args.R : args.R) * sizeof(float);
-  if (nz > 1 && (!args.splitk_ws || args.splitk_bytes < per_split * nz)) nz = args.splitk_ws ? (int)std::max<size_t>(1, args.splitk_bytes / per_split) : 1;
-  const int nt = args.n_rows <= 16 ? 2 : (args.n_rows <= 32 ? 4 : 8);
-  const size_t smem = (size_t)2 * 8 * nt * kStPitch + (size_t)warps * kStDepth * 1024;
-  const dim3 grid(args.R / (swiglu ? 8 : 16) / warps, nz);
-#define BLOK_ST_LAUNCH(NT, SW)                                                                                          \
-  {                                                                                                                     \
-    BLOK_CUDA(cudaFuncSetAttribute(wgemm_stream_kernel<NT, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    if (int rc = launch_pdl("wgemm_stream_kernel", wgemm_stream_kernel<NT, SW>, grid, warps * 32, smem, stream, args)) return rc; \
-  }
-  if (swiglu) {
-    if (nt == 2) BLOK_ST_LAUNCH(2, true) else if (nt == 4) BLOK_ST_LAUNCH(4, true) else BLOK_ST_LAUNCH(8, true)
+  BLOK_REQUIRE(args.K % 8 == 0 && args.R >= 1 && args.n_rows >= 1 && args.n_rows <= kWgStreamTokens && !(swiglu && args.R2), BLOK_ERR_SHAPE,
+               "streaming product: %d rows x %d columns over %d tokens", args.R, args.K, args.n_rows);
+  StArgs a;
+  a.tiles1 = st_tiles(mode, args.R);
+  const int tiles = a.tiles1 + (args.R2 ? st_tiles(mode, args.R2) : 0);
+  a.ld = swiglu ? 2 * args.R : args.R + args.R2;
+  const size_t per_split = (size_t)args.n_rows * a.ld * sizeof(float);
+  const size_t room = args.splitk_ws ? args.splitk_bytes / per_split : 0;
+  BLOK_REQUIRE(!args.keep_sums || room >= 1, BLOK_ERR_WORKSPACE, "streaming product: no room for the sums");
+  const int nz = (int)std::max<size_t>(1, std::min<size_t>(args.max_splits > 0 ? std::min(args.max_splits, st_split(args.K, tiles)) : st_split(args.K, tiles), room));
+  a.part = nz > 1 || args.keep_sums ? args.splitk_ws : nullptr;
+  a.out_bf16 = args.out_bf16;
+  a.out_f32 = args.out_f32;
+  a.out2 = args.out2;
+  a.T = args.n_rows;
+  a.N = (args.n_rows + 15) / 16 * 16;
+  a.K = args.K;
+  a.R = args.R;
+  a.R2 = args.R2;
+  a.early = args.weights_early;
+  a.err = args.err;
+  // as many steps as two CTAs per SM leave room for: 108, 100, 88 and 96 KB
+  a.stages = a.N == 16 ? 6 : (a.N == 32 ? 5 : 4);
+  const int smem = a.stages * (int)(kStWBytes + a.N * kStCols * 2) + 1024;
+  CUtensorMap mx, mwa, mwb;
+  int rc;
+  if ((rc = gemm_operand_map(args.x, args.n_rows, args.K, args.K, a.N, &mx))) return rc;
+  if ((rc = gemm_operand_map(args.w_a, args.R, args.K, args.K, swiglu ? kStRows / 2 : kStRows, &mwa))) return rc;
+  if (swiglu || args.R2) {
+    if ((rc = gemm_operand_map(args.w_b, swiglu ? args.R : args.R2, args.K, args.K, swiglu ? kStRows / 2 : kStRows, &mwb))) return rc;
   } else {
-    if (nt == 2) BLOK_ST_LAUNCH(2, false) else if (nt == 4) BLOK_ST_LAUNCH(4, false) else BLOK_ST_LAUNCH(8, false)
+    mwb = mwa;
   }
-#undef BLOK_ST_LAUNCH
+  auto kernel = swiglu ? wgemm_stream_kernel<true> : wgemm_stream_kernel<false>;
+  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   *splits = nz;
+  return launch_pdl("wgemm_stream_kernel", kernel, dim3(tiles, nz), kStThreads, (size_t)smem, stream, mx, mwa, mwb, a);
+}
+
+int wgemm_stream_take_error(unsigned *out) {
+  unsigned zero = 0;
+  BLOK_CUDA(cudaMemcpyFromSymbol(out, g_wgemm_stream_error, sizeof(unsigned)));
+  if (*out) BLOK_CUDA(cudaMemcpyToSymbol(g_wgemm_stream_error, &zero, sizeof(unsigned)));
   return BLOK_OK;
 }
 
