@@ -7,9 +7,9 @@
 // All 64 heads of a sequence share one latent row per token: per token 1,152 bytes are read once from HBM and feed
 // 64 x (576 + 512) multiply-adds.  A CTA owns one (sequence, token range) and walks it in tiles of 64 tokens:
 //
-//   S [heads x tokens]     = Q [heads x 576] . C^T          36 MMAs M64 N64 K16: A = Q (shared memory, K-major, no
-//                                                            swizzle), B = the tile read K-major; two partial sums
-//   P = exp2(S * scale * log2 e - m)                         one head row per thread (tcgen05.ld), bf16, to shared memory
+//   S [heads x tokens]     = Q [heads x 576] . C^T          36 MMAs M64 N64 K16: A = Q (shared memory, as a tile lies),
+//                                                            B = the tile read K-major; two partial sums
+//   P = exp2(S * scale * log2 e - m)                         a quad of lanes per pair of head rows, bf16, to shared memory
 //   O^T [latent x heads]  += C^T [latent x tokens] . P^T     16 MMAs M128 N64 K16: A = the SAME tile bytes read MN-major
 //                                                            (four blocks of 128 latent columns), B = P (K-major)
 //
@@ -17,6 +17,12 @@
 // cp.async.bulk.tensor (no multicast; the tensor map covers this GPU's cache only).  Read K-major a chunk is 64 columns
 // of a [64 tokens x 576] operand; read MN-major the same bytes are 64 rows of a [512 x 64 tokens] operand: one copy from
 // HBM serves both products, and no thread touches the bytes on their way.
+//
+// What bounds it: the chain load -> scores -> softmax -> P.C of a tile with two tile buffers beside Q, and in it the fixed cost of
+// an MMA of this size, about 40 cycles for the warp that issues it (43 with N = 32, 61 with N = 64; so tiles of 32 tokens in four
+// buffers are slower, 131 against 126 us below).  So two warps issue; a tile is loaded and released in two halves, its scores
+// begin with the first; whichever product can go next goes; and all 32 lanes of a softmax warp work.  A tile took 2.83 us, takes
+// 1.92 (8 x 32,768 tokens: the block 147 -> 126 us; 33 paged sequences 140 -> 122; HBM's share of an SM would be 1.67 us).
 //
 // The running maximum is kept lazily: a head's reference m changes only when a tile's maximum exceeds it by more than
 // 40 (natural units); then all four consumer warps rescale O^T in tensor memory.  exp(s - m) stays far inside fp32 and
@@ -28,7 +34,7 @@
 // the tile's release frees both.  seq_len then holds positions (the token itself included).  Any number of heads in groups of 64 (blockIdx.z).
 //
 // Warps: 0..3 consumers (the M = 64 accumulator S keeps head rows 16 w .. 16 w + 15 in lanes 0..15 of warp w's quarter of
-// tensor memory; all four own the 128 lanes of O^T), 4: the TMA producer, 5: one lane issues the MMAs.  Every mbarrier
+// tensor memory; all four own the 128 lanes of O^T), 4: the TMA producer, 5 and 6: one lane of each issues the MMAs.  Every mbarrier
 // wait is bounded; on a timeout the CTA records an error, still releases its tensor memory and returns.
 #include <cuda.h>
 
@@ -43,14 +49,15 @@ constexpr int kTaHeads = 64, kTaD = 576, kTaDV = 512;
 constexpr int kTaTile = 64;                              // tokens per tile
 constexpr int kTaChunks = kTaD / 64;                     // 128-byte column chunks of a cache row
 constexpr int kTaChunkBytes = kTaTile * 128;             // 8,192
+constexpr int kTaHalfChunks = 4;                         // chunks of a tile's first half (latent columns 0..255)
 constexpr int kTaTileBytes = kTaChunks * kTaChunkBytes;  // 73,728
-constexpr int kTaLbo = kTaHeads * 16;                    // Q and P (64 rows, no swizzle): bytes between 16-byte column groups
+constexpr int kTaLbo = kTaHeads * 16;                    // P (64 rows, no swizzle): bytes between 16-byte column groups
 constexpr int kTaSbo = 128;                              // ... and between 8-row groups
-constexpr int kTaQBytes = (kTaD / 8) * kTaLbo;           // 73,728
+constexpr int kTaQBytes = kTaChunks * kTaHeads * 128;    // 73,728
 constexpr int kTaPBytes = (kTaTile / 8) * kTaLbo;        // P: [64 heads x 64 tokens] bf16, K (token) major
 constexpr int kTaSmemBytes = 2 * kTaTileBytes + kTaQBytes + kTaPBytes + 1024;  // + 1024: the tiles start on a 1,024-byte boundary
 constexpr int kTaConsumers = 128;
-constexpr int kTaThreads = kTaConsumers + 64;
+constexpr int kTaThreads = kTaConsumers + 96;
 constexpr int kTaTmemCols = 512;                         // S: 2 buffers x 2 partial sums x 64 columns, O^T: 4 x 64 columns
 constexpr int kTaColO = 256;
 constexpr unsigned kTaSpinLimit = 1u << 21;
@@ -70,11 +77,20 @@ __device__ __forceinline__ uint32_t ta_pack_bf16x2(float lo, float hi) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
-__device__ __forceinline__ void ta_cp16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool ta_elect() {
+  uint32_t is;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(is));
+  return is != 0;
 }
 // Shared-memory matrix descriptors (start address, leading and stride byte offsets in 16-byte units, version 1).
-// No swizzle, K-major (Q and P): leading = between 16-byte column groups along K, stride = between 8-row groups.
+// No swizzle, K-major (P): leading = between 16-byte column groups along K, stride = between 8-row groups.
 __device__ __forceinline__ uint64_t ta_desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
 }
@@ -159,37 +175,22 @@ __device__ __forceinline__ bool ta_consumers_sync(bool failed) {
 
 size_t mla_attend_tc_smem_bytes() { return kTaSmemBytes; }
 
-// grid = (splits, B); arguments as mla_attend_kernel, plus the tensor map of the cache ([rows, 576] bf16, boxes of
-// 64 rows x 64 columns, 128-byte swizzle).  PAGED: page_rows is a multiple of the 64-token tile.
+// grid = (splits, B); arguments as mla_attend_kernel, plus the tensor maps of the cache ([rows, 576] bf16) and of the queries
+// ([B x heads, 576]), both in boxes of 64 rows x 64 columns, 128-byte swizzle.  PAGED: page_rows is a multiple of the 64-token tile.
 template <bool PAGED, bool FINE>
 __global__ void __launch_bounds__(kTaThreads, 1)
-    mla_attend_tc_kernel(const __grid_constant__ CUtensorMap tmap, const uint16_t *q, const uint16_t *cache,
+    mla_attend_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap qmap, const uint16_t *cache,
                          long ctx_stride, const int *seq_len, float scale, float *__restrict__ part_o,
                          float *__restrict__ part_ml, const int *block_table, const int *slot_of,
                          int table_stride, int page_rows, long long *__restrict__ trace, int heads) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(8) unsigned long long s_bar[11];
+  __shared__ __align__(8) unsigned long long s_bar[16];
   __shared__ uint32_t s_tmem;
   __shared__ float s_alpha[kTaHeads];
   __shared__ int s_need[2][4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int split = blockIdx.x, splits = gridDim.x, b = blockIdx.y;
   pdl_trigger();
-  pdl_wait();
-  const int seq = FINE ? min(seq_len[b] + 1, table_stride * page_rows) : seq_len[b];
-  const int ntiles = (seq + kTaTile - 1) / kTaTile;
-  const int per = (ntiles + splits - 1) / splits;
-  const int ts = split * per, te = min(ntiles, ts + per);
-  const int h0 = blockIdx.z * kTaHeads, nh = min(kTaHeads, heads - h0);  // this CTA's heads
-  float *my_ml = part_ml + (((size_t)b * splits + split) * heads + h0) * 2;
-  if (ts >= te) {  // nothing to do for this split: mark it empty for the merge
-    if (tid < nh) {
-      my_ml[tid * 2] = -INFINITY;
-      my_ml[tid * 2 + 1] = 0.f;
-    }
-    return;
-  }
-  const int nt = te - ts;
   // the swizzle is a function of the address: the tiles start on a 1,024-byte boundary
   const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
   const uint32_t sT = (raw + 1023u) & ~1023u;
@@ -198,20 +199,15 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   const uint32_t sP = sQ + kTaQBytes;
   unsigned char *Pp = smem + 2 * kTaTileBytes + kTaQBytes;
   const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(&s_bar[0]);
-  // tma[buf]: the tile's bytes have landed; fix[buf]: the rows past the sequence's end are zeroed (its last tile only);
-  // sfull[buf]: the S MMAs' commit; sfree[buf]: the softmax warps have read S; pfull: they have written P;
-  // empty[buf]: the commit behind the tile's P.C MMAs (tile buffer and P are free)
-  const uint32_t bar_tma = bar0, bar_fix = bar0 + 16, bar_sfull = bar0 + 32, bar_sfree = bar0 + 48, bar_pfull = bar0 + 64,
-                 bar_empty = bar0 + 72;
+  // A tile comes and goes in two halves: chunks 0..3 (latent columns 0..255) and 4..8.  tma[buf][half]: the half's bytes have
+  // landed; fix[buf]: the rows past the sequence's end are zeroed (its last tile only); sfull[buf]: the S MMAs' commits, one of each
+  // MMA warp; sfree[buf]: the softmax warps have read S; pfull: they have written P; empty[buf][half]: the commit behind the P.C
+  // MMAs of the half's columns (the half of the buffer is free, with both halves P too); q: the queries have landed
+  const uint32_t bar_tma = bar0, bar_fix = bar0 + 32, bar_sfull = bar0 + 48, bar_sfree = bar0 + 64, bar_empty = bar0 + 80, bar_pfull = bar0 + 112,
+                 bar_q = bar0 + 120;
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_tma + 8 * i) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_fix + 8 * i) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_sfull + 8 * i) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(bar_sfree + 8 * i) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_empty + 8 * i) : "memory");
-    }
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(bar_pfull) : "memory");
+    for (int i = 0; i < 16; ++i)  // sfree and pfull: an arrival per softmax warp
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0 + 8 * i), "r"(i == 8 || i == 9 || i == 14 ? 4 : (i == 6 || i == 7 ? 2 : 1)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -220,21 +216,22 @@ __global__ void __launch_bounds__(kTaThreads, 1)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  {
-    // Q [64 heads x 576] into 8 x 16-byte core matrices: consecutive threads take consecutive heads of one column group
-    const uint16_t *qb = q + ((size_t)b * heads + h0) * kTaD;
-    for (int u = tid; u < kTaHeads * (kTaD / 8); u += kTaThreads) {
-      const int kg = u >> 6, h = u & 63;
-      ta_cp16(sQ + kg * kTaLbo + h * 16, qb + (size_t)min(h, nh - 1) * kTaD + kg * 8);  // rows past the last head repeat it
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_tmem;
+  pdl_wait();
+  const int seq = FINE ? min(seq_len[b] + 1, table_stride * page_rows) : seq_len[b];
+  const int ntiles = (seq + kTaTile - 1) / kTaTile;
+  const int per = (ntiles + splits - 1) / splits;
+  const int ts = split * per, te = min(ntiles, ts + per);
+  const int h0 = blockIdx.z * kTaHeads, nh = min(kTaHeads, heads - h0);  // this CTA's heads
+  float *my_ml = part_ml + (((size_t)b * splits + split) * heads + h0) * 2;
+  const int nt = max(0, te - ts);
+  if (nt == 0 && tid < nh) {  // nothing to do for this split: mark it empty for the merge
+    my_ml[tid * 2] = -INFINITY;
+    my_ml[tid * 2 + 1] = 0.f;
+  }
   bool failed = false;
   // diagnostics (trace != NULL): CTA (0, 0) stamps, per tile, [0] buffer free, [1] TMA issued, [2] S issued, [3] S seen
   // by the softmax warps, [4] P handed over, [5] P.C issued, [8] S read, [9] softmax done (nanoseconds)
@@ -249,27 +246,42 @@ __global__ void __launch_bounds__(kTaThreads, 1)
   const int last_partial = (seq % kTaTile != 0 && te == ntiles) ? nt - 1 : -1;
 
   if (warp == 4) {
-    // ---- the producer: nine boxes per tile, all counted on the buffer's mbarrier ----
+    // ---- the producer: nine boxes for the queries, nine per tile, counted on the mbarrier of their half ----
     const uint16_t *cache_b = PAGED ? cache : cache + (size_t)b * ctx_stride * kTaD;
     const int *table_b = PAGED ? block_table + (size_t)(slot_of ? slot_of[b] : b) * table_stride : nullptr;
     auto first_row = [&](int tok0) -> long {  // the tensor map's row of the tile's first token
       if (PAGED) return (long)table_b[tok0 / page_rows] * page_rows + tok0 % page_rows;
       return (long)b * ctx_stride + tok0;
     };
+    if (nt > 0 && lane == 0) {
+      ta_expect_tx(bar_q, kTaQBytes);
+#pragma unroll 1
+      for (int c = 0; c < kTaChunks; ++c) ta_tma_2d(sQ + c * kTaChunkBytes, &qmap, 64 * c, b * heads + h0, bar_q);
+    }
+    int issued = 0;
     for (int n = 0; n < nt; ++n) {
       const int buf = n & 1;
-      if (n >= 2 && !ta_wait(bar_empty + 8 * buf, (uint32_t)(((n >> 1) - 1) & 1), 1u)) {
-        failed = true;
-        break;
-      }
-      const int tok0 = (ts + n) * kTaTile;
+      const int tok0 = (ts + n) * kTaTile, row = (int)first_row(tok0);
       const uint32_t dst = sT + buf * kTaTileBytes;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        // (the second half also holds FINE's low parts, which both warps read; it comes after the first)
+        if (n >= 2 && !__all_sync(0xffffffffu, ta_wait(bar_empty + 16 * buf + 8 * half, (uint32_t)(((n >> 1) - 1) & 1), 1u))) {
+          failed = true;
+          break;
+        }
+        if (lane == 0) {
+          if (half == 0) stamp(n, 0);
+          const int c0 = half ? kTaHalfChunks : 0, c1 = half ? kTaChunks : kTaHalfChunks;
+          const uint32_t bar = bar_tma + 16 * buf + 8 * half;
+          ta_expect_tx(bar, (uint32_t)(c1 - c0) * kTaChunkBytes);
+#pragma unroll 1
+          for (int c = c0; c < c1; ++c) ta_tma_2d(dst + c * kTaChunkBytes, &tmap, 64 * c, row, bar);
+        }
+        issued = 2 * n + half + 1;
+      }
+      if (failed) break;
       if (lane == 0) {
-        stamp(n, 0);
-        const int row = (int)first_row(tok0);
-        ta_expect_tx(bar_tma + 8 * buf, kTaTileBytes);
-#pragma unroll
-        for (int c = 0; c < kTaChunks; ++c) ta_tma_2d(dst + c * kTaChunkBytes, &tmap, 64 * c, row, bar_tma + 8 * buf);
         if (n + 2 < nt) {
           // The buffer's next tile starts its way from HBM to L2 now: by the time the buffer is free again (this
           // tile's two products later) the copy finds it there, and HBM has been busy meanwhile.  A tile is contiguous
@@ -284,7 +296,8 @@ __global__ void __launch_bounds__(kTaThreads, 1)
       if (n == last_partial) {
         // rows past the sequence's end hold whatever the allocation holds: zero them (their P is zero, and zero times
         // a stray NaN would not be), whole 128-byte rows, which the swizzle only permutes within
-        if (!ta_wait(bar_tma + 8 * buf, (uint32_t)((n >> 1) & 1), 10u)) {
+        const uint32_t turn = (uint32_t)((n >> 1) & 1);
+        if (!__all_sync(0xffffffffu, ta_wait(bar_tma + 16 * buf, turn, 10u) && ta_wait(bar_tma + 16 * buf + 8, turn, 10u))) {
           failed = true;
           break;
         }
@@ -299,120 +312,126 @@ __global__ void __launch_bounds__(kTaThreads, 1)
         if (lane == 0) ta_arrive(bar_fix + 8 * buf);
       }
     }
-  } else if (warp == 5) {
-    if (lane == 0) {
-      // ---- the MMA thread ----
-      const uint32_t idesc_128 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTaTile >> 3) << 17) | ((128u >> 4) << 24);
-      const uint32_t idesc_s = (idesc_128 & ~(31u << 24)) | ((64u >> 4) << 24);  // M = 64
-      const uint32_t idesc_pv = idesc_128 | (1u << 15);                          // A (the tile) MN-major
-      const uint64_t q_desc = ta_desc_plain(sQ, kTaLbo, kTaSbo);
-      const uint64_t p_desc = ta_desc_plain(sP, kTaLbo, kTaSbo);
-      auto tile_ready = [&](int n, bool block) -> bool {  // the tile has landed (and, if it is the partial one, is zeroed)
-        const int buf = n & 1;
-        if (block) {
-          if (!ta_wait(bar_tma + 8 * buf, (uint32_t)((n >> 1) & 1), 2u)) return false;
-          if (n == last_partial && !ta_wait(bar_fix + 8 * buf, 0u, 4u)) return false;
-          return true;
-        }
-        return ta_test(bar_tma + 8 * buf, (uint32_t)((n >> 1) & 1)) && (n != last_partial || ta_test(bar_fix + 8 * buf, 0u));
-      };
-      auto issue_s = [&](int n) {
-        const int buf = n & 1;
-        // every descriptor below is a per-tile base plus a constant: the start address sits in the low bits (16-byte units,
-        // 14 bits for 256 KB) and no offset used here carries out of them
-        const uint64_t c_desc = ta_desc_sw128(sT + buf * kTaTileBytes, 16, 1024);
+    // no copy may be in flight when the CTA leaves; the MMA warp has seen all of them unless a wait gave up
+    for (int i = max(0, issued - 4); i < issued; ++i) ta_wait(bar_tma + 16 * ((i >> 1) & 1) + 8 * (i & 1), (uint32_t)((i >> 2) & 1), 11u);
+  } else if (warp >= 5) {
+    // ---- two MMA warps: the fixed cost of an MMA of this size is larger than its work, and two warps share it.  All lanes walk,
+    // so that addresses and descriptors stay warp-uniform; one issues ----
+    const int wi = warp - 5;
+    const bool issues = ta_elect();
+    const uint32_t idesc_128 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTaTile >> 3) << 17) | ((128u >> 4) << 24);
+    const uint32_t idesc_s = (idesc_128 & ~(31u << 24)) | ((64u >> 4) << 24);  // M = 64
+    const uint32_t idesc_pv = idesc_128 | (1u << 15);                          // A (the tile) MN-major
+    const uint64_t q_desc = ta_desc_sw128(sQ, 16, 1024);
+    const uint64_t p_desc = ta_desc_plain(sP, kTaLbo, kTaSbo);
+    // every descriptor below is a per-tile base plus a constant: the start address sits in the low bits (16-byte units,
+    // 14 bits for 256 KB) and no offset used here carries out of them
+    auto issue_s = [&](int n, int half) {
+      const int buf = n & 1;
+      const uint64_t c_desc = ta_desc_sw128(sT + buf * kTaTileBytes, 16, 1024);
+      if (issues) {
+        const int c0 = half ? kTaHalfChunks : 0, c1 = half ? kTaChunks : kTaHalfChunks;
+#pragma unroll 1
+        for (int c = c0; c < c1; ++c) {
 #pragma unroll
-        for (int c = 0; c < kTaChunks; ++c) {
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4) {
-            const int kk = 4 * c + k4;  // K step of 16 columns: two column groups of Q, 32 bytes of the chunk's rows
-            // even and odd K steps accumulate into two partial sums: an MMA of this size is shorter than the wait for the
-            // previous one's accumulator, and two chains halve that wait
-            ta_mma(tmem + 128 * buf + 64 * (kk & 1), q_desc + (uint64_t)(kk * ((2 * kTaLbo) >> 4)),
-                   c_desc + (uint64_t)((c * kTaChunkBytes + k4 * 32) >> 4), idesc_s, kk > 1 ? 1u : 0u);
+          for (int k4 = 0; k4 < 4; k4 += 2) {
+            // K step of 16 columns: 32 bytes of the chunk's rows, of the queries and of the tile alike.  The first warp takes the
+            // even steps, the second one the odd ones, each into a partial sum of its own
+            const uint64_t at = (uint64_t)((c * kTaChunkBytes + (k4 + wi) * 32) >> 4);
+            ta_mma(tmem + 128 * buf + 64 * wi, q_desc + at, c_desc + at, idesc_s, c > 0 || k4 > 0 ? 1u : 0u);
           }
         }
-        ta_commit(bar_sfull + 8 * buf);
-        stamp(n, 2);
-      };
-      auto issue_pv = [&](int n) {
-        const int buf = n & 1;
-        const uint64_t a_desc = ta_desc_sw128(sT + buf * kTaTileBytes, kTaChunkBytes, 1024);
-        // block j: latent columns [128 j, +128) = chunks 2 j and 2 j + 1; a K step is 16 tokens = two 8-row groups.  The
-        // four blocks take turns: consecutive MMAs then accumulate into different columns of tensor memory and do not
-        // wait for one another.
-#pragma unroll
-        for (int kk = 0; kk < kTaTile / 16; ++kk) {
-#pragma unroll
-          for (int j = 0; j < kTaDV / 128; ++j)
-            ta_mma(tmem + kTaColO + 64 * j, a_desc + (uint64_t)((2 * j * kTaChunkBytes + kk * 2048) >> 4),
-                   p_desc + (uint64_t)(kk * ((2 * kTaLbo) >> 4)), idesc_pv, (n > 0 || kk > 0) ? 1u : 0u);
+        if (half) {
+          ta_commit(bar_sfull + 8 * buf);
+          if (wi == 0) stamp(n, 2);
         }
-        if (FINE) {  // the low parts, in the tile's last chunk
-          const uint64_t lo_desc = ta_desc_plain(sT + buf * kTaTileBytes + (kTaChunks - 1) * kTaChunkBytes, kTaLbo, kTaSbo);
+      }
+      __syncwarp();
+    };
+    // Latent blocks of 128 columns = chunks 2 j and 2 j + 1, two of them to a warp; a K step is 16 tokens = two 8-row groups.  The
+    // blocks take turns, so that consecutive MMAs accumulate into different columns of tensor memory.
+    auto issue_pv = [&](int n) {
+      const int buf = n & 1;
+      const uint64_t a_desc = ta_desc_sw128(sT + buf * kTaTileBytes + 4 * wi * kTaChunkBytes, kTaChunkBytes, 1024);
+      const uint64_t lo_desc = ta_desc_plain(sT + buf * kTaTileBytes + (kTaChunks - 1) * kTaChunkBytes, kTaLbo, kTaSbo);  // FINE: the low parts
+      if (issues) {
+#pragma unroll
+        for (int part = 0; part < (FINE ? 2 : 1); ++part) {
 #pragma unroll
           for (int kk = 0; kk < kTaTile / 16; ++kk) {
 #pragma unroll
-            for (int j = 0; j < kTaDV / 128; ++j)
-              ta_mma(tmem + kTaColO + 64 * j, a_desc + (uint64_t)((2 * j * kTaChunkBytes + kk * 2048) >> 4),
-                     lo_desc + (uint64_t)(kk * ((2 * kTaLbo) >> 4)), idesc_pv, 1u);
+            for (int j = 0; j < 2; ++j)
+              ta_mma(tmem + kTaColO + 128 * wi + 64 * j, a_desc + (uint64_t)((2 * j * kTaChunkBytes + kk * 2048) >> 4),
+                     (part ? lo_desc : p_desc) + (uint64_t)(kk * ((2 * kTaLbo) >> 4)), idesc_pv, (n > 0 || kk > 0 || part > 0) ? 1u : 0u);
           }
         }
-        ta_commit(bar_empty + 8 * buf);
-        stamp(n, 5);
-      };
-      if (!tile_ready(0, true)) failed = true;
-      if (!failed) {
-        tc_fence_after();
-        issue_s(0);
+        ta_commit(bar_empty + 16 * buf + 8 * wi);
+        if (wi == 0) stamp(n, 5);
       }
-      for (int n = 0; n < nt && !failed; ++n) {
-        // the next tile's scores go first when that tile has landed already: they run under this tile's softmax
-        bool early = false;
-        const int nn = n + 1, nb = nn & 1;
-        if (nn < nt && tile_ready(nn, false) && (nn < 2 || ta_test(bar_sfree + 8 * nb, (uint32_t)(((nn >> 1) - 1) & 1)))) {
-          tc_fence_after();
-          issue_s(nn);
-          early = true;
-        }
-        if (!ta_wait(bar_pfull, (uint32_t)(n & 1), 3u)) {
-          failed = true;
-          break;
-        }
+      __syncwarp();
+    };
+    // true where the whole warp sees the phase complete
+    auto seen = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, ta_test(bar, parity)); };
+    if (nt > 0 && !__all_sync(0xffffffffu, ta_wait(bar_q, 0u, 4u))) failed = true;
+    // Whatever can go next goes: a tile's P.C product frees its buffer and comes first; the scores of the tile behind it are
+    // issued half by half as they land, so that neither product waits long behind the other in the tensor pipe.
+    int sn = 0, sh = 0, pn = 0;  // next scores (tile, half), next P.C product
+    unsigned idle = 0;
+    while (pn < nt && !failed) {
+      bool went = false;
+      if (pn < sn && seen(bar_pfull, (uint32_t)(pn & 1))) {
         tc_fence_after();
-        issue_pv(n);
-        if (!early && nn < nt) {
-          if (!tile_ready(nn, true) || (nn >= 2 && !ta_wait(bar_sfree + 8 * nb, (uint32_t)(((nn >> 1) - 1) & 1), 5u))) {
-            failed = true;
-            break;
-          }
+        issue_pv(pn++);
+        went = true;
+      } else if (sn < nt && sn <= pn + 1) {
+        const int sb = sn & 1;
+        const uint32_t turn = (uint32_t)((sn >> 1) & 1);
+        bool ready = seen(bar_tma + 16 * sb + 8 * sh, turn);
+        if (ready && sn == last_partial) ready = seen(bar_fix + 8 * sb, 0u);
+        if (ready && sh == 0 && sn >= 2) ready = seen(bar_sfree + 8 * sb, turn ^ 1);
+        if (ready) {
           tc_fence_after();
-          issue_s(nn);
+          issue_s(sn, sh);
+          if (sh) ++sn;
+          sh ^= 1;
+          went = true;
+        }
+      }
+      if (went) {
+        idle = 0;
+      } else if (++idle > 64) {
+        __nanosleep(32);
+        if (idle > kTaSpinLimit) {
+          if (lane == 0) atomicExch(&g_mla_tc_error, 3u);
+          failed = true;
         }
       }
     }
-  } else {
-    // ---- consumers: lanes 0..15 of warp w hold head rows 16 w .. 16 w + 15 of S ----
+  } else if (nt > 0) {
+    // ---- consumers: warp w holds head rows 16 w .. 16 w + 15 of S; a lane has rows r0 and r0 + 8, 16 tokens of each ----
     const float sl2 = scale * 1.4426950408889634f;
-    float m_ref = -INFINITY, l = 0.f;
-    const bool row_ok = lane < 16;
-    const int head = 16 * warp + lane;
+    const int r0 = 16 * warp + (lane >> 2), tq = 2 * (lane & 3);
+    float m_ref[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+    auto done_with = [&](int n, unsigned code) -> bool {  // both warps' P.C products of tile n
+      const uint32_t turn = (uint32_t)((n >> 1) & 1);
+      return ta_wait(bar_empty + 16 * (n & 1), turn, code) && ta_wait(bar_empty + 16 * (n & 1) + 8, turn, code);
+    };
     for (int n = 0; n < nt; ++n) {
       const int buf = n & 1;
-      uint32_t pk[kTaTile / 2], pl[FINE ? kTaTile / 2 : 1];
+      uint32_t pk[2][8], pl[2][FINE ? 8 : 1];  // [row][column group of 8 tokens]: this lane's pair of tokens
       bool need = false;
-      if (!failed && !ta_wait(bar_sfull + 8 * buf, (uint32_t)((n >> 1) & 1), 6u)) failed = true;
+      if (!failed && !__all_sync(0xffffffffu, ta_wait(bar_sfull + 8 * buf, (uint32_t)((n >> 1) & 1), 6u))) failed = true;
       if (!failed) {
         if (tid == 0) stamp(n, 3);
         tc_fence_after();
-        uint32_t r[kTaTile];
+        uint32_t r[32];
         {
-          uint32_t r2[kTaTile];  // the two partial sums of the score product
-          tmem_ld64(tmem + ((uint32_t)(32 * warp) << 16) + 128 * buf, r);
-          tmem_ld64(tmem + ((uint32_t)(32 * warp) << 16) + 128 * buf + 64, r2);
+          uint32_t r2[32];  // the two partial sums of the score product
+          tmem_ld_rows16(tmem + ((uint32_t)(32 * warp) << 16) + 128 * buf, r);
+          tmem_ld_rows16(tmem + ((uint32_t)(32 * warp) << 16) + 128 * buf + 64, r2);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < kTaTile; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
         }
         tc_fence_before();
         __syncwarp();
@@ -421,53 +440,49 @@ __global__ void __launch_bounds__(kTaThreads, 1)
         const int tok0 = (ts + n) * kTaTile;
         if (tok0 + kTaTile > seq) {  // the sequence's last tile: tokens past the end take no weight
 #pragma unroll
-          for (int j = 0; j < kTaTile; ++j)
-            if (tok0 + j >= seq) r[j] = 0xff800000u;
+          for (int j = 0; j < 32; ++j)
+            if (tok0 + 8 * (j >> 2) + tq + (j & 1) >= seq) r[j] = 0xff800000u;
         }
-        float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < kTaTile; j += 4) {
-          mx0 = fmaxf(mx0, __uint_as_float(r[j]));
-          mx1 = fmaxf(mx1, __uint_as_float(r[j + 1]));
-          mx2 = fmaxf(mx2, __uint_as_float(r[j + 2]));
-          mx3 = fmaxf(mx3, __uint_as_float(r[j + 3]));
-        }
-        const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * sl2;  // the scale is positive
-        float alpha = 1.f;
-        if (n == 0) {
-          m_ref = mx;  // the split's first tile holds at least one token
-        } else if (mx > m_ref + kTaLazy) {
-          alpha = exp2f(m_ref - mx);
-          m_ref = mx;
-          need = row_ok;
-        }
-        if (row_ok) s_alpha[head] = alpha;
-        const float nm = -m_ref;
-        float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
+        for (int y = 0; y < 2; ++y) {
+          float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < kTaTile; j += 4) {
-          // the probabilities enter the second product rounded to bf16 (as the reference rounds them, :466); the
-          // normaliser sums the same rounded values (FINE: two parts, and the normaliser sums the weights themselves)
-          const float p0 = ta_ex2(fmaf(__uint_as_float(r[j]), sl2, nm)), p1 = ta_ex2(fmaf(__uint_as_float(r[j + 1]), sl2, nm));
-          const float p2 = ta_ex2(fmaf(__uint_as_float(r[j + 2]), sl2, nm)), p3 = ta_ex2(fmaf(__uint_as_float(r[j + 3]), sl2, nm));
-          const uint32_t pa = ta_pack_bf16x2(p0, p1), pb = ta_pack_bf16x2(p2, p3);
-          if (FINE) {
-            sum0 += p0;
-            sum1 += p1;
-            sum2 += p2;
-            sum3 += p3;
-            pl[FINE ? j >> 1 : 0] = ta_pack_bf16x2(p0 - __uint_as_float(pa << 16), p1 - __uint_as_float(pa & 0xffff0000u));
-            pl[FINE ? (j >> 1) + 1 : 0] = ta_pack_bf16x2(p2 - __uint_as_float(pb << 16), p3 - __uint_as_float(pb & 0xffff0000u));
-          } else {
-            sum0 += __uint_as_float(pa << 16);
-            sum1 += __uint_as_float(pa & 0xffff0000u);
-            sum2 += __uint_as_float(pb << 16);
-            sum3 += __uint_as_float(pb & 0xffff0000u);
+          for (int i = 0; i < 8; ++i) {
+            mx0 = fmaxf(mx0, __uint_as_float(r[4 * i + 2 * y]));
+            mx1 = fmaxf(mx1, __uint_as_float(r[4 * i + 2 * y + 1]));
           }
-          pk[j >> 1] = pa;
-          pk[(j >> 1) + 1] = pb;
+          float mx = fmaxf(mx0, mx1);
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2)) * sl2;  // the scale is positive
+          float alpha = 1.f;
+          if (n == 0) {
+            m_ref[y] = mx;  // the split's first tile holds at least one token
+          } else if (mx > m_ref[y] + kTaLazy) {
+            alpha = exp2f(m_ref[y] - mx);
+            m_ref[y] = mx;
+            need = true;
+          }
+          if ((lane & 3) == 0) s_alpha[r0 + 8 * y] = alpha;
+          const float nm = -m_ref[y];
+          float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            // the probabilities enter the second product rounded to bf16 (as the reference rounds them, :466); the
+            // normaliser sums the same rounded values (FINE: two parts, and the normaliser sums the weights themselves)
+            const float p0 = ta_ex2(fmaf(__uint_as_float(r[4 * i + 2 * y]), sl2, nm)), p1 = ta_ex2(fmaf(__uint_as_float(r[4 * i + 2 * y + 1]), sl2, nm));
+            const uint32_t pa = ta_pack_bf16x2(p0, p1);
+            if (FINE) {
+              sum0 += p0;
+              sum1 += p1;
+              pl[y][FINE ? i : 0] = ta_pack_bf16x2(p0 - __uint_as_float(pa << 16), p1 - __uint_as_float(pa & 0xffff0000u));
+            } else {
+              sum0 += __uint_as_float(pa << 16);
+              sum1 += __uint_as_float(pa & 0xffff0000u);
+            }
+            pk[y][i] = pa;
+          }
+          l[y] = l[y] * alpha + (sum0 + sum1);
         }
-        l = l * alpha + ((sum0 + sum1) + (sum2 + sum3));
         if (tid == 0) stamp(n, 9);
       }
       need = __any_sync(0xffffffffu, need);
@@ -479,7 +494,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
       if (s_need[buf][0] | s_need[buf][1] | s_need[buf][2] | s_need[buf][3]) {
         // a head's reference maximum moved (never in tile 0): every lane of O^T scales its 4 x 64 head columns, once the
         // previous tile's MMAs have finished with them
-        if (!ta_wait(bar_empty + 8 * ((n - 1) & 1), (uint32_t)(((n - 1) >> 1) & 1), 7u)) failed = true;
+        if (!__all_sync(0xffffffffu, done_with(n - 1, 7u))) failed = true;
         if (!failed) {
           tc_fence_after();
 #pragma unroll 1
@@ -501,19 +516,17 @@ __global__ void __launch_bounds__(kTaThreads, 1)
         }
       }
       if (!failed) {
-        if (n > 0 && !ta_wait(bar_empty + 8 * ((n - 1) & 1), (uint32_t)(((n - 1) >> 1) & 1), 8u)) {
+        if (n > 0 && !__all_sync(0xffffffffu, done_with(n - 1, 8u))) {
           failed = true;  // reaches the others at the next tile's barrier
         } else {
-          if (row_ok) {
+          unsigned char *lo = smem + (size_t)buf * kTaTileBytes + (kTaChunks - 1) * kTaChunkBytes;
 #pragma unroll
-            for (int kg = 0; kg < kTaTile / 8; ++kg)
-              *reinterpret_cast<uint4 *>(Pp + kg * kTaLbo + head * 16) = make_uint4(pk[4 * kg], pk[4 * kg + 1], pk[4 * kg + 2], pk[4 * kg + 3]);
-            if (FINE) {
-              unsigned char *lo = smem + (size_t)buf * kTaTileBytes + (kTaChunks - 1) * kTaChunkBytes;
+          for (int y = 0; y < 2; ++y) {
 #pragma unroll
-              for (int kg = 0; kg < kTaTile / 8; ++kg)
-                *reinterpret_cast<uint4 *>(lo + kg * kTaLbo + head * 16) =
-                    make_uint4(pl[FINE ? 4 * kg : 0], pl[FINE ? 4 * kg + 1 : 0], pl[FINE ? 4 * kg + 2 : 0], pl[FINE ? 4 * kg + 3 : 0]);
+            for (int kg = 0; kg < kTaTile / 8; ++kg) {
+              const int at = kg * kTaLbo + (r0 + 8 * y) * 16 + 2 * tq;
+              *reinterpret_cast<uint32_t *>(Pp + at) = pk[y][kg];
+              if (FINE) *reinterpret_cast<uint32_t *>(lo + at) = pl[y][FINE ? kg : 0];
             }
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -524,7 +537,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
       }
     }
     // ---- the split's partial result: O^T [latent lane x head column] -> part_o [head][512], (m, sum) per head ----
-    if (!failed && !ta_wait(bar_empty + 8 * ((nt - 1) & 1), (uint32_t)(((nt - 1) >> 1) & 1), 9u)) failed = true;
+    if (!failed && !__all_sync(0xffffffffu, done_with(nt - 1, 9u))) failed = true;
     failed = ta_consumers_sync(failed);
     if (!failed) {
       tc_fence_after();
@@ -541,9 +554,15 @@ __global__ void __launch_bounds__(kTaThreads, 1)
             if (32 * half + c < nh) po[(size_t)(32 * half + c) * kTaDV + 128 * j + 32 * warp + lane] = __uint_as_float(o[c]);
         }
       }
-      if (row_ok && head < nh) {
-        my_ml[head * 2] = m_ref * 0.6931471805599453f;  // back to natural units
-        my_ml[head * 2 + 1] = l;
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        float sum = l[y] + __shfl_xor_sync(0xffffffffu, l[y], 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        const int head = r0 + 8 * y;
+        if ((lane & 3) == 0 && head < nh) {
+          my_ml[head * 2] = m_ref[y] * 0.6931471805599453f;  // back to natural units
+          my_ml[head * 2 + 1] = sum;
+        }
       }
     }
   }
@@ -589,7 +608,8 @@ int mla_attend_tc_trace(long long *host_out, int max_entries) {
 typedef CUresult (*ta_encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static int cache_tensor_map(const uint16_t *base, long rows, CUtensorMap *out) {
+// keep: false for operands that move from call to call (the queries).
+static int cache_tensor_map(const uint16_t *base, long rows, bool keep, CUtensorMap *out) {
   struct Entry {
     const void *base;
     long rows;
@@ -600,7 +620,7 @@ static int cache_tensor_map(const uint16_t *base, long rows, CUtensorMap *out) {
   static int n_kept = 0, next = 0;
   static ta_encode_fn encode = nullptr;
   std::lock_guard<std::mutex> lock(mu);
-  for (int i = 0; i < n_kept; ++i)
+  for (int i = 0; i < n_kept && keep; ++i)
     if (kept[i].base == base && kept[i].rows == rows) {
       *out = kept[i].map;
       return BLOK_OK;
@@ -622,10 +642,11 @@ static int cache_tensor_map(const uint16_t *base, long rows, CUtensorMap *out) {
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   BLOK_REQUIRE(r == CUDA_SUCCESS, BLOK_ERR_CUDA, "blok_mla_decode: cuTensorMapEncodeTiled failed (%d) for a cache of %ld rows at %p", (int)r,
                rows, (const void *)base);
+  *out = map;
+  if (!keep) return BLOK_OK;
   kept[next] = Entry{base, rows, map};
   next = (next + 1) % 128;
   if (n_kept < 128) ++n_kept;
-  *out = map;
   return BLOK_OK;
 }
 
@@ -637,9 +658,10 @@ int launch_mla_attend_tc(const uint16_t *q, const uint16_t *cache, long ctx_stri
     BLOK_CUDA(cudaFuncSetAttribute(mla_attend_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemBytes));
     configured = true;
   }
-  CUtensorMap map;
-  if (int rc = cache_tensor_map(cache, total_rows, &map)) return rc;
-  return launch_pdl("mla_attend_tc_kernel", mla_attend_tc_kernel<false, false>, dim3(splits, B), kTaThreads, kTaSmemBytes, stream, map, q, cache, ctx_stride, seq_len, scale, part_o, part_ml, nullptr, nullptr, 0, 0, trace_buffer(), kTaHeads);
+  CUtensorMap map, qmap;
+  if (int rc = cache_tensor_map(cache, total_rows, true, &map)) return rc;
+  if (int rc = cache_tensor_map(q, (long)B * kTaHeads, false, &qmap)) return rc;
+  return launch_pdl("mla_attend_tc_kernel", mla_attend_tc_kernel<false, false>, dim3(splits, B), kTaThreads, kTaSmemBytes, stream, map, qmap, cache, ctx_stride, seq_len, scale, part_o, part_ml, nullptr, nullptr, 0, 0, trace_buffer(), kTaHeads);
 }
 
 // The same over a paged pool of pool_rows rows: page_rows must be a positive multiple of the 64-token tile.
@@ -652,9 +674,10 @@ static int launch_paged(const uint16_t *q, const uint16_t *pool, long pool_rows,
     BLOK_CUDA(cudaFuncSetAttribute(mla_attend_tc_kernel<true, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemBytes));
     configured = true;
   }
-  CUtensorMap map;
-  if (int rc = cache_tensor_map(pool, pool_rows, &map)) return rc;
-  return launch_pdl("mla_attend_tc_kernel(paged)", mla_attend_tc_kernel<true, FINE>, dim3(splits, B, (heads + kTaHeads - 1) / kTaHeads), kTaThreads, kTaSmemBytes, stream, map, q, pool, 0, seq_len, scale, part_o, part_ml, block_table, slot_of, table_stride, page_rows, trace_buffer(), heads);
+  CUtensorMap map, qmap;
+  if (int rc = cache_tensor_map(pool, pool_rows, true, &map)) return rc;
+  if (int rc = cache_tensor_map(q, (long)B * heads, false, &qmap)) return rc;
+  return launch_pdl("mla_attend_tc_kernel(paged)", mla_attend_tc_kernel<true, FINE>, dim3(splits, B, (heads + kTaHeads - 1) / kTaHeads), kTaThreads, kTaSmemBytes, stream, map, qmap, pool, 0, seq_len, scale, part_o, part_ml, block_table, slot_of, table_stride, page_rows, trace_buffer(), heads);
 }
 int launch_mla_attend_tc_paged(const uint16_t *q, const uint16_t *pool, long pool_rows, const int *block_table, const int *slot_of,
                                int table_stride, int page_rows, const int *seq_len, int B, int splits, float scale, float *part_o,
