@@ -40,11 +40,11 @@ __global__ void transpose_wuk_kernel(const uint16_t *__restrict__ kv_b, uint16_t
 size_t mla_attend_smem_bytes();
 int launch_mla_attend(const uint16_t *q, const uint16_t *cache, long ctx_stride, const int *seq_len, int B, int splits,
                       float scale, float *part_o, float *part_ml, cudaStream_t stream);
-int launch_mla_attend_tc(const uint16_t *q, const uint16_t *cache, long ctx_stride, long total_rows, const int *seq_len, int B, int splits,
-                         float scale, float *part_o, float *part_ml, cudaStream_t stream);
+int launch_mla_attend_tc(const uint16_t *q, const uint16_t *cache, long ctx_stride, long total_rows, const int *seq_len, int B, int ctas,
+                         float scale, float *part_o, float *part_ml, const MlaPlan *plan, int2 *parts, cudaStream_t stream);
 int launch_mla_attend_tc_paged(const uint16_t *q, const uint16_t *pool, long pool_rows, const int *block_table, const int *slot_of,
-                               int table_stride, int page_rows, const int *seq_len, int B, int splits, float scale, float *part_o,
-                               float *part_ml, cudaStream_t stream);
+                               int table_stride, int page_rows, const int *seq_len, int B, int ctas, float scale, float *part_o,
+                               float *part_ml, const MlaPlan *plan, int2 *parts, cudaStream_t stream);
 int mla_attend_tc_take_error(unsigned *out);
 int mla_attend_tc_trace(long long *host_out, int max_entries);
 int launch_mla_attend_paged(const uint16_t *q, const uint16_t *pool, const int *block_table, const int *slot_of,
@@ -73,8 +73,10 @@ struct blok_mla_layer {
   unsigned *err = nullptr;     // [2] 1 + b when entry b of a call had a position outside its sequence's rows; a product gave up
   float *wg_ws = nullptr;      // fp32 sums of the projections (wgemm_stream.cu), one projection's at a time
   size_t wg_bytes = 0;
-  float *part_o = nullptr;     // [max_splits * max_batch..]
+  float *part_o = nullptr;     // [max_splits + max_batch partial results, heads, kv_rank]
   float *part_ml = nullptr;
+  blok::MlaPlan *plan = nullptr;  // of the call's sequences
+  int2 *parts = nullptr;       // [B] and the sequences' partial results
 };
 
 using namespace blok;
@@ -136,6 +138,8 @@ extern "C" int blok_mla_layer_create(const blok_mla_weights *w, int max_batch, i
   size_t o_av = take((size_t)max_batch * w->heads * w->v_head * 2);
   size_t o_seq = take((size_t)max_batch * 4);
   size_t o_err = take(8);
+  size_t o_plan = take(sizeof(MlaPlan));
+  size_t o_parts = take((size_t)max_batch * sizeof(int2));
   size_t o_po = take((size_t)(L->max_splits + max_batch) * w->heads * w->kv_rank * 4);
   size_t o_pml = take((size_t)(L->max_splits + max_batch) * w->heads * 2 * 4);
   const size_t q_rows = (size_t)w->heads * qk_head;
@@ -164,6 +168,8 @@ extern "C" int blok_mla_layer_create(const blok_mla_weights *w, int max_batch, i
   L->av = reinterpret_cast<uint16_t *>(b + o_av);
   L->seq = reinterpret_cast<int *>(b + o_seq);
   L->err = reinterpret_cast<unsigned *>(b + o_err);
+  L->plan = reinterpret_cast<MlaPlan *>(b + o_plan);
+  L->parts = reinterpret_cast<int2 *>(b + o_parts);
   L->part_o = reinterpret_cast<float *>(b + o_po);
   L->part_ml = reinterpret_cast<float *>(b + o_pml);
   L->wg_ws = reinterpret_cast<float *>(b + o_wg);
@@ -240,7 +246,7 @@ struct CacheRef {
   int table_stride = 0, page_rows = 0;
 };
 
-// Context splits per sequence: enough CTAs to fill the GPU, but never more than one per 64 rows of the cache
+// The mma.sync core's context splits per sequence: enough CTAs to fill the GPU, but never more than one per 64 rows of the cache
 // allocation (the sequence lengths live on the device; the capacity bounds them), so that a short cache is not cut
 // into slivers whose merge costs more than the attention.
 static int splits_for(const blok_mla_layer *L, int B, long ctx_cap) {
@@ -250,31 +256,37 @@ static int splits_for(const blok_mla_layer *L, int B, long ctx_cap) {
   return s < 1 ? 1 : (int)s;
 }
 
-// The attention core: the splits' partial results in L->part_o and L->part_ml.
-static int attend(blok_mla_layer *L, const uint16_t *q, const CacheRef &c, const int *seq_len, int B, int splits, float scale, cudaStream_t stream) {
+// The attention core: partial results in L->part_o and L->part_ml.  *splits: of every sequence, or 0: as the plan for L->max_splits
+// CTAs says; planned: that is in L->plan and L->parts already, else the core makes it.
+static int attend(blok_mla_layer *L, const uint16_t *q, const CacheRef &c, const int *seq_len, int B, float scale, bool planned, int *splits,
+                  cudaStream_t stream) {
+  const MlaPlan *plan = planned ? L->plan : nullptr;
   // the tcgen05 core by default; BLOK_MLA_ATTEND_IMPL=mma (read at every call) selects the mma.sync kernel, which also
   // serves page sizes that are not a multiple of the tcgen05 core's 64-token tile
   const char *impl = getenv("BLOK_MLA_ATTEND_IMPL");
   const bool tc = !(impl && strcmp(impl, "mma") == 0) && (!c.block_table || c.page_rows % 64 == 0);
+  *splits = tc ? 0 : splits_for(L, B, c.ctx_cap);
   if (tc) {
     // the rows the tensor map may address: the whole dense cache (reads past it give zeros); a paged tile never leaves
     // its page, so the pool needs no tighter bound than the coordinate range
     const long dense_rows = c.seq_stride > 0 ? (long)B * c.seq_stride : c.ctx_cap;
     return c.block_table ? launch_mla_attend_tc_paged(q, c.base, (1l << 31) - 64, c.block_table, c.slot_of, c.table_stride, c.page_rows, seq_len,
-                                                      B, splits, scale, L->part_o, L->part_ml, stream)
-                         : launch_mla_attend_tc(q, c.base, c.seq_stride, dense_rows, seq_len, B, splits, scale, L->part_o, L->part_ml, stream);
+                                                      B, L->max_splits, scale, L->part_o, L->part_ml, plan, L->parts, stream)
+                         : launch_mla_attend_tc(q, c.base, c.seq_stride, dense_rows, seq_len, B, L->max_splits, scale, L->part_o, L->part_ml, plan, L->parts,
+                                                stream);
   }
   return c.block_table ? launch_mla_attend_paged(q, c.base, c.block_table, c.slot_of, c.table_stride, c.page_rows, seq_len, B,
-                                                 splits, scale, L->part_o, L->part_ml, stream)
-                       : launch_mla_attend(q, c.base, c.seq_stride, seq_len, B, splits, scale, L->part_o, L->part_ml, stream);
+                                                 *splits, scale, L->part_o, L->part_ml, stream)
+                       : launch_mla_attend(q, c.base, c.seq_stride, seq_len, B, *splits, scale, L->part_o, L->part_ml, stream);
 }
 
 static int attend_and_merge(blok_mla_layer *L, const uint16_t *q, const CacheRef &c, const int *seq_len, int B, float scale,
                             uint16_t *o_lat, cudaStream_t stream) {
-  const int splits = splits_for(L, B, c.ctx_cap);
-  if (int rc = attend(L, q, c, seq_len, B, splits, scale, stream)) return rc;
-  return launch_pdl("mla_merge_kernel", mla_merge_kernel, dim3(L->w.heads, B), 128, (size_t)splits * sizeof(float), stream, L->part_o, L->part_ml, splits,
-                    L->w.heads, L->w.kv_rank, o_lat, 0, nullptr, 0);
+  int splits;
+  if (int rc = attend(L, q, c, seq_len, B, scale, false, &splits, stream)) return rc;
+  const int most = splits ? splits : L->max_splits;
+  return launch_pdl("mla_merge_kernel", mla_merge_kernel, dim3(L->w.heads, B), 128, (size_t)most * sizeof(float), stream, L->part_o, L->part_ml, most,
+                    L->w.heads, L->w.kv_rank, o_lat, 0, nullptr, 0, splits ? nullptr : L->parts);
 }
 
 static int check_paged(const char *who, const void *pool, const int *block_table, int table_stride, int page_rows) {
@@ -342,7 +354,7 @@ static int decode_body(blok_mla_layer *L, const uint16_t *n, const CacheRef &c, 
   m.part = L->wg_ws; m.nz = nz; m.ld = w.q_rank + lat_w; m.q_rank = w.q_rank; m.kv_rank = w.kv_rank; m.rope = w.qk_rope;
   m.eps = w.rms_eps; m.q_ln = w.q_a_ln; m.kv_ln = w.kv_a_ln; m.qa = L->qa; m.inv_freq = L->inv_freq; m.pos = pos;
   m.cache = c.base; m.ctx_stride = c.seq_stride; m.block_table = c.block_table; m.slot_of = c.slot_of;
-  m.table_stride = c.table_stride; m.page_rows = c.page_rows; m.seq = L->seq; m.err = L->err;
+  m.table_stride = c.table_stride; m.page_rows = c.page_rows; m.seq = L->seq; m.plan = L->plan; m.parts = L->parts; m.ctas = L->max_splits; m.err = L->err;
   if ((rc = launch_mla_norm(m, B, stream))) return rc;
   // q_b, then q_abs = W_UK^T q_nope and the rotated rope part.  The head kernels read a head's sums four times over: with many
   // entries one part and bf16
@@ -353,11 +365,11 @@ static int decode_body(blok_mla_layer *L, const uint16_t *n, const CacheRef &c, 
   q.part = nz > 1 ? L->wg_ws : nullptr; q.q = L->q; q.nz = nz; q.B = B; q.nope = w.qk_nope; q.rope = w.qk_rope; q.kv_rank = w.kv_rank;
   q.inv_freq = L->inv_freq; q.pos = pos; q.q_full = L->q_full; q.werr = L->err + 1;
   if ((rc = launch_mla_query(L->wuk_t, w.heads, q, stream))) return rc;
-  const int splits = splits_for(L, B, c.ctx_cap);
-  if ((rc = attend(L, L->q_full, c, L->seq, B, splits, L->scale, stream))) return rc;
+  int splits;
+  if ((rc = attend(L, L->q_full, c, L->seq, B, L->scale, true, &splits, stream))) return rc;
   // the splits merged, out_h = W_UV o_lat_h, then o_proj   (:826)
   MlaValue v = {};
-  v.part_o = L->part_o; v.part_ml = L->part_ml; v.B = B; v.splits = splits; v.nope = w.qk_nope; v.v_head = w.v_head; v.out = L->av;
+  v.part_o = L->part_o; v.part_ml = L->part_ml; v.B = B; v.splits = splits; v.ctas = L->max_splits; v.parts = L->parts; v.nope = w.qk_nope; v.v_head = w.v_head; v.out = L->av;
   v.werr = L->err + 1;
   if ((rc = launch_mla_value(w.kv_b, w.heads, v, stream))) return rc;
   g.w_a = w.o; g.R = w.hidden; g.x = L->av; g.K = w.heads * w.v_head; g.out_bf16 = out; g.max_splits = 0;

@@ -41,6 +41,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "mla_plan.cuh"
 #include "tmem_io.cuh"
 
 namespace blok {
@@ -175,22 +176,24 @@ __device__ __forceinline__ bool ta_consumers_sync(bool failed) {
 
 size_t mla_attend_tc_smem_bytes() { return kTaSmemBytes; }
 
-// grid = (splits, B); arguments as mla_attend_kernel, plus the tensor maps of the cache ([rows, 576] bf16) and of the queries
-// ([B x heads, 576]), both in boxes of 64 rows x 64 columns, 128-byte swizzle.  PAGED: page_rows is a multiple of the 64-token tile.
+// Arguments as mla_attend_kernel, plus the tensor maps of the cache ([rows, 576] bf16) and of the queries ([B x heads, 576]), both in
+// boxes of 64 rows x 64 columns, 128-byte swizzle.  PAGED: page_rows is a multiple of the 64-token tile.  planned > 0: so many
+// sequences, shared out over a one-dimensional grid as mla_plan.cuh says (plan: made by a kernel before this one; NULL: made here, and
+// CTA 0 leaves each sequence's partial results in parts); planned = 0: grid = (splits, B, groups of heads), every sequence in `splits` equal parts.
 template <bool PAGED, bool FINE>
 __global__ void __launch_bounds__(kTaThreads, 1)
     mla_attend_tc_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap qmap, const uint16_t *cache,
                          long ctx_stride, const int *seq_len, float scale, float *__restrict__ part_o,
                          float *__restrict__ part_ml, const int *block_table, const int *slot_of,
-                         int table_stride, int page_rows, long long *__restrict__ trace, int heads) {
+                         int table_stride, int page_rows, long long *__restrict__ trace, int heads, int planned,
+                         const MlaPlan *plan, int2 *__restrict__ parts) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long s_bar[16];
   __shared__ uint32_t s_tmem;
   __shared__ float s_alpha[kTaHeads];
   __shared__ int s_need[2][4];
+  __shared__ MlaPlan s_plan;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int split = blockIdx.x, splits = gridDim.x, b = blockIdx.y;
-  pdl_trigger();
   // the swizzle is a function of the address: the tiles start on a 1,024-byte boundary
   const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
   const uint32_t sT = (raw + 1023u) & ~1023u;
@@ -216,22 +219,65 @@ __global__ void __launch_bounds__(kTaThreads, 1)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  if (plan) {  // made by a kernel that had finished before the one in front of this launch let it begin; a word a thread
+    static_assert(sizeof(MlaPlan) / sizeof(int) <= kTaThreads, "a word of the plan to a thread");
+    if (tid < (int)(sizeof(MlaPlan) / sizeof(int))) reinterpret_cast<int *>(&s_plan)[tid] = reinterpret_cast<const int *>(plan)[tid];
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_tmem;
   pdl_wait();
-  const int seq = FINE ? min(seq_len[b] + 1, table_stride * page_rows) : seq_len[b];
-  const int ntiles = (seq + kTaTile - 1) / kTaTile;
-  const int per = (ntiles + splits - 1) / splits;
-  const int ts = split * per, te = min(ntiles, ts + per);
+  pdl_trigger();  // after the wait: the kernel behind this one may read what was there before this one, the plan's parts
   const int h0 = blockIdx.z * kTaHeads, nh = min(kTaHeads, heads - h0);  // this CTA's heads
-  float *my_ml = part_ml + (((size_t)b * splits + split) * heads + h0) * 2;
-  const int nt = max(0, te - ts);
-  if (nt == 0 && tid < nh) {  // nothing to do for this split: mark it empty for the merge
-    my_ml[tid * 2] = -INFINITY;
-    my_ml[tid * 2 + 1] = 0.f;
+  auto length = [&](int b) { return FINE ? min(seq_len[b] + 1, table_stride * page_rows) : seq_len[b]; };
+  if (planned && !plan) {
+    if (warp == 0) {
+      mla_plan(s_plan, planned, gridDim.x, length);
+      if (blockIdx.x == 0)
+        for (int b = lane; b < planned; b += 32) parts[b] = mla_plan_parts(s_plan, b);
+    }
+    __syncthreads();
   }
+  // The CTA's segments in order: nt tiles of sequence b from tile ts on, partial result `slot`; `partial`: the last of them holds
+  // rows past the sequence's end.
+  struct Segment {
+    int b, ts, nt, slot, seq;
+    bool partial;
+  };
+  const int lo = planned ? (int)blockIdx.x * s_plan.per : 0, hi = planned ? lo + s_plan.per : 0;
+  int b_first = 0;  // the first sequence that ends behind the piece's begin
+  if (planned) {
+    b_first = __popc(__ballot_sync(0xffffffffu, lane < planned && s_plan.start[lane + 1] <= lo)) +
+              __popc(__ballot_sync(0xffffffffu, lane + 32 < planned && s_plan.start[lane + 33] <= lo));
+  }
+  auto segment = [&](int &next, Segment &g) -> bool {
+    if (planned) {
+      for (; next < planned && s_plan.start[next] < hi; ++next) {
+        const int tile0 = s_plan.start[next] + s_plan.lead, ntiles = (s_plan.tokens[next] + kTaTile - 1) / kTaTile;
+        const int t0 = max(lo - tile0, 0), t1 = min(hi - tile0, ntiles);
+        if (t1 <= t0) continue;
+        g.b = next, g.ts = t0, g.nt = t1 - t0, g.slot = (int)blockIdx.x + next, g.seq = s_plan.tokens[next];
+        g.partial = g.seq % kTaTile != 0 && ntiles == t1;
+        ++next;
+        return true;
+      }
+      return false;
+    }
+    if (next > 0) return false;
+    next = 1;
+    const int split = blockIdx.x, splits = gridDim.x;
+    g.b = blockIdx.y, g.slot = g.b * splits + split, g.seq = length(g.b);
+    const int ntiles = (g.seq + kTaTile - 1) / kTaTile, per = (ntiles + splits - 1) / splits;
+    g.ts = split * per, g.nt = max(0, min(ntiles, g.ts + per) - g.ts);
+    g.partial = g.seq % kTaTile != 0 && g.ts + g.nt == ntiles;
+    if (g.nt == 0 && tid < nh) {  // nothing to do for this split: mark it empty for the merge
+      float *ml = part_ml + ((size_t)g.slot * heads + h0) * 2;
+      ml[tid * 2] = -INFINITY;
+      ml[tid * 2 + 1] = 0.f;
+    }
+    return g.nt > 0;
+  };
   bool failed = false;
   // diagnostics (trace != NULL): CTA (0, 0) stamps, per tile, [0] buffer free, [1] TMA issued, [2] S issued, [3] S seen
   // by the softmax warps, [4] P handed over, [5] P.C issued, [8] S read, [9] softmax done (nanoseconds)
@@ -242,77 +288,84 @@ __global__ void __launch_bounds__(kTaThreads, 1)
       trace[n * 16 + slot] = t;
     }
   };
-  // the sequence's last tile may hold rows past its end
-  const int last_partial = (seq % kTaTile != 0 && te == ntiles) ? nt - 1 : -1;
+  Segment g;
+  int next_b = b_first;
 
   if (warp == 4) {
     // ---- the producer: nine boxes for the queries, nine per tile, counted on the mbarrier of their half ----
-    const uint16_t *cache_b = PAGED ? cache : cache + (size_t)b * ctx_stride * kTaD;
-    const int *table_b = PAGED ? block_table + (size_t)(slot_of ? slot_of[b] : b) * table_stride : nullptr;
-    auto first_row = [&](int tok0) -> long {  // the tensor map's row of the tile's first token
-      if (PAGED) return (long)table_b[tok0 / page_rows] * page_rows + tok0 % page_rows;
-      return (long)b * ctx_stride + tok0;
-    };
-    if (nt > 0 && lane == 0) {
-      ta_expect_tx(bar_q, kTaQBytes);
-#pragma unroll 1
-      for (int c = 0; c < kTaChunks; ++c) ta_tma_2d(sQ + c * kTaChunkBytes, &qmap, 64 * c, b * heads + h0, bar_q);
-    }
-    int issued = 0;
-    for (int n = 0; n < nt; ++n) {
-      const int buf = n & 1;
-      const int tok0 = (ts + n) * kTaTile, row = (int)first_row(tok0);
-      const uint32_t dst = sT + buf * kTaTileBytes;
-#pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        // (the second half also holds FINE's low parts, which both warps read; it comes after the first)
-        if (n >= 2 && !__all_sync(0xffffffffu, ta_wait(bar_empty + 16 * buf + 8 * half, (uint32_t)(((n >> 1) - 1) & 1), 1u))) {
-          failed = true;
-          break;
-        }
-        if (lane == 0) {
-          if (half == 0) stamp(n, 0);
-          const int c0 = half ? kTaHalfChunks : 0, c1 = half ? kTaChunks : kTaHalfChunks;
-          const uint32_t bar = bar_tma + 16 * buf + 8 * half;
-          ta_expect_tx(bar, (uint32_t)(c1 - c0) * kTaChunkBytes);
-#pragma unroll 1
-          for (int c = c0; c < c1; ++c) ta_tma_2d(dst + c * kTaChunkBytes, &tmap, 64 * c, row, bar);
-        }
-        issued = 2 * n + half + 1;
+    int issued = 0, at = 0;  // halves asked for, tile of the CTA
+    for (int sg = 0; !failed && segment(next_b, g); ++sg) {
+      const uint16_t *cache_b = PAGED ? cache : cache + (size_t)g.b * ctx_stride * kTaD;
+      const int *table_b = PAGED ? block_table + (size_t)(slot_of ? slot_of[g.b] : g.b) * table_stride : nullptr;
+      auto first_row = [&](int tok0) -> long {  // the tensor map's row of the tile's first token
+        if (PAGED) return (long)table_b[tok0 / page_rows] * page_rows + tok0 % page_rows;
+        return (long)g.b * ctx_stride + tok0;
+      };
+      // the queries of the segment before are free behind its last scores
+      if (at > 0 && !__all_sync(0xffffffffu, ta_wait(bar_sfull + 8 * ((at - 1) & 1), (uint32_t)(((at - 1) >> 1) & 1), 12u))) {
+        failed = true;
+        break;
       }
-      if (failed) break;
       if (lane == 0) {
-        if (n + 2 < nt) {
-          // The buffer's next tile starts its way from HBM to L2 now: by the time the buffer is free again (this
-          // tile's two products later) the copy finds it there, and HBM has been busy meanwhile.  A tile is contiguous
-          // (dense cache, or inside a page); only rows of the sequence are touched.
-          const int ptok = tok0 + 2 * kTaTile;
-          const int prow = min(kTaTile, seq - ptok);
-          const uint16_t *pp = PAGED ? cache + (size_t)first_row(ptok) * kTaD : cache_b + (size_t)ptok * kTaD;
-          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(pp), "r"((uint32_t)(prow * kTaD * 2)) : "memory");
-        }
-        stamp(n, 1);
+        ta_expect_tx(bar_q, kTaQBytes);
+#pragma unroll 1
+        for (int c = 0; c < kTaChunks; ++c) ta_tma_2d(sQ + c * kTaChunkBytes, &qmap, 64 * c, g.b * heads + h0, bar_q);
       }
-      if (n == last_partial) {
-        // rows past the sequence's end hold whatever the allocation holds: zero them (their P is zero, and zero times
-        // a stray NaN would not be), whole 128-byte rows, which the swizzle only permutes within
-        const uint32_t turn = (uint32_t)((n >> 1) & 1);
-        if (!__all_sync(0xffffffffu, ta_wait(bar_tma + 16 * buf, turn, 10u) && ta_wait(bar_tma + 16 * buf + 8, turn, 10u))) {
-          failed = true;
-          break;
+      for (int n = 0; n < g.nt; ++n, ++at) {
+        const int buf = at & 1;
+        const int tok0 = (g.ts + n) * kTaTile, row = (int)first_row(tok0);
+        const uint32_t dst = sT + buf * kTaTileBytes;
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          // (the second half also holds FINE's low parts, which both warps read; it comes after the first)
+          if (at >= 2 && !__all_sync(0xffffffffu, ta_wait(bar_empty + 16 * buf + 8 * half, (uint32_t)(((at >> 1) - 1) & 1), 1u))) {
+            failed = true;
+            break;
+          }
+          if (lane == 0) {
+            if (half == 0) stamp(at, 0);
+            const int c0 = half ? kTaHalfChunks : 0, c1 = half ? kTaChunks : kTaHalfChunks;
+            const uint32_t bar = bar_tma + 16 * buf + 8 * half;
+            ta_expect_tx(bar, (uint32_t)(c1 - c0) * kTaChunkBytes);
+#pragma unroll 1
+            for (int c = c0; c < c1; ++c) ta_tma_2d(dst + c * kTaChunkBytes, &tmap, 64 * c, row, bar);
+          }
+          issued = 2 * at + half + 1;
         }
-        const int valid = seq - tok0;
-        unsigned char *tile = smem + (size_t)buf * kTaTileBytes;
-        for (int idx = lane; idx < (kTaTile - valid) * kTaChunks * 8; idx += 32) {
-          const int r = valid + idx / (kTaChunks * 8), rem = idx % (kTaChunks * 8);
-          *reinterpret_cast<uint4 *>(tile + (rem >> 3) * kTaChunkBytes + r * 128 + (rem & 7) * 16) = make_uint4(0, 0, 0, 0);
+        if (failed) break;
+        if (lane == 0) {
+          if (n + 2 < g.nt) {
+            // The buffer's next tile starts its way from HBM to L2 now: by the time the buffer is free again (this
+            // tile's two products later) the copy finds it there, and HBM has been busy meanwhile.  A tile is contiguous
+            // (dense cache, or inside a page); only rows of the sequence are touched.
+            const int ptok = tok0 + 2 * kTaTile;
+            const int prow = min(kTaTile, g.seq - ptok);
+            const uint16_t *pp = PAGED ? cache + (size_t)first_row(ptok) * kTaD : cache_b + (size_t)ptok * kTaD;
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(pp), "r"((uint32_t)(prow * kTaD * 2)) : "memory");
+          }
+          stamp(at, 1);
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) ta_arrive(bar_fix + 8 * buf);
+        if (g.partial && n == g.nt - 1) {
+          // rows past the sequence's end hold whatever the allocation holds: zero them (their P is zero, and zero times
+          // a stray NaN would not be), whole 128-byte rows, which the swizzle only permutes within
+          const uint32_t turn = (uint32_t)((at >> 1) & 1);
+          if (!__all_sync(0xffffffffu, ta_wait(bar_tma + 16 * buf, turn, 10u) && ta_wait(bar_tma + 16 * buf + 8, turn, 10u))) {
+            failed = true;
+            break;
+          }
+          const int valid = g.seq - tok0;
+          unsigned char *tile = smem + (size_t)buf * kTaTileBytes;
+          for (int idx = lane; idx < (kTaTile - valid) * kTaChunks * 8; idx += 32) {
+            const int r = valid + idx / (kTaChunks * 8), rem = idx % (kTaChunks * 8);
+            *reinterpret_cast<uint4 *>(tile + (rem >> 3) * kTaChunkBytes + r * 128 + (rem & 7) * 16) = make_uint4(0, 0, 0, 0);
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) ta_arrive(bar_fix + 8 * buf);
+        }
       }
     }
-    // no copy may be in flight when the CTA leaves; the MMA warp has seen all of them unless a wait gave up
+    // no copy may be in flight when the CTA leaves; the MMA warps have seen all of them unless a wait gave up
     for (int i = max(0, issued - 4); i < issued; ++i) ta_wait(bar_tma + 16 * ((i >> 1) & 1) + 8 * (i & 1), (uint32_t)((i >> 2) & 1), 11u);
   } else if (warp >= 5) {
     // ---- two MMA warps: the fixed cost of an MMA of this size is larger than its work, and two warps share it.  All lanes walk,
@@ -350,7 +403,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
     };
     // Latent blocks of 128 columns = chunks 2 j and 2 j + 1, two of them to a warp; a K step is 16 tokens = two 8-row groups.  The
     // blocks take turns, so that consecutive MMAs accumulate into different columns of tensor memory.
-    auto issue_pv = [&](int n) {
+    auto issue_pv = [&](int n, bool first) {
       const int buf = n & 1;
       const uint64_t a_desc = ta_desc_sw128(sT + buf * kTaTileBytes + 4 * wi * kTaChunkBytes, kTaChunkBytes, 1024);
       const uint64_t lo_desc = ta_desc_plain(sT + buf * kTaTileBytes + (kTaChunks - 1) * kTaChunkBytes, kTaLbo, kTaSbo);  // FINE: the low parts
@@ -362,7 +415,7 @@ __global__ void __launch_bounds__(kTaThreads, 1)
 #pragma unroll
             for (int j = 0; j < 2; ++j)
               ta_mma(tmem + kTaColO + 128 * wi + 64 * j, a_desc + (uint64_t)((2 * j * kTaChunkBytes + kk * 2048) >> 4),
-                     (part ? lo_desc : p_desc) + (uint64_t)(kk * ((2 * kTaLbo) >> 4)), idesc_pv, (n > 0 || kk > 0 || part > 0) ? 1u : 0u);
+                     (part ? lo_desc : p_desc) + (uint64_t)(kk * ((2 * kTaLbo) >> 4)), idesc_pv, (!first || kk > 0 || part > 0) ? 1u : 0u);
           }
         }
         ta_commit(bar_empty + 16 * buf + 8 * wi);
@@ -372,196 +425,206 @@ __global__ void __launch_bounds__(kTaThreads, 1)
     };
     // true where the whole warp sees the phase complete
     auto seen = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, ta_test(bar, parity)); };
-    if (nt > 0 && !__all_sync(0xffffffffu, ta_wait(bar_q, 0u, 4u))) failed = true;
     // Whatever can go next goes: a tile's P.C product frees its buffer and comes first; the scores of the tile behind it are
     // issued half by half as they land, so that neither product waits long behind the other in the tensor pipe.
-    int sn = 0, sh = 0, pn = 0;  // next scores (tile, half), next P.C product
-    unsigned idle = 0;
-    while (pn < nt && !failed) {
-      bool went = false;
-      if (pn < sn && seen(bar_pfull, (uint32_t)(pn & 1))) {
-        tc_fence_after();
-        issue_pv(pn++);
-        went = true;
-      } else if (sn < nt && sn <= pn + 1) {
-        const int sb = sn & 1;
-        const uint32_t turn = (uint32_t)((sn >> 1) & 1);
-        bool ready = seen(bar_tma + 16 * sb + 8 * sh, turn);
-        if (ready && sn == last_partial) ready = seen(bar_fix + 8 * sb, 0u);
-        if (ready && sh == 0 && sn >= 2) ready = seen(bar_sfree + 8 * sb, turn ^ 1);
-        if (ready) {
+    int sn = 0, pn = 0;   // next scores, next P.C product: tiles of the CTA
+    uint32_t fix_turn = 0;  // a bit per buffer
+    for (int sg = 0; !failed && segment(next_b, g); ++sg) {
+      const int first = pn, end = pn + g.nt, last_partial = g.partial ? end - 1 : -1;
+      int sh = 0;  // half of the scores
+      if (!__all_sync(0xffffffffu, ta_wait(bar_q, (uint32_t)(sg & 1), 4u))) failed = true;
+      unsigned idle = 0;
+      while (pn < end && !failed) {
+        bool went = false;
+        if (pn < sn && seen(bar_pfull, (uint32_t)(pn & 1))) {
           tc_fence_after();
-          issue_s(sn, sh);
-          if (sh) ++sn;
-          sh ^= 1;
+          issue_pv(pn, pn == first);
+          ++pn;
           went = true;
+        } else if (sn < end && sn <= pn + 1) {
+          const int sb = sn & 1;
+          const uint32_t turn = (uint32_t)((sn >> 1) & 1);
+          bool ready = seen(bar_tma + 16 * sb + 8 * sh, turn);
+          if (ready && sn == last_partial) ready = seen(bar_fix + 8 * sb, (fix_turn >> sb) & 1u);
+          if (ready && sh == 0 && sn >= 2) ready = seen(bar_sfree + 8 * sb, turn ^ 1);
+          if (ready) {
+            tc_fence_after();
+            issue_s(sn, sh);
+            if (sh && sn == last_partial) fix_turn ^= 1u << sb;
+            sn += sh;
+            sh ^= 1;
+            went = true;
+          }
         }
-      }
-      if (went) {
-        idle = 0;
-      } else if (++idle > 64) {
-        __nanosleep(32);
-        if (idle > kTaSpinLimit) {
-          if (lane == 0) atomicExch(&g_mla_tc_error, 3u);
-          failed = true;
+        if (went) {
+          idle = 0;
+        } else if (++idle > 64) {
+          __nanosleep(32);
+          if (idle > kTaSpinLimit) {
+            if (lane == 0) atomicExch(&g_mla_tc_error, 3u);
+            failed = true;
+          }
         }
       }
     }
-  } else if (nt > 0) {
+  } else {
     // ---- consumers: warp w holds head rows 16 w .. 16 w + 15 of S; a lane has rows r0 and r0 + 8, 16 tokens of each ----
     const float sl2 = scale * 1.4426950408889634f;
     const int r0 = 16 * warp + (lane >> 2), tq = 2 * (lane & 3);
-    float m_ref[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
     auto done_with = [&](int n, unsigned code) -> bool {  // both warps' P.C products of tile n
       const uint32_t turn = (uint32_t)((n >> 1) & 1);
       return ta_wait(bar_empty + 16 * (n & 1), turn, code) && ta_wait(bar_empty + 16 * (n & 1) + 8, turn, code);
     };
-    for (int n = 0; n < nt; ++n) {
-      const int buf = n & 1;
-      uint32_t pk[2][8], pl[2][FINE ? 8 : 1];  // [row][column group of 8 tokens]: this lane's pair of tokens
-      bool need = false;
-      if (!failed && !__all_sync(0xffffffffu, ta_wait(bar_sfull + 8 * buf, (uint32_t)((n >> 1) & 1), 6u))) failed = true;
-      if (!failed) {
-        if (tid == 0) stamp(n, 3);
-        tc_fence_after();
-        uint32_t r[32];
-        {
-          uint32_t r2[32];  // the two partial sums of the score product
-          tmem_ld_rows16(tmem + ((uint32_t)(32 * warp) << 16) + 128 * buf, r);
-          tmem_ld_rows16(tmem + ((uint32_t)(32 * warp) << 16) + 128 * buf + 64, r2);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) ta_arrive(bar_sfree + 8 * buf);
-        if (tid == 0) stamp(n, 8);
-        const int tok0 = (ts + n) * kTaTile;
-        if (tok0 + kTaTile > seq) {  // the sequence's last tile: tokens past the end take no weight
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (tok0 + 8 * (j >> 2) + tq + (j & 1) >= seq) r[j] = 0xff800000u;
-        }
-#pragma unroll
-        for (int y = 0; y < 2; ++y) {
-          float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            mx0 = fmaxf(mx0, __uint_as_float(r[4 * i + 2 * y]));
-            mx1 = fmaxf(mx1, __uint_as_float(r[4 * i + 2 * y + 1]));
-          }
-          float mx = fmaxf(mx0, mx1);
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2)) * sl2;  // the scale is positive
-          float alpha = 1.f;
-          if (n == 0) {
-            m_ref[y] = mx;  // the split's first tile holds at least one token
-          } else if (mx > m_ref[y] + kTaLazy) {
-            alpha = exp2f(m_ref[y] - mx);
-            m_ref[y] = mx;
-            need = true;
-          }
-          if ((lane & 3) == 0) s_alpha[r0 + 8 * y] = alpha;
-          const float nm = -m_ref[y];
-          float sum0 = 0.f, sum1 = 0.f;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            // the probabilities enter the second product rounded to bf16 (as the reference rounds them, :466); the
-            // normaliser sums the same rounded values (FINE: two parts, and the normaliser sums the weights themselves)
-            const float p0 = ta_ex2(fmaf(__uint_as_float(r[4 * i + 2 * y]), sl2, nm)), p1 = ta_ex2(fmaf(__uint_as_float(r[4 * i + 2 * y + 1]), sl2, nm));
-            const uint32_t pa = ta_pack_bf16x2(p0, p1);
-            if (FINE) {
-              sum0 += p0;
-              sum1 += p1;
-              pl[y][FINE ? i : 0] = ta_pack_bf16x2(p0 - __uint_as_float(pa << 16), p1 - __uint_as_float(pa & 0xffff0000u));
-            } else {
-              sum0 += __uint_as_float(pa << 16);
-              sum1 += __uint_as_float(pa & 0xffff0000u);
-            }
-            pk[y][i] = pa;
-          }
-          l[y] = l[y] * alpha + (sum0 + sum1);
-        }
-        if (tid == 0) stamp(n, 9);
-      }
-      need = __any_sync(0xffffffffu, need);
-      if (lane == 0) s_need[buf][warp] = need ? 1 : 0;
-      if (ta_consumers_sync(failed)) {
-        failed = true;
-        break;
-      }
-      if (s_need[buf][0] | s_need[buf][1] | s_need[buf][2] | s_need[buf][3]) {
-        // a head's reference maximum moved (never in tile 0): every lane of O^T scales its 4 x 64 head columns, once the
-        // previous tile's MMAs have finished with them
-        if (!__all_sync(0xffffffffu, done_with(n - 1, 7u))) failed = true;
+    int n = 0;  // tile of the CTA
+    while (!failed && segment(next_b, g)) {
+      float m_ref[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+      for (int i = 0; i < g.nt; ++i, ++n) {
+        const int buf = n & 1;
+        uint32_t pk[2][8], pl[2][FINE ? 8 : 1];  // [row][column group of 8 tokens]: this lane's pair of tokens
+        bool need = false;
+        if (!failed && !__all_sync(0xffffffffu, ta_wait(bar_sfull + 8 * buf, (uint32_t)((n >> 1) & 1), 6u))) failed = true;
         if (!failed) {
+          if (tid == 0) stamp(n, 3);
           tc_fence_after();
-#pragma unroll 1
-          for (int j = 0; j < kTaDV / 128; ++j) {
-            uint32_t o[64];
-            const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) + kTaColO + 64 * j;
-            tmem_ld64(ta, o);
+          uint32_t r[32];
+          {
+            uint32_t r2[32];  // the two partial sums of the score product
+            tmem_ld_rows16(tmem + ((uint32_t)(32 * warp) << 16) + 128 * buf, r);
+            tmem_ld_rows16(tmem + ((uint32_t)(32 * warp) << 16) + 128 * buf + 64, r2);
             tmem_wait_ld();
 #pragma unroll
-            for (int c = 0; c < 64; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * s_alpha[c]);
-            tmem_st64(ta, o);
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
           }
-          tmem_wait_st();
           tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ta_arrive(bar_sfree + 8 * buf);
+          if (tid == 0) stamp(n, 8);
+          const int tok0 = (g.ts + i) * kTaTile;
+          if (tok0 + kTaTile > g.seq) {  // the sequence's last tile: tokens past the end take no weight
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (tok0 + 8 * (j >> 2) + tq + (j & 1) >= g.seq) r[j] = 0xff800000u;
+          }
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {
+            float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              mx0 = fmaxf(mx0, __uint_as_float(r[4 * e + 2 * y]));
+              mx1 = fmaxf(mx1, __uint_as_float(r[4 * e + 2 * y + 1]));
+            }
+            float mx = fmaxf(mx0, mx1);
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2)) * sl2;  // the scale is positive
+            float alpha = 1.f;
+            if (i == 0) {
+              m_ref[y] = mx;  // the segment's first tile holds at least one token
+            } else if (mx > m_ref[y] + kTaLazy) {
+              alpha = exp2f(m_ref[y] - mx);
+              m_ref[y] = mx;
+              need = true;
+            }
+            if ((lane & 3) == 0) s_alpha[r0 + 8 * y] = alpha;
+            const float nm = -m_ref[y];
+            float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              // the probabilities enter the second product rounded to bf16 (as the reference rounds them, :466); the
+              // normaliser sums the same rounded values (FINE: two parts, and the normaliser sums the weights themselves)
+              const float p0 = ta_ex2(fmaf(__uint_as_float(r[4 * e + 2 * y]), sl2, nm)), p1 = ta_ex2(fmaf(__uint_as_float(r[4 * e + 2 * y + 1]), sl2, nm));
+              const uint32_t pa = ta_pack_bf16x2(p0, p1);
+              if (FINE) {
+                sum0 += p0;
+                sum1 += p1;
+                pl[y][FINE ? e : 0] = ta_pack_bf16x2(p0 - __uint_as_float(pa << 16), p1 - __uint_as_float(pa & 0xffff0000u));
+              } else {
+                sum0 += __uint_as_float(pa << 16);
+                sum1 += __uint_as_float(pa & 0xffff0000u);
+              }
+              pk[y][e] = pa;
+            }
+            l[y] = l[y] * alpha + (sum0 + sum1);
+          }
+          if (tid == 0) stamp(n, 9);
         }
+        need = __any_sync(0xffffffffu, need);
+        if (lane == 0) s_need[buf][warp] = need ? 1 : 0;
         if (ta_consumers_sync(failed)) {
           failed = true;
           break;
         }
-      }
-      if (!failed) {
-        if (n > 0 && !__all_sync(0xffffffffu, done_with(n - 1, 8u))) {
-          failed = true;  // reaches the others at the next tile's barrier
-        } else {
-          unsigned char *lo = smem + (size_t)buf * kTaTileBytes + (kTaChunks - 1) * kTaChunkBytes;
+        if (s_need[buf][0] | s_need[buf][1] | s_need[buf][2] | s_need[buf][3]) {
+          // a head's reference maximum moved (never in a segment's first tile): every lane of O^T scales its 4 x 64 head columns, once the
+          // previous tile's MMAs have finished with them
+          if (!__all_sync(0xffffffffu, done_with(n - 1, 7u))) failed = true;
+          if (!failed) {
+            tc_fence_after();
+#pragma unroll 1
+            for (int j = 0; j < kTaDV / 128; ++j) {
+              uint32_t o[64];
+              const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) + kTaColO + 64 * j;
+              tmem_ld64(ta, o);
+              tmem_wait_ld();
 #pragma unroll
-          for (int y = 0; y < 2; ++y) {
-#pragma unroll
-            for (int kg = 0; kg < kTaTile / 8; ++kg) {
-              const int at = kg * kTaLbo + (r0 + 8 * y) * 16 + 2 * tq;
-              *reinterpret_cast<uint32_t *>(Pp + at) = pk[y][kg];
-              if (FINE) *reinterpret_cast<uint32_t *>(lo + at) = pl[y][FINE ? kg : 0];
+              for (int c = 0; c < 64; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * s_alpha[c]);
+              tmem_st64(ta, o);
             }
+            tmem_wait_st();
+            tc_fence_before();
           }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) ta_arrive(bar_pfull);
-          if (tid == 0) stamp(n, 4);
+          if (ta_consumers_sync(failed)) {
+            failed = true;
+            break;
+          }
+        }
+        if (!failed) {
+          if (n > 0 && !__all_sync(0xffffffffu, done_with(n - 1, 8u))) {
+            failed = true;  // reaches the others at the next tile's barrier
+          } else {
+            unsigned char *lo = smem + (size_t)buf * kTaTileBytes + (kTaChunks - 1) * kTaChunkBytes;
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+#pragma unroll
+              for (int kg = 0; kg < kTaTile / 8; ++kg) {
+                const int at = kg * kTaLbo + (r0 + 8 * y) * 16 + 2 * tq;
+                *reinterpret_cast<uint32_t *>(Pp + at) = pk[y][kg];
+                if (FINE) *reinterpret_cast<uint32_t *>(lo + at) = pl[y][FINE ? kg : 0];
+              }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) ta_arrive(bar_pfull);
+            if (tid == 0) stamp(n, 4);
+          }
         }
       }
-    }
-    // ---- the split's partial result: O^T [latent lane x head column] -> part_o [head][512], (m, sum) per head ----
-    if (!failed && !__all_sync(0xffffffffu, done_with(nt - 1, 9u))) failed = true;
-    failed = ta_consumers_sync(failed);
-    if (!failed) {
-      tc_fence_after();
-      float *po = part_o + (((size_t)b * splits + split) * heads + h0) * kTaDV;
+      // ---- the segment's partial result: O^T [latent lane x head column] -> part_o [head][512], (m, sum) per head ----
+      if (!failed && !__all_sync(0xffffffffu, done_with(n - 1, 9u))) failed = true;
+      failed = ta_consumers_sync(failed);
+      if (!failed) {
+        tc_fence_after();
+        float *po = part_o + ((size_t)g.slot * heads + h0) * kTaDV, *my_ml = part_ml + ((size_t)g.slot * heads + h0) * 2;
 #pragma unroll 1
-      for (int j = 0; j < kTaDV / 128; ++j) {
+        for (int j = 0; j < kTaDV / 128; ++j) {
 #pragma unroll 1
-        for (int half = 0; half < 2; ++half) {
-          uint32_t o[32];
-          tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + kTaColO + 64 * j + 32 * half, o);
-          tmem_wait_ld();
+          for (int half = 0; half < 2; ++half) {
+            uint32_t o[32];
+            tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + kTaColO + 64 * j + 32 * half, o);
+            tmem_wait_ld();
 #pragma unroll
-          for (int c = 0; c < 32; ++c)
-            if (32 * half + c < nh) po[(size_t)(32 * half + c) * kTaDV + 128 * j + 32 * warp + lane] = __uint_as_float(o[c]);
+            for (int c = 0; c < 32; ++c)
+              if (32 * half + c < nh) po[(size_t)(32 * half + c) * kTaDV + 128 * j + 32 * warp + lane] = __uint_as_float(o[c]);
+          }
         }
-      }
 #pragma unroll
-      for (int y = 0; y < 2; ++y) {
-        float sum = l[y] + __shfl_xor_sync(0xffffffffu, l[y], 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        const int head = r0 + 8 * y;
-        if ((lane & 3) == 0 && head < nh) {
-          my_ml[head * 2] = m_ref[y] * 0.6931471805599453f;  // back to natural units
-          my_ml[head * 2 + 1] = sum;
+        for (int y = 0; y < 2; ++y) {
+          float sum = l[y] + __shfl_xor_sync(0xffffffffu, l[y], 1);
+          sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+          const int head = r0 + 8 * y;
+          if ((lane & 3) == 0 && head < nh) {
+            my_ml[head * 2] = m_ref[y] * 0.6931471805599453f;  // back to natural units
+            my_ml[head * 2 + 1] = sum;
+          }
         }
       }
     }
@@ -650,9 +713,10 @@ static int cache_tensor_map(const uint16_t *base, long rows, bool keep, CUtensor
   return BLOK_OK;
 }
 
-// total_rows: the rows of the cache allocation from `cache` on (reads past them give zeros).
-int launch_mla_attend_tc(const uint16_t *q, const uint16_t *cache, long ctx_stride, long total_rows, const int *seq_len, int B, int splits,
-                         float scale, float *part_o, float *part_ml, cudaStream_t stream) {
+// total_rows: the rows of the cache allocation from `cache` on (reads past them give zeros).  Up to kMlaPlanMax sequences over `ctas`
+// CTAs; plan, parts: see the kernel.
+int launch_mla_attend_tc(const uint16_t *q, const uint16_t *cache, long ctx_stride, long total_rows, const int *seq_len, int B, int ctas,
+                         float scale, float *part_o, float *part_ml, const MlaPlan *plan, int2 *parts, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
     BLOK_CUDA(cudaFuncSetAttribute(mla_attend_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemBytes));
@@ -661,14 +725,14 @@ int launch_mla_attend_tc(const uint16_t *q, const uint16_t *cache, long ctx_stri
   CUtensorMap map, qmap;
   if (int rc = cache_tensor_map(cache, total_rows, true, &map)) return rc;
   if (int rc = cache_tensor_map(q, (long)B * kTaHeads, false, &qmap)) return rc;
-  return launch_pdl("mla_attend_tc_kernel", mla_attend_tc_kernel<false, false>, dim3(splits, B), kTaThreads, kTaSmemBytes, stream, map, qmap, cache, ctx_stride, seq_len, scale, part_o, part_ml, nullptr, nullptr, 0, 0, trace_buffer(), kTaHeads);
+  return launch_pdl("mla_attend_tc_kernel", mla_attend_tc_kernel<false, false>, dim3(ctas), kTaThreads, kTaSmemBytes, stream, map, qmap, cache, ctx_stride, seq_len, scale, part_o, part_ml, nullptr, nullptr, 0, 0, trace_buffer(), kTaHeads, B, plan, parts);
 }
 
 // The same over a paged pool of pool_rows rows: page_rows must be a positive multiple of the 64-token tile.
 template <bool FINE>
 static int launch_paged(const uint16_t *q, const uint16_t *pool, long pool_rows, const int *block_table, const int *slot_of, int table_stride,
-                        int page_rows, const int *seq_len, int B, int heads, int splits, float scale, float *part_o, float *part_ml,
-                        cudaStream_t stream) {
+                        int page_rows, const int *seq_len, int B, int heads, dim3 grid, float scale, float *part_o, float *part_ml,
+                        int planned, const MlaPlan *plan, int2 *parts, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
     BLOK_CUDA(cudaFuncSetAttribute(mla_attend_tc_kernel<true, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemBytes));
@@ -677,20 +741,20 @@ static int launch_paged(const uint16_t *q, const uint16_t *pool, long pool_rows,
   CUtensorMap map, qmap;
   if (int rc = cache_tensor_map(pool, pool_rows, true, &map)) return rc;
   if (int rc = cache_tensor_map(q, (long)B * heads, false, &qmap)) return rc;
-  return launch_pdl("mla_attend_tc_kernel(paged)", mla_attend_tc_kernel<true, FINE>, dim3(splits, B, (heads + kTaHeads - 1) / kTaHeads), kTaThreads, kTaSmemBytes, stream, map, qmap, pool, 0, seq_len, scale, part_o, part_ml, block_table, slot_of, table_stride, page_rows, trace_buffer(), heads);
+  return launch_pdl("mla_attend_tc_kernel(paged)", mla_attend_tc_kernel<true, FINE>, grid, kTaThreads, kTaSmemBytes, stream, map, qmap, pool, 0, seq_len, scale, part_o, part_ml, block_table, slot_of, table_stride, page_rows, trace_buffer(), heads, planned, plan, parts);
 }
 int launch_mla_attend_tc_paged(const uint16_t *q, const uint16_t *pool, long pool_rows, const int *block_table, const int *slot_of,
-                               int table_stride, int page_rows, const int *seq_len, int B, int splits, float scale, float *part_o,
-                               float *part_ml, cudaStream_t stream) {
-  return launch_paged<false>(q, pool, pool_rows, block_table, slot_of, table_stride, page_rows, seq_len, B, kTaHeads, splits, scale, part_o, part_ml,
-                             stream);
+                               int table_stride, int page_rows, const int *seq_len, int B, int ctas, float scale, float *part_o,
+                               float *part_ml, const MlaPlan *plan, int2 *parts, cudaStream_t stream) {
+  return launch_paged<false>(q, pool, pool_rows, block_table, slot_of, table_stride, page_rows, seq_len, B, kTaHeads, dim3(ctas), scale, part_o,
+                             part_ml, B, plan, parts, stream);
 }
 // Any number of heads; the weights in two bf16 parts; entry b attends to rows 0..pos[b].
 int launch_mla_attend_tc_fine(const uint16_t *q, const uint16_t *pool, long pool_rows, const int *block_table, const int *slot_of, int table_stride,
                               int page_rows, const int *pos, int B, int heads, int splits, float scale, float *part_o, float *part_ml,
                               cudaStream_t stream) {
-  return launch_paged<true>(q, pool, pool_rows, block_table, slot_of, table_stride, page_rows, pos, B, heads, splits, scale, part_o, part_ml,
-                            stream);
+  return launch_paged<true>(q, pool, pool_rows, block_table, slot_of, table_stride, page_rows, pos, B, heads, dim3(splits, B, (heads + kTaHeads - 1) / kTaHeads), scale,
+                            part_o, part_ml, 0, nullptr, nullptr, stream);
 }
 
 }  // namespace blok

@@ -59,7 +59,8 @@ __global__ void __launch_bounds__(kMnThreads) mla_norm_kernel(const MlaNorm a) {
   extern __shared__ float val[];
   __shared__ float red[kMnThreads / 32];
   const int b = blockIdx.y, tid = threadIdx.x, lat = a.kv_rank + a.rope, half = a.rope / 2;
-  const bool kv = blockIdx.x != 0;
+  __shared__ MlaPlan s_plan;
+  const bool kv = blockIdx.x != 0, plans = !kv && b == 0 && tid >= kMnThreads - 32;
   const int n = kv ? a.kv_rank : a.q_rank, all = kv ? lat : n;  // values under the norm, and in all
   pdl_trigger();
   const uint16_t *ln = kv ? a.kv_ln : a.q_ln;
@@ -76,7 +77,16 @@ __global__ void __launch_bounds__(kMnThreads) mla_norm_kernel(const MlaNorm a) {
                                      pos % a.page_rows) * lat
                         : a.cache + ((size_t)b * a.ctx_stride + pos) * lat;
   }
+  if (plans)
+    mla_plan(s_plan, gridDim.y, a.ctas, [&](int i) {
+      bool in;
+      return mh_position(a.pos, i, &in) + 1;
+    });
   pdl_wait();
+  if (plans) {
+    for (int i = tid & 31; i < (int)gridDim.y; i += 32) a.parts[i] = mla_plan_parts(s_plan, i);
+    for (int i = tid & 31; i < (int)(sizeof(MlaPlan) / sizeof(int)); i += 32) reinterpret_cast<int *>(a.plan)[i] = reinterpret_cast<const int *>(&s_plan)[i];
+  }
   if (kv) {
     if (tid == 0) {
       a.seq[b] = pos + 1;
@@ -144,7 +154,7 @@ __global__ void __launch_bounds__(kMqThreads) mla_query_kernel(const __grid_cons
   const int N = (a.B + 15) / 16 * 16;
   const int qk = a.nope + a.rope;
   const size_t q_row = (size_t)gridDim.x * qk, stride = (size_t)a.B * q_row;
-  pdl_trigger();
+  // The trigger stands behind the wait: the attention core may then read before its own wait what the norm kernel left
   if (blockIdx.y == gridDim.y - 1) {
     const int half = a.rope / 2;
     uint32_t *cs = reinterpret_cast<uint32_t *>(smem_raw);  // [B][half] cosine and sine, before the wait
@@ -154,6 +164,7 @@ __global__ void __launch_bounds__(kMqThreads) mla_query_kernel(const __grid_cons
       cs[u] = pack_bf16x2(cosf(ang), sinf(ang));
     }
     pdl_wait();
+    pdl_trigger();
     for (int u = tid; u < a.B * half; u += kMqThreads) {  // the thread's own entries of cs
       const int tok = u / half, p = u % half;
       const size_t at = (size_t)tok * q_row + (size_t)h * qk + a.nope + 2 * p;
@@ -196,6 +207,7 @@ __global__ void __launch_bounds__(kMqThreads) mla_query_kernel(const __grid_cons
   };
   if (tid == 0) fetch(0);
   pdl_wait();
+  pdl_trigger();
   // 16 bytes of one token's query: columns c .. c + 7 of the head
   auto query8 = [&](int tok, int c) -> uint4 {
     const size_t at = (size_t)tok * q_row + (size_t)h * qk + c;
@@ -242,10 +254,11 @@ constexpr int kMvRank = 512;                     // kv_rank
 constexpr int kMvWBytes = (kMvRank / 64) * 16384;  // 128 rows of W_UV: 128 KB
 
 struct MvMerge {
-  int heads, S, G, N, quarter, j4;
-  const float4 *po;   // this thread's columns of the first entry's first split
-  const float2 *ml;   // (max, sum) of the first entry's first split
-  float *wt, *inv;    // [G][S] weights of the splits, [G] 1 / their sum
+  int heads, G, N, quarter, j4;
+  const int2 *parts;  // [G] first partial result and number of them
+  const float4 *po;   // this thread's columns of partial result 0
+  const float2 *ml;   // (max, sum) of partial result 0
+  float *wt, *inv;    // weights of the partial results from parts[0].x on, [G] 1 / their sum
   float4 (*acc)[128];
   unsigned char *x;   // the merged rows, bf16, as the product reads them
 };
@@ -263,72 +276,84 @@ __device__ __forceinline__ void mv_put(const MvMerge &m, int g, const float4 &ac
 template <int SP>
 __device__ __noinline__ void mv_merge(const MvMerge m) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int parts = SP == 8 ? (m.G == 1 ? 4 : (m.G == 2 ? 2 : 1)) : 1, per = (m.S + parts - 1) / parts, part = m.quarter % parts;
-  const int s0 = part * per, s1 = min(m.S, s0 + per), gstep = 4 / parts;
+  const int parts = SP == 8 ? (m.G == 1 ? 4 : (m.G == 2 ? 2 : 1)) : 1, part = m.quarter % parts, gstep = 4 / parts;
   const size_t split4 = (size_t)m.heads * (kMvRank / 4);
   float4 v[8];
+  int2 e[8 / SP];  // the partial results of the entries in flight that this thread adds
   auto ask = [&](int g, int s) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int gi = g + (i / SP) * gstep, si = s + i % SP;
-      if (gi < m.G && si < s1) v[i] = m.po[((size_t)gi * m.S + si) * split4];
+    for (int k = 0; k < 8 / SP; ++k) {
+      e[k] = g + k * gstep < m.G ? m.parts[g + k * gstep] : make_int2(0, 0);
+      if (parts > 1) {
+        const int per = (e[k].y + parts - 1) / parts, n = max(0, min(e[k].y - part * per, per));
+        e[k] = make_int2(e[k].x + part * per, n);
+      }
+#pragma unroll
+      for (int i = 0; i < SP; ++i)
+        if (s + i < e[k].y) v[k * SP + i] = m.po[(size_t)(e[k].x + s + i) * split4];
     }
   };
-  int g = m.quarter / parts, s = s0;
+  int g = m.quarter / parts, s = 0;
   ask(g, s);
+  const int base = m.parts[0].x;
 #pragma unroll 1
-  for (int e = warp; e < m.G; e += kMvThreads / 32) {
+  for (int i = warp; i < m.G; i += kMvThreads / 32) {
+    const int2 p = m.parts[i];
     float M = -INFINITY, L = 0.f;
-    float2 ms[5];  // up to 160 splits
+    float2 ms[5];  // up to 160 of them
 #pragma unroll
-    for (int i = 0; i < 5; ++i) ms[i] = lane + 32 * i < m.S ? m.ml[((size_t)e * m.S + lane + 32 * i) * m.heads] : make_float2(-INFINITY, 0.f);
+    for (int k = 0; k < 5; ++k) ms[k] = lane + 32 * k < p.y ? m.ml[(size_t)(p.x + lane + 32 * k) * m.heads] : make_float2(-INFINITY, 0.f);
 #pragma unroll
-    for (int i = 0; i < 5; ++i) M = fmaxf(M, ms[i].x);
+    for (int k = 0; k < 5; ++k) M = fmaxf(M, ms[k].x);
     M = warp_max(M);
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      const float w = ms[i].x != -INFINITY ? expf(ms[i].x - M) : 0.f;  // 0 for an empty split
-      if (lane + 32 * i < m.S) m.wt[e * m.S + lane + 32 * i] = w;
-      L += w * ms[i].y;
+    for (int k = 0; k < 5; ++k) {
+      const float w = ms[k].x != -INFINITY ? expf(ms[k].x - M) : 0.f;  // 0 for an empty split
+      if (lane + 32 * k < p.y) m.wt[p.x - base + lane + 32 * k] = w;
+      L += w * ms[k].y;
     }
     L = warp_sum(L);
-    if (lane == 0) m.inv[e] = L > 0.f ? 1.0f / L : 0.f;
+    if (lane == 0) m.inv[i] = L > 0.f ? 1.0f / L : 0.f;
   }
   __syncthreads();
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
   while (g < m.G) {
+    const int more = e[0].y;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int gi = g + (i / SP) * gstep, si = s + i % SP;
-      const float w = gi < m.G && si < s1 ? m.wt[gi * m.S + si] : 0.f;
-      // an empty split holds no result: its weight of zero must not meet whatever lies there
-      if (w != 0.f) acc.x = fmaf(w, v[i].x, acc.x), acc.y = fmaf(w, v[i].y, acc.y), acc.z = fmaf(w, v[i].z, acc.z), acc.w = fmaf(w, v[i].w, acc.w);
-      if (SP < 8 && i % SP == SP - 1) {
-        if (gi < m.G) mv_put(m, gi, acc);
+    for (int k = 0; k < 8 / SP; ++k) {
+#pragma unroll
+      for (int i = 0; i < SP; ++i) {
+        const float w = s + i < e[k].y ? m.wt[e[k].x + s + i - base] : 0.f;
+        const float4 t = v[k * SP + i];
+        // an empty split holds no result: its weight of zero must not meet whatever lies there
+        if (w != 0.f) acc.x = fmaf(w, t.x, acc.x), acc.y = fmaf(w, t.y, acc.y), acc.z = fmaf(w, t.z, acc.z), acc.w = fmaf(w, t.w, acc.w);
+      }
+      if (SP < 8) {
+        if (g + k * gstep < m.G) mv_put(m, g + k * gstep, acc);
         acc = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
     if (SP < 8) {
       g += (8 / SP) * gstep;
-    } else if ((s += 8) >= s1) {
+    } else if ((s += 8) >= more) {
       if (parts > 1) break;
       mv_put(m, g, acc);
       acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      s = s0, g += gstep;
+      s = 0, g += gstep;
     }
     ask(g, s);
   }
   if (parts > 1) {  // uniform
-    const int e = m.quarter / parts;
-    if (part) m.acc[m.quarter - e - 1][m.j4] = acc;
+    const int i = m.quarter / parts;
+    if (part) m.acc[m.quarter - i - 1][m.j4] = acc;
     __syncthreads();
     if (part == 0) {
       for (int p = 1; p < parts; ++p) {
-        const float4 t = m.acc[m.quarter + p - e - 1][m.j4];
+        const float4 t = m.acc[m.quarter + p - i - 1][m.j4];
         acc.x += t.x, acc.y += t.y, acc.z += t.z, acc.w += t.w;
       }
-      mv_put(m, e, acc);
+      mv_put(m, i, acc);
     }
   }
 }
@@ -341,13 +366,15 @@ __global__ void __launch_bounds__(kMvThreads, 1) mla_value_kernel(const __grid_c
   __shared__ uint32_t s_tmem;
   __shared__ float s_inv[32];
   __shared__ float4 s_acc[3][128];
+  __shared__ int2 s_parts[32];
+  __shared__ int s_most;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.x, heads = gridDim.x;
   const int b0 = (int)blockIdx.z * a.group, G = min(a.group, a.B - b0), N = a.group <= 16 ? 16 : 32;
   pdl_trigger();
   const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw), sw = (raw + 1023u) & ~1023u;
   const uint32_t sx = sw + kMvWBytes;
   unsigned char *xp = smem_raw + (sx - raw);
-  float *wt = reinterpret_cast<float *>(xp + (kMvRank / 64) * N * 128);  // [G][splits]
+  float *wt = reinterpret_cast<float *>(xp + (kMvRank / 64) * N * 128);
   const uint32_t full = (uint32_t)__cvta_generic_to_shared(&s_bar[0]), done = full + 8;
   if (tid == 0) {
     tp_mbar_init(full, 1);
@@ -358,18 +385,26 @@ __global__ void __launch_bounds__(kMvThreads, 1) mla_value_kernel(const __grid_c
       tp_load_2d(sw + (uint32_t)j * 16384, &mw, 64 * j, h * (a.nope + a.v_head) + a.nope + 128 * (int)blockIdx.y, full);
   }
   if (warp == 0) tp_tmem_alloc((uint32_t)__cvta_generic_to_shared(&s_tmem), 32);
+  if (warp == 1) {  // what the attention core leaves: known before the core began (it triggers behind its own wait)
+    int2 p = make_int2((b0 + lane) * a.splits, a.splits);
+    if (!a.splits && lane < G) p = a.parts[b0 + lane];
+    if (lane < G) s_parts[lane] = p;
+    const int most = __reduce_max_sync(0xffffffffu, lane < G ? p.y : 0);
+    if (lane == 0) s_most = most;
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   pdl_wait();
   MvMerge m;
-  m.heads = heads, m.S = a.splits, m.G = G, m.N = N, m.quarter = tid >> 7, m.j4 = tid & 127;
-  m.po = reinterpret_cast<const float4 *>(a.part_o) + ((size_t)b0 * a.splits * heads + h) * (kMvRank / 4) + m.j4;
-  m.ml = reinterpret_cast<const float2 *>(a.part_ml) + (size_t)b0 * a.splits * heads + h;
+  m.heads = heads, m.G = G, m.N = N, m.quarter = tid >> 7, m.j4 = tid & 127;
+  m.parts = s_parts;
+  m.po = reinterpret_cast<const float4 *>(a.part_o) + (size_t)h * (kMvRank / 4) + m.j4;
+  m.ml = reinterpret_cast<const float2 *>(a.part_ml) + h;
   m.wt = wt, m.inv = s_inv, m.acc = s_acc, m.x = xp;
   // one instance per size of the lists, so that a launch fetches little code
-  if (G <= 2 || a.splits > 4) mv_merge<8>(m);
-  else if (a.splits > 2) mv_merge<4>(m);
+  if (G <= 2 || s_most > 4) mv_merge<8>(m);
+  else if (s_most > 2) mv_merge<4>(m);
   else mv_merge<2>(m);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
@@ -415,7 +450,8 @@ int launch_mla_value(const uint16_t *kv_b, int heads, MlaValue a, cudaStream_t s
   const int groups = a.B > 1 ? 2 : 1;
   a.group = (a.B + groups - 1) / groups;
   const int N = a.group <= 16 ? 16 : 32;
-  const int smem = kMvWBytes + (kMvRank / 64) * N * 128 + a.group * a.splits * (int)sizeof(float) + 1024;
+  // weights of the partial results: in the planned form those of consecutive entries are consecutive, fewer than CTAs + entries
+  const int smem = kMvWBytes + (kMvRank / 64) * N * 128 + (a.splits ? a.group * a.splits : a.ctas + a.B) * (int)sizeof(float) + 1024;
   BLOK_CUDA(cudaFuncSetAttribute(mla_value_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   return launch_pdl("mla_value_kernel", mla_value_kernel, dim3(heads, (a.v_head + 127) / 128, groups), kMvThreads, (size_t)smem, stream, mw, a);
 }

@@ -4,6 +4,8 @@
 
 #include <cstdint>
 
+#include "mla_plan.cuh"
+
 namespace blok {
 
 // Entry b stands at position len[b], or (a chunk of one sequence) at len[0] + b; a sequence has cap rows.
@@ -27,6 +29,9 @@ struct MlaNorm {
   const int *block_table, *slot_of;
   int table_stride, page_rows;
   int *seq;       // [B] position + 1
+  MlaPlan *plan;  // how `ctas` CTAs of the attention core share the sequences,
+  int2 *parts;    // [B] and what partial results they leave
+  int ctas;
   unsigned *err;  // 1 + b of an entry outside its rows
 };
 int launch_mla_norm(const MlaNorm &a, int B, cudaStream_t stream);
@@ -44,8 +49,11 @@ struct MlaQuery {
 int launch_mla_query(const uint16_t *wuk_t, int heads, const MlaQuery &a, cudaStream_t stream);
 
 struct MlaValue {
-  const float *part_o, *part_ml;  // [B, splits, heads, 512], [B, splits, heads, 2]
-  int B, splits, nope, v_head;
+  const float *part_o, *part_ml;  // [partial result, heads, 512], [.., heads, 2]
+  int B, nope, v_head;
+  int splits;         // of every entry; 0: entry b has parts[b].y of them from parts[b].x on, fewer than ctas + B in all
+  int ctas;
+  const int2 *parts;  // there since before the attention core began
   uint16_t *out;  // [B, heads, v_head]
   unsigned *werr;
   int group;  // entries per CTA (set by the launch)

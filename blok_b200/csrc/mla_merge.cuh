@@ -7,17 +7,21 @@ namespace blok {
 // ---------------------------------------------------------------------------
 // Merge of the split-KV partial results.  grid = (heads, B), 128 threads.
 //   part_o fp32 [B, splits, heads, kv_rank] unnormalised, part_ml fp32 [B, splits, heads, 2] = (max, sum)
+// parts, optional: entry b has parts[b].y <= splits partial results, one after another from parts[b].x on.
 // Rows of o_lat are ldo values apart (0: heads * kv_rank).  gate, optional: bf16 [B, ld_gate]; head h's output times
 // sigmoid(gate[b][h]).
 // ---------------------------------------------------------------------------
 static __global__ void mla_merge_kernel(const float *part_o, const float *part_ml, int splits, int heads, int kv_rank,
-                                        uint16_t *__restrict__ o_lat, int ldo = 0, const uint16_t *gate = nullptr, int ld_gate = 0) {
+                                        uint16_t *__restrict__ o_lat, int ldo = 0, const uint16_t *gate = nullptr, int ld_gate = 0,
+                                        const int2 *parts = nullptr) {
   extern __shared__ float s_wt[];  // [splits] weight of every split: exp(m_s - M), 0 for an empty split
   __shared__ float s_red[2][4];
   pdl_trigger();
   pdl_wait();
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
-  const float *ml = part_ml + ((size_t)b * splits * heads + h) * 2;  // split s at + s * heads * 2
+  size_t first = (size_t)b * splits;
+  if (parts) first = parts[b].x, splits = parts[b].y;
+  const float *ml = part_ml + (first * heads + h) * 2;  // split s at + s * heads * 2
   float M = -INFINITY;
   for (int s = tid; s < splits; s += blockDim.x) M = fmaxf(M, ml[(size_t)s * heads * 2]);
   M = warp_max(M);
@@ -38,7 +42,7 @@ static __global__ void mla_merge_kernel(const float *part_o, const float *part_m
   float inv = L > 0.f ? 1.0f / L : 0.f;
   if (gate) inv *= 1.0f / (1.0f + expf(-bf16_bits_to_f32(gate[(size_t)b * ld_gate + h])));
   if (!ldo) ldo = heads * kv_rank;
-  const float *po = part_o + ((size_t)b * splits * heads + h) * kv_rank;  // split s at + s * heads * kv_rank
+  const float *po = part_o + (first * heads + h) * kv_rank;  // split s at + s * heads * kv_rank
   // four columns per thread, eight splits' worth of loads in flight per thread: the partial results (B x splits x 128 KB)
   // come from L2 or HBM, and the kernel is as fast as it keeps bytes in flight.  Each column still adds its splits in
   // ascending order.

@@ -89,3 +89,30 @@ def test_chain(cuda, hidden, q_rank, nope, v_head, B):
     _check(rows[first:], new, "chunk rows")
     layer.check()
     layer.close()
+
+
+@pytest.mark.parametrize("lens", [
+    [1] * 60 + [900, 64, 65, 3000],                    # pieces over the sequences' borders, several sequences to a CTA
+    [0, 5, 0, 700, 128, 0],                            # empty sequences: zeros
+    [1300] * 50, [64 * 37] * 4, list(range(1, 65))])
+def test_core_over_lengths(cuda, lens):
+    """The attention core alone over batches of sequences whose tiles fall on the CTAs in every way."""
+    from blok_b200 import lib
+    w, g = _weights(cuda, 288, 96, 32, 16, len(lens))
+    layer = lib.MlaLayer(w, yarn_factor=32.0, max_batch=64, max_ctx=64, qk_nope=32, v_head=16)
+    B, ctx = len(lens), max(lens) + 3
+    cache = torch.randn((B, ctx, RANK + ROPE), generator=g, device=cuda).bfloat16()
+    for b, n in enumerate(lens):
+        cache[b, n:] = float("nan")                    # rows past a sequence's end are nobody's business
+    q = (torch.randn((B, HEADS, RANK + ROPE), generator=g, device=cuda) * 0.3).bfloat16()
+    o = layer.attend(q, cache, torch.tensor(lens, dtype=torch.int32, device=cuda))
+    layer.check()
+    for b, n in enumerate(lens):
+        rows = cache[b, :n].double()
+        want = torch.softmax(q[b].double() @ rows.T * layer.scale, dim=-1) @ rows[:, :RANK]
+        if n == 0:
+            assert not o[b].any(), b
+        else:                                          # probabilities and results to bf16: 2^-9 each
+            err = float((o[b].double() - want).norm() / want.norm())
+            assert err < 6e-3, (b, n, err)
+    layer.close()
