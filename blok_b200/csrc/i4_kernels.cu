@@ -113,20 +113,24 @@ __global__ void __launch_bounds__(kMaxWarps * 32)
 // rows, A-high rows the same 8 up rows, so the SiLU*up epilogue needs no second
 // pass.  slot_expert (device, may be NULL = identity) maps slot -> local expert.
 // mid is bf16 [slots, inter] in natural order.
+//
+// One expert is 25 MB, 4 us of HBM, in two dependent launches: what counts is that nothing waits for anything it does not need.
+// The blocks are resident when the launch before has finished (launch_pdl), the first batch of weights is asked for before the
+// activations are staged, and the down kernel has its own in registers when the intermediate vector is there.  One expert of
+// 7,168 x 2,048 whose weights come from HBM: 17.5 -> 12.9 us, 1,024 x 512 8.2 -> 4.5, 5,120 x 2,816 22.6 -> 18.2.
 // ---------------------------------------------------------------------------
 template <int BATCH>
 __global__ void __launch_bounds__(kMaxWarps * 32)
     i4_gateup_kernel(const uint32_t *__restrict__ gate_w, const uint16_t *__restrict__ gate_s,
                      const uint32_t *__restrict__ up_w, const uint16_t *__restrict__ up_s,
-                     const uint16_t *__restrict__ x, const int *__restrict__ slot_expert, uint16_t *__restrict__ mid,
+                     const uint16_t *x, const int *slot_expert, uint16_t *mid,
                      int cols, int inter, int nbatch) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ float partial[kMaxWarps][16];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  I4Stage st = i4_stage_carve(smem, cols, BATCH);
-  stage_x_i4(reinterpret_cast<const uint4 *>(x), st, cols, BATCH, tid, blockDim.x);
-  __syncthreads();
+  pdl_wait();
+  pdl_trigger();  // behind the wait: the down kernel reads weights before its own
   const int slot = blockIdx.y;
   const int e = slot_expert ? slot_expert[slot] : slot;
   const int row0 = blockIdx.x * 8;
@@ -135,8 +139,15 @@ __global__ void __launch_bounds__(kMaxWarps * 32)
   const uint4 *w_lo = reinterpret_cast<const uint4 *>(gate_w) + ebase + (size_t)(row0 + g) * wrow;
   const uint4 *w_hi = reinterpret_cast<const uint4 *>(up_w) + ebase + (size_t)(row0 + g) * wrow;
   const uint16_t *s_sel = ((t >> 1) ? up_s : gate_s) + ebase + (size_t)(row0 + g) * wrow + 2 * (t & 1);
+  const int kb0 = warp * nbatch * BATCH;
+  I4Batch<BATCH> first;  // the weights are on their way while the activations are staged
+  i4_batch_load<BATCH>(first, w_lo, w_hi, s_sel, kb0, t);
+  I4Stage st = i4_stage_carve(smem, cols, BATCH);
+  stage_x_i4(reinterpret_cast<const uint4 *>(x), st, cols, BATCH, tid, blockDim.x);
+  __syncthreads();
   XFragLane xl = xfrag_lane(st, lane, BATCH);
-  float acc = i4_rows16_accumulate<BATCH>(w_lo, w_hi, s_sel, xl, st.xsum, warp * nbatch * BATCH, nbatch, lane);
+  float acc = i4_batch_compute<BATCH>(first, xl, st.xsum, kb0, lane, 0.f);
+  acc += i4_rows16_accumulate<BATCH>(w_lo, w_hi, s_sel, xl, st.xsum, kb0 + BATCH, nbatch - 1, lane);
   acc += __shfl_xor_sync(0xffffffffu, acc, 1);
   if ((t & 1) == 0) partial[warp][g + 8 * (t >> 1)] = acc;
   __syncthreads();
@@ -158,35 +169,42 @@ __global__ void __launch_bounds__(kMaxWarps * 32)
 // down projection + weighted combine.  grid = hidden/16.  Warp w works on slot
 // w / ksplit, K part w % ksplit.  out[r] = bf16( bf16(sum_slot bf16(y_slot[r]) *
 // wts[slot]) + addend[r] ); wts == NULL means weight 1 (single expert), addend
-// may be NULL.  Mirrors expert_accum_k :399, round_bf16_k :404, add_k :248.
+// may be NULL.  Mirrors expert_accum_k :399, round_bf16_k :404, add_k :248.  Launched to become resident while the kernel
+// before it (gate/up) runs: its first batch of weights is in registers before the wait, so what is written by launches
+// before gate/up only (weights, slot_expert) is read early, everything else behind the wait.
 // ---------------------------------------------------------------------------
 template <int BATCH>
 __global__ void __launch_bounds__(kMaxWarps * 32)
     i4_down_kernel(const uint32_t *__restrict__ down_w, const uint16_t *__restrict__ down_s,
-                   const uint16_t *__restrict__ mid, const int *__restrict__ slot_expert,
-                   const float *__restrict__ wts, const uint16_t *__restrict__ addend, uint16_t *__restrict__ out,
+                   const uint16_t *mid, const int *__restrict__ slot_expert, const float *wts, const uint16_t *addend, uint16_t *out,
                    int cols /*inter*/, int rows /*hidden*/, int slots, int ksplit, int nbatch) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ float partial[kMaxWarps][16];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
+  pdl_trigger();
+  const int slot = warp / ksplit, kpart = warp - slot * ksplit;
+  const int e = slot_expert ? slot_expert[slot] : slot;
+  const int row0 = blockIdx.x * 16;
+  const size_t wrow = cols / 32;
+  const size_t ebase = (size_t)e * rows * wrow;
+  const uint4 *w_lo = reinterpret_cast<const uint4 *>(down_w) + ebase + (size_t)(row0 + g) * wrow;
+  const uint4 *w_hi = w_lo + 8 * wrow;
+  const uint16_t *s_sel = down_s + ebase + (size_t)(row0 + g + 8 * (t >> 1)) * wrow + 2 * (t & 1);
+  const int kb0 = kpart * nbatch * BATCH;
+  I4Batch<BATCH> first;  // weights do not depend on the gate/up kernel that runs meanwhile
+  i4_batch_load<BATCH>(first, w_lo, w_hi, s_sel, kb0, t);
+  pdl_wait();
   const size_t stage_stride = i4_stage_bytes(cols, BATCH);
   for (int s = 0; s < slots; ++s) {
     I4Stage st = i4_stage_carve(smem + s * stage_stride, cols, BATCH);
     stage_x_i4(reinterpret_cast<const uint4 *>(mid + (size_t)s * cols), st, cols, BATCH, tid, blockDim.x);
   }
   __syncthreads();
-  const int slot = warp / ksplit, kpart = warp - slot * ksplit;
-  const int e = slot_expert ? slot_expert[slot] : slot;
-  const int row0 = blockIdx.x * 16;
-  const size_t wrow = cols / 32;
-  const size_t ebase = (size_t)e * rows * wrow;
   I4Stage st = i4_stage_carve(smem + slot * stage_stride, cols, BATCH);
-  const uint4 *w_lo = reinterpret_cast<const uint4 *>(down_w) + ebase + (size_t)(row0 + g) * wrow;
-  const uint4 *w_hi = w_lo + 8 * wrow;
-  const uint16_t *s_sel = down_s + ebase + (size_t)(row0 + g + 8 * (t >> 1)) * wrow + 2 * (t & 1);
   XFragLane xl = xfrag_lane(st, lane, BATCH);
-  float acc = i4_rows16_accumulate<BATCH>(w_lo, w_hi, s_sel, xl, st.xsum, kpart * nbatch * BATCH, nbatch, lane);
+  float acc = i4_batch_compute<BATCH>(first, xl, st.xsum, kb0, lane, 0.f);
+  acc += i4_rows16_accumulate<BATCH>(w_lo, w_hi, s_sel, xl, st.xsum, kb0 + BATCH, nbatch - 1, lane);
   acc += __shfl_xor_sync(0xffffffffu, acc, 1);
   if ((t & 1) == 0) partial[warp][g + 8 * (t >> 1)] = acc;
   __syncthreads();
@@ -277,11 +295,10 @@ int launch_i4_gateup(const uint32_t *gate_w, const uint16_t *gate_s, const uint3
   BLOK_DISPATCH_BATCH(ks.batch, {
     int rc = ensure_smem(i4_gateup_kernel<B>, smem);
     if (rc) return rc;
-    i4_gateup_kernel<B><<<dim3(inter / 8, slots), ks.nwarps * 32, smem, stream>>>(gate_w, gate_s, up_w, up_s, x,
-                                                                                   slot_expert, mid, hidden, inter,
-                                                                                   ks.nbatch);
+    return launch_pdl("i4_gateup_kernel", i4_gateup_kernel<B>, dim3(inter / 8, slots), ks.nwarps * 32, smem, stream, gate_w, gate_s, up_w, up_s, x,
+                      slot_expert, mid, hidden, inter, ks.nbatch);
   });
-  return launch_status("i4_gateup_kernel");
+  return BLOK_OK;
 }
 
 int launch_i4_down(const uint32_t *down_w, const uint16_t *down_s, const uint16_t *mid, const int *slot_expert,
@@ -298,11 +315,10 @@ int launch_i4_down(const uint32_t *down_w, const uint16_t *down_s, const uint16_
   BLOK_DISPATCH_BATCH(ks.batch, {
     int rc = ensure_smem(i4_down_kernel<B>, smem);
     if (rc) return rc;
-    i4_down_kernel<B><<<hidden / 16, slots * ks.nwarps * 32, smem, stream>>>(down_w, down_s, mid, slot_expert, wts,
-                                                                             addend, out, inter, hidden, slots,
-                                                                             ks.nwarps, ks.nbatch);
+    return launch_pdl("i4_down_kernel", i4_down_kernel<B>, hidden / 16, slots * ks.nwarps * 32, smem, stream, down_w, down_s, mid, slot_expert, wts,
+                      addend, out, inter, hidden, slots, ks.nwarps, ks.nbatch);
   });
-  return launch_status("i4_down_kernel");
+  return BLOK_OK;
 }
 
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

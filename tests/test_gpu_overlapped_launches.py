@@ -77,3 +77,40 @@ def test_attention_block(cuda, B, paged):
     for i, (a, b) in enumerate(zip(outs[True], outs[False])):
         assert torch.equal(a, b), "call %d" % i
     layer.close()
+
+
+@pytest.mark.parametrize("what,rows", [("expert", 1), ("mla", 1), ("mla", 20), ("moe", 5), ("moe", 60)])
+def test_weights_written_just_before(cuda, what, rows):
+    """Kernels that fetch their weights before the launches in front of them have finished: weights that an ordinary launch wrote
+    just before the call are the ones that count."""
+    from blok_b200 import lib, synth
+    if what == "mla":
+        names = ("q_a", "q_b", "kv_a", "o")
+        w, other = synth.mla_weights(cuda, seed=1), synth.mla_weights(cuda, seed=2)
+        layer = lib.MlaLayer(w, max_batch=rows, max_ctx=128)
+        hidden, cache0 = 7168, synth.latent_cache(rows, 128, cuda)
+        pos = torch.full((rows,), 90, dtype=torch.int32, device=cuda)
+        call = lambda y: layer.decode(y, cache0.clone(), pos)  # noqa: E731
+    else:
+        hidden = 2048
+        w, other = (synth.moe_layer_weights(cuda, seed=s, hidden=hidden, inter=1024, experts=128, shared_inter=1024) for s in (1, 2))
+        if what == "moe":
+            names = ("router_w", "shared_gate", "shared_up", "shared_down")
+            layer = lib.MoeLayer(w, max_tokens=rows)
+            call = layer.batched
+        else:
+            w, other = ({k: v[3].contiguous() for k, v in t.items() if v.dim() == 3} for t in (w, other))
+            names = ("gate_w", "gate_s", "up_w", "up_s", "down_w", "down_s")
+            call = lambda y: lib.expert_ffn(*(w[k] for k in names), y[0])[None]  # noqa: E731
+    sets = [{k: t[k].clone() for k in names} for t in (w, other)]
+    ln = torch.ones(hidden, device=cuda, dtype=torch.bfloat16)
+    turn = [0]
+
+    def step(y):
+        y = lib.rmsnorm(y, ln)
+        turn[0] += 1
+        for k in names:
+            w[k].copy_(sets[turn[0] % 2][k])
+        return call(y)
+
+    _same(step, synth.activations(rows, hidden, cuda, 4))
