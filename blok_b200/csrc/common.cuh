@@ -43,11 +43,12 @@ int sm_count();
 // dependent launch), which takes the launch and the start of its blocks off the critical path; captured into graphs like any
 // other launch.  For kernels whose blocks fill an SM (shared memory) or are few and small.  Not for the mat-vec kernels: blocks
 // that come early crowd on the SMs that have room, and the stream of weights is then uneven (o_proj over 8 rows 29 -> 80 us).
+// overlap false: an ordinary launch of the same kernel.
 template <typename... P, typename... A>
-inline int launch_pdl(const char *what, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+inline int launch_pdl_if(bool overlap, const char *what, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].val.programmaticStreamSerializationAllowed = overlap ? 1 : 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -58,6 +59,10 @@ inline int launch_pdl(const char *what, void (*kernel)(P...), dim3 grid, dim3 bl
   count_launch();
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
   return e == cudaSuccess ? BLOK_OK : cuda_fail(e, what);
+}
+template <typename... P, typename... A>
+inline int launch_pdl(const char *what, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  return launch_pdl_if(true, what, kernel, grid, block, smem, stream, args...);
 }
 
 // ---- device helpers ----------------------------------------------------------

@@ -144,7 +144,7 @@ extern "C" int blok_mla_layer_create(const blok_mla_weights *w, int max_batch, i
   size_t o_pml = take((size_t)(L->max_splits + max_batch) * w->heads * 2 * 4);
   const size_t q_rows = (size_t)w->heads * qk_head;
   L->wg_bytes = (size_t)max_batch * sizeof(float) *
-                std::max(std::max((size_t)wgemm_stream_pair_split(w->hidden, w->q_rank, lat_w) * (w->q_rank + lat_w),
+                std::max(std::max((size_t)wgemm_stream_pair_split(WG_BF16_PLAIN, w->hidden, w->q_rank, lat_w) * (w->q_rank + lat_w),
                                   wgemm_stream_split(WG_BF16_PLAIN, w->q_rank, (int)q_rows) * q_rows),
                          (size_t)wgemm_stream_split(WG_BF16_PLAIN, w->heads * w->v_head, w->hidden) * w->hidden);
   size_t o_wg = take(L->wg_bytes);
@@ -347,7 +347,7 @@ static int decode_body(blok_mla_layer *L, const uint16_t *n, const CacheRef &c, 
   g.splitk_bytes = L->wg_bytes;
   g.err = L->err + 1;
   // q_a and kv_a, then the norms and the cache row   (:813-824)
-  g.w_a = w.q_a; g.R = w.q_rank; g.w_b = w.kv_a; g.R2 = lat_w; g.x = n; g.K = w.hidden;
+  g.w_a = w.q_a; g.R = w.q_rank; g.w_2 = w.kv_a; g.R2 = lat_w; g.x = n; g.K = w.hidden;
   g.keep_sums = true;
   if ((rc = launch_wgemm_stream(WG_BF16_PLAIN, g, &nz, stream))) return rc;
   MlaNorm m = {};
@@ -358,7 +358,7 @@ static int decode_body(blok_mla_layer *L, const uint16_t *n, const CacheRef &c, 
   if ((rc = launch_mla_norm(m, B, stream))) return rc;
   // q_b, then q_abs = W_UK^T q_nope and the rotated rope part.  The head kernels read a head's sums four times over: with many
   // entries one part and bf16
-  g.w_a = w.q_b; g.R = w.heads * qk_head; g.w_b = nullptr; g.R2 = 0; g.x = L->qa; g.K = w.q_rank; g.out_bf16 = L->q;
+  g.w_a = w.q_b; g.R = w.heads * qk_head; g.w_2 = nullptr; g.R2 = 0; g.x = L->qa; g.K = w.q_rank; g.out_bf16 = L->q;
   g.keep_sums = false; g.max_splits = B > 16 ? 1 : 0; g.weights_early = true;
   if ((rc = launch_wgemm_stream(WG_BF16_PLAIN, g, &nz, stream))) return rc;
   MlaQuery q = {};

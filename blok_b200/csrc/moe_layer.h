@@ -55,6 +55,7 @@ struct blok_moe_layer {
   uint16_t *b_sout = nullptr;    // [T, hidden]
   float *b_splitk = nullptr;     // K-split partial sums of the bf16 products over one tile of tokens
   size_t b_splitk_bytes = 0;
+  int b_front_split = 0;         // K split of the router and the shared expert's first half over up to 64 tokens
   unsigned *b_err = nullptr;     // [1] set when a wait of a tcgen05 product of this handle gave up
   // fused decode kernel scratch
   blok::FusedPlan plan;

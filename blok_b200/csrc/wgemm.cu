@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kWgThreads) wgemm_kernel(const WgArgs a) {
 size_t wgemm_smem_bytes() { return (size_t)kWgTokens * kWgTokPitch; }
 
 // 0 = pick by size, 1 = mma.sync kernel always, 2 = tcgen05 kernels wherever they apply
-static int wgemm_forced_impl() {  // read at every launch, so that a test can switch it inside one process
+int wgemm_forced_impl() {  // read at every launch, so that a test can switch it inside one process
   const char *e = getenv("BLOK_WGEMM_IMPL");
   if (e && strcmp(e, "mma") == 0) return 1;
   if (e && strcmp(e, "tc") == 0) return 2;

@@ -37,13 +37,18 @@ struct WgArgs {
   size_t splitk_bytes = 0;
   // INT4 modes, where the host knows only a bound of them: the assignments that pick the kernel, a device word (launch_wgemm_experts)
   const int *total = nullptr;
-  // The weight-streaming kernel only.  A second matrix over the same rows (w_b, R2 rows, bf16 to out2): its tiles follow the first's,
-  // its partial sums the first's R columns.  max_splits: a bound of the K split (0: none).  keep_sums: fp32 sums in
+  // The weight-streaming kernel only.  A second matrix over the same rows (w_2, R2 rows, bf16 to out2; beside a gated product with
+  // keep_sums only): its tiles follow the first's, its partial sums the first's columns.  max_splits: a bound of the K split (0: none).  keep_sums: fp32 sums in
   // splitk_ws also where K is not split.  weights_early: the weights may be fetched
   // before the kernels in front of this launch have finished (the caller has launched one since they were written, in this call).
+  const void *w_2 = nullptr;
   int R2 = 0, max_splits = 0;
   uint16_t *out2 = nullptr;
   bool keep_sums = false, weights_early = false;
+  // INT4 modes: the launches become resident while the ones before them run.  For few tokens, where they are short: layers of 3, 64 (2048 x
+  // 1024, 128 experts) and 6 (7168 x 2048) tokens 59 -> 56, 139 -> 130, 259 -> 254 us; over 2,048 tokens 1 to 2 % slower (blocks that come
+  // early hold registers that the many blocks of the layout and the combination want).
+  bool overlap = false;
   unsigned *err = nullptr;  // set to 1 when a tcgen05 kernel's wait gives up: a word of the handle the launch is for
 };
 
@@ -52,6 +57,7 @@ struct WgArgs {
 // (gemm_tma.cu), K split where its tiles are few; for shapes the others do not cover the mma.sync kernel with its K-split.
 // BLOK_WGEMM_IMPL=mma / =tc in the environment forces one GEMM kernel for every row (no small-group or streaming kernel).
 int launch_wgemm(int mode, const WgArgs &args, int max_tiles, cudaStream_t stream);
+int wgemm_forced_impl();  // 0: none forced
 
 // A bf16 product over few tiles of tokens has (R / 128 or R / 64) x tiles CTAs, far fewer than the GPU has SMs (3 per
 // tile for a 384-expert router): the mma.sync kernel then splits K over blockIdx.z so that about two CTAs per SM run,
@@ -73,7 +79,7 @@ int launch_wgemv_small(int mode, const WgArgs &args, cudaStream_t stream);
 // wgemm_stream_supports: what launch_wgemm hands to it; the launch itself takes any K % 8 == 0 and R.
 bool wgemm_stream_supports(int mode, const WgArgs &args);
 int wgemm_stream_split(int mode, int K, int R);
-int wgemm_stream_pair_split(int K, int R, int R2);
+int wgemm_stream_pair_split(int mode, int K, int R, int R2);
 // *out becomes non-zero if a CTA without an error word of its own has given up since the last call (the flag is cleared).
 int wgemm_stream_take_error(unsigned *out);
 // The reduction behind a K-split launch: adds the nz partial sums in split order and applies the epilogue.

@@ -41,14 +41,15 @@ struct StArgs {
   float *part;         // fp32 [split][token][ld] where K is split, else NULL
   uint16_t *out_bf16;  // [token][R]
   float *out_f32;
-  uint16_t *out2;      // the second matrix's output (tiles from tiles1 on), bf16; its partial sums follow the first's R columns
+  uint16_t *out2;      // the second matrix's output (tiles from tiles1 on), bf16; its partial sums follow the first's columns
   int T, N, K, R, R2, tiles1, ld, stages, early;
   unsigned *err;
 };
 
 template <bool SWIGLU>
 __global__ void __launch_bounds__(kStThreads) wgemm_stream_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mwa,
-                                                                  const __grid_constant__ CUtensorMap mwb, const StArgs a) {
+                                                                  const __grid_constant__ CUtensorMap mwb, const __grid_constant__ CUtensorMap mw2,
+                                                                  const StArgs a) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long s_bar[2 * kStMaxStages + 1];
   __shared__ uint32_t s_tmem;
@@ -73,7 +74,7 @@ __global__ void __launch_bounds__(kStThreads) wgemm_stream_kernel(const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_tmem;
-  const bool second = !SWIGLU && (int)blockIdx.x >= a.tiles1;
+  const bool second = (int)blockIdx.x >= a.tiles1, gated = SWIGLU && !second;
   const int tile = second ? (int)blockIdx.x - a.tiles1 : (int)blockIdx.x;
   const int all_steps = (a.K + kStCols - 1) / kStCols, nz = (int)gridDim.y, z = (int)blockIdx.y;
   const int first = all_steps * z / nz, nsteps = all_steps * (z + 1) / nz - first;
@@ -85,11 +86,11 @@ __global__ void __launch_bounds__(kStThreads) wgemm_stream_kernel(const __grid_c
       auto weights = [&](int c, uint32_t dst, uint32_t bar) {
         const int k = (first + c) * kStCols;
         tp_expect_tx(bar, stage);
-        if (SWIGLU) {
+        if (gated) {
           tp_load_2d(dst, &mwa, k, tile * (kStRows / 2), bar);
           tp_load_2d(dst + kStWBytes / 2, &mwb, k, tile * (kStRows / 2), bar);
         } else {
-          tp_load_2d(dst, second ? &mwb : &mwa, k, tile * kStRows, bar);
+          tp_load_2d(dst, second ? &mw2 : &mwa, k, tile * kStRows, bar);
         }
       };
       const int pre = min(S, nsteps);
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(kStThreads) wgemm_stream_kernel(const __grid_c
     const int r = 32 * warp + lane;
     const uint32_t at = tmem + ((uint32_t)(32 * warp) << 16);
     const int R = second ? a.R2 : a.R;
-    if (SWIGLU && !a.part) {
+    if (gated && !a.part) {
       // the up half hands its sums over through the ring's memory (every copy into it has been consumed)
       float *up = reinterpret_cast<float *>(smem_raw);
       const int row = tile * (kStRows / 2) + (r & 63);
@@ -167,8 +168,8 @@ __global__ void __launch_bounds__(kStThreads) wgemm_stream_kernel(const __grid_c
         asm volatile("bar.sync 1, 128;" ::: "memory");
       }
     } else {
-      const int row = SWIGLU ? tile * (kStRows / 2) + (r & 63) : tile * kStRows + r;
-      const int col = SWIGLU && r >= 64 ? R + row : (second ? a.R + row : row);  // of the partial sums
+      const int row = gated ? tile * (kStRows / 2) + (r & 63) : tile * kStRows + r;
+      const int col = second ? a.ld - a.R2 + row : (gated && r >= 64 ? R + row : row);  // of the partial sums
       const size_t ld = a.part ? a.ld : R;
       float *f32 = a.part ? a.part + (size_t)z * a.T * ld + col : (a.out_f32 && !second ? a.out_f32 + row : nullptr);
       uint16_t *b16 = (second ? a.out2 : a.out_bf16) + row;
@@ -215,17 +216,17 @@ int wgemm_stream_split(int mode, int K, int R) {
   if (mode != WG_BF16_PLAIN && mode != WG_BF16_SWIGLU) return 1;
   return st_split(K, st_tiles(mode, R));
 }
-int wgemm_stream_pair_split(int K, int R, int R2) { return st_split(K, st_tiles(WG_BF16_PLAIN, R) + st_tiles(WG_BF16_PLAIN, R2)); }
+int wgemm_stream_pair_split(int mode, int K, int R, int R2) { return st_split(K, st_tiles(mode, R) + st_tiles(WG_BF16_PLAIN, R2)); }
 
 // Launches the kernel; *splits = the K-split it used (> 1: the partial sums wait in args.splitk_ws for the reduce kernel).
 int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t stream) {
   const bool swiglu = mode == WG_BF16_SWIGLU;
-  BLOK_REQUIRE(args.K % 8 == 0 && args.R >= 1 && args.n_rows >= 1 && args.n_rows <= kWgStreamTokens && !(swiglu && args.R2), BLOK_ERR_SHAPE,
+  BLOK_REQUIRE(args.K % 8 == 0 && args.R >= 1 && args.n_rows >= 1 && args.n_rows <= kWgStreamTokens && (!swiglu || !args.R2 || args.keep_sums), BLOK_ERR_SHAPE,
                "streaming product: %d rows x %d columns over %d tokens", args.R, args.K, args.n_rows);
   StArgs a;
   a.tiles1 = st_tiles(mode, args.R);
-  const int tiles = a.tiles1 + (args.R2 ? st_tiles(mode, args.R2) : 0);
-  a.ld = swiglu ? 2 * args.R : args.R + args.R2;
+  const int tiles = a.tiles1 + (args.R2 ? st_tiles(WG_BF16_PLAIN, args.R2) : 0);
+  a.ld = (swiglu ? 2 * args.R : args.R) + args.R2;
   const size_t per_split = (size_t)args.n_rows * a.ld * sizeof(float);
   const size_t room = args.splitk_ws ? args.splitk_bytes / per_split : 0;
   BLOK_REQUIRE(!args.keep_sums || room >= 1, BLOK_ERR_WORKSPACE, "streaming product: no room for the sums");
@@ -244,19 +245,17 @@ int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t 
   // as many steps as two CTAs per SM leave room for: 108, 100, 88 and 96 KB
   a.stages = a.N == 16 ? 6 : (a.N == 32 ? 5 : 4);
   const int smem = a.stages * (int)(kStWBytes + a.N * kStCols * 2) + 1024;
-  CUtensorMap mx, mwa, mwb;
+  CUtensorMap mx, mwa, mwb, mw2;
   int rc;
   if ((rc = gemm_operand_map(args.x, args.n_rows, args.K, args.K, a.N, &mx))) return rc;
   if ((rc = gemm_operand_map(args.w_a, args.R, args.K, args.K, swiglu ? kStRows / 2 : kStRows, &mwa))) return rc;
-  if (swiglu || args.R2) {
-    if ((rc = gemm_operand_map(args.w_b, swiglu ? args.R : args.R2, args.K, args.K, swiglu ? kStRows / 2 : kStRows, &mwb))) return rc;
-  } else {
-    mwb = mwa;
-  }
+  mwb = mw2 = mwa;
+  if (swiglu && (rc = gemm_operand_map(args.w_b, args.R, args.K, args.K, kStRows / 2, &mwb))) return rc;
+  if (args.R2 && (rc = gemm_operand_map(args.w_2, args.R2, args.K, args.K, kStRows, &mw2))) return rc;
   auto kernel = swiglu ? wgemm_stream_kernel<true> : wgemm_stream_kernel<false>;
   BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   *splits = nz;
-  return launch_pdl("wgemm_stream_kernel", kernel, dim3(tiles, nz), kStThreads, (size_t)smem, stream, mx, mwa, mwb, a);
+  return launch_pdl("wgemm_stream_kernel", kernel, dim3(tiles, nz), kStThreads, (size_t)smem, stream, mx, mwa, mwb, mw2, a);
 }
 
 int wgemm_stream_take_error(unsigned *out) {

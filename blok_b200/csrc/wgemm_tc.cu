@@ -93,6 +93,9 @@ struct I4Args {
   const void *w_a, *w_b;  // the operands again, for i4_plain_rows
   const uint16_t *s_a, *s_b, *x;
   unsigned *err;
+  // the launch before is the gate/up product of the same experts: weights, scales and the tile table are there, what that product
+  // writes and reads (activations, results' buffer) only behind the wait
+  int early;
 };
 
 // The epilogue of a thread's two sums for one token: gate and up, or two rows of the down projection 128 apart.
@@ -199,7 +202,7 @@ __device__ __forceinline__ bool i4_mma(const I4Mma &m, const I4Args &a, int unit
   I4Ring<2> dr;
   uint32_t aturn = 0;
   for (int u = blockIdx.x; u < units; u += gridDim.x) {
-    const uint32_t idesc = tp_idesc_bf16(((__ldg(a.tile_count + u / blocks) + 15) >> 4) << 4);
+    const uint32_t idesc = tp_idesc_bf16(((a.tile_count[u / blocks] + 15) >> 4) << 4);
     if (!__all_sync(0xffffffffu, i4_wait<0>(m.d_empty + 8 * dr.slot, dr.turn ^ 1))) return false;
     const uint32_t d = (uint32_t)(dr.slot * 2 + BLK) * kTcN;
     for (int st = 0; st < stages; ++st) {
@@ -234,6 +237,8 @@ template <bool SWIGLU>
 __global__ void __launch_bounds__(kI4Threads, 1)
     wgemm_tc_kernel(const __grid_constant__ CUtensorMap mwa, const __grid_constant__ CUtensorMap mwb, const __grid_constant__ CUtensorMap msa,
                     const __grid_constant__ CUtensorMap msb, const __grid_constant__ CUtensorMap mx, const __grid_constant__ I4Args a) {
+  if (!a.early) pdl_wait();
+  pdl_trigger();  // behind the wait of the gate/up product: the down projection reads weights and tile table before its own
   if (a.total && *a.total <= kWgSmallRows) return;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long s_bar[2 * (kI4WStages + kI4XStages + 8 + 2)];
@@ -328,6 +333,7 @@ __global__ void __launch_bounds__(kI4Threads, 1)
   } else if (warp >= 4) {
     const int quarter = warp & 3, row = 32 * quarter + lane;
     I4Ring<2> dr;
+    pdl_wait();
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
       const int tile = u / blocks, row0 = (u - tile * blocks) * kRows;
       const int p0 = a.tile_start[tile], cnt = a.tile_count[tile];
@@ -396,6 +402,7 @@ __global__ void __launch_bounds__(kI4Threads, 1)
     if (lane == 0) {
       I4Ring<kI4XStages> xr;
       long issued = 0;
+      pdl_wait();
       for (int u = blockIdx.x; u < units && !failed; u += gridDim.x) {
         const int tile = u / blocks, p0 = a.tile_start[tile], rows16 = (a.tile_count[tile] + 15) >> 4;
         for (int c = 0; c < 2 * stages; ++c) {
@@ -428,9 +435,10 @@ __global__ void __launch_bounds__(kI4Threads, 1)
 
 // xs[p] = x[x_index ? x_index[p] : p] for the sorted positions p of every tile, the columns of each packed word in the
 // order 0 4 1 5 2 6 3 7.  grid = (tile slots, parts of a tile).
-__global__ void __launch_bounds__(256) i4_rows_kernel(const uint16_t *__restrict__ x, const int *__restrict__ x_index, int K,
-                                                      const int *__restrict__ tile_start, const int *__restrict__ tile_count,
-                                                      const int *__restrict__ num_tiles, const int *__restrict__ total, uint16_t *__restrict__ xs) {
+__global__ void __launch_bounds__(256) i4_rows_kernel(const uint16_t *x, const int *x_index, int K, const int *tile_start, const int *tile_count,
+                                                      const int *num_tiles, const int *total, uint16_t *xs) {
+  pdl_wait();
+  pdl_trigger();
   if (total && *total <= kWgSmallRows) return;
   const int ntiles = *num_tiles, per_row = K / 8;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -474,21 +482,16 @@ static int i4_launch(bool swiglu, const WgArgs &g, const uint16_t *x, long x_row
   }
   if ((rc = tensor_map_2d(x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x_rows, g.K, (long)g.K * 2, 16, 64, CU_TENSOR_MAP_SWIZZLE_128B, &mx))) return rc;
   const I4Args a = {g.out_bf16, g.out_index, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.K, g.R, (int)g.expert_stride_rows, g.total,
-                    g.w_a, g.w_b, g.s_a, g.s_b, x, g.err};
-  if (swiglu) {
-    BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kI4Smem));
-    wgemm_tc_kernel<true><<<sm_count(), kI4Threads, kI4Smem, stream>>>(wa, wb, sa, sb, mx, a);
-  } else {
-    BLOK_CUDA(cudaFuncSetAttribute(wgemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kI4Smem));
-    wgemm_tc_kernel<false><<<sm_count(), kI4Threads, kI4Smem, stream>>>(wa, wb, sa, sb, mx, a);
-  }
-  return launch_status("wgemm_tc_kernel");
+                    g.w_a, g.w_b, g.s_a, g.s_b, x, g.err, g.overlap && !swiglu};
+  auto kernel = swiglu ? wgemm_tc_kernel<true> : wgemm_tc_kernel<false>;
+  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kI4Smem));
+  return launch_pdl_if(g.overlap, "wgemm_tc_kernel", kernel, sm_count(), kI4Threads, (size_t)kI4Smem, stream, wa, wb, sa, sb, mx, a);
 }
 
 int launch_wgemm_i4(const WgArgs &up, const WgArgs &down, uint16_t *xs, long rows, int max_tiles, cudaStream_t stream) {
   // a tile's rows are shared by a few CTAs: 64 rows of 7,168 columns are 57,344 16-byte pieces
-  i4_rows_kernel<<<dim3(std::min(max_tiles, 1024), 4), 256, 0, stream>>>(up.x, up.x_index, up.K, up.tile_start, up.tile_count, up.num_tiles, up.total, xs);
-  int rc = launch_status("i4_rows_kernel");
+  int rc = launch_pdl_if(up.overlap, "i4_rows_kernel", i4_rows_kernel, dim3(std::min(max_tiles, 1024), 4), 256, 0, stream, up.x, up.x_index, up.K, up.tile_start,
+                      up.tile_count, up.num_tiles, up.total, xs);
   if (rc) return rc;
   if ((rc = i4_launch(true, up, xs, rows, stream))) return rc;
   return i4_launch(false, down, up.out_bf16, rows, stream);

@@ -199,6 +199,8 @@ __device__ __forceinline__ void gs_stream_by_count(int cnt, const GsStream &q, i
 
 template <bool SWIGLU>
 __global__ void __launch_bounds__(kGsThreads, 1) wgemv_small_kernel(const WgArgs a) {
+  pdl_wait();
+  pdl_trigger();
   if (a.total && *a.total > kWgSmallRows) return;  // the tcgen05 kernel's
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ unsigned short s_group[kGsMaxGroups];  // the launch's passes: tile index | pass of the tile << 12
@@ -322,14 +324,9 @@ bool wgemv_small_supports(int mode, const WgArgs &a, int max_rows) {
 int launch_wgemv_small(int mode, const WgArgs &args, cudaStream_t stream) {
   const size_t smem = wgemv_small_smem_bytes(args.K);
   const int grid = sm_count();
-  if (mode == WG_I4_SWIGLU) {
-    BLOK_CUDA(cudaFuncSetAttribute(wgemv_small_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    wgemv_small_kernel<true><<<grid, kGsThreads, smem, stream>>>(args);
-  } else {
-    BLOK_CUDA(cudaFuncSetAttribute(wgemv_small_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    wgemv_small_kernel<false><<<grid, kGsThreads, smem, stream>>>(args);
-  }
-  return launch_status("wgemv_small_kernel");
+  auto kernel = mode == WG_I4_SWIGLU ? wgemv_small_kernel<true> : wgemv_small_kernel<false>;
+  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  return launch_pdl_if(args.overlap, "wgemv_small_kernel", kernel, grid, kGsThreads, smem, stream, args);
 }
 
 }  // namespace blok

@@ -186,3 +186,29 @@ def test_a_product_that_gave_up_is_reported_by_its_own_handle(cuda):
     assert lib.load().blok_moe_layer_debug_set_error(one._handle, C.c_uint(256), None) == -4  # no such products on this handle
     for layer in (a, b, one):
         layer.close()
+
+
+@pytest.mark.parametrize("T,experts,topk,hidden,inter,shared", [
+    (1, 128, 8, 512, 512, 512), (2, 384, 8, 1024, 512, 0), (31, 128, 1, 1536, 512, 1024), (32, 256, 6, 512, 1024, 512),
+    (33, 384, 32, 512, 512, 512), (63, 128, 32, 2048, 512, 2048), (64, 384, 8, 1024, 512, 512), (64, 128, 7, 512, 512, 0)])
+def test_front_of_a_small_batch(cuda, monkeypatch, T, experts, topk, hidden, inter, shared):
+    """Up to 64 tokens the router and the shared expert's first half are one launch and what follows them another (routing, sorted
+    order, tile table, gated vector): against the separate launches that BLOK_WGEMM_IMPL=tc takes, at the edges of warps and tiles."""
+    from blok_b200 import lib, synth
+    w = synth.moe_layer_weights(cuda, seed=T + experts, hidden=hidden, inter=inter, experts=experts, shared_inter=shared)
+    for k in ("gate_s", "up_s", "down_s"):
+        w[k] = (w[k].float() * 8).bfloat16()
+    w["router_w"] = (w["router_w"].float() * 20).bfloat16()
+    layer = lib.MoeLayer(w, topk=topk, max_tokens=T + 1)
+    x = synth.activations(T, hidden, cuda, T)
+    monkeypatch.delenv("BLOK_WGEMM_IMPL", raising=False)
+    y, ids, wts = layer.batched(x, return_routing=True)
+    assert torch.equal(y, layer.batched(x))
+    monkeypatch.setenv("BLOK_WGEMM_IMPL", "tc")
+    want, wid, wwt = layer.batched(x, return_routing=True)
+    assert torch.equal(ids, wid)                       # fp32 logits, summed in another order
+    assert float(((wts - wwt).abs() / wwt.abs().clamp(min=1e-6)).max()) < 1e-4
+    # eight roundings to bf16 on each side, the intermediate vectors' and the outputs' among them (2^-9 / sqrt(3) each, rms)
+    assert float((y.float() - want.float()).norm() / want.float().norm()) < 1e-2
+    layer.check()
+    layer.close()
