@@ -190,7 +190,7 @@ def test_a_product_that_gave_up_is_reported_by_its_own_handle(cuda):
 
 @pytest.mark.parametrize("T,experts,topk,hidden,inter,shared", [
     (1, 128, 8, 512, 512, 512), (2, 384, 8, 1024, 512, 0), (31, 128, 1, 1536, 512, 1024), (32, 256, 6, 512, 1024, 512),
-    (33, 384, 32, 512, 512, 512), (63, 128, 32, 2048, 512, 2048), (64, 384, 8, 1024, 512, 512), (64, 128, 7, 512, 512, 0)])
+    (33, 384, 16, 512, 512, 512), (63, 128, 16, 2048, 512, 2048), (64, 384, 8, 1024, 512, 512), (64, 128, 7, 512, 512, 0)])
 def test_front_of_a_small_batch(cuda, monkeypatch, T, experts, topk, hidden, inter, shared):
     """Up to 64 tokens the router and the shared expert's first half are one launch and what follows them another (routing, sorted
     order, tile table, gated vector): against the separate launches that BLOK_WGEMM_IMPL=tc takes, at the edges of warps and tiles."""
