@@ -12,8 +12,8 @@
 // in flight, releases its tensor memory and returns.
 #include <mutex>
 
-#include "gemm_tma.h"
-#include "tc_pipe.cuh"
+#include "gemm_epilogue.cuh"
+#include "gemm_pair.h"
 
 namespace blok {
 
@@ -29,23 +29,6 @@ struct GtCfg {
 };
 
 __device__ unsigned g_gemm_tma_error = 0;
-
-struct GtArgs {
-  void *out;
-  const int *tile_expert, *tile_start, *tile_count, *num_tiles;
-  int T, R, K, ldo, act_cols, up_row;
-  unsigned *err;
-};
-
-template <int ACT>
-__device__ __forceinline__ float gt_act(float v) {
-  if (ACT == GEMM_ACT_RELU2) {
-    v = fmaxf(v, 0.f);
-    return v * v;
-  }
-  if (ACT == GEMM_ACT_SILU) return __fdividef(v, 1.0f + __expf(-v));  // the result is rounded to bf16
-  return v;
-}
 
 template <int BN, int ACT, bool F32>
 __global__ void __launch_bounds__(kGtThreads)
@@ -139,71 +122,7 @@ __global__ void __launch_bounds__(kGtThreads)
     failed = __any_sync(0xffffffffu, failed);
     tc_fence_after();
     const int r = 32 * warp + lane;
-    const size_t o = ((size_t)blockIdx.z * a.T + row0 + r) * a.ldo;
-    const int n0 = blockIdx.x * kCols;
-    if constexpr (kGated) {
-#pragma unroll 1
-      for (int c0 = 0; c0 < kCols; c0 += 16) {
-        if (n0 + c0 >= a.R) break;
-        uint32_t gate[16], up[16];
-        const uint32_t at = tmem + ((uint32_t)(32 * warp) << 16) + c0;
-        tmem_ld16(at, gate);
-        tmem_ld16(at + kCols, up);
-        tmem_wait_ld();
-        if (failed) {  // nothing that looks like a result
-#pragma unroll
-          for (int j = 0; j < 16; ++j) gate[j] = up[j] = 0x7fc00000u;
-        }
-        if (r < count) {
-#pragma unroll
-          for (int j = 0; j < 16; j += 4) {
-            const int col = n0 + c0 + j;
-            if (col < a.R) {
-              if (F32) {  // the parts of a K split
-                *reinterpret_cast<uint4 *>(static_cast<float *>(a.out) + o + col) = make_uint4(gate[j], gate[j + 1], gate[j + 2], gate[j + 3]);
-                *reinterpret_cast<uint4 *>(static_cast<float *>(a.out) + o + a.R + col) = make_uint4(up[j], up[j + 1], up[j + 2], up[j + 3]);
-                continue;
-              }
-              float f[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                if (ACT == GEMM_ACT_SWIGLU_REF) {
-                  const float g = round_bf16(__uint_as_float(gate[j + i]));
-                  f[i] = round_bf16(g / (1.0f + expf(-g))) * round_bf16(__uint_as_float(up[j + i]));
-                } else {
-                  f[i] = gt_act<GEMM_ACT_SILU>(__uint_as_float(gate[j + i])) * __uint_as_float(up[j + i]);
-                }
-              }
-              *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(a.out) + o + col) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
-            }
-          }
-        }
-      }
-    } else {
-#pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
-        if (n0 + c0 >= a.R) break;
-        uint32_t v[32];
-        tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + c0, v);
-        tmem_wait_ld();
-        if (failed) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = 0x7fc00000u;
-        }
-        if (r < count) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const int col = n0 + c0 + j;
-            if (col < a.R) {  // R is a multiple of 4
-              float f0 = __uint_as_float(v[j]), f1 = __uint_as_float(v[j + 1]), f2 = __uint_as_float(v[j + 2]), f3 = __uint_as_float(v[j + 3]);
-              if (ACT != GEMM_ACT_SILU || col < a.act_cols) f0 = gt_act<ACT>(f0), f1 = gt_act<ACT>(f1), f2 = gt_act<ACT>(f2), f3 = gt_act<ACT>(f3);
-              if (F32) *reinterpret_cast<float4 *>(static_cast<float *>(a.out) + o + col) = make_float4(f0, f1, f2, f3);
-              else *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(a.out) + o + col) = make_uint2(pack_bf16x2(f0, f1), pack_bf16x2(f2, f3));
-            }
-          }
-        }
-      }
-    }
+    gt_epilogue<BN, ACT, F32>(a, tmem, warp, (size_t)blockIdx.z * a.T + row0 + r, r < count, blockIdx.x * kCols, failed);
   }
   if (failed) atomicExch(a.err ? a.err : &g_gemm_tma_error, 1u);
   tc_fence_before();
@@ -242,9 +161,11 @@ int gemm_operand_map(const void *base, long rows, int cols, long pitch, int box,
   return tensor_map_2d(base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rows, cols, pitch * 2, box, kGtKStep, CU_TENSOR_MAP_SWIZZLE_128B, out);
 }
 
+int gt_wide(const GemmTma &g) { return !g.out_f32 && g.R % 8 == 0 && g.ldo % 8 == 0 && reinterpret_cast<uintptr_t>(g.out) % 16 == 0; }
+
 template <int BN, int ACT, bool F32>
 static int gt_launch(const GemmTma &g, dim3 grid, cudaStream_t stream) {
-  const GtArgs a = {g.out, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.T, g.R, g.K, g.ldo, g.act_cols, g.up_row, g.err};
+  const GtArgs a = {g.out, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.T, g.R, g.K, g.ldo, g.act_cols, g.up_row, g.err, gt_wide(g)};
   BLOK_CUDA(cudaFuncSetAttribute(gemm_tma_kernel<BN, ACT, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, GtCfg<BN>::kSmem));
   gemm_tma_kernel<BN, ACT, F32><<<grid, kGtThreads, GtCfg<BN>::kSmem, stream>>>(
       *g.x, BN == 128 || ACT == GEMM_ACT_SWIGLU || ACT == GEMM_ACT_SWIGLU_REF ? *g.w128 : *g.w256, g.up128 ? *g.up128 : *g.w128, a);
@@ -255,6 +176,7 @@ int launch_gemm_tma(const GemmTma &g, cudaStream_t stream) {
   BLOK_REQUIRE(g.x && g.w128 && g.out && g.R % 4 == 0 && g.K % 8 == 0 && g.T >= 1, BLOK_ERR_SHAPE, "gemm: T %d, R %d, K %d", g.T, g.R, g.K);
   BLOK_REQUIRE(g.splits == 1 || (g.out_f32 && !g.tile_start && (g.act == GEMM_ACT_NONE || g.act == GEMM_ACT_SWIGLU_REF)), BLOK_ERR_SHAPE,
                "gemm: a K split leaves plain fp32 sums");
+  if (gemm_pair_takes(g)) return launch_gemm_pair(g, stream);
   if (g.act == GEMM_ACT_SWIGLU_REF) {
     BLOK_REQUIRE(g.up128 && !g.tile_start && (g.splits > 1) == g.out_f32, BLOK_ERR_SHAPE, "gemm: a gated product is bf16 and not grouped");
     const dim3 grid((g.R + 127) / 128, (g.T + kGtTileRows - 1) / kGtTileRows, g.splits);

@@ -23,6 +23,7 @@ int gemm_operand_map(const void *base, long rows, int cols, long pitch, int box,
 struct GemmTma {
   const CUtensorMap *x = nullptr;              // boxes of kGtTileRows rows
   const CUtensorMap *w128 = nullptr, *w256 = nullptr;  // the weights in boxes of 128 and of 256 rows
+  const CUtensorMap *w64 = nullptr;            // and of 64 (more than 128 rows of x over few weight rows), or NULL
   int T = 0;                                   // rows of x
   int R = 0, K = 0;                            // weight rows (a multiple of 4) and columns (a multiple of 8)
   void *out = nullptr;                         // bf16 or fp32 [T, ldo]
@@ -47,5 +48,6 @@ struct GemmTma {
 int launch_gemm_tma(const GemmTma &g, cudaStream_t stream);
 // *out becomes non-zero if a CTA has given up on a barrier since the last call (the flag is cleared).
 int gemm_tma_take_error(unsigned *out);
+int gemm_pair_take_error(unsigned *out);  // the same for the kernel that takes more than 128 rows
 
 }  // namespace blok

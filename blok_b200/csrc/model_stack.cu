@@ -46,7 +46,7 @@ int pad(int n, int to) { return (n + to - 1) / to * to; }
 struct Mat {
   uint16_t *w = nullptr;
   int R = 0, K = 0;  // padded; experts: R per expert
-  CUtensorMap m128, m256;
+  CUtensorMap m128, m256, m64;
 };
 struct Norm {
   float *w = nullptr, *b = nullptr, alpha = 0.f;
@@ -177,6 +177,7 @@ class Weights {
     t->w = static_cast<uint16_t *>(p);
     if (m_->dtype == BLOK_DTYPE_F32) return BLOK_OK;
     if (int rc = gemm_operand_map(t->w, (long)rows, K, K, 128, &t->m128)) return rc;
+    if (int rc = gemm_operand_map(t->w, (long)rows, K, K, 64, &t->m64)) return rc;
     return gemm_operand_map(t->w, (long)rows, K, K, 256, &t->m256);
   }
   // The stored matrix `name` (or rows of it, see fill_rows) into rows row0.. of t.
@@ -550,6 +551,7 @@ int product(StackModel *S, const Mat &w, const void *x, int T, void *y, bool y_f
   TRY(x_map(S, x, w.K, &g.x));
   g.w128 = &w.m128;
   g.w256 = &w.m256;
+  g.w64 = &w.m64;
   g.T = T;
   g.R = g.ldo = w.R;
   g.K = w.K;
@@ -872,6 +874,7 @@ int run_latent(const Call &c, const LayerState &L, const Run &r) {
     TRY(x_map(S, S->c_all, s.rank, &g.x));
     g.w128 = &L.kvb.m128;
     g.w256 = &L.kvb.m256;
+    g.w64 = &L.kvb.m64;
     g.T = n;
     g.R = g.ldo = L.kvb.R;
     g.K = s.rank;
@@ -1203,6 +1206,8 @@ int stack_check(blok_model *, blok_stream_t stream) {
   BLOK_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
   unsigned err = 0;
   TRY(gemm_tma_take_error(&err));
+  BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");
+  TRY(gemm_pair_take_error(&err));
   BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");
   TRY(wgemm_stream_take_error(&err));
   BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");

@@ -118,15 +118,16 @@ extern "C" int blok_gemm_bf16(const blok_bf16_t *x, const blok_bf16_t *w, int T,
                               blok_stream_t stream) {
   BLOK_REQUIRE(x && w && (out_bf16 != nullptr) != (out_f32 != nullptr), BLOK_ERR_ARG, "blok_gemm_bf16: need x, w and exactly one output");
   BLOK_REQUIRE(T >= 1 && R >= 4 && R % 4 == 0 && K >= 8 && K % 8 == 0, BLOK_ERR_SHAPE, "blok_gemm_bf16: T %d, R %d (a multiple of 4), K %d (of 8)", T, R, K);
-  CUtensorMap mx, m128, m256;
+  CUtensorMap mx, m128, m256, m64;
   int rc;
   if ((rc = gemm_operand_map(x, T, K, K, kGtTileRows, &mx)) || (rc = gemm_operand_map(w, R, K, K, 128, &m128)) ||
-      (rc = gemm_operand_map(w, R, K, K, 256, &m256)))
+      (rc = gemm_operand_map(w, R, K, K, 256, &m256)) || (rc = gemm_operand_map(w, R, K, K, 64, &m64)))
     return rc;
   GemmTma g;
   g.x = &mx;
   g.w128 = &m128;
   g.w256 = &m256;
+  g.w64 = &m64;
   g.T = T;
   g.R = g.ldo = R;
   g.K = K;

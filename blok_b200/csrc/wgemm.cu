@@ -217,16 +217,17 @@ static bool wgemm_tma_supports(int mode, const WgArgs &a) {
 // forced: no K split, so that a row's sums do not depend on how many rows the launch has
 static int launch_wgemm_tma(int mode, const WgArgs &a, int forced, cudaStream_t stream) {
   const bool swiglu = mode == WG_BF16_SWIGLU;
-  CUtensorMap mx, mw, mw256, mup;
+  CUtensorMap mx, mw, mw256, mup, mw64;
   int rc;
   if ((rc = gemm_operand_map(a.x, a.n_rows, a.K, a.K, kGtTileRows, &mx))) return rc;
   if ((rc = gemm_operand_map(a.w_a, a.R, a.K, a.K, 128, &mw))) return rc;
   if ((rc = gemm_operand_map(swiglu ? a.w_b : a.w_a, a.R, a.K, a.K, swiglu ? 128 : 256, swiglu ? &mup : &mw256))) return rc;
+  if (!swiglu && (rc = gemm_operand_map(a.w_a, a.R, a.K, a.K, 64, &mw64))) return rc;
   GemmTma g;
   g.x = &mx;
   g.w128 = &mw;
   if (swiglu) g.up128 = &mup;
-  else g.w256 = &mw256;
+  else g.w256 = &mw256, g.w64 = &mw64;
   g.T = a.n_rows; g.R = a.R; g.K = a.K; g.ldo = a.R;
   g.act = swiglu ? GEMM_ACT_SWIGLU_REF : GEMM_ACT_NONE;
   g.out = a.out_f32 ? (void *)a.out_f32 : (void *)a.out_bf16;

@@ -305,10 +305,15 @@ int wgemm_splitk_factor(int mode, int K, int R, int tiles) {
   const int ctas = R / rows_per_cta * tiles, chunks = K / 512;
   return std::max(1, std::min(chunks, 2 * sm_count() / ctas));
 }
-// The TMA-fed GEMM has tiles of 128 rows of x by 128 outputs (256 where that fills the GPU) and two CTAs per SM: parts of at
-// least 16 of its 64-column steps, so that its pipeline fills (the 384-expert router over 517 tokens: 15 tiles, 7 parts).
+// The TMA-fed GEMM: parts of at least 16 of its 64-column steps, so that its pipeline fills.  Up to 128 rows of x tiles of 128
+// outputs and two CTAs per SM; more, pairs of CTAs with tiles of 256 rows by 256 weight rows (the 384-expert router over 517
+// tokens: 6 tiles, 7 parts).
 int wgemm_tma_split(int mode, int K, int R, int rows) {
   if (mode != WG_BF16_PLAIN && mode != WG_BF16_SWIGLU) return 1;
+  if (rows > 128) {
+    const int tiles = ((mode == WG_BF16_SWIGLU ? 2 * R : R) + 255) / 256 * ((rows + 255) / 256);
+    return std::max(1, std::min((K + 63) / 64 / 16, sm_count() / 2 / tiles));
+  }
   const int ctas = (R + 127) / 128 * ((rows + 127) / 128);
   return std::max(1, std::min((K + 63) / 64 / 16, 2 * sm_count() / ctas));
 }
