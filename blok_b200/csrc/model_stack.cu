@@ -94,7 +94,8 @@ struct StackModel {
   Norm final_norm;
   Mat head;
   ExpertPlanArgs *plans_dev = nullptr;
-  int n_plans = 0, max_top = 1;
+  int n_plans = 0, max_top = 1, y_parts = 1;  // y_parts: of the sublayer output that y holds
+  size_t y_rows = 0;
   // step buffers (Act: bf16 or fp32)
   float *x = nullptr, *y = nullptr, *ckr = nullptr, *lin_o = nullptr, *chunk_state = nullptr, *logits = nullptr;
   float4 *token = nullptr;
@@ -565,6 +566,31 @@ int product(StackModel *S, const Mat &w, const void *x, int T, void *y, bool y_f
   return launch_gemm_tma(g, stream);
 }
 
+// The product that ends a sublayer, S->h -> S->y fp32.  Between sandwiched sublayers its only reader is the residual norm, which
+// takes it in parts: more than 128 rows of few weight rows leave most pairs of SMs without a tile, and K is cut then (2,048 x 8,192
+// over 1,000 rows: 32 wide tiles for 74 pairs).
+int sublayer_product(StackModel *S, const Mat &w, const void *x, int T, cudaStream_t stream) {
+  S->y_parts = 1;
+  if (S->spec.sandwich && !S->f32 && T > 128) {
+    const int tiles = (T + 255) / 256 * ((w.R + 255) / 256);
+    const int parts = std::min({4, w.K / 64 / 16, sm_count() / 2 / tiles, (int)(S->y_rows / T)});
+    if (parts > 1) {
+      GemmTma g;
+      TRY(x_map(S, x, w.K, &g.x));
+      g.w128 = &w.m128;
+      g.w64 = &w.m64;
+      g.T = T;
+      g.R = g.ldo = w.R;
+      g.K = w.K;
+      g.out = S->y;
+      g.out_f32 = true;
+      g.splits = S->y_parts = parts;
+      return launch_gemm_tma(g, stream);
+    }
+  }
+  return product(S, w, x, T, S->y, true, stream);
+}
+
 }  // namespace
 
 int stack_describe(blok_model *m, const StackSpec &spec) {
@@ -734,7 +760,8 @@ int stack_build(blok_model *m, const char *dir, uint64_t seed) {
   }
   const size_t slack = kGtTileRows;  // a product's last tile copies whole boxes of rows
   TRY(buffer(m, N * spec.streams * S->W * 4, &S->x));
-  TRY(buffer(m, N * S->max_top * S->W * 4, &S->y));
+  S->y_rows = (spec.sandwich ? 2 : 1) * N * S->max_top;
+  TRY(buffer(m, S->y_rows * S->W * 4, &S->y));
   TRY(buffer(m, (N * S->max_top + slack) * S->W * esz, &S->h));
   TRY(buffer(m, (N + slack) * proj * esz, &S->proj));
   TRY(buffer(m, N * ckr * 4, &S->ckr));
@@ -835,7 +862,7 @@ int run_linear(const Call &c, const LinearMixer &x, const LayerState &L, const R
   g.ldo = L.o.K;
   g.f32 = S->f32;
   TRY(launch_gated_norm(g, c.T, c.stream));
-  return product(S, L.o, S->mix, c.T, S->y, true, c.stream);
+  return sublayer_product(S, L.o, S->mix, c.T, c.stream);
 }
 
 // One product per head: y[t, h, :] = W_h x[t, h, :].
@@ -890,7 +917,7 @@ int run_latent(const Call &c, const LayerState &L, const Run &r) {
     TRY(head_product(c, L.kvb.w + (size_t)s.heads * s.dim * s.rank, (long)s.vdim * s.rank, S->o_lat, (long)s.heads * s.rank, s.rank, S->mix, L.o.K,
                      s.vdim, s.vdim, s.rank, s.heads));
   }
-  return product(S, L.o, S->mix, c.T, S->y, true, c.stream);
+  return sublayer_product(S, L.o, S->mix, c.T, c.stream);
 }
 
 // S->h -> S->y: a selective state space.
@@ -929,7 +956,7 @@ int run_state(const Call &c, const StateMixer &x, const LayerState &L, const Run
   g.ldo = L.o.K;
   g.f32 = S->f32;
   TRY(launch_gate_then_norm(g, x.norm_groups, c.T, c.stream));
-  return product(S, L.o, S->mix, c.T, S->y, true, c.stream);
+  return sublayer_product(S, L.o, S->mix, c.T, c.stream);
 }
 
 template <typename Act>
@@ -960,7 +987,7 @@ int run_grouped(const Call &c, const GroupedMixer &x, const LayerState &L, const
   } else {
     TRY(launch_grouped_attend(s, grouped_query<uint16_t>(S, x, L), r.pool, c.rows, c.T, c.m->cfg.max_ctx, S->part_o, S->part_ml, c.stream));
   }
-  return product(S, L.o, S->mix, c.T, S->y, true, c.stream);
+  return sublayer_product(S, L.o, S->mix, c.T, c.stream);
 }
 
 int run_mixer(const Call &c, const StackLayer &x, const LayerState &L, const Run &r) {
@@ -997,7 +1024,7 @@ int run_dense(const Call &c, const LayerState &L) {
     g.out = mid;
     TRY(launch_gemm_tma(g, c.stream));
   }
-  return product(S, L.down, S->mid, c.T, S->y, true, c.stream);
+  return sublayer_product(S, L.down, S->mid, c.T, c.stream);
 }
 
 bool planned(const StackModel *S, int T, int top) { return !S->f32 && T * top > kGemvAssignments; }
@@ -1065,6 +1092,7 @@ int sandwich_layers(const Call &c) {
   a.ids = m->ids;
   auto step = [&](const Norm &n) {
     a.norm_w = n.w;
+    a.y_parts = S->y_parts;
     const int rc = launch_residual_norm(a, c.stream);
     a.ids = nullptr;
     a.copy = nullptr;

@@ -1,7 +1,8 @@
 // One residual between sandwiched sublayers, in one pass over a token's row: the sublayer's output is normed, scaled and
 // added to the residual, the new residual is normed again into the next sublayer's input.  Both are layer norms without a
 // bias (mean, then the mean of the squared deviations, from registers).  The first pass of a step makes the residual from the
-// embeddings instead.  All of it is fp32; h alone is rounded.  One CTA per token.
+// embeddings instead.  All of it is fp32; h alone is rounded.  One CTA per token.  The sublayer's output may come as the parts of its
+// last product's K split (sublayer_product in model_stack.cu), which costs a read of 8 MB a part over 1,000 tokens of 2,048.
 #include "common.cuh"
 #include "stack_kernels.h"
 
@@ -110,6 +111,15 @@ __global__ void __launch_bounds__(THREADS) residual_norm_kernel(const ResidualNo
         const int c = 4 * (tid + THREADS * k);
         y[k] = c < a.width ? *reinterpret_cast<const float4 *>(a.y + (size_t)t * a.width + c) : make_float4(0.f, 0.f, 0.f, 0.f);
         p[k] = a.post_w && c < a.width ? *reinterpret_cast<const float4 *>(a.post_w + c) : make_float4(1.f, 1.f, 1.f, 1.f);
+      }
+      for (int part = 1; part < a.y_parts; ++part) {
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+          const int c = 4 * (tid + THREADS * k);
+          if (c >= a.width) continue;
+          const float4 v = *reinterpret_cast<const float4 *>(a.y + ((size_t)part * a.T + t) * a.width + c);
+          y[k] = make_float4(y[k].x + v.x, y[k].y + v.y, y[k].z + v.z, y[k].w + v.w);
+        }
       }
       if (a.post_w) rn_layer_norm<THREADS, KEEP>(y, a.true_width, a.eps, s_red);
 #pragma unroll

@@ -65,7 +65,8 @@ struct ResidualNorm {
   uint32_t *last_ids = nullptr;          // [slots] the newest token of every sequence
   const uint32_t *keep_ids = nullptr;    // set: last_ids takes in this call's newest tokens (in a later launch than ids)
   // else x += mult * layer_norm(y) * post_w (post_w NULL: += mult * y) when y is set
-  const float *y = nullptr;              // [T, width]
+  const float *y = nullptr;              // [y_parts, T, width]: the parts are added in order
+  int y_parts = 1;
   const float *post_w = nullptr;
   float mult = 1.f, eps = 0.f;
   float *copy = nullptr;                 // [T, true_width]: x (for parity checks)
