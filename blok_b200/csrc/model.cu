@@ -374,7 +374,11 @@ extern "C" int blok_model_extend_slot(blok_model_t *m, int slot, const uint32_t 
     rows.clear(), places.clear();
     for (int i = 0; i < n_want; ++i)
       if (want[i] >= at && want[i] < at + T) rows.push_back(want[i] - at), places.push_back(i);
-    if (!rows.empty()) {
+    bool in_row = true;  // the places are neighbours in the caller's array
+    for (size_t i = 1; i < places.size(); ++i) in_row = in_row && places[i] == places[0] + (int)i;
+    if (!rows.empty() && in_row) {
+      if ((rc = m->family->logits(m, rows.data(), (int)rows.size(), logits + (size_t)places[0] * c.vocab, stream_))) return rc;
+    } else if (!rows.empty()) {
       got.resize(rows.size() * (size_t)c.vocab);
       if ((rc = m->family->logits(m, rows.data(), (int)rows.size(), got.data(), stream_))) return rc;
       for (size_t i = 0; i < rows.size(); ++i)

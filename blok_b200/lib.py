@@ -53,6 +53,14 @@ def load():
     lib.blok_kernel_launch_count.restype = C.c_longlong
     for name in ("blok_expert_ffn_workspace_bytes", "blok_bf16_mlp_workspace_bytes", "blok_router_workspace_bytes"):
         getattr(lib, name).restype = C.c_size_t
+    # the short calls pass plain integers: an argument object of its own costs as much as the conversion
+    p, i, n = C.c_void_p, C.c_int, C.c_size_t
+    lib.blok_expert_ffn.argtypes = [p] * 8 + [i, i, p, n, p]
+    lib.blok_moe_decode.argtypes = [p] * 6
+    lib.blok_moe_batched.argtypes = [p, p, i, p, p, p, p]
+    lib.blok_mla_decode.argtypes = [p, p, p, C.c_long, p, i, p, p]
+    lib.blok_mla_prefill.argtypes = [p, p, p, C.c_long, p, i, p, p]
+    lib.blok_mla_decode_paged.argtypes = [p, p, p, p, p, i, i, p, i, p, p]
     _lib = lib
     return lib
 
@@ -62,8 +70,22 @@ def _check(rc):
         raise BlokError(rc, load().blok_last_error().decode())
 
 
+def _raw_stream():
+    """The current device's current stream (torch.cuda.current_stream() makes an object of it: 3.3 us of a call that takes 13 on the GPU)."""
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(_raw_stream())
+
+
+def _addr(t, dtype, name="tensor"):
+    """The address of a tensor that _ptr would take, for functions with declared argument types."""
+    if t.dtype is dtype and t.is_cuda and t.is_contiguous():
+        return t.data_ptr()
+    return _ptr(t, dtype, name).value
 
 
 def _ptr(t, dtype=None, name="tensor"):
@@ -111,14 +133,12 @@ def expert_ffn(gate_w, gate_s, up_w, up_s, down_w, down_s, x, workspace=None):
     """One routed expert, y = down(SiLU(gate x) * up x) (src/kimi_exec.cu:853-869)."""
     inter, hidden = gate_w.shape[0], gate_w.shape[1] * 8
     lib = load()
-    need = lib.blok_expert_ffn_workspace_bytes(C.c_int(hidden), C.c_int(inter))
     if workspace is None:
-        workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
+        workspace = torch.empty(lib.blok_expert_ffn_workspace_bytes(hidden, inter), dtype=torch.uint8, device=x.device)
     y = torch.empty(hidden, dtype=torch.bfloat16, device=x.device)
-    _check(lib.blok_expert_ffn(_ptr(gate_w, torch.int32), _ptr(gate_s, torch.bfloat16), _ptr(up_w, torch.int32),
-                               _ptr(up_s, torch.bfloat16), _ptr(down_w, torch.int32), _ptr(down_s, torch.bfloat16),
-                               _ptr(x, torch.bfloat16), _ptr(y), C.c_int(hidden), C.c_int(inter), _ptr(workspace),
-                               C.c_size_t(workspace.numel() * workspace.element_size()), _stream()))
+    i4, b16 = torch.int32, torch.bfloat16
+    _check(lib.blok_expert_ffn(_addr(gate_w, i4), _addr(gate_s, b16), _addr(up_w, i4), _addr(up_s, b16), _addr(down_w, i4), _addr(down_s, b16),
+                               _addr(x, b16), y.data_ptr(), hidden, inter, _addr(workspace, workspace.dtype), workspace.nbytes, _raw_stream()))
     return y
 
 
@@ -268,8 +288,7 @@ class MoeLayer:
         if return_routing:
             ids = torch.empty(self.topk, dtype=torch.int16, device=x.device)
             wts = torch.empty(self.topk, dtype=torch.float32, device=x.device)
-        _check(load().blok_moe_decode(self._handle, _ptr(x, torch.bfloat16, "x"), _ptr(y, torch.bfloat16, "y"), _ptr(ids),
-                                      _ptr(wts), _stream()))
+        _check(load().blok_moe_decode(self._handle, _addr(x, torch.bfloat16, "x"), _addr(y, torch.bfloat16, "y"), _ptr(ids), _ptr(wts), _raw_stream()))
         return (y, ids, wts) if return_routing else y
 
     def has_partial(self):
@@ -296,8 +315,7 @@ class MoeLayer:
         if return_routing:
             ids = torch.empty((T, self.topk), dtype=torch.int16, device=x.device)
             wts = torch.empty((T, self.topk), dtype=torch.float32, device=x.device)
-        _check(load().blok_moe_batched(self._handle, _ptr(x, torch.bfloat16, "x"), C.c_int(T), _ptr(y), _ptr(ids), _ptr(wts),
-                                       _stream()))
+        _check(load().blok_moe_batched(self._handle, _addr(x, torch.bfloat16, "x"), T, y.data_ptr(), _ptr(ids), _ptr(wts), _raw_stream()))
         return (y, ids, wts) if return_routing else y
 
     def check(self):
@@ -523,9 +541,9 @@ class MlaLayer:
         """n bf16 [B, hidden]; cache bf16 [B, ctx_stride, 576] (row ctx_len[b] is written); ctx_len int32 [B] (device)."""
         B = n.shape[0]
         y = torch.empty((B, self.hidden), dtype=torch.bfloat16, device=n.device) if out is None else out
-        _check(load().blok_mla_decode(self._handle, _ptr(n, torch.bfloat16, "n"), _ptr(cache, torch.bfloat16, "cache"),
-                                      C.c_long(cache.shape[1]), _ptr(ctx_len, torch.int32, "ctx_len"), C.c_int(B),
-                                      _ptr(y, torch.bfloat16, "out"), _stream()))
+        b16 = torch.bfloat16
+        _check(load().blok_mla_decode(self._handle, _addr(n, b16, "n"), _addr(cache, b16, "cache"), cache.shape[1], _addr(ctx_len, torch.int32, "ctx_len"), B,
+                                      _addr(y, b16, "out"), _raw_stream()))
         return y
 
     def check(self):
@@ -547,9 +565,9 @@ class MlaLayer:
         first_pos .. first_pos+T-1 are written), first_pos int32 [1] (device)."""
         T = n.shape[0]
         y = torch.empty((T, self.hidden), dtype=torch.bfloat16, device=n.device) if out is None else out
-        _check(load().blok_mla_prefill(self._handle, _ptr(n, torch.bfloat16, "n"), _ptr(cache, torch.bfloat16, "cache"),
-                                       C.c_long(cache.shape[0]), _ptr(first_pos, torch.int32, "first_pos"), C.c_int(T),
-                                       _ptr(y, torch.bfloat16, "out"), _stream()))
+        b16 = torch.bfloat16
+        _check(load().blok_mla_prefill(self._handle, _addr(n, b16, "n"), _addr(cache, b16, "cache"), cache.shape[0],
+                                       _addr(first_pos, torch.int32, "first_pos"), T, _addr(y, b16, "out"), _raw_stream()))
         return y
 
     def decode_paged(self, n, pool, block_table, ctx_len, slot_of=None, out=None):
@@ -557,11 +575,11 @@ class MlaLayer:
         (device), slot_of int32 [B] (device) or None for slot b."""
         B = n.shape[0]
         y = torch.empty((B, self.hidden), dtype=torch.bfloat16, device=n.device) if out is None else out
+        b16, i32 = torch.bfloat16, torch.int32
         _check(load().blok_mla_decode_paged(
-            self._handle, _ptr(n, torch.bfloat16, "n"), _ptr(pool, torch.bfloat16, "pool"),
-            _ptr(block_table, torch.int32, "block_table"), _ptr(slot_of, torch.int32, "slot_of") if slot_of is not None else None,
-            C.c_int(block_table.shape[1]), C.c_int(pool.shape[1]), _ptr(ctx_len, torch.int32, "ctx_len"), C.c_int(B),
-            _ptr(y, torch.bfloat16, "out"), _stream()))
+            self._handle, _addr(n, b16, "n"), _addr(pool, b16, "pool"), _addr(block_table, i32, "block_table"),
+            None if slot_of is None else _addr(slot_of, i32, "slot_of"), block_table.shape[1], pool.shape[1], _addr(ctx_len, i32, "ctx_len"), B,
+            _addr(y, b16, "out"), _raw_stream()))
         return y
 
     def attend_paged(self, q, pool, block_table, seq_len, slot_of=None, scale=None, out=None):
