@@ -73,6 +73,7 @@ struct blok_mla_layer {
   unsigned *err = nullptr;     // [2] 1 + b when entry b of a call had a position outside its sequence's rows; a product gave up
   float *wg_ws = nullptr;      // fp32 sums of the projections (wgemm_stream.cu), one projection's at a time
   size_t wg_bytes = 0;
+  bool weights_stay = false;   // see mla_layer_weights_stay
   float *part_o = nullptr;     // [max_splits + max_batch partial results, heads, kv_rank]
   float *part_ml = nullptr;
   blok::MlaPlan *plan = nullptr;  // of the call's sequences
@@ -80,6 +81,13 @@ struct blok_mla_layer {
 };
 
 using namespace blok;
+
+// For a layer whose calls follow an ordinary launch of the same program that stands behind the last write of its weights, positions
+// and tables (a model's embedding): the first launch of a call, too, may fetch its weights early.
+namespace blok {
+void mla_layer_weights_stay(blok_mla_layer_t *L);
+}
+void blok::mla_layer_weights_stay(blok_mla_layer_t *L) { L->weights_stay = true; }
 
 // YaRN inverse frequencies, src/kimi_exec.cu:325-344 with the factor as a parameter.
 static void yarn_inv_freq_host(const blok_mla_weights &w, float *out) {
@@ -349,6 +357,7 @@ static int decode_body(blok_mla_layer *L, const uint16_t *n, const CacheRef &c, 
   // q_a and kv_a, then the norms and the cache row   (:813-824)
   g.w_a = w.q_a; g.R = w.q_rank; g.w_2 = w.kv_a; g.R2 = lat_w; g.x = n; g.K = w.hidden;
   g.keep_sums = true;
+  g.weights_early = L->weights_stay;
   if ((rc = launch_wgemm_stream(WG_BF16_PLAIN, g, &nz, stream))) return rc;
   MlaNorm m = {};
   m.part = L->wg_ws; m.nz = nz; m.ld = w.q_rank + lat_w; m.q_rank = w.q_rank; m.kv_rank = w.kv_rank; m.rope = w.qk_rope;

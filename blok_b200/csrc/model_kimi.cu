@@ -49,6 +49,12 @@ __global__ void sharded_finish_kernel(const float *__restrict__ part, const uint
   *reinterpret_cast<uint32_t *>(out + (size_t)t * hidden + c) = pack_bf16x2(o0, o1);
 }
 
+// Forms of the public calls for a model whose weights were there before the call's first launch (the embedding, an ordinary one).
+int bf16_mlp(const blok_bf16_t *gate, const blok_bf16_t *up, const blok_bf16_t *down, const blok_bf16_t *x, blok_bf16_t *y, int hidden, int ffn, int T,
+             void *workspace, size_t workspace_bytes, bool weights_early, blok_stream_t stream);
+int lm_head_argmax(const blok_bf16_t *w, const blok_bf16_t *n, int vocab, int hidden, int T, uint32_t *ids, void *workspace, size_t workspace_bytes,
+                   bool weights_early, blok_stream_t stream);
+void mla_layer_weights_stay(blok_mla_layer_t *L);
 int launch_bf16_gemv(const uint16_t *w, const uint16_t *x, uint16_t *y_bf16, float *y_f32, int rows, int cols, int T,
                      cudaStream_t stream);
 int launch_router_topk(const float *logits, const float *bias, int T, int experts, int topk, float routed_scale,
@@ -205,6 +211,7 @@ int build(blok_model *m, const char *, uint64_t) {
     mw.kv_a_ln = tp<uint16_t>(L.t, "kv_a_layernorm"); mw.kv_b = tp<uint16_t>(L.t, "kv_b_proj");
     mw.o = tp<uint16_t>(L.t, "o_proj");
     if ((rc = blok_mla_layer_create(&mw, m->rows, c.max_ctx, &L.mla))) return rc;
+    mla_layer_weights_stay(L.mla);
     if (l >= c.first_dense) {
       blok_moe_weights ew;
       memset(&ew, 0, sizeof(ew));
@@ -464,8 +471,8 @@ static int ffn_rows(blok_model_t *m, int l, int T, bool chunk, blok_stream_t str
     while (group > 1 && row_bytes * group > 200 * 1024) --group;
     if (wide && T > 8 && K->mlp_rows > 8) group = K->mlp_rows;  // one pass over the weights for up to 64 rows
     for (int b = 0; b < T && !rc; b += group)
-      rc = blok_bf16_mlp(tp<uint16_t>(L.t, "gate_proj"), tp<uint16_t>(L.t, "up_proj"), tp<uint16_t>(L.t, "down_proj"), K->n + b * H,
-                         K->tmp + b * H, c.hidden, c.dense_inter, T - b < group ? T - b : group, K->mlp_ws, K->mlp_ws_bytes, stream_);
+      rc = bf16_mlp(tp<uint16_t>(L.t, "gate_proj"), tp<uint16_t>(L.t, "up_proj"), tp<uint16_t>(L.t, "down_proj"), K->n + b * H,
+                         K->tmp + b * H, c.hidden, c.dense_inter, T - b < group ? T - b : group, K->mlp_ws, K->mlp_ws_bytes, true, stream_);
     return rc;
   }
   if (c.ep_world > 1) return moe_sharded_rows(m, L, T, stream_);
@@ -510,8 +517,8 @@ static int sample(blok_model *m, int row, int n, uint32_t *next, blok_stream_t s
   const blok_model_config &c = m->cfg;
   const int head_rows = (c.vocab % 16 == 0 && c.hidden % 256 == 0) ? kWgStreamTokens : 8;
   for (int b = 0; b < n; b += head_rows)
-    if (int rc = blok_lm_head_argmax(tp<uint16_t>(K->top, "lm_head"), K->n + (size_t)(row + b) * c.hidden, c.vocab, c.hidden,
-                                     n - b < head_rows ? n - b : head_rows, next + b, K->head_ws, K->head_ws_bytes, stream))
+    if (int rc = lm_head_argmax(tp<uint16_t>(K->top, "lm_head"), K->n + (size_t)(row + b) * c.hidden, c.vocab, c.hidden,
+                                     n - b < head_rows ? n - b : head_rows, next + b, K->head_ws, K->head_ws_bytes, true, stream))
       return rc;
   return BLOK_OK;
 }

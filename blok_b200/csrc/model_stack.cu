@@ -547,6 +547,8 @@ int product(StackModel *S, const Mat &w, const void *x, int T, void *y, bool y_f
   const uint16_t *xb = static_cast<const uint16_t *>(x);
   uint16_t *yb = y_f32 ? nullptr : static_cast<uint16_t *>(y);
   float *yf = y_f32 ? static_cast<float *>(y) : nullptr;
+  if (T <= 8 && wgemm_stream_takes_few(WG_BF16_PLAIN, wgemm_rows(w.w, nullptr, xb, yb, yf, w.R, w.K, T)))
+    return launch_wgemm_rows(WG_BF16_PLAIN, w.w, nullptr, xb, yb, yf, w.R, w.K, T, nullptr, 0, stream);
   if (T <= 8) return launch_bf16_gemv_splitk(w.w, xb, yb, yf, w.R, w.K, T, S->gemv_ws, S->gemv_ws_bytes, stream);
   if (T <= kWgStreamTokens && w.K % 256 == 0 && w.R % 16 == 0)
     return launch_wgemm_rows(WG_BF16_PLAIN, w.w, nullptr, xb, yb, yf, w.R, w.K, T, S->splitk_ws, S->splitk_bytes, stream);

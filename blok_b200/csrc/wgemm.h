@@ -80,6 +80,10 @@ int launch_wgemv_small(int mode, const WgArgs &args, cudaStream_t stream);
 bool wgemm_stream_supports(int mode, const WgArgs &args);
 int wgemm_stream_split(int mode, int K, int R);
 int wgemm_stream_pair_split(int mode, int K, int R, int R2);
+// Matrices with a tile for every SM: up to 8 rows of x too go through it rather than the mat-vec kernels (bf16_kernels.cu), which
+// spend an instruction on every 16 bytes.  One row, 2 x 18,432 gated rows of 7,168 (528 MB) 93 us and 77, 32,768 (470 MB) 92 and 75; below, the
+// mat-vec kernels' finer blocks are ahead.
+bool wgemm_stream_takes_few(int mode, const WgArgs &args);
 // *out becomes non-zero if a CTA without an error word of its own has given up since the last call (the flag is cleared).
 int wgemm_stream_take_error(unsigned *out);
 // The reduction behind a K-split launch: adds the nz partial sums in split order and applies the epilogue.
@@ -88,7 +92,8 @@ int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t 
 // One dense product through launch_wgemm without tile tables: out[T, R] = W[R, K] x[T, K] (mode WG_BF16_PLAIN; bf16 or
 // fp32 output) or the SwiGLU front half of (w_a = gate, w_b = up) (mode WG_BF16_SWIGLU), for 1 <= T <= kWgStreamTokens.
 int launch_wgemm_rows(int mode, const void *w_a, const void *w_b, const uint16_t *x, uint16_t *out_bf16, float *out_f32, int R, int K,
-                      int T, float *splitk_ws, size_t splitk_bytes, cudaStream_t stream);
+                      int T, float *splitk_ws, size_t splitk_bytes, cudaStream_t stream, bool weights_early = false);
+WgArgs wgemm_rows(const void *w_a, const void *w_b, const uint16_t *x, uint16_t *out_bf16, float *out_f32, int R, int K, int T);  // its launch
 
 // Both products of the grouped experts, INT4: mid = SwiGLU front half of x (up: WG_I4_SWIGLU), then the down projection
 // (down: WG_I4_PLAIN, its x is up's output).  Up to kWgSmallRows rows through the mat-vec-style kernel (wgemv_small.cu), else

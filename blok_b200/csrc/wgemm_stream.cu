@@ -218,6 +218,8 @@ int wgemm_stream_split(int mode, int K, int R) {
 }
 int wgemm_stream_pair_split(int mode, int K, int R, int R2) { return st_split(K, st_tiles(mode, R) + st_tiles(WG_BF16_PLAIN, R2)); }
 
+bool wgemm_stream_takes_few(int mode, const WgArgs &args) { return wgemm_stream_supports(mode, args) && st_tiles(mode, args.R) >= sm_count(); }
+
 // Launches the kernel; *splits = the K-split it used (> 1: the partial sums wait in args.splitk_ws for the reduce kernel).
 int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t stream) {
   const bool swiglu = mode == WG_BF16_SWIGLU;
@@ -337,13 +339,19 @@ size_t wgemm_splitk_bytes(int mode, int K, int R, int max_rows) {
   return worst;
 }
 
-int launch_wgemm_rows(int mode, const void *w_a, const void *w_b, const uint16_t *x, uint16_t *out_bf16, float *out_f32, int R, int K,
-                      int T, float *splitk_ws, size_t splitk_bytes, cudaStream_t stream) {
+WgArgs wgemm_rows(const void *w_a, const void *w_b, const uint16_t *x, uint16_t *out_bf16, float *out_f32, int R, int K, int T) {
   WgArgs r;
   r.w_a = w_a; r.w_b = w_b; r.s_a = r.s_b = nullptr; r.expert_stride_rows = 0; r.x = x; r.x_index = nullptr;
   r.K = K; r.R = R; r.out_bf16 = out_bf16; r.out_f32 = out_f32;
   r.tile_expert = r.tile_start = r.tile_count = r.num_tiles = nullptr; r.out_index = nullptr;
-  r.identity_tiles = 1; r.n_rows = T; r.splitk_ws = splitk_ws; r.splitk_bytes = splitk_bytes;
+  r.identity_tiles = 1; r.n_rows = T;
+  return r;
+}
+
+int launch_wgemm_rows(int mode, const void *w_a, const void *w_b, const uint16_t *x, uint16_t *out_bf16, float *out_f32, int R, int K,
+                      int T, float *splitk_ws, size_t splitk_bytes, cudaStream_t stream, bool weights_early) {
+  WgArgs r = wgemm_rows(w_a, w_b, x, out_bf16, out_f32, R, K, T);
+  r.splitk_ws = splitk_ws; r.splitk_bytes = splitk_bytes; r.weights_early = weights_early;
   BLOK_REQUIRE(wgemm_stream_supports(mode, r), BLOK_ERR_SHAPE, "wgemm rows: %d rows x %d columns over %d tokens is outside the streaming kernel",
                R, K, T);
   int nz = 1;
