@@ -146,3 +146,19 @@ def test_add_rmsnorm_is_add_then_rmsnorm(cuda, T, n):
     y = lib.add_rmsnorm(x_got, t, w, eps=1e-5)
     assert torch.equal(x_got, x_ref) and torch.equal(y, y_ref)
     assert torch.equal(x_ref, (x.float() + t.float()).bfloat16())
+
+
+@pytest.mark.parametrize("cols,T", [(6784, 3), (7168, 3), (8000, 3), (5056, 4), (2560, 8), (24576, 1)])
+def test_staged_rows_around_the_shared_memory_limit(cuda, cols, T):
+    """Rows of x that fill 40 to 48 KB of shared memory: with the kernels' static arrays more than a launch gets without asking."""
+    from blok_b200 import lib, synth
+    g = torch.Generator(device=cuda).manual_seed(cols)
+    w = (torch.randn((64, cols), generator=g, device=cuda) / cols ** 0.5).bfloat16()
+    x = synth.activations(T, cols, cuda, 5)
+    want = x.double() @ w.double().T
+    got = lib.bf16_gemv(w, x, out_f32=True)
+    assert float((got.double() - want).norm() / want.norm()) < 1e-5  # fp32 sums
+    y = lib.bf16_mlp(w, w, w.T.contiguous(), x)
+    mid = want * torch.sigmoid(want) * want
+    ref = mid @ w.double()
+    assert float((y.double() - ref).norm() / ref.norm()) < 1e-2      # five roundings to bf16
