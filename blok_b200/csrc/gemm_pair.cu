@@ -136,6 +136,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGpThreads, 1)
   gp_cluster_sync();
   tc_fence_after();
   const uint32_t tmem = s_tmem;
+  pdl_wait();
+  pdl_trigger();
   const int all_steps = (a.K + kGpStep - 1) / kGpStep;
   const int tiles = tl.rows * tl.cols * tl.parts, pairs = (int)gridDim.x / 2, pair = (int)blockIdx.x / 2;
   bool failed = false;
@@ -266,8 +268,7 @@ static int gp_launch(const GemmTma &g, cudaStream_t stream) {
   auto kernel = gemm_pair_kernel<BN, ACT, F32>;
   BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GpCfg<BN>::kSmem));
   const CUtensorMap &w = BN == 128 && !kGated ? *g.w64 : *g.w128;
-  kernel<<<2 * pairs, kGpThreads, GpCfg<BN>::kSmem, stream>>>(*g.x, w, g.up128 ? *g.up128 : *g.w128, a, tl);
-  return launch_status("gemm_pair_kernel");
+  return launch_pdl("gemm_pair_kernel", kernel, 2 * pairs, kGpThreads, (size_t)GpCfg<BN>::kSmem, stream, *g.x, w, g.up128 ? *g.up128 : *g.w128, a, tl);
 }
 
 int launch_gemm_pair(const GemmTma &g, cudaStream_t stream) {

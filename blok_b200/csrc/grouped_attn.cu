@@ -33,8 +33,10 @@ __device__ __forceinline__ size_t ga_row(const StackRows &r, int slot, int pos) 
 
 // ---- norms over all of q and all of k, cache append; one CTA per token ----
 template <typename Act>
-__global__ void __launch_bounds__(256) grouped_append_kernel(const GroupedShape s, Act *__restrict__ qkv, int ld, const float *__restrict__ q_norm,
-                                                             const float *__restrict__ k_norm, const StackRows r, Act *__restrict__ pool) {
+__global__ void __launch_bounds__(256) grouped_append_kernel(const GroupedShape s, Act *qkv, int ld, const float *q_norm, const float *k_norm, const StackRows r,
+                                                             Act *pool) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float s_red[2][8];
   const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nq = s.heads * s.dim, nk = pool ? s.kv_heads * s.dim : 0, nv = s.kv_heads * s.vdim;
@@ -93,9 +95,11 @@ __global__ void __launch_bounds__(256) grouped_append_kernel(const GroupedShape 
 int launch_grouped_append(const GroupedShape &s, void *qkv, int ld, const float *q_norm, const float *k_norm, const StackRows &r, int T, void *pool,
                           bool f32, cudaStream_t stream) {
   BLOK_REQUIRE(s.dim % 4 == 0 && s.vdim % 4 == 0 && ld % 4 == 0, BLOK_ERR_SHAPE, "grouped attention: rows of %d values", ld);
-  if (f32) grouped_append_kernel<float><<<T, 256, 0, stream>>>(s, static_cast<float *>(qkv), ld, q_norm, k_norm, r, static_cast<float *>(pool));
-  else grouped_append_kernel<uint16_t><<<T, 256, 0, stream>>>(s, static_cast<uint16_t *>(qkv), ld, q_norm, k_norm, r, static_cast<uint16_t *>(pool));
-  return launch_status("grouped_append_kernel");
+  if (f32)
+    return launch_pdl("grouped_append_kernel", grouped_append_kernel<float>, T, 256, 0, stream, s, static_cast<float *>(qkv), ld, q_norm, k_norm, r,
+                      static_cast<float *>(pool));
+  return launch_pdl("grouped_append_kernel", grouped_append_kernel<uint16_t>, T, 256, 0, stream, s, static_cast<uint16_t *>(qkv), ld, q_norm, k_norm, r,
+                    static_cast<uint16_t *>(pool));
 }
 
 __device__ __forceinline__ float ga_gate(float z) { return 1.0f / (1.0f + expf(-z)); }

@@ -167,6 +167,8 @@ __device__ __forceinline__ float lc_between(float4 a, float4 b) { return expf((a
 // chunk_state[c][h] = sum_j k_scale decay^(L-1-j) k_j v_j^T.  grid = (chunks, heads, columns / 64)
 template <bool TOKEN>
 __global__ void __launch_bounds__(kLcThreads) linear_chunk_state_kernel(const LaArgs a) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ float s_wt[kLinChunk];
   const int c = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * kLcCols;
@@ -252,6 +254,8 @@ __global__ void __launch_bounds__(kLcThreads) linear_chunk_state_kernel(const La
 // chunk_state[c] <- the state in front of chunk c; state <- the state behind the last chunk.
 template <bool TOKEN>
 __global__ void __launch_bounds__(128) linear_scan_kernel(const LaArgs a) {
+  pdl_wait();
+  pdl_trigger();
   const int h = blockIdx.y, i = (blockIdx.x * blockDim.x + threadIdx.x) * 4, n = a.dim * a.vdim;
   if (i >= n) return;
   float4 *st = reinterpret_cast<float4 *>(a.state + ((size_t)a.slot * a.heads + h) * n + i);
@@ -288,6 +292,8 @@ __global__ void __launch_bounds__(128) linear_scan_kernel(const LaArgs a) {
 // grid = (chunks, heads, columns / 64); a warp owns 16 tokens of the chunk and half of the columns.
 template <bool TOKEN>
 __global__ void __launch_bounds__(kLcThreads, 2) linear_chunk_out_kernel(const LaArgs a) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ float s_pw[TOKEN ? 1 : kLinChunk + 1];
   __shared__ float4 s_tok[TOKEN ? kLinChunk : 1];
@@ -606,12 +612,9 @@ static int chunked(const LaArgs &r, cudaStream_t stream) {
   const size_t smem3 = (size_t)2 * kLinChunk * kp + (size_t)kLinChunk * kLcVPitch + (size_t)kSplitParts * r.dim * kLcVPitch;
   BLOK_CUDA(cudaFuncSetAttribute(linear_chunk_state_kernel<TOKEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
   BLOK_CUDA(cudaFuncSetAttribute(linear_chunk_out_kernel<TOKEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3));
-  linear_chunk_state_kernel<TOKEN><<<grid, kLcThreads, smem1, stream>>>(r);
-  if (int rc = launch_status("linear_chunk_state_kernel")) return rc;
-  linear_scan_kernel<TOKEN><<<dim3((r.dim * r.vdim / 4 + 127) / 128, r.heads), 128, 0, stream>>>(r);
-  if (int rc = launch_status("linear_scan_kernel")) return rc;
-  linear_chunk_out_kernel<TOKEN><<<grid, kLcThreads, smem3, stream>>>(r);
-  return launch_status("linear_chunk_out_kernel");
+  if (int rc = launch_pdl("linear_chunk_state_kernel", linear_chunk_state_kernel<TOKEN>, grid, kLcThreads, smem1, stream, r)) return rc;
+  if (int rc = launch_pdl("linear_scan_kernel", linear_scan_kernel<TOKEN>, dim3((r.dim * r.vdim / 4 + 127) / 128, r.heads), 128, 0, stream, r)) return rc;
+  return launch_pdl("linear_chunk_out_kernel", linear_chunk_out_kernel<TOKEN>, grid, kLcThreads, smem3, stream, r);
 }
 
 int launch_linear_chunk(const LinearAttn &a, int slot, long first_pos, int T, cudaStream_t stream) {

@@ -84,6 +84,8 @@ __global__ void __launch_bounds__(kPtThreads, 1)
   tc_fence_after();
   const uint32_t tmem = s_tmem;
   bool failed = false;
+  pdl_wait();
+  pdl_trigger();
 
   if (warp == 8) {
     if (lane == 0) {
@@ -342,14 +344,9 @@ int launch_prompt_attn(const CUtensorMap &mq, const CUtensorMap &mkv, const CUte
   a.stages = std::min(kPtMaxStages, (kPtMaxSmem - 1024 - qc * kPtQChunk) / stage_bytes);
   const int smem = qc * kPtQChunk + a.stages * stage_bytes + 1024;
   const dim3 grid((a.T + kPtRows - 1) / kPtRows, a.heads);
-  if (a.bias) {
-    BLOK_CUDA(cudaFuncSetAttribute(prompt_attn_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    prompt_attn_tc_kernel<true><<<grid, kPtThreads, smem, stream>>>(mq, mkv, mkr, a);
-  } else {
-    BLOK_CUDA(cudaFuncSetAttribute(prompt_attn_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    prompt_attn_tc_kernel<false><<<grid, kPtThreads, smem, stream>>>(mq, mkv, mkr, a);
-  }
-  return launch_status("prompt_attn_tc_kernel");
+  auto kernel = a.bias ? prompt_attn_tc_kernel<true> : prompt_attn_tc_kernel<false>;
+  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  return launch_pdl("prompt_attn_tc_kernel", kernel, grid, kPtThreads, (size_t)smem, stream, mq, mkv, mkr, a);
 }
 
 bool latent_prompt_tc_supports(const LatentShape &s) {

@@ -61,6 +61,8 @@ __global__ void __launch_bounds__(THREADS) residual_norm_kernel(const ResidualNo
       if (c < a.width) w[k] = *reinterpret_cast<const float4 *>(a.norm_w + c);
     }
   }
+  pdl_wait();
+  pdl_trigger();
   if (a.ids) {
     const uint32_t last = (uint32_t)a.vocab - 1, id = min(a.ids[t], last);
     const int pos = a.pos ? a.pos[t] : 0;
@@ -161,13 +163,13 @@ __global__ void __launch_bounds__(THREADS) residual_norm_kernel(const ResidualNo
 int launch_residual_norm(const ResidualNorm &a, cudaStream_t stream) {
   BLOK_REQUIRE(a.T >= 1 && a.width % 4 == 0 && a.true_width >= 1 && a.true_width <= a.width && a.width <= kMaxNormWidth, BLOK_ERR_SHAPE,
                "residual norm: T %d, width %d (at most %d)", a.T, a.width, kMaxNormWidth);
-  if (a.width <= 512) residual_norm_kernel<128, 1><<<a.T, 128, 0, stream>>>(a);
-  else if (a.width <= 1024) residual_norm_kernel<256, 1><<<a.T, 256, 0, stream>>>(a);
-  else if (a.width <= 2048) residual_norm_kernel<256, 2><<<a.T, 256, 0, stream>>>(a);
-  else if (a.width <= 4096) residual_norm_kernel<512, 2><<<a.T, 512, 0, stream>>>(a);
-  else if (a.width <= 8192) residual_norm_kernel<512, 4><<<a.T, 512, 0, stream>>>(a);
-  else residual_norm_kernel<1024, 8><<<a.T, 1024, 0, stream>>>(a);
-  return launch_status("residual_norm_kernel");
+  auto launch = [&](void (*kernel)(ResidualNorm), int threads) { return launch_pdl("residual_norm_kernel", kernel, a.T, threads, 0, stream, a); };
+  if (a.width <= 512) return launch(residual_norm_kernel<128, 1>, 128);
+  if (a.width <= 1024) return launch(residual_norm_kernel<256, 1>, 256);
+  if (a.width <= 2048) return launch(residual_norm_kernel<256, 2>, 256);
+  if (a.width <= 4096) return launch(residual_norm_kernel<512, 2>, 512);
+  if (a.width <= 8192) return launch(residual_norm_kernel<512, 4>, 512);
+  return launch(residual_norm_kernel<1024, 8>, 1024);
 }
 
 }  // namespace blok

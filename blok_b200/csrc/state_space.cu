@@ -158,6 +158,8 @@ __device__ __forceinline__ void si_steps(const StateInputs &a, int head0, int ch
 // The steps in the first `step_blocks` blocks, then the convolution: unit 0 of a chunk has its first `lead` tokens.
 template <typename Act, int TAPS, int TOKENS>
 __global__ void __launch_bounds__(kSiThreads, sizeof(Act) == 2 ? 2 : 1) state_inputs_kernel(const StateInputs a, const StackRows r, int T, int chunk, int lead, int step_blocks) {
+  pdl_wait();
+  pdl_trigger();
   const int b = (int)blockIdx.x - step_blocks;
   if (b < 0) {
     const int groups = (a.heads + 31) / 32;
@@ -186,8 +188,8 @@ static int state_inputs(const StateInputs &a, const StackRows &r, int T, bool ch
   const long units = chunk ? 1 + (T > lead ? (T - lead + TOKENS - 1) / TOKENS : 0) : T, threads = a.channels / 8 * units;
   const int steps = (a.heads + 31) / 32 * ((T + kLinChunk - 1) / kLinChunk);
   BLOK_REQUIRE(threads < (1l << 30), BLOK_ERR_SHAPE, "state space: %d channels of %d tokens", a.channels, T);
-  state_inputs_kernel<Act, TAPS, TOKENS><<<steps + (int)((threads + kSiThreads - 1) / kSiThreads), kSiThreads, 0, stream>>>(a, r, T, chunk, lead, steps);
-  return launch_status("state_inputs_kernel");
+  return launch_pdl("state_inputs_kernel", state_inputs_kernel<Act, TAPS, TOKENS>, steps + (int)((threads + kSiThreads - 1) / kSiThreads), kSiThreads, 0,
+                    stream, a, r, T, (int)chunk, lead, steps);
 }
 template <typename Act>
 static int state_inputs_of(const StateInputs &a, const StackRows &r, int T, bool chunk, cudaStream_t stream) {
@@ -209,6 +211,8 @@ constexpr int kGnKeep = 8;
 // VEC 4: no padding and parts in multiples of four; 1: any.
 template <typename Act, int VEC>
 __global__ void __launch_bounds__(256) gate_then_norm_kernel(const GatedNorm a, int part_len) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float s_red[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, from = blockIdx.y * part_len, n = a.heads * a.vdim;
   const float *o = a.o + (size_t)blockIdx.x * n;
@@ -294,11 +298,9 @@ int launch_gate_then_norm(const GatedNorm &a, int parts, int T, cudaStream_t str
   const int len = a.heads * a.true_vdim / parts;
   const dim3 grid(T, parts);
   const bool wide = a.true_vdim == a.vdim && len % 4 == 0 && a.ldg % 4 == 0 && a.ldo % 4 == 0;
-  if (a.f32 && wide) gate_then_norm_kernel<float, 4><<<grid, 256, 0, stream>>>(a, len);
-  else if (a.f32) gate_then_norm_kernel<float, 1><<<grid, 256, 0, stream>>>(a, len);
-  else if (wide) gate_then_norm_kernel<uint16_t, 4><<<grid, 256, 0, stream>>>(a, len);
-  else gate_then_norm_kernel<uint16_t, 1><<<grid, 256, 0, stream>>>(a, len);
-  return launch_status("gate_then_norm_kernel");
+  auto launch = [&](void (*kernel)(GatedNorm, int)) { return launch_pdl("gate_then_norm_kernel", kernel, grid, 256, 0, stream, a, len); };
+  if (a.f32) return wide ? launch(gate_then_norm_kernel<float, 4>) : launch(gate_then_norm_kernel<float, 1>);
+  return wide ? launch(gate_then_norm_kernel<uint16_t, 4>) : launch(gate_then_norm_kernel<uint16_t, 1>);
 }
 
 }  // namespace blok
