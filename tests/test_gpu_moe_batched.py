@@ -133,6 +133,31 @@ def test_experts_grouped_handles_empty_and_ragged_groups(cuda, oracle, monkeypat
     layer.close()
 
 
+# blocks of 512 assignments sort (mb_sort_kernel): one short of a block, one block, one more, several with a remainder; ids that are no
+# expert of the layer's (-1, the count itself) lie between the others
+@pytest.mark.parametrize("N,only", [(511, None), (512, None), (513, None), (1025, None), (4136, None), (1500, 9)])
+def test_sort_of_the_assignments(cuda, N, only):
+    """A row of the result holds its own assignment's value: the same, bit for bit, as a call for that (expert, row) pair gives.  A
+    row's arithmetic in the tcgen05 kernel does not depend on the tile it lies in, so there is no tolerance."""
+    from blok_b200 import lib, synth
+    hidden, inter, experts, nrows = 512, 512, 40, 3
+    w = synth.moe_layer_weights(cuda, seed=47, hidden=hidden, inter=inter, experts=experts, shared_inter=0)
+    layer = lib.MoeLayer(w, max_tokens=600)
+    x = synth.activations(nrows, hidden, cuda, 47)
+    g = torch.Generator().manual_seed(N)
+    e = torch.full((N,), only) if only is not None else torch.randint(-1, experts + 1, (N,), generator=g)
+    rows = torch.randint(0, nrows, (N,), generator=g)
+    pairs_e = torch.arange(experts).repeat_interleave(nrows)
+    each = layer.experts_grouped(x, pairs_e.int().to(cuda), torch.arange(nrows).repeat(experts).int().to(cuda))
+    got = layer.experts_grouped(x, e.int().to(cuda), rows.int().to(cuda))
+    layer.check()
+    ours = (e >= 0) & (e < experts)
+    want = each[(e.clamp(0, experts - 1) * nrows + rows).to(cuda)]
+    assert len(torch.unique(each.view(torch.int16), dim=0)) == experts * nrows, "every pair has a value of its own"
+    assert torch.equal(got[ours.to(cuda)], want[ours.to(cuda)])
+    layer.close()
+
+
 @pytest.mark.parametrize("hidden,inter,groups,small", [
     (512, 512, {7: 40}, True),                               # ten passes of four tokens over one expert
     (2048, 1024, {0: 2, 5: 3, 64: 4, 90: 9, 127: 5}, True),  # passes of 1 to 4 tokens; scales staged in chunks of 16 k-blocks
