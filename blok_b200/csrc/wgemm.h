@@ -54,7 +54,7 @@ struct WgArgs {
 
 // Picks the kernel of a launch.  INT4 modes: the mma.sync kernel (see launch_wgemm_experts for the others).  bf16 modes: up to
 // kWgStreamTokens rows of a dense product the weight-streaming kernel (wgemm_stream.cu); more, the TMA-fed tcgen05 GEMM
-// (gemm_tma.cu), K split where its tiles are few; for shapes the others do not cover the mma.sync kernel with its K-split.
+// (gemm_tma.cu; over more than 128 rows gemm_pair.cu), K split where its tiles are few; for shapes the others do not cover the mma.sync kernel with its K-split.
 // BLOK_WGEMM_IMPL=mma / =tc in the environment forces one GEMM kernel for every row (no small-group or streaming kernel).
 int launch_wgemm(int mode, const WgArgs &args, int max_tiles, cudaStream_t stream);
 int wgemm_forced_impl();  // 0: none forced
