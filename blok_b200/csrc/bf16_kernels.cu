@@ -452,10 +452,16 @@ int blok::bf16_mlp(const blok_bf16_t *gate, const blok_bf16_t *up, const blok_bf
     if (int rc = launch_wgemm_rows(WG_BF16_SWIGLU, gate, up, x, mid, nullptr, ffn, hidden, T, sk, sk_bytes, (cudaStream_t)stream, weights_early)) return rc;
     return launch_wgemm_rows(WG_BF16_PLAIN, down, nullptr, mid, y, nullptr, hidden, ffn, T, sk, sk_bytes, (cudaStream_t)stream, true);
   }
-  int rc = wgemm_stream_takes_few(WG_BF16_SWIGLU, wgemm_rows(gate, up, x, mid, nullptr, ffn, hidden, T))
-               ? launch_wgemm_rows(WG_BF16_SWIGLU, gate, up, x, mid, nullptr, ffn, hidden, T, nullptr, 0, (cudaStream_t)stream, weights_early)
+  // a workspace with room behind the vector (a model's has it) lets the weight stream cut K into parts
+  const size_t at = mlp_mid_bytes(ffn, T), room = workspace_bytes > at ? workspace_bytes - at : 0;
+  float *sk = room ? reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + at) : nullptr;
+  const WgArgs front = wgemm_rows(gate, up, x, mid, nullptr, ffn, hidden, T);
+  int rc = wgemm_stream_takes_few(WG_BF16_SWIGLU, front) || wgemm_stream_takes_parts(WG_BF16_SWIGLU, front, room)
+               ? launch_wgemm_rows(WG_BF16_SWIGLU, gate, up, x, mid, nullptr, ffn, hidden, T, sk, room, (cudaStream_t)stream, weights_early)
                : launch_bf16_gateup(gate, up, x, mid, ffn, hidden, T, (cudaStream_t)stream);
   if (rc) return rc;
+  if (wgemm_stream_takes_parts(WG_BF16_PLAIN, wgemm_rows(down, nullptr, mid, y, nullptr, hidden, ffn, T), room))
+    return launch_wgemm_rows(WG_BF16_PLAIN, down, nullptr, mid, y, nullptr, hidden, ffn, T, sk, room, (cudaStream_t)stream, true);
   return launch_bf16_gemv(down, mid, y, nullptr, hidden, ffn, T, (cudaStream_t)stream);
 }
 

@@ -236,6 +236,10 @@ int build(blok_model *m, const char *, uint64_t) {
   // the dense layer takes up to 64 rows per call where its sizes fit the weight-streaming kernel, else 8
   K->mlp_rows = (c.hidden % 256 == 0 && c.dense_inter % 256 == 0 && c.dense_inter > 0) ? std::min((int)m->rows, kWgStreamTokens) : 8;
   K->mlp_ws_bytes = blok_bf16_mlp_workspace_bytes(c.hidden, c.dense_inter > 0 ? c.dense_inter : 32, std::max(K->mlp_rows, 8));
+  if (c.dense_inter > 0)  // the vector of up to 8 rows and behind it the sums of the K splits
+    K->mlp_ws_bytes = std::max(K->mlp_ws_bytes, (blok_bf16_mlp_workspace_bytes(c.hidden, c.dense_inter, 8) + 255) / 256 * 256 +
+                                                    std::max(wgemm_splitk_bytes(WG_BF16_PLAIN, c.dense_inter, c.hidden, 8),
+                                                             wgemm_splitk_bytes(WG_BF16_SWIGLU, c.hidden, c.dense_inter, 8)));
   if ((rc = dev_alloc(m, K->mlp_ws_bytes, &K->mlp_ws))) return rc;
   K->head_ws_bytes = blok_lm_head_workspace_bytes(c.vocab, c.max_batch);
   if ((rc = dev_alloc(m, K->head_ws_bytes, &K->head_ws))) return rc;

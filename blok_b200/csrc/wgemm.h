@@ -81,9 +81,10 @@ bool wgemm_stream_supports(int mode, const WgArgs &args);
 int wgemm_stream_split(int mode, int K, int R);
 int wgemm_stream_pair_split(int mode, int K, int R, int R2);
 // Matrices with a tile for every SM: up to 8 rows of x too go through it rather than the mat-vec kernels (bf16_kernels.cu), which
-// spend an instruction on every 16 bytes.  One row, 2 x 18,432 gated rows of 7,168 (528 MB) 93 us and 77, 32,768 (470 MB) 92 and 75; below, the
-// mat-vec kernels' finer blocks are ahead.
+// spend an instruction on every 16 bytes.  One row, 2 x 18,432 gated rows of 7,168 (528 MB) 93 us and 77, 32,768 (470 MB) 92 and 75.
 bool wgemm_stream_takes_few(int mode, const WgArgs &args);
+// Fewer tiles, K in parts; room: bytes for their sums.
+bool wgemm_stream_takes_parts(int mode, const WgArgs &args, size_t room);
 // *out becomes non-zero if a CTA without an error word of its own has given up since the last call (the flag is cleared).
 int wgemm_stream_take_error(unsigned *out);
 // The reduction behind a K-split launch: adds the nz partial sums in split order and applies the epilogue.

@@ -219,6 +219,18 @@ int wgemm_stream_split(int mode, int K, int R) {
 int wgemm_stream_pair_split(int mode, int K, int R, int R2) { return st_split(K, st_tiles(mode, R) + st_tiles(WG_BF16_PLAIN, R2)); }
 
 bool wgemm_stream_takes_few(int mode, const WgArgs &args) { return wgemm_stream_supports(mode, args) && st_tiles(mode, args.R) >= sm_count(); }
+// Products of up to 8 rows with fewer tiles than SMs: K in parts and a launch that adds them, against the mat-vec kernel, the dense
+// layer's two products measured together (hidden x ffn, rows: mat-vec / here, us).
+//  - gate and up: 7168 x 8192, 1 row 72 / 62, 8 rows 101 / 63; 16384 x 4096, 1 row 81 / 69; 2048 x 8192, 1 row 27.3 / 25.8, 8 rows 30.7 /
+//    27.0; but 7168 x 2048, 59 MB, 1 row 24.6 / 26.7 (4 rows 24.7 / 23.6), 1024 x 4096, 17 MB, 4 rows 14.3 / 15.7.
+//  - down: 7168 x 18432, 1 row 145 / 124, 4 rows 188 / 124; 4096 x 14336, 1 row 72 / 62; 1024 x 4096, 1 row 14.4 / 13.4; but K = 2,048 of
+//    7,168 rows, 1 row 23.7 / 24.6 (4 rows 26.2 / 24.7).
+bool wgemm_stream_takes_parts(int mode, const WgArgs &args, size_t room) {
+  const bool gated = mode == WG_BF16_SWIGLU, one = args.n_rows == 1;
+  const size_t weights = (size_t)args.R * args.K * (gated ? 4 : 2), sums = (size_t)args.n_rows * args.R * (gated ? 8 : 4);
+  if (gated ? weights < (one ? size_t(64) : size_t(32)) * 1000000 : one && args.K < 4096) return false;
+  return wgemm_stream_supports(mode, args) && room >= wgemm_stream_split(mode, args.K, args.R) * sums;
+}
 
 // Launches the kernel; *splits = the K-split it used (> 1: the partial sums wait in args.splitk_ws for the reduce kernel).
 int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t stream) {

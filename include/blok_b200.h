@@ -133,7 +133,8 @@ size_t blok_bf16_mlp_workspace_bytes(int hidden, int ffn, int T);
 /* y[t] = W_d (SiLU(W_g x[t]) * W_u x[t]); replaces bf16_mlp (src/kimi_exec.cu:674-686)
  * without its running-sum side effect (the caller adds).  T <= 64; more than 8 rows
  * need hidden and ffn to be multiples of 256 and stream each matrix once for all rows
- * (the workspace then also holds the K-split partial sums of the down projection). */
+ * (the workspace then also holds the K-split partial sums of the down projection; with up to 8 rows a larger
+ * workspace is used so where that is faster, in another order of summation). */
 int blok_bf16_mlp(const blok_bf16_t *gate, const blok_bf16_t *up, const blok_bf16_t *down, const blok_bf16_t *x,
                   blok_bf16_t *y, int hidden, int ffn, int T, void *workspace, size_t workspace_bytes,
                   blok_stream_t stream);

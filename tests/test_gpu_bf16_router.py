@@ -1,4 +1,6 @@
 """GPU parity of the bf16 mat-vec / MLP / RMSNorm kernels and of the router."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -41,6 +43,45 @@ def test_bf16_mlp(cuda, oracle, hidden, ffn, T):
     for t in range(T):
         util.assert_close(y[t], oracle.bf16_mlp(g, u, d, x[t], mode=0, round_out=True), "bf16_mlp")
         util.assert_close(y[t], oracle.bf16_mlp(g, u, d, x[t], mode=1, round_out=True), "bf16_mlp vs ref_exact")
+
+
+# up to 8 rows with room behind the vector: K in parts (wgemm_stream_takes_parts) for down only (gate and up below 32 MB, or 64 with
+# one row), for both, and for neither (columns no multiple of 256); more: launches that add the parts
+@pytest.mark.parametrize("hidden,ffn,T,more", [(1024, 4096, 1, 1), (1024, 4096, 8, 1), (2048, 4096, 2, 2), (4096, 4096, 1, 2), (2048, 2112, 3, 0),
+                                               (288, 4128, 4, 0)])
+def test_bf16_mlp_with_room_for_a_split(cuda, oracle, hidden, ffn, T, more):
+    """With too little room, or where neither product takes parts, the bits are those of a workspace without room.  Nothing behind the
+    workspace is touched.  The bars are those of the other forms: only the order of the fp32 sums differs."""
+    from blok_b200 import lib
+    rng = np.random.default_rng(hidden + ffn + T)
+    g, u, d = _w(rng, ffn, hidden, 0.02), _w(rng, ffn, hidden, 0.02), _w(rng, hidden, ffn, 0.02)
+    x = oracle.bf16_round(rng.normal(size=(T, hidden)).astype(np.float32))
+    dg, du, dd, dx = (util.np_bf16_to_torch(g, cuda), util.np_bf16_to_torch(u, cuda), util.np_bf16_to_torch(d, cuda),
+                      torch.from_numpy(x).to(cuda).bfloat16())
+    vector = (ffn * T * 2 + 255) // 256 * 256
+
+    def run(nbytes):
+        ws = torch.full((nbytes + 4096,), 0x5A, dtype=torch.uint8, device=cuda)
+        y = torch.empty((T, hidden), dtype=torch.bfloat16, device=cuda)
+        lib._check(lib.load().blok_bf16_mlp(lib._ptr(dg), lib._ptr(du), lib._ptr(dd), lib._ptr(dx), lib._ptr(y), C.c_int(hidden), C.c_int(ffn),
+                                            C.c_int(T), lib._ptr(ws), C.c_size_t(nbytes), lib._stream()))
+        assert bool((ws[nbytes:] == 0x5A).all())
+        return y
+
+    def launches(nbytes):
+        before = lib.kernel_launch_count()
+        y = run(nbytes)
+        return y, lib.kernel_launch_count() - before
+
+    room = vector + 4 * T * 65536
+    (plain, few), (split, many) = launches(ffn * T * 2), launches(room)
+    assert many - few == more
+    assert torch.equal(plain, lib.bf16_mlp(dg, du, dd, dx))
+    yh = util.t2np_f32(split)
+    for t in range(T):
+        util.assert_close(yh[t], oracle.bf16_mlp(g, u, d, x[t], mode=0, round_out=True), "bf16_mlp")
+    assert torch.equal(split, plain if more == 0 else run(room))
+    assert torch.equal(plain, run(vector + 16))
 
 
 @pytest.mark.parametrize("n,T", [(7168, 1), (1536, 4), (512, 8)])
