@@ -345,8 +345,9 @@ int batched_alloc(blok_moe_layer *L) {
                                std::max(wgemm_splitk_bytes(WG_BF16_SWIGLU, w.hidden, std::max(w.shared_inter, 8), (int)T),
                                         wgemm_splitk_bytes(WG_BF16_PLAIN, std::max(w.shared_inter, 8), w.hidden, (int)T)));
   L->b_front_split = wgemm_stream_pair_split(WG_BF16_SWIGLU, w.hidden, std::max(w.shared_inter, 8), w.experts);
-  L->b_splitk_bytes = std::max(L->b_splitk_bytes, (size_t)L->b_front_split * std::min<size_t>(T, kWgStreamTokens) *
-                                                      (2 * w.shared_inter + w.experts) * sizeof(float));
+  // The launches over up to kWgStreamTokens tokens that leave their sums to another kernel want room for one part also where K is not split.
+  const size_t few = std::min<size_t>(T, kWgStreamTokens) * sizeof(float);
+  L->b_splitk_bytes = std::max({L->b_splitk_bytes, L->b_front_split * few * (2 * w.shared_inter + w.experts), w.shared_inter > 0 ? few * w.hidden : 0});
   size_t o_sk = take(std::max(L->b_splitk_bytes, (size_t)16)), o_err = take(4);
   BLOK_CUDA(cudaMalloc(&L->bws, off));
   unsigned char *b = static_cast<unsigned char *>(L->bws);

@@ -237,3 +237,21 @@ def test_front_of_a_small_batch(cuda, monkeypatch, T, experts, topk, hidden, int
     assert float((y.float() - want.float()).norm() / want.float().norm()) < 1e-2
     layer.check()
     layer.close()
+
+
+def test_a_wide_layer_has_room_for_its_sums(cuda, monkeypatch):
+    """The shared expert's down projection leaves its sums also where K is not split: hidden / 128 tiles for all SMs, and a front (twice the
+    shared expert and the router) of fewer columns than hidden.  Against the separate launches, as above."""
+    from blok_b200 import lib, synth
+    T, hidden, shared = 64, 20480, 9728
+    w = synth.moe_layer_weights(cuda, seed=9, hidden=hidden, inter=512, experts=128, shared_inter=shared)
+    layer = lib.MoeLayer(w, max_tokens=T)
+    x = synth.activations(T, hidden, cuda, 9)
+    monkeypatch.delenv("BLOK_WGEMM_IMPL", raising=False)
+    y, ids, _ = layer.batched(x, return_routing=True)
+    monkeypatch.setenv("BLOK_WGEMM_IMPL", "tc")
+    want, wid, _ = layer.batched(x, return_routing=True)
+    layer.check()
+    assert torch.equal(ids, wid)
+    assert float((y.float() - want.float()).norm() / want.float().norm()) < 1e-2
+    layer.close()
