@@ -6,6 +6,8 @@
 // exists only to add them, and the per-head products have their weights in shared memory before the wait for that input.  From one
 // kernel's last store to the next one's first load pass about 1 us; of the rest (time stamps, one sequence / 8 / 64 tokens, us) the
 // norms take 4 / 4 / 2, the query 2.5 / 3.5 / 5, merge and value product 7 / 13 / 9, where nine launches stood before.
+#include <algorithm>
+
 #include "gemm_tma.h"
 #include "mla_heads.h"
 #include "tc_pipe.cuh"
@@ -30,6 +32,9 @@ __device__ __forceinline__ float4 mh_sum4(const float *p, size_t stride, int nz)
 }
 
 constexpr int kMnThreads = 512;
+// Values of a row that stay in shared memory between its two passes: 44 KB, which a launch gets without asking beside what the kernel
+// keeps in static arrays.  Of longer rows the rest is added up from the parts a second time.
+constexpr int kMnKept = 11264;
 
 __device__ __forceinline__ float mh_block_sum(float v, float *red) {
   v = warp_sum(v);
@@ -52,7 +57,7 @@ __device__ __forceinline__ void mh_rotate(float x0, float x1, float c, float s, 
   *hi = f32_to_bf16_bits(round_bf16(x1 * c) + round_bf16(x0 * s));
 }
 
-// grid = (2, B); dynamic shared memory: max(q_rank, kv_rank + rope) floats.  Block 0 of an entry: q_a's sums -> bf16 -> RMSNorm
+// grid = (2, B); dynamic shared memory: the longer of the two rows, up to kMnKept floats.  Block 0 of an entry: q_a's sums -> bf16 -> RMSNorm
 // (:813-815).  Block 1: kv_a's -> bf16, c_kv normalised, k_pe rotated, the row appended to the cache, the length of the sequence
 // published (:816-824).  What the call was given (positions, tables, weights) is read before the wait, see decode_body.
 __global__ void __launch_bounds__(kMnThreads) mla_norm_kernel(const MlaNorm a) {
@@ -95,16 +100,20 @@ __global__ void __launch_bounds__(kMnThreads) mla_norm_kernel(const MlaNorm a) {
     if (!in_range) return;
   }
   const float *row = a.part + (size_t)b * a.ld + (kv ? a.q_rank : 0);
-  float v = 0.f;
-  for (int i = 4 * tid; i < all; i += 4 * kMnThreads) {
+  auto sums = [&](int i) {
     float4 f = mh_sum4<16>(row + i, (size_t)gridDim.y * a.ld, a.nz);
     f.x = round_bf16(f.x), f.y = round_bf16(f.y), f.z = round_bf16(f.z), f.w = round_bf16(f.w);
-    *reinterpret_cast<float4 *>(val + i) = f;
+    return f;
+  };
+  float v = 0.f;
+  for (int i = 4 * tid; i < all; i += 4 * kMnThreads) {
+    const float4 f = sums(i);
+    if (i < kMnKept) *reinterpret_cast<float4 *>(val + i) = f;
     if (i < n) v = fmaf(f.x, f.x, fmaf(f.y, f.y, fmaf(f.z, f.z, fmaf(f.w, f.w, v))));
   }
   const float scale = rsqrtf(mh_block_sum(v, red) / n + a.eps);  // its barrier also orders val
   for (int i = 4 * tid; i < n; i += 4 * kMnThreads) {
-    const float4 f = *reinterpret_cast<const float4 *>(val + i);
+    const float4 f = i < kMnKept ? *reinterpret_cast<const float4 *>(val + i) : sums(i);
     if (i != 4 * tid) first_ln = make_uint2(ln[i] | (uint32_t)ln[i + 1] << 16, ln[i + 2] | (uint32_t)ln[i + 3] << 16);
     *reinterpret_cast<uint2 *>(out + i) = make_uint2(pack_bf16x2(round_bf16(f.x * scale) * bf16lo(first_ln.x), round_bf16(f.y * scale) * bf16hi(first_ln.x)),
                                                      pack_bf16x2(round_bf16(f.z * scale) * bf16lo(first_ln.y), round_bf16(f.w * scale) * bf16hi(first_ln.y)));
@@ -430,8 +439,9 @@ __global__ void __launch_bounds__(kMvThreads, 1) mla_value_kernel(const __grid_c
 }
 
 int launch_mla_norm(const MlaNorm &a, int B, cudaStream_t stream) {
-  const size_t smem = (size_t)(a.q_rank > a.kv_rank + a.rope ? a.q_rank : a.kv_rank + a.rope) * sizeof(float);
-  if (smem > 48 * 1024) BLOK_CUDA(cudaFuncSetAttribute(mla_norm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int lat = a.kv_rank + a.rope;
+  BLOK_REQUIRE(lat <= kMnKept, BLOK_ERR_SHAPE, "mla norm: cache rows of %d values (at most %d)", lat, kMnKept);
+  const size_t smem = (size_t)std::min(std::max(a.q_rank, lat), kMnKept) * sizeof(float);
   return launch_pdl("mla_norm_kernel", mla_norm_kernel, dim3(2, B), kMnThreads, smem, stream, a);
 }
 

@@ -91,6 +91,24 @@ def test_chain(cuda, hidden, q_rank, nope, v_head, B):
     layer.close()
 
 
+# around 48 KB of a norm's shared memory (12,160 to 12,288 values leave no room for its static arrays), and rows longer than an SM's
+@pytest.mark.parametrize("q_rank", [11264, 11296, 12160, 12288, 61440])
+def test_long_query_rows(cuda, q_rank):
+    from blok_b200 import lib
+    hidden, nope, v_head, B = 288, 32, 16, 2
+    w, g = _weights(cuda, hidden, q_rank, nope, v_head, q_rank)
+    layer = lib.MlaLayer(w, yarn_factor=32.0, max_batch=B, max_ctx=100, qk_nope=nope, v_head=v_head)
+    n = torch.randn((B, hidden), generator=g, device=cuda).bfloat16()
+    pos = torch.tensor([7, 99], dtype=torch.int32, device=cuda)
+    cache = torch.randn((B, 100, RANK + ROPE), generator=g, device=cuda).bfloat16()
+    before = cache.clone()
+    out = layer.decode(n, cache, pos)
+    want, _ = _plain(w, n.double(), pos, nope, v_head, lambda b, new: torch.cat([before[b, :int(pos[b])].double(), new[b:b + 1]]))
+    _check(out, want, "decode")
+    layer.check()
+    layer.close()
+
+
 @pytest.mark.parametrize("lens", [
     [1] * 60 + [900, 64, 65, 3000],                    # pieces over the sequences' borders, several sequences to a CTA
     [0, 5, 0, 700, 128, 0],                            # empty sequences: zeros
