@@ -2,6 +2,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstring>
+#include <mutex>
 
 #include "common.cuh"
 
@@ -38,6 +39,47 @@ int sm_count() {
     cached_dev = dev;
   }
   return cached;
+}
+
+// The bytes of a kernel's static arrays, which do not change; a table without allocations.
+static int static_smem_of(const void *kernel, size_t *bytes) {
+  struct Known {
+    std::atomic<const void *> kernel{nullptr};
+    size_t bytes = 0;  // written before the kernel is
+  };
+  constexpr size_t kSlots = 512;
+  static Known known[kSlots];
+  static std::mutex mu;
+  const size_t home = reinterpret_cast<uintptr_t>(kernel) / 16 % kSlots;
+  auto find = [&]() -> Known * {  // its slot, or the free one; NULL: the table is full
+    for (size_t i = 0; i < kSlots; ++i) {
+      Known *k = known + (home + i) % kSlots;
+      const void *is = k->kernel.load(std::memory_order_acquire);
+      if (is == kernel || !is) return k;
+    }
+    return nullptr;
+  };
+  Known *k = find();
+  if (k && k->kernel.load(std::memory_order_acquire) == kernel) {
+    *bytes = k->bytes;
+    return BLOK_OK;
+  }
+  cudaFuncAttributes a;
+  BLOK_CUDA(cudaFuncGetAttributes(&a, kernel));
+  *bytes = a.sharedSizeBytes;
+  std::lock_guard<std::mutex> lock(mu);
+  if ((k = find()) && !k->kernel.load(std::memory_order_relaxed)) {
+    k->bytes = a.sharedSizeBytes;
+    k->kernel.store(kernel, std::memory_order_release);
+  }
+  return BLOK_OK;
+}
+
+int allow_smem_of(const void *kernel, size_t dynamic) {
+  size_t fixed = 0;
+  if (int rc = static_smem_of(kernel, &fixed)) return rc;
+  if (fixed + dynamic > 48 * 1024) BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynamic));
+  return BLOK_OK;
 }
 
 }  // namespace blok

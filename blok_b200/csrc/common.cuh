@@ -39,6 +39,13 @@ inline int launch_status(const char *what) {
 
 int sm_count();
 
+// Lets a kernel be launched with `dynamic` bytes of dynamic shared memory: a launch gets 48 KB, its static arrays among them, without asking.
+int allow_smem_of(const void *kernel, size_t dynamic);
+template <typename... P>
+inline int allow_smem(void (*kernel)(P...), size_t dynamic) {
+  return allow_smem_of(reinterpret_cast<const void *>(kernel), dynamic);
+}
+
 // Launches a kernel that begins with pdl_wait(): its blocks may become resident while the kernel before it runs (programmatic
 // dependent launch), which takes the launch and the start of its blocks off the critical path; captured into graphs like any
 // other launch.  Some forty launches of 5 to 50 us in a prompt of 60 / 130 / 1,000 tokens: 547 / 612 / 1,050 -> 500 / 517 / 956 us; over

@@ -79,12 +79,10 @@ int launch_i4_gemv16_imma(const uint32_t *w, const uint16_t *scale, const uint16
     }
   const size_t smem = imma_stage_bytes(cols);
   if (y_bf16) {
-    if (smem > 48 * 1024)
-      BLOK_CUDA(cudaFuncSetAttribute(i4_gemv16_imma_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(i4_gemv16_imma_kernel<uint16_t>, smem)) return rc;
     i4_gemv16_imma_kernel<uint16_t><<<rows / 16, nwarps * 32, smem, stream>>>(w, scale, x, y_bf16, cols, kblocks / nwarps);
   } else {
-    if (smem > 48 * 1024)
-      BLOK_CUDA(cudaFuncSetAttribute(i4_gemv16_imma_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(i4_gemv16_imma_kernel<float>, smem)) return rc;
     i4_gemv16_imma_kernel<float><<<rows / 16, nwarps * 32, smem, stream>>>(w, scale, x, y_f32, cols, kblocks / nwarps);
   }
   return launch_status("i4_gemv16_imma_kernel");

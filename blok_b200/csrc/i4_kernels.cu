@@ -263,23 +263,17 @@ static KSplit pick_split(int kblocks, int max_warps) {
     default: { constexpr int B = 1; __VA_ARGS__; } break;      \
   }
 
-template <typename K>
-static int ensure_smem(K kernel, size_t bytes) {
-  if (bytes > 48 * 1024) BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return BLOK_OK;
-}
-
 int launch_i4_gemv16(const uint32_t *w, const uint16_t *scale, const uint16_t *x, uint16_t *y_bf16, float *y_f32,
                      int rows, int cols, cudaStream_t stream) {
   KSplit ks = pick_split(cols / 128, 8);
   size_t smem = i4_stage_bytes(cols, ks.batch);
   BLOK_DISPATCH_BATCH(ks.batch, {
     if (y_bf16) {
-      int rc = ensure_smem(i4_gemv16_kernel<B, uint16_t>, smem);
+      int rc = allow_smem(i4_gemv16_kernel<B, uint16_t>, smem);
       if (rc) return rc;
       i4_gemv16_kernel<B, uint16_t><<<rows / 16, ks.nwarps * 32, smem, stream>>>(w, scale, x, y_bf16, cols, ks.nbatch);
     } else {
-      int rc = ensure_smem(i4_gemv16_kernel<B, float>, smem);
+      int rc = allow_smem(i4_gemv16_kernel<B, float>, smem);
       if (rc) return rc;
       i4_gemv16_kernel<B, float><<<rows / 16, ks.nwarps * 32, smem, stream>>>(w, scale, x, y_f32, cols, ks.nbatch);
     }
@@ -293,7 +287,7 @@ int launch_i4_gateup(const uint32_t *gate_w, const uint16_t *gate_s, const uint3
   KSplit ks = pick_split(hidden / 128, 8);
   size_t smem = i4_stage_bytes(hidden, ks.batch);
   BLOK_DISPATCH_BATCH(ks.batch, {
-    int rc = ensure_smem(i4_gateup_kernel<B>, smem);
+    int rc = allow_smem(i4_gateup_kernel<B>, smem);
     if (rc) return rc;
     return launch_pdl("i4_gateup_kernel", i4_gateup_kernel<B>, dim3(inter / 8, slots), ks.nwarps * 32, smem, stream, gate_w, gate_s, up_w, up_s, x,
                       slot_expert, mid, hidden, inter, ks.nbatch);
@@ -313,7 +307,7 @@ int launch_i4_down(const uint32_t *down_w, const uint16_t *down_s, const uint16_
   KSplit ks = pick_split(inter / 128, max_split > 8 ? 8 : max_split);
   size_t smem = i4_stage_bytes(inter, ks.batch) * slots;
   BLOK_DISPATCH_BATCH(ks.batch, {
-    int rc = ensure_smem(i4_down_kernel<B>, smem);
+    int rc = allow_smem(i4_down_kernel<B>, smem);
     if (rc) return rc;
     return launch_pdl("i4_down_kernel", i4_down_kernel<B>, hidden / 16, slots * ks.nwarps * 32, smem, stream, down_w, down_s, mid, slot_expert, wts,
                       addend, out, inter, hidden, slots, ks.nwarps, ks.nbatch);

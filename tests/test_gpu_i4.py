@@ -119,3 +119,23 @@ def test_bad_shapes_raise(cuda):
         lib.i4_gemv(w, s, torch.zeros(32, dtype=torch.bfloat16, device=cuda))
     with pytest.raises(lib.BlokError):
         lib.i4_gemv(w.cpu(), s, torch.zeros(64, dtype=torch.bfloat16, device=cuda))
+
+
+# a launch's dynamic and static shared memory together at 48 KB: the largest that needs no asking, and those just above
+@pytest.mark.parametrize("what,n", [("gemv", 21504), ("gemv", 21632), ("gemv", 21760), ("gateup", 22272), ("gateup", 22528), ("gateup", 22784),
+                                    ("down", 22528), ("down", 22784)])
+def test_shared_memory_around_what_a_launch_gets_unasked(cuda, oracle, what, n):
+    from blok_b200 import lib
+    rng = np.random.default_rng(n)
+    x = oracle.bf16_round(rng.normal(size=n if what != "down" else 256).astype(np.float32))
+    dx = torch.from_numpy(x).to(cuda).bfloat16()
+    if what == "gemv":
+        w, s, dw, ds = _dev_i4(rng, 16, n, cuda)
+        util.assert_close(util.t2np_f32(lib.i4_gemv(dw, ds, dx)), oracle.i4_gemv(w, s, x, mode=0, round_out=True), "gemv of %d columns" % n)
+        return
+    hidden, inter = (n, 256) if what == "gateup" else (256, n)
+    gw, gs, dgw, dgs = _dev_i4(rng, inter, hidden, cuda, 0.03)
+    uw, us, duw, dus = _dev_i4(rng, inter, hidden, cuda, 0.03)
+    dw, ds, ddw, dds = _dev_i4(rng, hidden, inter, cuda, 0.03)
+    y = lib.expert_ffn(dgw, dgs, duw, dus, ddw, dds, dx)
+    util.assert_close(util.t2np_f32(y), oracle.expert_ffn(gw, gs, uw, us, dw, ds, x, mode=0, round_out=True), "expert %d x %d" % (hidden, inter))

@@ -63,6 +63,12 @@ def test_moe_decode_small(cuda, oracle, monkeypatch, impl, hidden, inter, expert
     _check(cuda, oracle, hidden, inter, experts, shared_inter, seed)
 
 
+def test_moe_decode_down_projection_of_48_kb(cuda, oracle, monkeypatch):
+    """Four slots of 5,632 columns: the down projection's dynamic shared memory alone is what a launch gets without asking."""
+    monkeypatch.setenv("BLOK_MOE_DECODE_IMPL", "multi")
+    _check(cuda, oracle, 512, 5632, 8, 0, 15, topk=4)
+
+
 def test_moe_decode_many_tokens_fused(cuda, oracle):
     """Back-to-back launches on one handle: the kernel's self-cleaning counters must leave no state behind."""
     from blok_b200 import lib, synth
