@@ -75,10 +75,14 @@ static int static_smem_of(const void *kernel, size_t *bytes) {
   return BLOK_OK;
 }
 
+constexpr size_t kFreeSmem = 48 * 1024, kMostSmem = 227 * 1024;  // of a block, static arrays included: unasked, and at most
+
 int allow_smem_of(const void *kernel, size_t dynamic) {
   size_t fixed = 0;
   if (int rc = static_smem_of(kernel, &fixed)) return rc;
-  if (fixed + dynamic > 48 * 1024) BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynamic));
+  if (fixed + dynamic <= kFreeSmem) return BLOK_OK;
+  BLOK_REQUIRE(fixed + dynamic <= kMostSmem, BLOK_ERR_SHAPE, "a kernel wants %zu bytes of shared memory (at most %zu)", fixed + dynamic, kMostSmem);
+  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMostSmem - fixed)));
   return BLOK_OK;
 }
 

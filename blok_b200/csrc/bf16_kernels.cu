@@ -276,9 +276,6 @@ __global__ void add_bf16_kernel(uint16_t *__restrict__ a, const uint16_t *__rest
   if (i < n) a[i] = f32_to_bf16_bits(bf16_bits_to_f32(a[i]) + bf16_bits_to_f32(b[i]));
 }
 
-// Dynamic shared memory that a launch gets without asking: 48 KB less what the kernels keep in static arrays (up to 8 KB).
-constexpr size_t kBfFreeSmem = 40 * 1024 - 256;
-
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 int launch_bf16_gemv(const uint16_t *w, const uint16_t *x, uint16_t *y_bf16, float *y_f32, int rows, int cols, int T,
@@ -286,8 +283,7 @@ int launch_bf16_gemv(const uint16_t *w, const uint16_t *x, uint16_t *y_bf16, flo
   size_t smem = bf16_x_row_bytes(cols) * T;
   bool tc = rows % 16 == 0 && cols % 32 == 0 && aligned16(w) && aligned16(x) && smem <= 200 * 1024;
   if (tc) {
-    if (smem > kBfFreeSmem)
-      BLOK_CUDA(cudaFuncSetAttribute(bf16_gemv16_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(bf16_gemv16_kernel<0>, smem)) return rc;
     int nwarps = cols >= 4096 ? 16 : (cols >= 1024 ? 8 : 4);
     bf16_gemv16_kernel<0><<<rows / 16, nwarps * 32, smem, stream>>>(w, nullptr, x, y_bf16, y_f32, rows, cols, T);
     return launch_status("bf16_gemv16_kernel");
@@ -327,8 +323,7 @@ int launch_bf16_gemv_splitk(const uint16_t *w, const uint16_t *x, uint16_t *y_bf
     return launch_status("bf16_gemv16_splitk_kernel<l1>");
   }
   const size_t smem = bf16_x_row_bytes(per * 32) * T;
-  if (smem > kBfFreeSmem)
-    BLOK_CUDA(cudaFuncSetAttribute(bf16_gemv16_splitk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int rc = allow_smem(bf16_gemv16_splitk_kernel<true>, smem)) return rc;
   bf16_gemv16_splitk_kernel<true><<<dim3(rb, ksplit), 128, smem, stream>>>(w, x, y_bf16, y_f32, rows, cols, T, per, part, tickets);
   return launch_status("bf16_gemv16_splitk_kernel");
 }
@@ -400,8 +395,7 @@ int bf16_mlp(const blok_bf16_t *gate, const blok_bf16_t *up, const blok_bf16_t *
 int launch_bf16_gateup(const uint16_t *gate, const uint16_t *up, const uint16_t *x, uint16_t *mid, int ffn, int cols,
                        int T, cudaStream_t stream) {
   size_t smem = bf16_x_row_bytes(cols) * T;
-  if (smem > kBfFreeSmem)
-    BLOK_CUDA(cudaFuncSetAttribute(bf16_gemv16_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int rc = allow_smem(bf16_gemv16_kernel<1>, smem)) return rc;
   int nwarps = cols >= 4096 ? 16 : (cols >= 1024 ? 8 : 4);
   bf16_gemv16_kernel<1><<<ffn / 8, nwarps * 32, smem, stream>>>(gate, up, x, mid, nullptr, ffn, cols, T);
   return launch_status("bf16_gemv16_kernel<swiglu>");

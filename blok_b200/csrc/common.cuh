@@ -40,6 +40,8 @@ inline int launch_status(const char *what) {
 int sm_count();
 
 // Lets a kernel be launched with `dynamic` bytes of dynamic shared memory: a launch gets 48 KB, its static arrays among them, without asking.
+// The limit is the function's, for all threads of the program, so it is always set to the same value: a smaller one could come between
+// another thread's call and its launch.
 int allow_smem_of(const void *kernel, size_t dynamic);
 template <typename... P>
 inline int allow_smem(void (*kernel)(P...), size_t dynamic) {

@@ -236,7 +236,7 @@ static int gp_pairs(int *out) {
   static std::atomic<int> known{0};
   if (!known.load()) {
     auto kernel = gemm_pair_kernel<BN, ACT, F32>;
-    BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GpCfg<BN>::kSmem));
+    if (int rc = allow_smem(kernel, GpCfg<BN>::kSmem)) return rc;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -267,7 +267,7 @@ static int gp_launch(const GemmTma &g, cudaStream_t stream) {
   if (int rc = gp_pairs<BN, ACT, F32>(&pairs)) return rc;
   pairs = std::min(tl.rows * tl.cols * tl.parts, pairs);
   auto kernel = gemm_pair_kernel<BN, ACT, F32>;
-  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GpCfg<BN>::kSmem));
+  if (int rc = allow_smem(kernel, GpCfg<BN>::kSmem)) return rc;
   const CUtensorMap &w = BN == 128 && !kGated ? *g.w64 : *g.w128;
   return launch_pdl("gemm_pair_kernel", kernel, 2 * pairs, kGpThreads, (size_t)GpCfg<BN>::kSmem, stream, *g.x, w, g.up128 ? *g.up128 : *g.w128, a, tl);
 }

@@ -166,7 +166,7 @@ int gt_wide(const GemmTma &g) { return !g.out_f32 && g.R % 8 == 0 && g.ldo % 8 =
 template <int BN, int ACT, bool F32>
 static int gt_launch(const GemmTma &g, dim3 grid, cudaStream_t stream) {
   const GtArgs a = {g.out, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.T, g.R, g.K, g.ldo, g.act_cols, g.up_row, g.err, gt_wide(g)};
-  BLOK_CUDA(cudaFuncSetAttribute(gemm_tma_kernel<BN, ACT, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, GtCfg<BN>::kSmem));
+  if (int rc = allow_smem(gemm_tma_kernel<BN, ACT, F32>, GtCfg<BN>::kSmem)) return rc;
   gemm_tma_kernel<BN, ACT, F32><<<grid, kGtThreads, GtCfg<BN>::kSmem, stream>>>(
       *g.x, BN == 128 || ACT == GEMM_ACT_SWIGLU || ACT == GEMM_ACT_SWIGLU_REF ? *g.w128 : *g.w256, g.up128 ? *g.up128 : *g.w128, a);
   return launch_status("gemm_tma_kernel");

@@ -365,7 +365,7 @@ template <typename Act>
 static int ga_simple(const GroupedShape &s, const GroupedQuery<Act> &a, const void *pool, const StackRows &r, int T, cudaStream_t stream) {
   const size_t smem = (size_t)(s.dim + s.vdim) * sizeof(float);
   BLOK_REQUIRE(smem <= 200 * 1024, BLOK_ERR_SHAPE, "grouped attention: heads of %d / %d are too wide", s.dim, s.vdim);
-  if (smem > 40 * 1024) BLOK_CUDA(cudaFuncSetAttribute(grouped_attend_simple_kernel<Act>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int rc = allow_smem(grouped_attend_simple_kernel<Act>, smem)) return rc;
   grouped_attend_simple_kernel<Act><<<dim3(s.heads, T), kGsKeys, smem, stream>>>(s, a, static_cast<const Act *>(pool), r);
   return launch_status("grouped_attend_simple_kernel");
 }
@@ -374,7 +374,7 @@ template <int MT, int NT>
 static int ga_launch(const GroupedShape &s, const GroupedQuery<uint16_t> &a, const uint16_t *pool, const StackRows &r, int T, int splits, float *po,
                      float *pml, cudaStream_t stream) {
   const size_t smem = ga_smem_bytes(s, MT);
-  BLOK_CUDA(cudaFuncSetAttribute(grouped_attend_kernel<MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int rc = allow_smem(grouped_attend_kernel<MT, NT>, smem)) return rc;
   grouped_attend_kernel<MT, NT><<<dim3(splits, ga_blocks(s), T), kGaThreads, smem, stream>>>(s, a, pool, r, po, pml);
   return launch_status("grouped_attend_kernel");
 }

@@ -377,7 +377,7 @@ template <int MT, int NT>
 static int la_launch(const LatentShape &s, const uint16_t *q, const uint16_t *pool, const StackRows &r, int T, int splits, float *po, float *pml,
                      cudaStream_t stream) {
   const size_t smem = la_smem_bytes(s, MT);
-  BLOK_CUDA(cudaFuncSetAttribute(latent_attend_kernel<MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int rc = allow_smem(latent_attend_kernel<MT, NT>, smem)) return rc;
   latent_attend_kernel<MT, NT><<<dim3(splits, (s.heads + 16 * MT - 1) / (16 * MT), T), kLaThreads, smem, stream>>>(s, q, pool, r, po, pml);
   return launch_status("latent_attend_kernel");
 }
@@ -389,11 +389,11 @@ int launch_latent_attend(const LatentShape &s, const void *q_abs, const void *po
     const size_t smem = (size_t)(s.row() + s.rank) * sizeof(float);
     BLOK_REQUIRE(smem <= 200 * 1024, BLOK_ERR_SHAPE, "latent attention: a latent of %d values is too wide", s.rank);
     if (f32) {
-      if (smem > 40 * 1024) BLOK_CUDA(cudaFuncSetAttribute(latent_attend_simple_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      if (int rc = allow_smem(latent_attend_simple_kernel<float>, smem)) return rc;
       latent_attend_simple_kernel<float><<<grid, kLsKeys, smem, stream>>>(s, static_cast<const float *>(q_abs), static_cast<const float *>(pool), r,
                                                                           static_cast<float *>(o));
     } else {
-      if (smem > 40 * 1024) BLOK_CUDA(cudaFuncSetAttribute(latent_attend_simple_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      if (int rc = allow_smem(latent_attend_simple_kernel<uint16_t>, smem)) return rc;
       latent_attend_simple_kernel<uint16_t><<<grid, kLsKeys, smem, stream>>>(s, static_cast<const uint16_t *>(q_abs), static_cast<const uint16_t *>(pool), r,
                                                                              static_cast<uint16_t *>(o));
     }
@@ -594,7 +594,7 @@ template <int DQ, int DV>
 static int lp_launch(const LatentShape &s, const uint16_t *q, const uint16_t *kv, const uint16_t *kr_all, int T, int n, uint16_t *o, int ldo,
                      cudaStream_t stream) {
   constexpr int smem = (kLpRows + 2 * kLpKeys) * (DQ * 2 + 16) + 2 * kLpKeys * (DV * 2 + 16);
-  BLOK_CUDA(cudaFuncSetAttribute(latent_prompt_kernel<DQ, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  if (int rc = allow_smem(latent_prompt_kernel<DQ, DV>, smem)) return rc;
   latent_prompt_kernel<DQ, DV><<<dim3((T + kLpRows - 1) / kLpRows, s.heads), kLpThreads, smem, stream>>>(s, q, kv, kr_all, T, n, o, ldo);
   return launch_status("latent_prompt_kernel");
 }

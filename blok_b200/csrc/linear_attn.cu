@@ -610,8 +610,8 @@ static int chunked(const LaArgs &r, cudaStream_t stream) {
   const dim3 grid(r.chunks, r.heads, (r.vdim + kLcCols - 1) / kLcCols);
   const size_t smem1 = (size_t)kSplitParts * kLinChunk * kp + (size_t)kLinChunk * kLcVPitch;
   const size_t smem3 = (size_t)2 * kLinChunk * kp + (size_t)kLinChunk * kLcVPitch + (size_t)kSplitParts * r.dim * kLcVPitch;
-  BLOK_CUDA(cudaFuncSetAttribute(linear_chunk_state_kernel<TOKEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
-  BLOK_CUDA(cudaFuncSetAttribute(linear_chunk_out_kernel<TOKEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3));
+  if (int rc = allow_smem(linear_chunk_state_kernel<TOKEN>, smem1)) return rc;
+  if (int rc = allow_smem(linear_chunk_out_kernel<TOKEN>, smem3)) return rc;
   if (int rc = launch_pdl("linear_chunk_state_kernel", linear_chunk_state_kernel<TOKEN>, grid, kLcThreads, smem1, stream, r)) return rc;
   if (int rc = launch_pdl("linear_scan_kernel", linear_scan_kernel<TOKEN>, dim3((r.dim * r.vdim / 4 + 127) / 128, r.heads), 128, 0, stream, r)) return rc;
   return launch_pdl("linear_chunk_out_kernel", linear_chunk_out_kernel<TOKEN>, grid, kLcThreads, smem3, stream, r);

@@ -226,12 +226,8 @@ __global__ void __launch_bounds__(kAttThreads, 1)
 
 int launch_mla_attend(const uint16_t *q, const uint16_t *cache, long ctx_stride, const int *seq_len, int B, int splits,
                       float scale, float *part_o, float *part_ml, cudaStream_t stream) {
-  static bool configured = false;
   const size_t smem = mla_attend_smem_bytes();
-  if (!configured) {
-    BLOK_CUDA(cudaFuncSetAttribute(mla_attend_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
+  if (int rc = allow_smem(mla_attend_kernel<false>, smem)) return rc;
   mla_attend_kernel<false><<<dim3(splits, B), kAttThreads, smem, stream>>>(q, cache, ctx_stride, seq_len, scale, part_o,
                                                                           part_ml, nullptr, nullptr, 0, 0);
   return launch_status("mla_attend_kernel");
@@ -241,12 +237,8 @@ int launch_mla_attend(const uint16_t *q, const uint16_t *cache, long ctx_stride,
 int launch_mla_attend_paged(const uint16_t *q, const uint16_t *pool, const int *block_table, const int *slot_of,
                             int table_stride, int page_rows, const int *seq_len, int B, int splits, float scale,
                             float *part_o, float *part_ml, cudaStream_t stream) {
-  static bool configured = false;
   const size_t smem = mla_attend_smem_bytes();
-  if (!configured) {
-    BLOK_CUDA(cudaFuncSetAttribute(mla_attend_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
+  if (int rc = allow_smem(mla_attend_kernel<true>, smem)) return rc;
   mla_attend_kernel<true><<<dim3(splits, B), kAttThreads, smem, stream>>>(q, pool, 0, seq_len, scale, part_o, part_ml,
                                                                          block_table, slot_of, table_stride, page_rows);
   return launch_status("mla_attend_kernel(paged)");

@@ -717,11 +717,7 @@ static int cache_tensor_map(const uint16_t *base, long rows, bool keep, CUtensor
 // CTAs; plan, parts: see the kernel.
 int launch_mla_attend_tc(const uint16_t *q, const uint16_t *cache, long ctx_stride, long total_rows, const int *seq_len, int B, int ctas,
                          float scale, float *part_o, float *part_ml, const MlaPlan *plan, int2 *parts, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    BLOK_CUDA(cudaFuncSetAttribute(mla_attend_tc_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemBytes));
-    configured = true;
-  }
+  if (int rc = allow_smem(mla_attend_tc_kernel<false, false>, kTaSmemBytes)) return rc;
   CUtensorMap map, qmap;
   if (int rc = cache_tensor_map(cache, total_rows, true, &map)) return rc;
   if (int rc = cache_tensor_map(q, (long)B * kTaHeads, false, &qmap)) return rc;
@@ -733,11 +729,7 @@ template <bool FINE>
 static int launch_paged(const uint16_t *q, const uint16_t *pool, long pool_rows, const int *block_table, const int *slot_of, int table_stride,
                         int page_rows, const int *seq_len, int B, int heads, dim3 grid, float scale, float *part_o, float *part_ml,
                         int planned, const MlaPlan *plan, int2 *parts, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    BLOK_CUDA(cudaFuncSetAttribute(mla_attend_tc_kernel<true, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTaSmemBytes));
-    configured = true;
-  }
+  if (int rc = allow_smem(mla_attend_tc_kernel<true, FINE>, kTaSmemBytes)) return rc;
   CUtensorMap map, qmap;
   if (int rc = cache_tensor_map(pool, pool_rows, true, &map)) return rc;
   if (int rc = cache_tensor_map(q, (long)B * heads, false, &qmap)) return rc;

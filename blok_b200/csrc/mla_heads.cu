@@ -449,7 +449,7 @@ int launch_mla_query(const uint16_t *wuk_t, int heads, const MlaQuery &a, cudaSt
   CUtensorMap mw;
   if (int rc = gemm_operand_map(wuk_t, (long)heads * a.kv_rank, a.nope, a.nope, 128, &mw)) return rc;
   const int smem = 2 * 16384 + 2 * ((a.B + 15) / 16 * 16) * 128 + 1024;
-  BLOK_CUDA(cudaFuncSetAttribute(mla_query_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  if (int rc = allow_smem(mla_query_kernel, smem)) return rc;
   return launch_pdl("mla_query_kernel", mla_query_kernel, dim3(heads, a.kv_rank / 128 + 1), kMqThreads, (size_t)smem, stream, mw, a);
 }
 
@@ -462,7 +462,7 @@ int launch_mla_value(const uint16_t *kv_b, int heads, MlaValue a, cudaStream_t s
   const int N = a.group <= 16 ? 16 : 32;
   // weights of the partial results: in the planned form those of consecutive entries are consecutive, fewer than CTAs + entries
   const int smem = kMvWBytes + (kMvRank / 64) * N * 128 + (a.splits ? a.group * a.splits : a.ctas + a.B) * (int)sizeof(float) + 1024;
-  BLOK_CUDA(cudaFuncSetAttribute(mla_value_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  if (int rc = allow_smem(mla_value_kernel, smem)) return rc;
   return launch_pdl("mla_value_kernel", mla_value_kernel, dim3(heads, (a.v_head + 127) / 128, groups), kMvThreads, (size_t)smem, stream, mw, a);
 }
 

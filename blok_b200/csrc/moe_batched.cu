@@ -235,7 +235,7 @@ static int launch_mb_route(const MbRoute &a, cudaStream_t stream) {
   const size_t smem = (size_t)((a.T * a.topk + 3) / 4 * 4 + (3 + a.T) * a.experts) * sizeof(int);
   const int blocks = 1 + (a.T * a.shared / 4 + 1023) / 1024;
   auto kernel = a.experts <= 128 ? mb_route_kernel<4> : mb_route_kernel<12>;
-  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int rc = allow_smem(kernel, smem)) return rc;
   return launch_pdl("mb_route_kernel", kernel, blocks, 1024, smem, stream, a);
 }
 

@@ -956,7 +956,7 @@ int fused_plan(const blok_moe_weights &w, FusedPlan *plan) {
   if (!coop) return BLOK_OK;
   size_t smem = fused_smem_bytes(w);
   if (smem > 227 * 1024) return BLOK_OK;
-  BLOK_CUDA(cudaFuncSetAttribute(moe_decode_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int rc = allow_smem(moe_decode_fused_kernel, smem)) return rc;
   int per_sm = 0;
   BLOK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_decode_fused_kernel, kFusedThreads, smem));
   if (per_sm < 1) return BLOK_OK;

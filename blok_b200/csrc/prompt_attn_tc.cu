@@ -345,7 +345,7 @@ int launch_prompt_attn(const CUtensorMap &mq, const CUtensorMap &mkv, const CUte
   const int smem = qc * kPtQChunk + a.stages * stage_bytes + 1024;
   const dim3 grid((a.T + kPtRows - 1) / kPtRows, a.heads);
   auto kernel = a.bias ? prompt_attn_tc_kernel<true> : prompt_attn_tc_kernel<false>;
-  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  if (int rc = allow_smem(kernel, smem)) return rc;
   return launch_pdl("prompt_attn_tc_kernel", kernel, grid, kPtThreads, (size_t)smem, stream, mq, mkv, mkr, a);
 }
 

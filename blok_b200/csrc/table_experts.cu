@@ -150,10 +150,10 @@ int launch_expert_gemv(const uint16_t *w, int R, int K, const int *table, const 
   BLOK_REQUIRE(K % 8 == 0 && smem <= 200 * 1024, BLOK_ERR_SHAPE, "expert mat-vec: %d columns", K);
   const dim3 grid(T * top, (R + kEgWarps * kEgRows - 1) / (kEgWarps * kEgRows));
   if (x_f32) {
-    if (smem > 48 * 1024) BLOK_CUDA(cudaFuncSetAttribute(expert_gemv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(expert_gemv_kernel<true>, smem)) return rc;
     expert_gemv_kernel<true><<<grid, kEgWarps * 32, smem, stream>>>(w, R, K, table, ids, vocab, top, x, shared_x, relu2, y, y_f32);
   } else {
-    if (smem > 48 * 1024) BLOK_CUDA(cudaFuncSetAttribute(expert_gemv_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(expert_gemv_kernel<false>, smem)) return rc;
     expert_gemv_kernel<false><<<grid, kEgWarps * 32, smem, stream>>>(w, R, K, table, ids, vocab, top, x, shared_x, relu2, y, y_f32);
   }
   return launch_status("expert_gemv_kernel");

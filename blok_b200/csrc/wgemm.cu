@@ -268,7 +268,7 @@ int launch_wgemm(int mode, const WgArgs &args, int max_tiles, cudaStream_t strea
   }
 #define BLOK_WG_LAUNCH(M)                                                                                         \
   {                                                                                                                \
-    BLOK_CUDA(cudaFuncSetAttribute(wgemm_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));      \
+    if (int rc = allow_smem(wgemm_kernel<M>, smem)) return rc;                                                     \
     wgemm_kernel<M><<<grid, kWgThreads, smem, stream>>>(args);                                                     \
   }
   switch (mode) {

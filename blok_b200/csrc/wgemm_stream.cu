@@ -267,7 +267,7 @@ int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t 
   if (swiglu && (rc = gemm_operand_map(args.w_b, args.R, args.K, args.K, kStRows / 2, &mwb))) return rc;
   if (args.R2 && (rc = gemm_operand_map(args.w_2, args.R2, args.K, args.K, kStRows, &mw2))) return rc;
   auto kernel = swiglu ? wgemm_stream_kernel<true> : wgemm_stream_kernel<false>;
-  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  if (int rc = allow_smem(kernel, smem)) return rc;
   *splits = nz;
   return launch_pdl("wgemm_stream_kernel", kernel, dim3(tiles, nz), kStThreads, (size_t)smem, stream, mx, mwa, mwb, mw2, a);
 }

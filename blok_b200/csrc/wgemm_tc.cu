@@ -484,7 +484,7 @@ static int i4_launch(bool swiglu, const WgArgs &g, const uint16_t *x, long x_row
   const I4Args a = {g.out_bf16, g.out_index, g.tile_expert, g.tile_start, g.tile_count, g.num_tiles, g.K, g.R, (int)g.expert_stride_rows, g.total,
                     g.w_a, g.w_b, g.s_a, g.s_b, x, g.err, g.overlap && !swiglu};
   auto kernel = swiglu ? wgemm_tc_kernel<true> : wgemm_tc_kernel<false>;
-  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kI4Smem));
+  if (int rc = allow_smem(kernel, kI4Smem)) return rc;
   return launch_pdl_if(g.overlap, "wgemm_tc_kernel", kernel, sm_count(), kI4Threads, (size_t)kI4Smem, stream, wa, wb, sa, sb, mx, a);
 }
 

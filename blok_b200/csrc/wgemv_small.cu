@@ -325,7 +325,7 @@ int launch_wgemv_small(int mode, const WgArgs &args, cudaStream_t stream) {
   const size_t smem = wgemv_small_smem_bytes(args.K);
   const int grid = sm_count();
   auto kernel = mode == WG_I4_SWIGLU ? wgemv_small_kernel<true> : wgemv_small_kernel<false>;
-  BLOK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int rc = allow_smem(kernel, smem)) return rc;
   return launch_pdl_if(args.overlap, "wgemv_small_kernel", kernel, grid, kGsThreads, smem, stream, args);
 }
 
