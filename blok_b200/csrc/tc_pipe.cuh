@@ -8,7 +8,10 @@
 
 namespace blok {
 
-constexpr unsigned kTpSpinLimit = 1u << 21;
+#ifndef BLOK_SPIN_LIMIT  // a test sets a lower one
+#define BLOK_SPIN_LIMIT (1u << 21)
+#endif
+constexpr unsigned kTpSpinLimit = BLOK_SPIN_LIMIT;
 
 __device__ __forceinline__ void tp_mbar_init(uint32_t mbar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");

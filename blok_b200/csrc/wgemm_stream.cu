@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(kStThreads) wgemm_stream_kernel(const __grid_c
     // the whole warp walks the steps, so that addresses and descriptors stay warp-uniform; one lane issues
     const bool issues = tp_elect();
     const uint32_t idesc = tp_idesc_bf16(a.N);
+    pdl_wait();  // the bound below is for this kernel's own copies, not for what the kernels in front still have to do
     int s = 0;
     uint32_t turn = 0;
     for (int c = 0; c < nsteps; ++c) {
