@@ -389,7 +389,7 @@ int launch_head_gemv(const uint16_t *w, long w_head_stride, const uint16_t *x, l
 }
 
 int bf16_mlp(const blok_bf16_t *gate, const blok_bf16_t *up, const blok_bf16_t *down, const blok_bf16_t *x, blok_bf16_t *y, int hidden, int ffn, int T,
-             void *workspace, size_t workspace_bytes, bool weights_early, blok_stream_t stream);
+             void *workspace, size_t workspace_bytes, bool weights_early, unsigned *err, blok_stream_t stream);
 
 // mid[T, ffn] = SwiGLU front half.
 int launch_bf16_gateup(const uint16_t *gate, const uint16_t *up, const uint16_t *x, uint16_t *mid, int ffn, int cols,
@@ -424,9 +424,9 @@ extern "C" size_t blok_bf16_mlp_workspace_bytes(int hidden, int ffn, int T) {
   return mlp_mid_bytes(ffn, T) + std::max(wgemm_splitk_bytes(WG_BF16_SWIGLU, hidden, ffn, T), wgemm_splitk_bytes(WG_BF16_PLAIN, ffn, hidden, T));
 }
 
-// weights_early: see WgArgs.
+// weights_early, err: see WgArgs.
 int blok::bf16_mlp(const blok_bf16_t *gate, const blok_bf16_t *up, const blok_bf16_t *down, const blok_bf16_t *x, blok_bf16_t *y, int hidden, int ffn,
-                   int T, void *workspace, size_t workspace_bytes, bool weights_early, blok_stream_t stream) {
+                   int T, void *workspace, size_t workspace_bytes, bool weights_early, unsigned *err, blok_stream_t stream) {
   BLOK_REQUIRE(gate && up && down && x && y && workspace, BLOK_ERR_ARG, "blok_bf16_mlp: null pointer");
   BLOK_REQUIRE(hidden > 0 && ffn > 0 && hidden % 32 == 0 && ffn % 32 == 0 && hidden % 16 == 0 && T >= 1 && T <= kWgStreamTokens,
                BLOK_ERR_SHAPE, "blok_bf16_mlp: hidden %d, ffn %d must be multiples of 32 and 1 <= T=%d <= %d", hidden, ffn, T,
@@ -443,26 +443,27 @@ int blok::bf16_mlp(const blok_bf16_t *gate, const blok_bf16_t *up, const blok_bf
   if (T > 8) {  // 9..64 rows: each matrix streamed once for all rows (wgemm_stream.cu)
     float *sk = reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + mlp_mid_bytes(ffn, T));
     const size_t sk_bytes = workspace_bytes - mlp_mid_bytes(ffn, T);
-    if (int rc = launch_wgemm_rows(WG_BF16_SWIGLU, gate, up, x, mid, nullptr, ffn, hidden, T, sk, sk_bytes, (cudaStream_t)stream, weights_early)) return rc;
-    return launch_wgemm_rows(WG_BF16_PLAIN, down, nullptr, mid, y, nullptr, hidden, ffn, T, sk, sk_bytes, (cudaStream_t)stream, true);
+    if (int rc = launch_wgemm_rows(WG_BF16_SWIGLU, gate, up, x, mid, nullptr, ffn, hidden, T, sk, sk_bytes, (cudaStream_t)stream, weights_early, err))
+      return rc;
+    return launch_wgemm_rows(WG_BF16_PLAIN, down, nullptr, mid, y, nullptr, hidden, ffn, T, sk, sk_bytes, (cudaStream_t)stream, true, err);
   }
   // a workspace with room behind the vector (a model's has it) lets the weight stream cut K into parts
   const size_t at = mlp_mid_bytes(ffn, T), room = workspace_bytes > at ? workspace_bytes - at : 0;
   float *sk = room ? reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + at) : nullptr;
   const WgArgs front = wgemm_rows(gate, up, x, mid, nullptr, ffn, hidden, T);
   int rc = wgemm_stream_takes_few(WG_BF16_SWIGLU, front) || wgemm_stream_takes_parts(WG_BF16_SWIGLU, front, room)
-               ? launch_wgemm_rows(WG_BF16_SWIGLU, gate, up, x, mid, nullptr, ffn, hidden, T, sk, room, (cudaStream_t)stream, weights_early)
+               ? launch_wgemm_rows(WG_BF16_SWIGLU, gate, up, x, mid, nullptr, ffn, hidden, T, sk, room, (cudaStream_t)stream, weights_early, err)
                : launch_bf16_gateup(gate, up, x, mid, ffn, hidden, T, (cudaStream_t)stream);
   if (rc) return rc;
   if (wgemm_stream_takes_parts(WG_BF16_PLAIN, wgemm_rows(down, nullptr, mid, y, nullptr, hidden, ffn, T), room))
-    return launch_wgemm_rows(WG_BF16_PLAIN, down, nullptr, mid, y, nullptr, hidden, ffn, T, sk, room, (cudaStream_t)stream, true);
+    return launch_wgemm_rows(WG_BF16_PLAIN, down, nullptr, mid, y, nullptr, hidden, ffn, T, sk, room, (cudaStream_t)stream, true, err);
   return launch_bf16_gemv(down, mid, y, nullptr, hidden, ffn, T, (cudaStream_t)stream);
 }
 
 extern "C" int blok_bf16_mlp(const blok_bf16_t *gate, const blok_bf16_t *up, const blok_bf16_t *down,
                              const blok_bf16_t *x, blok_bf16_t *y, int hidden, int ffn, int T, void *workspace,
                              size_t workspace_bytes, blok_stream_t stream) {
-  return blok::bf16_mlp(gate, up, down, x, y, hidden, ffn, T, workspace, workspace_bytes, false, stream);
+  return blok::bf16_mlp(gate, up, down, x, y, hidden, ffn, T, workspace, workspace_bytes, false, nullptr, stream);
 }
 
 extern "C" int blok_rmsnorm(const blok_bf16_t *x, const blok_bf16_t *w, blok_bf16_t *y, int T, int n, float eps,

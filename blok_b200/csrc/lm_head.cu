@@ -141,11 +141,11 @@ extern "C" size_t blok_lm_head_workspace_bytes(int vocab, int T) {
 
 namespace blok {
 int lm_head_argmax(const blok_bf16_t *w, const blok_bf16_t *n, int vocab, int hidden, int T, uint32_t *ids, void *workspace, size_t workspace_bytes,
-                   bool weights_early, blok_stream_t stream);
+                   bool weights_early, unsigned *err, blok_stream_t stream);
 }
-// weights_early: see WgArgs.
+// weights_early, err: see WgArgs.
 int blok::lm_head_argmax(const blok_bf16_t *w, const blok_bf16_t *n, int vocab, int hidden, int T, uint32_t *ids, void *workspace,
-                         size_t workspace_bytes, bool weights_early, blok_stream_t stream) {
+                         size_t workspace_bytes, bool weights_early, unsigned *err, blok_stream_t stream) {
   BLOK_REQUIRE(w && n && ids && workspace, BLOK_ERR_ARG, "blok_lm_head_argmax: null pointer");
   BLOK_REQUIRE(vocab > 0 && hidden > 0 && hidden % 8 == 0 && T >= 1 && T <= kWgStreamTokens, BLOK_ERR_SHAPE,
                "blok_lm_head_argmax: unsupported shape vocab=%d hidden=%d T=%d", vocab, hidden, T);
@@ -156,7 +156,8 @@ int blok::lm_head_argmax(const blok_bf16_t *w, const blok_bf16_t *n, int vocab, 
   uint16_t *logits = static_cast<uint16_t *>(workspace);
   // one pass of the weight-streaming kernel over the table; up to 8 rows of a small one: the mat-vec kernel
   const bool streams = T > 8 || wgemm_stream_takes_few(WG_BF16_PLAIN, wgemm_rows(w, nullptr, n, logits, nullptr, vocab, hidden, T));
-  int rc = streams ? launch_wgemm_rows(WG_BF16_PLAIN, w, nullptr, n, logits, nullptr, vocab, hidden, T, nullptr, 0, (cudaStream_t)stream, weights_early)
+  int rc = streams ? launch_wgemm_rows(WG_BF16_PLAIN, w, nullptr, n, logits, nullptr, vocab, hidden, T, nullptr, 0, (cudaStream_t)stream, weights_early,
+                                        err)
                    : launch_bf16_gemv(w, n, logits, nullptr, vocab, hidden, T, (cudaStream_t)stream);
   if (rc) return rc;
   argmax_bf16_kernel<<<T, 1024, 0, (cudaStream_t)stream>>>(logits, vocab, ids);
@@ -165,7 +166,7 @@ int blok::lm_head_argmax(const blok_bf16_t *w, const blok_bf16_t *n, int vocab, 
 
 extern "C" int blok_lm_head_argmax(const blok_bf16_t *w, const blok_bf16_t *n, int vocab, int hidden, int T,
                                    uint32_t *ids, void *workspace, size_t workspace_bytes, blok_stream_t stream) {
-  return blok::lm_head_argmax(w, n, vocab, hidden, T, ids, workspace, workspace_bytes, false, stream);
+  return blok::lm_head_argmax(w, n, vocab, hidden, T, ids, workspace, workspace_bytes, false, nullptr, stream);
 }
 
 extern "C" int blok_embed(const blok_bf16_t *table, const uint32_t *ids, int vocab, int hidden, int T, blok_bf16_t *x,

@@ -8,6 +8,7 @@
 #include <sstream>
 
 #include "model.h"
+#include "wgemm.h"
 
 namespace blok {
 
@@ -49,6 +50,15 @@ int dev_alloc(blok_model *m, size_t bytes, void **out) {
   return BLOK_OK;
 }
 
+int model_products_check(blok_model *m) {
+  unsigned err = 0;
+  BLOK_CUDA(cudaMemcpy(&err, m->err, sizeof(err), cudaMemcpyDeviceToHost));
+  if (!err) return BLOK_OK;
+  BLOK_CUDA(cudaMemset(m->err, 0, sizeof(err)));
+  set_error("a product gave up on a barrier");
+  return BLOK_ERR_TIMEOUT;
+}
+
 int alloc_serving_state(blok_model *m) {
   const blok_model_config &c = m->cfg;
   int rc;
@@ -56,6 +66,8 @@ int alloc_serving_state(blok_model *m) {
       (rc = dev_alloc_as(m, c.prefill_chunk > 0 ? std::max(c.max_ctx, m->rows) : 1, &m->prompt_ids)))
     return rc;
   BLOK_CUDA(cudaMemset(m->pos, 0, c.max_batch * 4));
+  if ((rc = dev_alloc_as(m, 1, &m->err))) return rc;
+  BLOK_CUDA(cudaMemset(m->err, 0, sizeof(unsigned)));
   m->host_pos.assign(c.max_batch, 0);
   if (c.kv_page_rows > 0) {
     m->table_stride = (c.max_ctx + c.kv_page_rows - 1) / c.kv_page_rows;
@@ -90,6 +102,12 @@ extern "C" int blok_model_destroy(blok_model_t *m) {
 extern "C" int blok_model_get_config(blok_model_t *m, blok_model_config *cfg) {
   BLOK_REQUIRE(m && cfg, BLOK_ERR_ARG, "blok_model_get_config: null pointer");
   *cfg = m->cfg;
+  return BLOK_OK;
+}
+
+extern "C" int blok_debug_set_products_error(blok_model_t *m, unsigned code) {
+  if (!m) return wgemm_stream_set_error(code);
+  BLOK_CUDA(cudaMemcpy(m->err, &code, sizeof(code), cudaMemcpyHostToDevice));
   return BLOK_OK;
 }
 

@@ -57,6 +57,7 @@ struct blok_model {
   int chunk_slot = 0;                        // slot of the prompt chunk in flight
   int *pos = nullptr;                        // [max_batch]
   uint32_t *ids = nullptr, *next = nullptr;  // [rows]
+  unsigned *err = nullptr;                   // [1] set to 1 by a product of this model (not of a layer's handle) whose wait gave up
   // One CUDA graph of the whole step per batch size: a step is many small launches per layer and the host cannot issue
   // them as fast as the GPU runs them.  steps_seen counts eager steps (the first one also sets kernel attributes).
   cudaGraphExec_t step_graph[blok::kMaxBatch + 1] = {};
@@ -79,6 +80,8 @@ int dev_alloc_as(blok_model *m, size_t count, T **out) {
   *out = static_cast<T *>(p);
   return BLOK_OK;
 }
+// Reports (BLOK_ERR_TIMEOUT), once, that a wait of one of the model's own products gave up; the stream they ran on is synchronised.
+int model_products_check(blok_model *m);
 // Token buffers, positions and, for a paged model, the page table; m->cfg and m->rows are set.
 int alloc_serving_state(blok_model *m);
 

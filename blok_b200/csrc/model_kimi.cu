@@ -51,9 +51,9 @@ __global__ void sharded_finish_kernel(const float *__restrict__ part, const uint
 
 // Forms of the public calls for a model whose weights were there before the call's first launch (the embedding, an ordinary one).
 int bf16_mlp(const blok_bf16_t *gate, const blok_bf16_t *up, const blok_bf16_t *down, const blok_bf16_t *x, blok_bf16_t *y, int hidden, int ffn, int T,
-             void *workspace, size_t workspace_bytes, bool weights_early, blok_stream_t stream);
+             void *workspace, size_t workspace_bytes, bool weights_early, unsigned *err, blok_stream_t stream);
 int lm_head_argmax(const blok_bf16_t *w, const blok_bf16_t *n, int vocab, int hidden, int T, uint32_t *ids, void *workspace, size_t workspace_bytes,
-                   bool weights_early, blok_stream_t stream);
+                   bool weights_early, unsigned *err, blok_stream_t stream);
 void mla_layer_weights_stay(blok_mla_layer_t *L);
 int launch_bf16_gemv(const uint16_t *w, const uint16_t *x, uint16_t *y_bf16, float *y_f32, int rows, int cols, int T,
                      cudaStream_t stream);
@@ -388,11 +388,9 @@ static int check(blok_model *m, blok_stream_t stream) {
       message = "layer " + std::to_string(l) + ": " + blok_last_error();
     }
   }
-  if (first == BLOK_OK) {  // the dense layers' and the head's products have no handle
-    unsigned err = 0;
-    if (int rc = wgemm_stream_take_error(&err)) return rc;
-    BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");
-  }
+  BLOK_CUDA(cudaStreamSynchronize((cudaStream_t)stream));  // the dense layers' and the head's products have no handle
+  const int own = model_products_check(m);
+  if (first == BLOK_OK && own != BLOK_OK) return own;
   if (first == BLOK_OK && K->comm) return blok_comm_check(K->comm);
   if (first != BLOK_OK) set_error("%s", message.c_str());
   return first;
@@ -434,7 +432,7 @@ static int moe_sharded_rows(blok_model_t *m, blok::LayerWeights &L, int T, blok_
   for (int t0 = 0; t0 < T; t0 += stream_rows ? kWgStreamTokens : 8) {
     const int nrows = std::min(T - t0, stream_rows ? kWgStreamTokens : 8);
     rc = nrows > 8 ? launch_wgemm_rows(WG_BF16_PLAIN, router, nullptr, K->n + (size_t)t0 * c.hidden, nullptr, K->ep_logits + (size_t)t0 * c.experts,
-                                       c.experts, c.hidden, nrows, K->ep_sk, K->ep_sk_bytes, stream)
+                                       c.experts, c.hidden, nrows, K->ep_sk, K->ep_sk_bytes, stream, false, m->err)
                    : launch_bf16_gemv(router, K->n + (size_t)t0 * c.hidden, nullptr, K->ep_logits + (size_t)t0 * c.experts, c.experts, c.hidden,
                                       nrows, stream);
     if (rc) return rc;
@@ -476,7 +474,7 @@ static int ffn_rows(blok_model_t *m, int l, int T, bool chunk, blok_stream_t str
     if (wide && T > 8 && K->mlp_rows > 8) group = K->mlp_rows;  // one pass over the weights for up to 64 rows
     for (int b = 0; b < T && !rc; b += group)
       rc = bf16_mlp(tp<uint16_t>(L.t, "gate_proj"), tp<uint16_t>(L.t, "up_proj"), tp<uint16_t>(L.t, "down_proj"), K->n + b * H,
-                         K->tmp + b * H, c.hidden, c.dense_inter, T - b < group ? T - b : group, K->mlp_ws, K->mlp_ws_bytes, true, stream_);
+                         K->tmp + b * H, c.hidden, c.dense_inter, T - b < group ? T - b : group, K->mlp_ws, K->mlp_ws_bytes, true, m->err, stream_);
     return rc;
   }
   if (c.ep_world > 1) return moe_sharded_rows(m, L, T, stream_);
@@ -522,7 +520,7 @@ static int sample(blok_model *m, int row, int n, uint32_t *next, blok_stream_t s
   const int head_rows = (c.vocab % 16 == 0 && c.hidden % 256 == 0) ? kWgStreamTokens : 8;
   for (int b = 0; b < n; b += head_rows)
     if (int rc = lm_head_argmax(tp<uint16_t>(K->top, "lm_head"), K->n + (size_t)(row + b) * c.hidden, c.vocab, c.hidden,
-                                     n - b < head_rows ? n - b : head_rows, next + b, K->head_ws, K->head_ws_bytes, true, stream))
+                                     n - b < head_rows ? n - b : head_rows, next + b, K->head_ws, K->head_ws_bytes, true, m->err, stream))
       return rc;
   return BLOK_OK;
 }

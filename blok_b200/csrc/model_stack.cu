@@ -111,6 +111,7 @@ struct StackModel {
   float *host_logits = nullptr;  // pinned, kPinnedRows rows of the vocabulary
   float *splitk_ws = nullptr;
   size_t splitk_bytes = 0;
+  unsigned *err = nullptr;  // the model's
   std::map<std::pair<const void *, int>, CUtensorMap> x_maps;
   std::map<const void *, size_t> buffer_bytes;
 };
@@ -548,11 +549,12 @@ int product(StackModel *S, const Mat &w, const void *x, int T, void *y, bool y_f
   uint16_t *yb = y_f32 ? nullptr : static_cast<uint16_t *>(y);
   float *yf = y_f32 ? static_cast<float *>(y) : nullptr;
   if (T <= 8 && wgemm_stream_takes_few(WG_BF16_PLAIN, wgemm_rows(w.w, nullptr, xb, yb, yf, w.R, w.K, T)))
-    return launch_wgemm_rows(WG_BF16_PLAIN, w.w, nullptr, xb, yb, yf, w.R, w.K, T, nullptr, 0, stream);
+    return launch_wgemm_rows(WG_BF16_PLAIN, w.w, nullptr, xb, yb, yf, w.R, w.K, T, nullptr, 0, stream, false, S->err);
   if (T <= 8) return launch_bf16_gemv_splitk(w.w, xb, yb, yf, w.R, w.K, T, S->gemv_ws, S->gemv_ws_bytes, stream);
   if (T <= kWgStreamTokens && w.K % 256 == 0 && w.R % 16 == 0)
-    return launch_wgemm_rows(WG_BF16_PLAIN, w.w, nullptr, xb, yb, yf, w.R, w.K, T, S->splitk_ws, S->splitk_bytes, stream);
+    return launch_wgemm_rows(WG_BF16_PLAIN, w.w, nullptr, xb, yb, yf, w.R, w.K, T, S->splitk_ws, S->splitk_bytes, stream, false, S->err);
   GemmTma g;
+  g.err = S->err;
   TRY(x_map(S, x, w.K, &g.x));
   g.w128 = &w.m128;
   g.w256 = &w.m256;
@@ -580,6 +582,7 @@ int sublayer_product(StackModel *S, const Mat &w, const void *x, int T, cudaStre
     const int parts = std::min({4, w.K / 64 / 16, sm_count() / 2 / tiles, (int)(S->y_rows / T)});
     if (parts > 1) {
       GemmTma g;
+      g.err = S->err;
       TRY(x_map(S, x, w.K, &g.x));
       g.w128 = &w.m128;
       g.w64 = &w.m64;
@@ -821,6 +824,7 @@ int stack_build(blok_model *m, const char *dir, uint64_t seed) {
     BLOK_CUDA(cudaMemcpy(S->plans_dev, plans.data(), plans.size() * sizeof(ExpertPlanArgs), cudaMemcpyHostToDevice));
   }
   TRY(alloc_serving_state(m));
+  S->err = m->err;
   BLOK_CUDA(cudaDeviceSynchronize());
   return BLOK_OK;
 }
@@ -904,6 +908,7 @@ int run_latent(const Call &c, const LayerState &L, const Run &r) {
     TRY(launch_latent_rotate(s, S->proj, c.rows, c.T, S->proj, s.head(), s.dim, false, c.stream));
     TRY(launch_latent_gather(s, static_cast<const uint16_t *>(r.pool), c.rows, slot, n, S->c_all, S->kr_all, c.stream));
     GemmTma g;
+    g.err = S->err;
     TRY(x_map(S, S->c_all, s.rank, &g.x));
     g.w128 = &L.kvb.m128;
     g.w256 = &L.kvb.m256;
@@ -1018,9 +1023,10 @@ int run_dense(const Call &c, const LayerState &L) {
   } else if (c.T <= 8 && ((size_t)L.up.K * 2 + 64) * c.T <= 200 * 1024) {
     TRY(launch_bf16_gateup(L.up.w, up, h, mid, ff, L.up.K, c.T, c.stream));
   } else if (c.T > 8 && c.T <= kWgStreamTokens && L.up.K % 256 == 0) {
-    TRY(launch_wgemm_rows(WG_BF16_SWIGLU, L.up.w, up, h, mid, nullptr, ff, L.up.K, c.T, S->splitk_ws, S->splitk_bytes, c.stream));
+    TRY(launch_wgemm_rows(WG_BF16_SWIGLU, L.up.w, up, h, mid, nullptr, ff, L.up.K, c.T, S->splitk_ws, S->splitk_bytes, c.stream, false, S->err));
   } else {
     GemmTma g;
+    g.err = S->err;
     TRY(x_map(S, S->h, L.up.K, &g.x));
     g.w128 = &L.up.m128;
     g.T = c.T;
@@ -1044,6 +1050,7 @@ int run_experts(const Call &c, const TableExperts &x, const LayerState &L) {
     return launch_expert_gemv(L.down.w, L.down.R, L.down.K, L.table, ids, S->spec.vocab, x.top, c.T, S->mid, S->f32, false, false, S->y, true, c.stream);
   }
   GemmTma g;
+  g.err = S->err;
   g.tile_expert = L.plan.tile_expert;
   g.tile_start = L.plan.tile_start;
   g.tile_count = L.plan.tile_count;
@@ -1241,15 +1248,10 @@ int stack_logits(blok_model *m, const int *rows, int n, float *out, blok_stream_
   return BLOK_OK;
 }
 
-int stack_check(blok_model *, blok_stream_t stream) {
+int stack_check(blok_model *m, blok_stream_t stream) {
   BLOK_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  TRY(model_products_check(m));
   unsigned err = 0;
-  TRY(gemm_tma_take_error(&err));
-  BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");
-  TRY(gemm_pair_take_error(&err));
-  BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");
-  TRY(wgemm_stream_take_error(&err));
-  BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");
   TRY(prompt_attn_take_error(&err));
   BLOK_REQUIRE(!err, BLOK_ERR_TIMEOUT, "attention over a prompt gave up on a barrier");
   TRY(mla_attend_tc_take_error(&err));

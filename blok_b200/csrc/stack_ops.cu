@@ -4,6 +4,7 @@
 
 #include "gemm_tma.h"
 #include "stack_kernels.h"
+#include "wgemm.h"
 #include "common.cuh"
 
 using namespace blok;
@@ -112,6 +113,15 @@ extern "C" int blok_latent_prompt(const blok_bf16_t *q, const blok_bf16_t *kv, c
   const LatentShape s = latent_shape(heads, dim, rot, vdim, 32, scale);
   if (int rc = latent_sizes_ok(s, "blok_latent_prompt")) return rc;
   return launch_latent_prompt(s, q, kv, k_rot, T, n, o, ld_out, (cudaStream_t)stream);
+}
+
+extern "C" int blok_products_check(blok_stream_t stream) {
+  BLOK_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+  unsigned tma = 0, pair = 0, few = 0;
+  int rc;
+  if ((rc = gemm_tma_take_error(&tma)) || (rc = gemm_pair_take_error(&pair)) || (rc = wgemm_stream_take_error(&few))) return rc;
+  BLOK_REQUIRE(!tma && !pair && !few, BLOK_ERR_TIMEOUT, "a product gave up on a barrier");
+  return BLOK_OK;
 }
 
 extern "C" int blok_gemm_bf16(const blok_bf16_t *x, const blok_bf16_t *w, int T, int R, int K, int relu2, blok_bf16_t *out_bf16, float *out_f32,

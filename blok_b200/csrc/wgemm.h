@@ -87,13 +87,14 @@ bool wgemm_stream_takes_few(int mode, const WgArgs &args);
 bool wgemm_stream_takes_parts(int mode, const WgArgs &args, size_t room);
 // *out becomes non-zero if a CTA without an error word of its own has given up since the last call (the flag is cleared).
 int wgemm_stream_take_error(unsigned *out);
+int wgemm_stream_set_error(unsigned code);  // for tests
 // The reduction behind a K-split launch: adds the nz partial sums in split order and applies the epilogue.
 int launch_wgemm_splitk_reduce(int mode, const WgArgs &args, int nz, cudaStream_t stream);
 int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t stream);
 // One dense product through launch_wgemm without tile tables: out[T, R] = W[R, K] x[T, K] (mode WG_BF16_PLAIN; bf16 or
 // fp32 output) or the SwiGLU front half of (w_a = gate, w_b = up) (mode WG_BF16_SWIGLU), for 1 <= T <= kWgStreamTokens.
 int launch_wgemm_rows(int mode, const void *w_a, const void *w_b, const uint16_t *x, uint16_t *out_bf16, float *out_f32, int R, int K,
-                      int T, float *splitk_ws, size_t splitk_bytes, cudaStream_t stream, bool weights_early = false);
+                      int T, float *splitk_ws, size_t splitk_bytes, cudaStream_t stream, bool weights_early = false, unsigned *err = nullptr);
 WgArgs wgemm_rows(const void *w_a, const void *w_b, const uint16_t *x, uint16_t *out_bf16, float *out_f32, int R, int K, int T);  // its launch
 
 // Both products of the grouped experts, INT4: mid = SwiGLU front half of x (up: WG_I4_SWIGLU), then the down projection

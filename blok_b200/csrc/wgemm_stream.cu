@@ -280,6 +280,11 @@ int wgemm_stream_take_error(unsigned *out) {
   return BLOK_OK;
 }
 
+int wgemm_stream_set_error(unsigned code) {
+  BLOK_CUDA(cudaMemcpyToSymbol(g_wgemm_stream_error, &code, sizeof(unsigned)));
+  return BLOK_OK;
+}
+
 // Adds the K-split partial sums in split order and applies the epilogue of the GEMM kernels.  grid = (ceil(R / 256), n_rows).
 template <bool SWIGLU>
 __global__ void wgemm_splitk_reduce_kernel(const WgArgs a, int nz) {
@@ -362,9 +367,9 @@ WgArgs wgemm_rows(const void *w_a, const void *w_b, const uint16_t *x, uint16_t 
 }
 
 int launch_wgemm_rows(int mode, const void *w_a, const void *w_b, const uint16_t *x, uint16_t *out_bf16, float *out_f32, int R, int K,
-                      int T, float *splitk_ws, size_t splitk_bytes, cudaStream_t stream, bool weights_early) {
+                      int T, float *splitk_ws, size_t splitk_bytes, cudaStream_t stream, bool weights_early, unsigned *err) {
   WgArgs r = wgemm_rows(w_a, w_b, x, out_bf16, out_f32, R, K, T);
-  r.splitk_ws = splitk_ws; r.splitk_bytes = splitk_bytes; r.weights_early = weights_early;
+  r.splitk_ws = splitk_ws; r.splitk_bytes = splitk_bytes; r.weights_early = weights_early; r.err = err;
   BLOK_REQUIRE(wgemm_stream_supports(mode, r), BLOK_ERR_SHAPE, "wgemm rows: %d rows x %d columns over %d tokens is outside the streaming kernel",
                R, K, T);
   int nz = 1;

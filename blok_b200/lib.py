@@ -858,6 +858,12 @@ def gemm_bf16(x, w, relu2=False, f32=True):
     return out
 
 
+def products_check():
+    """Synchronises the stream; raises, once, if a device-side wait gave up in a product called without a handle (bf16_mlp, lm_head_argmax,
+    gemm_bf16, gemm_swiglu)."""
+    _check(load().blok_products_check(_stream()))
+
+
 class ModelConfig(C.Structure):
     _fields_ = [(n, C.c_int) for n in ("layers", "first_dense", "hidden", "vocab", "dense_inter", "inter", "experts", "topk",
                                        "shared_inter")] + [("routed_scale", C.c_float)] + \

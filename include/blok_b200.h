@@ -598,6 +598,10 @@ int blok_gemm_swiglu(const blok_bf16_t *x, const blok_bf16_t *w, int T, int R, i
 /* out[t, r] = act(sum_k x[t, k] w[r, k]) on tcgen05 with TMA-fed tiles; act: none, or the square of ReLU. */
 int blok_gemm_bf16(const blok_bf16_t *x, const blok_bf16_t *w, int T, int R, int K, int relu2, blok_bf16_t *out_bf16,
                    float *out_f32, blok_stream_t stream);
+/* Synchronises `stream` and reports, once, whether a device-side wait gave up (BLOK_ERR_TIMEOUT) in a product that was called without a
+ * handle, by any thread of the process: blok_bf16_mlp, blok_lm_head_argmax, blok_gemm_bf16, blok_gemm_swiglu.  The outputs of such a
+ * product are NaN (blok_lm_head_argmax passes over them).  Products of a layer's or a model's handle are reported by its own check. */
+int blok_products_check(blok_stream_t stream);
 
 /* ------------------------------------------------------------------------- */
 /* A11/A12  whole model: decode step and greedy generation (config 4)          */
@@ -736,6 +740,8 @@ int blok_model_check(blok_model_t *model, blok_stream_t stream);
 
 /* Test hook: blok_moe_layer_debug_set_error on the MoE layer `layer` of the model. */
 int blok_model_debug_set_layer_error(blok_model_t *model, int layer, unsigned code, blok_stream_t stream);
+/* Test hook: the same for the model's own products (dense layers, vocabulary), or with NULL for those called without a handle. */
+int blok_debug_set_products_error(blok_model_t *model, unsigned code);
 
 /* Forgets all cached tokens (positions restart at 0). */
 int blok_model_reset(blok_model_t *model);

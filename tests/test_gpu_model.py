@@ -222,6 +222,33 @@ def test_sharded_model_holds_the_slices_of_the_unsharded_tensors(cuda, tmp_path)
     other.close()
 
 
+def test_a_product_that_gave_up_is_reported_by_its_own_model(cuda):
+    """The dense layers' and the vocabulary's products report to their model: another model's check, and the check of the products called
+    without a handle, neither report nor clear it.  The words are set from the host: no wait is made to run out on the device."""
+    import ctypes as C
+    from blok_b200 import lib
+    a, b = lib.Model(seed=5, **CFG), lib.Model(seed=5, **CFG)
+    want = a.generate([3, 1, 4], 4)
+
+    def gave_up(check):
+        with pytest.raises(lib.BlokError) as e:
+            check()
+        assert e.value.code == -5 and "product" in str(e.value)
+
+    assert lib.load().blok_debug_set_products_error(a._handle, C.c_uint(1)) == 0
+    b.check()
+    lib.products_check()
+    gave_up(a.check)
+    a.check()                                   # reported once; the handle stays usable
+    assert lib.load().blok_debug_set_products_error(None, C.c_uint(1)) == 0
+    a.check()
+    gave_up(lib.products_check)
+    lib.products_check()
+    assert a.generate([3, 1, 4], 4) == want
+    a.close()
+    b.close()
+
+
 def test_a_wait_that_gave_up_in_a_layer_voids_the_generation(cuda):
     """The decode kernels' waits are bounded and leave an error word; generate() must not return tokens after one.
     The word is set from the host here (blok_moe_layer_debug_set_error): no wait is made to run out on the device."""
