@@ -5,7 +5,8 @@
 // which stays as the fallback.
 //
 // All 64 heads of a sequence share one latent row per token: per token 1,152 bytes are read once from HBM and feed
-// 64 x (576 + 512) multiply-adds.  A CTA owns one (sequence, token range) and walks it in tiles of 64 tokens:
+// 64 x (576 + 512) multiply-adds.  A CTA walks its share of the batch, a range of tokens of one sequence after another's
+// (mla_plan.cuh; FINE: of one sequence), in tiles of 64 tokens:
 //
 //   S [heads x tokens]     = Q [heads x 576] . C^T          36 MMAs M64 N64 K16: A = Q (shared memory, as a tile lies),
 //                                                            B = the tile read K-major; two partial sums

@@ -181,11 +181,9 @@ __global__ void __launch_bounds__(1024) mb_route_kernel(const MbRoute a) {
     warp_topk(score + tok * a.experts, sel, a.topk, a.scale, lane, my_id, my_w);
     if (lane < a.topk) {
       const int at = tok * a.topk + lane;
-      {
-        a.ids[at] = (uint16_t)my_id;
-        a.local_ids[at] = my_id;
-        a.wts[at] = my_w;
-      }
+      a.ids[at] = (uint16_t)my_id;
+      a.local_ids[at] = my_id;
+      a.wts[at] = my_w;
       s_local[at] = my_id;
       atomicAdd(s_counts + my_id, 1);
     }
@@ -205,14 +203,12 @@ __global__ void __launch_bounds__(1024) mb_route_kernel(const MbRoute a) {
   off += before - c, first += tiles - nt;
   if (tid < a.experts) {
     s_offsets[tid] = off;
-    {
-      for (int k = 0; k < nt && first + k < a.max_tiles; ++k) {
-        a.tile_expert[first + k] = tid;
-        a.tile_start[first + k] = off + k * kWgTileTokens;
-        a.tile_count[first + k] = min(kWgTileTokens, c - k * kWgTileTokens);
-      }
-      if (tid == a.experts - 1) *a.num_tiles = min(first + nt, a.max_tiles);
+    for (int k = 0; k < nt && first + k < a.max_tiles; ++k) {
+      a.tile_expert[first + k] = tid;
+      a.tile_start[first + k] = off + k * kWgTileTokens;
+      a.tile_count[first + k] = min(kWgTileTokens, c - k * kWgTileTokens);
     }
+    if (tid == a.experts - 1) *a.num_tiles = min(first + nt, a.max_tiles);
   }
   __syncthreads();
   // an assignment per thread: its place among its expert's is the number of them before it
@@ -224,10 +220,8 @@ __global__ void __launch_bounds__(1024) mb_route_kernel(const MbRoute a) {
       const int4 v = *reinterpret_cast<const int4 *>(s_local + j);
       rank += (v.x == e) + (j + 1 < i && v.y == e) + (j + 2 < i && v.z == e) + (j + 3 < i && v.w == e);
     }
-    {
-      a.sorted_assign[s_offsets[e] + rank] = i;
-      a.sorted_row[s_offsets[e] + rank] = i / a.topk;
-    }
+    a.sorted_assign[s_offsets[e] + rank] = i;
+    a.sorted_row[s_offsets[e] + rank] = i / a.topk;
   }
 }
 

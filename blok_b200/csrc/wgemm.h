@@ -1,4 +1,5 @@
-// Interface of the weight-streaming GEMM (wgemm.cu).
+// Products of several tokens with bf16 or INT4 weights: which kernel takes a launch (wgemm.cu) and the kernels (wgemm.cu, wgemm_stream.cu,
+// wgemm_tc.cu, wgemv_small.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include <cstddef>
@@ -37,13 +38,12 @@ struct WgArgs {
   size_t splitk_bytes = 0;
   // INT4 modes, where the host knows only a bound of them: the assignments that pick the kernel, a device word (launch_wgemm_experts)
   const int *total = nullptr;
-  // The weight-streaming kernel only.  A second matrix over the same rows (w_2, R2 rows, bf16 to out2; beside a gated product with
-  // keep_sums only): its tiles follow the first's, its partial sums the first's columns.  max_splits: a bound of the K split (0: none).  keep_sums: fp32 sums in
-  // splitk_ws also where K is not split.  weights_early: the weights may be fetched
-  // before the kernels in front of this launch have finished (the caller has launched one since they were written, in this call).
+  // The weight-streaming kernel only.  keep_sums: fp32 sums in splitk_ws also where K is not split, for a kernel of the caller's that
+  // takes them.  A second matrix over the same rows (w_2, R2 rows; with keep_sums): its tiles follow the first's, its sums the first's
+  // columns.  max_splits: a bound of the K split (0: none).  weights_early: the weights may be fetched before the kernels in front of
+  // this launch have finished (the caller has launched one since they were written, in this call).
   const void *w_2 = nullptr;
   int R2 = 0, max_splits = 0;
-  uint16_t *out2 = nullptr;
   bool keep_sums = false, weights_early = false;
   // INT4 modes: the launches become resident while the ones before them run.  For few tokens, where they are short: layers of 3, 64 (2048 x
   // 1024, 128 experts) and 6 (7168 x 2048) tokens 59 -> 56, 139 -> 130, 259 -> 254 us; over 2,048 tokens 1 to 2 % slower (blocks that come

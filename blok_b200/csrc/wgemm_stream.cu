@@ -41,8 +41,7 @@ struct StArgs {
   float *part;         // fp32 [split][token][ld] where K is split, else NULL
   uint16_t *out_bf16;  // [token][R]
   float *out_f32;
-  uint16_t *out2;      // the second matrix's output (tiles from tiles1 on), bf16; its partial sums follow the first's columns
-  int T, N, K, R, R2, tiles1, ld, stages, early;
+  int T, N, K, R, R2, tiles1, ld, stages, early;  // tiles from tiles1 on: the second matrix's; its sums follow the first's columns
   unsigned *err;
 };
 
@@ -172,8 +171,8 @@ __global__ void __launch_bounds__(kStThreads) wgemm_stream_kernel(const __grid_c
       const int row = gated ? tile * (kStRows / 2) + (r & 63) : tile * kStRows + r;
       const int col = second ? a.ld - a.R2 + row : (gated && r >= 64 ? R + row : row);  // of the partial sums
       const size_t ld = a.part ? a.ld : R;
-      float *f32 = a.part ? a.part + (size_t)z * a.T * ld + col : (a.out_f32 && !second ? a.out_f32 + row : nullptr);
-      uint16_t *b16 = (second ? a.out2 : a.out_bf16) + row;
+      float *f32 = a.part ? a.part + (size_t)z * a.T * ld + col : (a.out_f32 ? a.out_f32 + row : nullptr);
+      uint16_t *b16 = a.out_bf16 + row;
 #pragma unroll 1
       for (int c0 = 0; c0 < a.T; c0 += 16) {
         uint32_t v[16];
@@ -236,7 +235,7 @@ bool wgemm_stream_takes_parts(int mode, const WgArgs &args, size_t room) {
 // Launches the kernel; *splits = the K-split it used (> 1: the partial sums wait in args.splitk_ws for the reduce kernel).
 int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t stream) {
   const bool swiglu = mode == WG_BF16_SWIGLU;
-  BLOK_REQUIRE(args.K % 8 == 0 && args.R >= 1 && args.n_rows >= 1 && args.n_rows <= kWgStreamTokens && (!swiglu || !args.R2 || args.keep_sums), BLOK_ERR_SHAPE,
+  BLOK_REQUIRE(args.K % 8 == 0 && args.R >= 1 && args.n_rows >= 1 && args.n_rows <= kWgStreamTokens && (!args.R2 || args.keep_sums), BLOK_ERR_SHAPE,
                "streaming product: %d rows x %d columns over %d tokens", args.R, args.K, args.n_rows);
   StArgs a;
   a.tiles1 = st_tiles(mode, args.R);
@@ -249,7 +248,6 @@ int launch_wgemm_stream(int mode, const WgArgs &args, int *splits, cudaStream_t 
   a.part = nz > 1 || args.keep_sums ? args.splitk_ws : nullptr;
   a.out_bf16 = args.out_bf16;
   a.out_f32 = args.out_f32;
-  a.out2 = args.out2;
   a.T = args.n_rows;
   a.N = (args.n_rows + 15) / 16 * 16;
   a.K = args.K;
