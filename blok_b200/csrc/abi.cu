@@ -18,6 +18,7 @@ void set_error(const char *fmt, ...) {
 }
 
 int cuda_fail(cudaError_t e, const char *what) {
+  cudaGetLastError();  // reported here: the program's next CUDA call must not find it
   set_error("%s: %s", what, cudaGetErrorString(e));
   return BLOK_ERR_CUDA;
 }

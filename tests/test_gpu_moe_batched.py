@@ -255,3 +255,14 @@ def test_a_wide_layer_has_room_for_its_sums(cuda, monkeypatch):
     assert torch.equal(ids, wid)
     assert float((y.float() - want.float()).norm() / want.float().norm()) < 1e-2
     layer.close()
+
+
+def test_a_refused_launch_is_reported_once(cuda):
+    """A launch that CUDA refuses (more tokens than a grid has rows) is the call's error and nobody else's."""
+    from blok_b200 import lib
+    T = 65536
+    y, wts = torch.zeros((T, 2), device=cuda, dtype=torch.bfloat16), torch.ones((T, 1), device=cuda)
+    with pytest.raises(lib.BlokError):
+        lib.moe_combine(y, wts)
+    assert int(torch.ones(3, device=cuda).sum()) == 3
+    assert lib.moe_combine(y[:4].contiguous(), wts[:4].contiguous()).shape == (4, 2)
