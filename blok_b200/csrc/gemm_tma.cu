@@ -151,8 +151,17 @@ int tensor_map_2d(const void *base, CUtensorMapDataType type, long rows, long co
   const cuuint64_t strides[1] = {(cuuint64_t)pitch};
   const cuuint32_t boxes[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = encode(out, type, 2, const_cast<void *>(base), dims, strides, boxes, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encoded = [&] {
+    return encode(out, type, 2, const_cast<void *>(base), dims, strides, boxes, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encoded();
+  if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {  // the first CUDA call of this host thread: it is the driver's own
+    int device = 0;
+    BLOK_CUDA(cudaGetDevice(&device));
+    BLOK_CUDA(cudaSetDevice(device));
+    r = encoded();
+  }
   BLOK_REQUIRE(r == CUDA_SUCCESS, BLOK_ERR_CUDA, "gemm: no tensor map (%d) for a matrix of %ld x %ld, pitch %ld bytes", (int)r, rows, cols, pitch);
   return BLOK_OK;
 }

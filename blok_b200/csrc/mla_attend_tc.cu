@@ -42,6 +42,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "gemm_tma.h"
 #include "mla_plan.cuh"
 #include "tmem_io.cuh"
 
@@ -667,11 +668,7 @@ int mla_attend_tc_trace(long long *host_out, int max_entries) {
 }
 
 // The tensor map of a cache of `rows` rows of 576 bf16 at `base`: boxes of 64 rows x 64 columns in the 128-byte swizzle;
-// rows at or past `rows` read as zeros.  cuTensorMapEncodeTiled is resolved from the driver at run time; the last few
-// maps are kept (a model's layers pass the same caches step after step).
-typedef CUresult (*ta_encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                 const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// rows at or past `rows` read as zeros.  The last few maps are kept (a model's layers pass the same caches step after step).
 // keep: false for operands that move from call to call (the queries).
 static int cache_tensor_map(const uint16_t *base, long rows, bool keep, CUtensorMap *out) {
   struct Entry {
@@ -682,30 +679,14 @@ static int cache_tensor_map(const uint16_t *base, long rows, bool keep, CUtensor
   static std::mutex mu;
   static Entry kept[128];
   static int n_kept = 0, next = 0;
-  static ta_encode_fn encode = nullptr;
   std::lock_guard<std::mutex> lock(mu);
   for (int i = 0; i < n_kept && keep; ++i)
     if (kept[i].base == base && kept[i].rows == rows) {
       *out = kept[i].map;
       return BLOK_OK;
     }
-  if (!encode) {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    BLOK_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
-    BLOK_REQUIRE(fn && qres == cudaDriverEntryPointSuccess, BLOK_ERR_CUDA, "blok_mla_decode: the driver has no cuTensorMapEncodeTiled");
-    encode = reinterpret_cast<ta_encode_fn>(fn);
-  }
-  const cuuint64_t dims[2] = {(cuuint64_t)kTaD, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)kTaD * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)kTaTile};
-  const cuuint32_t estr[2] = {1, 1};
   CUtensorMap map;
-  const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t *>(base), dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  BLOK_REQUIRE(r == CUDA_SUCCESS, BLOK_ERR_CUDA, "blok_mla_decode: cuTensorMapEncodeTiled failed (%d) for a cache of %ld rows at %p", (int)r,
-               rows, (const void *)base);
+  if (int rc = tensor_map_2d(base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rows, kTaD, kTaD * 2, kTaTile, 64, CU_TENSOR_MAP_SWIZZLE_128B, &map)) return rc;
   *out = map;
   if (!keep) return BLOK_OK;
   kept[next] = Entry{base, rows, map};

@@ -32,7 +32,7 @@ def test_launches_of_different_shared_memory(cuda, tmp_path):
         keep.append((x, y, ws, stream))
         calls.append(MlpCall(*(t.data_ptr() for t in (*w, x, y)), hidden, ffn, T, ws.data_ptr(), ws.numel(), stream.cuda_stream))
     torch.cuda.synchronize()
-    failed = native.two_threads(C.cast(library.blok_bf16_mlp, C.c_void_p), C.byref(calls[0]), C.byref(calls[1]), 10000)
+    failed = native.two_threads(C.cast(library.blok_bf16_mlp, C.c_void_p), C.cast(library.blok_last_error, C.c_void_p), C.byref(calls[0]), C.byref(calls[1]), 10000)
     torch.cuda.synchronize()
     assert failed == 0
     for (x, y, _, _), z in zip(keep, want):
