@@ -395,8 +395,8 @@ int launch_grouped_attend(const GroupedShape &s, const GroupedQuery<uint16_t> &a
   else BLOK_GA(1);
 #undef BLOK_GA
   if (rc) return rc;
-  mla_merge_kernel<<<dim3(s.heads, T), 128, (size_t)splits * sizeof(float), stream>>>(part_o, part_ml, splits, s.heads, s.vdim, a.out, a.ldo, a.gate,
-                                                                                      a.ld_gate);
+  const auto merge = mla_merge(s.heads, T);
+  merge<<<dim3(s.heads, T), 128, (size_t)splits * sizeof(float), stream>>>(part_o, part_ml, splits, s.heads, s.vdim, a.out, a.ldo, a.gate, a.ld_gate, nullptr);
   return launch_status("mla_merge_kernel");
 }
 

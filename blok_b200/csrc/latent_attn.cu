@@ -414,7 +414,9 @@ int launch_latent_attend(const LatentShape &s, const void *q_abs, const void *po
   else BLOK_LA(1);
 #undef BLOK_LA
   if (rc) return rc;
-  mla_merge_kernel<<<dim3(s.heads, T), 128, (size_t)splits * sizeof(float), stream>>>(part_o, part_ml, splits, s.heads, s.rank, static_cast<uint16_t *>(o));
+  const auto merge = mla_merge(s.heads, T);
+  merge<<<dim3(s.heads, T), 128, (size_t)splits * sizeof(float), stream>>>(part_o, part_ml, splits, s.heads, s.rank, static_cast<uint16_t *>(o), 0, nullptr, 0,
+                                                                           nullptr);
   return launch_status("mla_merge_kernel");
 }
 

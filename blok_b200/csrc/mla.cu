@@ -293,7 +293,7 @@ static int attend_and_merge(blok_mla_layer *L, const uint16_t *q, const CacheRef
   int splits;
   if (int rc = attend(L, q, c, seq_len, B, scale, false, &splits, stream)) return rc;
   const int most = splits ? splits : L->max_splits;
-  return launch_pdl("mla_merge_kernel", mla_merge_kernel, dim3(L->w.heads, B), 128, (size_t)most * sizeof(float), stream, L->part_o, L->part_ml, most,
+  return launch_pdl("mla_merge_kernel", mla_merge(L->w.heads, B), dim3(L->w.heads, B), 128, (size_t)most * sizeof(float), stream, L->part_o, L->part_ml, most,
                     L->w.heads, L->w.kv_rank, o_lat, 0, nullptr, 0, splits ? nullptr : L->parts);
 }
 

@@ -33,7 +33,10 @@ __device__ __forceinline__ void mla_plan(MlaPlan &p, int B, int ctas, F tokens) 
   int per = max(1, (total + kMlaPlanLead * B + ctas - 1) / ctas), lead = kMlaPlanLead;
   // pieces of t tiles are enough for every sequence by itself where the number of pieces does not exceed the CTAs'
   auto pieces = [&](int t) { return __reduce_add_sync(0xffffffffu, (a + t - 1) / t + (c + t - 1) / t); };
-  if (pieces(per + 1) <= ctas) {
+  if (B == 1) {  // the search's result
+    per = max(1, (total + ctas - 1) / ctas), lead = 0;
+    a = (a + per - 1) / per * per;
+  } else if (pieces(per + 1) <= ctas) {
     int lo = max(1, (total + ctas - 1) / ctas), hi = per + 1;
     while (lo < hi) {
       const int t = (lo + hi) / 2;
