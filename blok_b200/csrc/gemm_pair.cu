@@ -227,8 +227,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGpThreads, 1)
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * BN) : "memory");
 }
 
-// Rows past the first 128: below that half of every pair would have nothing to do.
-bool gemm_pair_takes(const GemmTma &g) { return !g.tile_start && g.T > 128; }
+// Rows past the first 128: below that half of every pair would have nothing to do.  Against the one-CTA kernel, us, weights in L2 / from HBM:
+//  - few columns are mostly the stores of a tile's sums, which 256 x 256 outputs make once per pair and 128 x 128 in smaller pieces:
+//    gated, 2 x 8,192 by 256 over 1,000 rows 25 / 31 here, 21 / 27 there; 1,024 by 256 (fp32) over 513 rows 7.4 / 12.2, 8.7 / 10.2.  At 512
+//    columns the launch's own ramp, hidden behind the kernel before, decides: geometric mean over 200 products 0.93 / 1.03 of the other.
+//  - rows that leave half of the last tile empty, among three tiles or fewer, cost a fifth or more of the products: 4,096 and 8,192 by 512
+//    over 513 rows 12.5 / 17.2 and 19 / 24.6 here, 10.7 / 14.3 and 14.9 / 20.5 there; by 2,048 they are even.
+//  - with a few tiles only the one-CTA kernel is 4 to 11 % faster from L2 (64 by 8,192: 33.3 / 37.0), and 20 % slower from HBM.
+bool gemm_pair_takes(const GemmTma &g) {
+  if (g.tile_start || g.T <= 128 || g.K < 512) return false;
+  const bool gated = g.act == GEMM_ACT_SWIGLU || g.act == GEMM_ACT_SWIGLU_REF;
+  const long row_tiles = (g.T + kGpRows - 1) / kGpRows, tiles = row_tiles * (((gated ? 2 * g.R : g.R) + 255) / 256);
+  const bool half_empty = (g.T - 1) % kGpRows < 128 && (row_tiles == 2 || row_tiles == 3);
+  return !(half_empty && g.K < 2048 && tiles > sm_count() / 4);
+}
 
 // Pairs of SMs that hold a pair of CTAs at once (an odd SM of a GPC has no partner): a persistent grid must not be larger.
 template <int BN, int ACT, bool F32>

@@ -30,3 +30,18 @@ def test_gated(cuda, T, R, K):
     want = gate * torch.sigmoid(gate) * up
     got = lib.gemm_swiglu(x, w)
     assert float((got.double() - want).norm() / want.norm()) < 3e-3
+
+
+# from 512 columns on pairs take a product, with exceptions below 2,048 columns where most of a half tile is empty: every edge of a pair's
+# tile, and both sides of the lines
+@pytest.mark.parametrize("T,R,K", [(129, 4, 512), (129, 256, 520), (255, 260, 584), (256, 128, 1000), (257, 36, 520), (513, 516, 712), (300, 18944, 512),
+                                   (384, 8192, 512), (385, 8192, 512), (513, 4096, 2040), (513, 4096, 2048), (640, 4096, 1024), (641, 4096, 1024),
+                                   (300, 2048, 504), (300, 2048, 512)])
+def test_lines_between_the_kernels(cuda, T, R, K):
+    test_plain(cuda, T, R, K)
+
+
+@pytest.mark.parametrize("T,R,K", [(128, 128, 512), (129, 4, 512), (256, 132, 584), (300, 200, 1000), (300, 4736, 512), (300, 4864, 512), (385, 4864, 520),
+                                   (1025, 8192, 504)])
+def test_gated_lines_between_the_kernels(cuda, T, R, K):
+    test_gated(cuda, T, R, K)
