@@ -113,7 +113,9 @@ struct MbRoute {
   int max_tiles;
   uint16_t *mid;  // [T][shared]
 };
-constexpr int kMbRouteExperts = 384;
+// Most experts: the scores of 64 tokens stay in shared memory (512 experts 137 KB, 1,024 would be 268), one instance per width of a lane's
+// share of them.
+constexpr int kMbRouteExperts = 512;
 
 template <int N>
 __global__ void __launch_bounds__(1024) mb_route_kernel(const MbRoute a) {
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(1024) mb_route_kernel(const MbRoute a) {
 static int launch_mb_route(const MbRoute &a, cudaStream_t stream) {
   const size_t smem = (size_t)((a.T * a.topk + 3) / 4 * 4 + (3 + a.T) * a.experts) * sizeof(int);
   const int blocks = 1 + (a.T * a.shared / 4 + 1023) / 1024;
-  auto kernel = a.experts <= 128 ? mb_route_kernel<4> : mb_route_kernel<12>;
+  auto kernel = a.experts <= 128 ? mb_route_kernel<4> : (a.experts <= 384 ? mb_route_kernel<12> : mb_route_kernel<16>);
   if (int rc = allow_smem(kernel, smem)) return rc;
   return launch_pdl("mb_route_kernel", kernel, blocks, 1024, smem, stream, a);
 }

@@ -266,3 +266,9 @@ def test_a_refused_launch_is_reported_once(cuda):
         lib.moe_combine(y, wts)
     assert int(torch.ones(3, device=cuda).sum()) == 3
     assert lib.moe_combine(y[:4].contiguous(), wts[:4].contiguous()).shape == (4, 2)
+
+
+@pytest.mark.parametrize("T,experts,topk,hidden,inter,shared", [(1, 512, 8, 1024, 512, 512), (33, 512, 16, 512, 512, 0), (64, 512, 16, 512, 512, 1024),
+                                                                (7, 640, 8, 512, 512, 512)])
+def test_front_of_a_small_batch_with_many_experts(cuda, monkeypatch, T, experts, topk, hidden, inter, shared):
+    test_front_of_a_small_batch(cuda, monkeypatch, T, experts, topk, hidden, inter, shared)
