@@ -1,5 +1,5 @@
-"""bf16 products over more than 128 rows, which pairs of CTAs take: against 64 bits at the edges of their tiles (256 rows of x by 128 or
-256 weight rows, 64-column steps) and on both sides of the line to the one-CTA kernel."""
+"""bf16 products over more than 128 rows, which pairs of CTAs take from 512 columns on: against 64 bits at the edges of their tiles (256 rows
+of x by 128 or 256 weight rows, 64-column steps) and on both sides of the lines to the one-CTA kernel."""
 import pytest
 import torch
 

@@ -134,3 +134,10 @@ def test_core_over_lengths(cuda, lens):
             err = float((o[b].double() - want).norm() / want.norm())
             assert err < 6e-3, (b, n, err)
     layer.close()
+
+
+# one sequence has a plan without a search; parts from one to all CTAs', around the sixteen that the merge has in flight, and (320 blocks)
+# around its eight
+@pytest.mark.parametrize("lens", [[1], [64 * 15], [64 * 16 + 1], [64 * 17], [3000], [64 * 148], [64 * 149 - 1], [64 * 300 + 5], [20000] * 5])
+def test_core_over_few_long_sequences(cuda, lens):
+    test_core_over_lengths(cuda, lens)
