@@ -8,8 +8,9 @@
 //
 // Measured, one CTA per tile / pairs, us: 1,000 rows, gated product of 2 x 8,192 by 2,048 70 / 52 (1.3 PFLOP/s), 8,512 by 2,048 43 / 31,
 // 2,048 by 8,192 49.5 / 41; a prompt of 130 / 1,000 / 2,040 tokens through four layers 966 / 1,340 / 2,090 -> 832 / 1,196 / 1,770 (with the
-// K parts of sublayer_product and overlapped launches 517 / 956 / 1,600 since).  Now some
-// 12 TB/s from L2 to the SMs are the limit: 0.41 us a step of the wide tile, 0.32 of the narrow one.
+// K parts of sublayer_product and overlapped launches 517 / 956 / 1,600 since).  A step
+// takes 0.41 us of the wide tile, 0.32 of the narrow one; over a whole launch the tensor pipe is 78 % busy (gated), 66 and 46 % (the other
+// two), and 8.3 to 9.5 TB/s come from L2 to the SMs.
 //
 // Both CTAs' copies count on the leader's mbarrier (the copy's cta_group::2 form; no multicast); the leader's MMA warp issues for
 // the pair, its commits free the slots of both.  A gated product's tile is 128 gate rows (the leader's half) and the up rows of the

@@ -8,7 +8,7 @@
 //    queries, its result), so each has a lead of that length.
 // Against a fixed number of parts per sequence (the longest one then sets the time), the block, us: 33 sequences of 1,500 to 6,000
 // tokens 122 -> 110, 50 of 5,000 158 -> 147; where that number was as good the plan's way through memory costs 1 to 2.5 us
-// (8 of 32,768 126 -> 128.5, one of 4,001 64.8 -> 65.4).
+// (8 of 32,768 126 -> 128.5, one of 4,001 64.8 -> 65.4; the core alone, which makes the plan itself, over one of 3,000 23.5 -> 25.6).
 #pragma once
 #include "common.cuh"
 

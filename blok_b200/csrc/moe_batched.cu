@@ -21,7 +21,8 @@ int launch_router_topk(const float *logits, const float *bias, int T, int expert
 // memory, scans the counts, and a pair of threads counts the equals before an assignment inside the block's own.  Every block does the
 // counting again, which costs less than a launch that it would have to wait for.  ids outside [0, n_local) belong to none.  Latency is all
 // there is to it: one block that counted and, in a launch behind it, a warp per expert that walked all assignments took 15 us over
-// 4,136 and 39 over 16,384 assignments (the gap between them with it), this one 8.4 and 9.9.
+// 4,136 and 39 over 16,384 assignments (the gap between them with it), this one 8.4 and 9.9.  The counting is quadratic in all, but over
+// 524,280 assignments of which nearly all belong to no expert a call takes 292 us where it took 1,321 with the two launches.
 // Dynamic shared memory: [n_local] counts, [n_local] counts before the block's own, [n_local] offsets.
 constexpr int kMbChunk = 512;
 __global__ void __launch_bounds__(1024) mb_sort_kernel(const int *__restrict__ expert_local, const int *__restrict__ x_index, int row_div, int N,
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(1024) mb_sort_kernel(const int *__restrict__ e
 // a few microseconds of latency, most of it the fetch of its instructions (the weights that stream between two calls leave
 // nothing of them in L2): reduce, top-k, plan and reduce took 22 us over 6 tokens, this one 8.7.  With the front launch and the
 // combination that adds the second half's sums, layers of 6 and 2 tokens (7168 x 2048, 384 experts) 285 -> 257, 151 -> 121 us, of 3, 40
-// and 64 (2048 x 1024, 128 experts) 76 -> 61, 152 -> 127, 157 -> 139.  A pass over stale sums before the wait, to have the
+// and 64 (2048 x 1024, 128 experts) 76 -> 61, 152 -> 127, 157 -> 139; of 1, 5 and 16 (2048 x 512, 512 experts) 73 -> 45, 94 -> 67, 124 -> 97.  A pass over stale sums before the wait, to have the
 // instructions there, is slower (64 tokens 139 -> 148).
 struct MbRoute {
   const float *part;  // [nz][T][ld]: the shared expert's gate columns, its up columns, the router's

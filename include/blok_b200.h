@@ -599,8 +599,8 @@ int blok_gemm_swiglu(const blok_bf16_t *x, const blok_bf16_t *w, int T, int R, i
 int blok_gemm_bf16(const blok_bf16_t *x, const blok_bf16_t *w, int T, int R, int K, int relu2, blok_bf16_t *out_bf16,
                    float *out_f32, blok_stream_t stream);
 /* Synchronises `stream` and reports, once, whether a device-side wait gave up (BLOK_ERR_TIMEOUT) in a product that was called without a
- * handle, by any thread of the process: blok_bf16_mlp, blok_lm_head_argmax, blok_gemm_bf16, blok_gemm_swiglu.  The outputs of such a
- * product are NaN (blok_lm_head_argmax passes over them).  Products of a layer's or a model's handle are reported by its own check. */
+ * handle, by any thread of the process: blok_bf16_mlp, blok_lm_head_argmax, blok_gemm_bf16, blok_gemm_swiglu.  The outputs of
+ * such a product are NaN (blok_lm_head_argmax passes over them).  Products of a layer's or a model's handle are reported by its own check. */
 int blok_products_check(blok_stream_t stream);
 
 /* ------------------------------------------------------------------------- */
