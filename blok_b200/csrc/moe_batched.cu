@@ -458,6 +458,7 @@ extern "C" int blok_moe_batched(blok_moe_layer_t *L, const blok_bf16_t *x, int T
   r.tile_expert = r.tile_start = r.tile_count = r.num_tiles = nullptr;
   r.out_index = nullptr; r.n_rows = T; r.identity_tiles = 1;
   r.splitk_ws = L->b_splitk; r.splitk_bytes = L->b_splitk_bytes; r.err = L->b_err;
+  r.max_splits = L->b_front_split;  // the expert-parallel layer's: the two agree bit for bit
   if ((rc = launch_wgemm(WG_BF16_PLAIN, r, tt, stream))) return rc;
   if ((rc = launch_router_topk(L->logits, w.router_bias, T, w.experts, w.topk, w.routed_scale, L->ids, L->wts, L->local_ids,
                                w.expert_base, stream)))
@@ -468,10 +469,10 @@ extern "C" int blok_moe_batched(blok_moe_layer_t *L, const blok_bf16_t *x, int T
     WgArgs s = r;
     s.w_a = w.shared_gate; s.w_b = w.shared_up; s.R = w.shared_inter; s.out_bf16 = L->b_smid; s.out_f32 = nullptr;
     s.weights_early = true;  // the router's launch and others are in between
-    s.max_splits = L->b_front_split;
     if ((rc = launch_wgemm(WG_BF16_SWIGLU, s, tt, stream))) return rc;
     WgArgs d = r;
     d.w_a = w.shared_down; d.x = L->b_smid; d.K = w.shared_inter; d.R = w.hidden; d.out_bf16 = L->b_sout; d.out_f32 = nullptr;
+    d.max_splits = 0;
     d.weights_early = true;
     if ((rc = launch_wgemm(WG_BF16_PLAIN, d, tt, stream))) return rc;
     shared = L->b_sout;

@@ -59,6 +59,24 @@ def test_one_rank_world_without_shared_expert_and_full_size_rows(cuda):
     ep.close(); full.close(); comm.close()
 
 
+@pytest.mark.parametrize("experts", [512, 640])
+def test_one_rank_world_of_many_experts(cuda, experts):
+    """On both sides of the expert count up to which blok_moe_batched runs its front in two launches, with a shared expert wide enough for
+    the router's K to be cut otherwise beside it than alone."""
+    from blok_b200 import lib, synth
+    w = synth.moe_layer_weights(cuda, seed=54, hidden=7168, inter=512, experts=experts, shared_inter=2048)
+    comm = lib.Comm(rank=0, world=1)
+    ep = lib.MoeEp(comm, w, max_tokens=80)
+    full = lib.MoeLayer(w, max_tokens=80)
+    for T in (1, 33, 64, 65):
+        x = synth.activations(T, 7168, cuda, T)
+        y, ids, wts = ep.forward(x, return_routing=True)
+        ep.check()
+        ref, rid, rw = full.batched(x, return_routing=True)
+        assert torch.equal(ids, rid) and torch.equal(wts, rw) and torch.equal(y, ref), T
+    ep.close(); full.close(); comm.close()
+
+
 def test_shard_must_match_the_rank(cuda):
     from blok_b200 import lib
     w = _small_layer(cuda, 53)
