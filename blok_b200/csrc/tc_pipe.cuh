@@ -59,6 +59,17 @@ __device__ __forceinline__ void tp_load_2d(uint32_t dst, const CUtensorMap *map,
                "l"(map), "r"(x), "r"(y), "r"(mbar)
                : "memory");
 }
+// The same for data that is read once: its lines are the first that L2 gives up (policy: tp_read_once()).
+__device__ __forceinline__ uint64_t tp_read_once() {
+  uint64_t policy;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  return policy;
+}
+__device__ __forceinline__ void tp_load_2d_hint(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t mbar, uint64_t policy) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(dst),
+               "l"(map), "r"(x), "r"(y), "r"(mbar), "l"(policy)
+               : "memory");
+}
 // K-major operand in the 128-byte swizzle: rows of 128 bytes (64 bf16), 1,024 bytes between 8-row groups.  A K = 16 step
 // inside the row advances the start address by 32 bytes.
 __device__ __forceinline__ uint64_t tp_desc_k_sw128(uint32_t saddr) {

@@ -18,6 +18,11 @@
 // been there (WgArgs::weights_early) the first steps' weights are on their way before the wait: the ramp of the stream is hidden
 // behind the kernel before.  Shared memory keeps it at two CTAs per SM, so early CTAs spread evenly.
 //
+// A launch reads every weight once, and they are the first that L2 gives up: what other kernels find there (caches, activations, the rest
+// of a small model) stays.  Without that the vocabulary's 134 MB, which had gone through the mat-vec kernel, pushed the layers' weights out
+// at every step: small Nomozen and Pamopel models of four layers, one sequence of 1,024 tokens, us a step: mat-vec 301 / 282, weight
+// stream 336 / 306, with the hint 301 / 277.
+//
 // Every wait is bounded; a CTA that gives up sets the error word, stores NaN, waits for its copies and frees its tensor memory.
 #include <algorithm>
 
@@ -82,14 +87,15 @@ __global__ void __launch_bounds__(kStThreads) wgemm_stream_kernel(const __grid_c
 
   if (warp == 4) {
     if (lane == 0) {
+      const uint64_t once = tp_read_once();
       auto weights = [&](int c, uint32_t dst, uint32_t bar) {
         const int k = (first + c) * kStCols;
         tp_expect_tx(bar, stage);
         if (gated) {
-          tp_load_2d(dst, &mwa, k, tile * (kStRows / 2), bar);
-          tp_load_2d(dst + kStWBytes / 2, &mwb, k, tile * (kStRows / 2), bar);
+          tp_load_2d_hint(dst, &mwa, k, tile * (kStRows / 2), bar, once);
+          tp_load_2d_hint(dst + kStWBytes / 2, &mwb, k, tile * (kStRows / 2), bar, once);
         } else {
-          tp_load_2d(dst, second ? &mw2 : &mwa, k, tile * kStRows, bar);
+          tp_load_2d_hint(dst, second ? &mw2 : &mwa, k, tile * kStRows, bar, once);
         }
       };
       const int pre = min(S, nsteps);
