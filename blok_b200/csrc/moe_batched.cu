@@ -34,14 +34,17 @@ __global__ void __launch_bounds__(1024) mb_sort_kernel(const int *__restrict__ e
   __shared__ int s_rank[kMbChunk], s_warp[2][32];
   int *s_counts = s_dyn, *s_before = s_dyn + n_local, *s_offsets = s_before + n_local;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, start = blockIdx.x * kMbChunk;
+  // the thread's own assignment, if any: both of its words are on their way before the first barrier
+  const int at = start + tid;
+  const bool has = tid < kMbChunk && at < N;
+  const int own = has ? expert_local[at] : -1, row = has ? (x_index ? x_index[at] : at / row_div) : 0;
+  const bool placed = own >= 0 && own < n_local;
   for (int e = tid; e < n_local; e += 1024) s_counts[e] = s_before[e] = 0;
-  if (tid < kMbChunk) {
-    s_own[tid] = start + tid < N ? expert_local[start + tid] : -1;
-    s_rank[tid] = 0;
-  }
+  if (tid < kMbChunk) s_own[tid] = own, s_rank[tid] = 0;
   __syncthreads();
   constexpr int kFly = 8;
-  for (int a0 = tid; a0 < N; a0 += kFly * 1024) {
+  if (gridDim.x == 1 && placed) atomicAdd(s_counts + own, 1);
+  for (int a0 = tid; gridDim.x > 1 && a0 < N; a0 += kFly * 1024) {
     int e[kFly];
 #pragma unroll
     for (int i = 0; i < kFly; ++i) e[i] = a0 + 1024 * i < N ? expert_local[a0 + 1024 * i] : -1;
@@ -53,7 +56,8 @@ __global__ void __launch_bounds__(1024) mb_sort_kernel(const int *__restrict__ e
     }
   }
   {  // two threads an assignment: the equals among the first and the second half of those before it
-    const int i = tid & (kMbChunk - 1), e = s_own[i], mid = (i / 2 + 3) / 4 * 4, j0 = tid < kMbChunk ? 0 : mid, j1 = tid < kMbChunk ? min(mid, i) : i;
+    const int i = tid & (kMbChunk - 1), e = s_own[i], mid = (i / 2 + 3) / 4 * 4, j0 = tid < kMbChunk ? 0 : mid;
+    const int j1 = e < 0 || e >= n_local ? 0 : (tid < kMbChunk ? min(mid, i) : i);
     int n = 0;
 #pragma unroll 4
     for (int j = j0; j < j1; j += 4) {
@@ -87,11 +91,10 @@ __global__ void __launch_bounds__(1024) mb_sort_kernel(const int *__restrict__ e
   }
   if (blockIdx.x == 0 && tid == 1023) *num_tiles = min(first + nt, max_tiles);
   __syncthreads();
-  const int at = start + tid;
-  if (tid < kMbChunk && at < N && s_own[tid] >= 0 && s_own[tid] < n_local) {
-    const int p = s_offsets[s_own[tid]] + s_rank[tid];
+  if (placed) {
+    const int p = s_offsets[own] + s_rank[tid];
     sorted_assign[p] = at;
-    sorted_row[p] = x_index ? x_index[at] : at / row_div;
+    sorted_row[p] = row;
   }
 }
 

@@ -272,3 +272,8 @@ def test_a_refused_launch_is_reported_once(cuda):
                                                                 (7, 640, 8, 512, 512, 512)])
 def test_front_of_a_small_batch_with_many_experts(cuda, monkeypatch, T, experts, topk, hidden, inter, shared):
     test_front_of_a_small_batch(cuda, monkeypatch, T, experts, topk, hidden, inter, shared)
+
+
+@pytest.mark.parametrize("N,only", [(1, 39), (2, None), (41, None), (100, None)])  # one block that counts its own, part of it empty
+def test_sort_of_few_assignments(cuda, N, only):
+    test_sort_of_the_assignments(cuda, N, only)
