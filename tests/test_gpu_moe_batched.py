@@ -274,6 +274,8 @@ def test_front_of_a_small_batch_with_many_experts(cuda, monkeypatch, T, experts,
     test_front_of_a_small_batch(cuda, monkeypatch, T, experts, topk, hidden, inter, shared)
 
 
-@pytest.mark.parametrize("N,only", [(1, 39), (2, None), (41, None), (100, None)])  # one block that counts its own, part of it empty
-def test_sort_of_few_assignments(cuda, N, only):
+# one block that counts its own, part of it empty; up to 40 assignments through the tcgen05 kernel as well, whose bits the comparison has
+@pytest.mark.parametrize("N,only", [(1, 39), (2, None), (41, None), (100, None)])
+def test_sort_of_few_assignments(cuda, monkeypatch, N, only):
+    monkeypatch.setenv("BLOK_WGEMM_SMALL", "0")
     test_sort_of_the_assignments(cuda, N, only)
